@@ -71,7 +71,7 @@ def build_native_module(force=False):
            "-I" + os.path.join(HERE, "cpp", "include"), "-I" + os.path.join(HERE, "..", "include"),
            "-I" + os.path.join(cuda, "include")] + NATIVE_SRCS + ["-o", out,
            "-L" + HERE, "-llmg_b200", "-L" + os.path.join(cuda, "lib64"), "-lcudart",
-           "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + os.path.join(cuda, "lib64")]
+           "-Wl,-rpath,$ORIGIN", "-pthread", "-Wl,-rpath," + os.path.join(cuda, "lib64")]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)

@@ -42,10 +42,11 @@ struct ViewInfo {
   py::object keep;
 };
 
-// torch's tensor type and dtypes, looked up once (null when torch is not importable)
+// torch's tensor type, dtypes and current-stream query, looked up once (null when torch is not
+// importable)
 struct TorchNames {
   PyTypeObject* tensor = nullptr;
-  py::object f32, f64, i32;
+  py::object f32, f64, i32, stream;
 };
 inline const TorchNames& torch_names() {
   static TorchNames* names = [] {
@@ -55,6 +56,7 @@ inline const TorchNames& torch_names() {
       n->f32 = torch.attr("float32");
       n->f64 = torch.attr("float64");
       n->i32 = torch.attr("int32");
+      n->stream = torch.attr("_C").attr("_cuda_getCurrentRawStream");
       n->tensor = reinterpret_cast<PyTypeObject*>(torch.attr("Tensor").ptr());
     } catch (py::error_already_set&) {
       n->tensor = nullptr;
@@ -62,6 +64,16 @@ inline const TorchNames& torch_names() {
     return n;
   }();
   return *names;
+}
+
+// The stream on which an asynchronous call that writes `o` is issued: torch's current one for a
+// tensor, the default stream for other arrays.
+inline cudaStream_t stream_for(const py::handle& o) {
+  const TorchNames& tn = torch_names();
+  if (tn.tensor == nullptr || !PyObject_TypeCheck(o.ptr(), tn.tensor)) return nullptr;
+  int dev = 0;
+  LMG_CUDA_CHECK(cudaGetDevice(&dev));
+  return reinterpret_cast<cudaStream_t>(tn.stream(dev).cast<size_t>());
 }
 
 // The common case of a training loop, a plain contiguous torch tensor, read with as few attribute

@@ -5,6 +5,7 @@
 #include <pybind11/numpy.h>
 #include <pybind11/operators.h>
 #include <pybind11/pybind11.h>
+#include <pybind11/stl.h>
 #include <pybind11/stl_bind.h>
 
 #include <cmath>
@@ -320,6 +321,111 @@ void make_vector_types(CoordinateSet& s, bool include_dummy_type, const std::vec
   }
 }
 
+// A line of an example list ready to be handed out: the raw records of its files in memory (one
+// array per coordinate set), the type and radius tables of their typers, and its labels.
+struct RecordExample {
+  struct Record {
+    float x, y, z;
+    int type;
+  };
+  struct Set {
+    const Record* rec;
+    size_t n;
+    const int* map;      // channel or -1 of the record types 0..27
+    const float* radius; // their radii
+    unsigned num_types;
+  };
+  std::vector<Set> sets;
+  std::vector<float> labels;
+  int group;
+  py::list keep;  // the arrays the sets point into
+
+  RecordExample(const py::list& records, const py::list& maps, const py::list& radii, const std::vector<unsigned>& num_types,
+                std::vector<float> labels_, int group_)
+      : labels(std::move(labels_)), group(group_) {
+    for (size_t i = 0; i < records.size(); i++) {
+      py::array rec = records[i].cast<py::array>();
+      py::array_t<int> map = maps[i].cast<py::array_t<int>>();
+      py::array_t<float> rad = radii[i].cast<py::array_t<float>>();
+      if (rec.itemsize() != sizeof(Record) || rec.ndim() != 1 || !(rec.flags() & py::array::c_style) ||
+          map.size() != LMG_RECORD_TYPES || rad.size() != LMG_RECORD_TYPES)
+        throw py::value_error("a coordinate set is an array of 16-byte records with tables of 28 types");
+      sets.push_back({static_cast<const Record*>(rec.data()), (size_t)rec.size(), map.data(), rad.data(), num_types.at(i)});
+      keep.append(rec);
+      keep.append(map);
+      keep.append(rad);
+    }
+  }
+
+  // Example with arrays of its own: typed atoms in file order, atoms without a channel left out,
+  // unknown type numbers taken as the generic metal (26).
+  void make(Example& ex) const {
+    size_t total = 0;
+    for (const Set& s : sets) total += s.n;
+    std::shared_ptr<char> block = detail::HostBlocks::get(total * 20 + 16);
+    float* p = reinterpret_cast<float*>(block.get());
+    ex.sets.reserve(sets.size());
+    for (const Set& s : sets) {
+      float *c = p, *t = c + 3 * s.n, *r = t + s.n;
+      size_t k = 0;
+      for (size_t i = 0; i < s.n; i++) {
+        const Record& a = s.rec[i];
+        const unsigned row = (unsigned)a.type < LMG_RECORD_TYPES ? (unsigned)a.type : 26u;
+        const int ch = s.map[row];
+        c[3 * k] = a.x; c[3 * k + 1] = a.y; c[3 * k + 2] = a.z;
+        t[k] = (float)ch;
+        r[k] = s.radius[row];
+        k += ch >= 0;  // the slot of a dropped atom is written again by the next one
+      }
+      if (k == 0) {
+        ex.sets.emplace_back();
+        ex.sets.back().max_type = s.num_types;
+      } else {
+        ex.sets.emplace_back(MGrid2f::within(block, c, k, 3), MGrid1f::within(block, t, k), MGrid1f::within(block, r, k),
+                             s.num_types);
+      }
+      p = r + s.n;
+    }
+    ex.labels = labels;
+    ex.group = group;
+  }
+};
+
+std::vector<Example> make_examples(const py::list& lines) {
+  std::vector<Example> out(lines.size());
+  std::vector<const RecordExample*> from;
+  size_t atoms = 0;
+  for (auto l : lines) {
+    from.push_back(&l.cast<const RecordExample&>());
+    for (const RecordExample::Set& s : from.back()->sets) atoms += s.n;
+  }
+  auto make = [&](size_t i) { from[i]->make(out[i]); };
+  if (atoms >= 8192) detail::Workers::run(out.size(), make);
+  else for (size_t i = 0; i < out.size(); i++) make(i);
+  return out;
+}
+
+// host floats into an array on either side; into a tensor on the GPU through pinned memory, ordered
+// on torch's current stream
+void copy_out(const py::object& dest, const ViewInfo& v, const std::vector<float>& host) {
+  const size_t bytes = host.size() * sizeof(float);
+  if (!v.cuda || bytes == 0 || bytes > ((size_t)1 << 20) || torch_names().tensor == nullptr ||
+      !PyObject_TypeCheck(dest.ptr(), torch_names().tensor)) {
+    detail::copy_bytes(v.ptr, host.data(), bytes, false, v.cuda);
+    return;
+  }
+  cudaStream_t st = stream_for(dest);
+  detail::Staging::Slot* slot = detail::small_staging().acquire(bytes);
+  std::memcpy(slot->host, host.data(), bytes);
+  cudaError_t e = cudaMemcpyAsync(v.ptr, slot->host, bytes, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaEventRecord(slot->copied, st);
+  if (e != cudaSuccess) {
+    detail::small_staging().abandon(slot);
+    LMG_CUDA_CHECK(e);
+  }
+  detail::small_staging().release(slot);
+}
+
 // CoordinateSet::sum_types (src/coordinateset.cpp:352-374) into a host or device array
 void sum_types(const CoordinateSet& s, const py::object& sum, bool zerofirst) {
   ViewInfo v = view_info(sum, "sum");
@@ -446,13 +552,16 @@ void gm_forward_objects(GridMaker& gm, const py::args& a, const py::kwargs& kw) 
     return;
   }
   if (is_example_list(a0)) {
-    std::vector<Example> exs = to_examples(a0);
-    Arg o(arg_or(a, 1, kw, {"grid"}), "grid", 5, true);
+    std::vector<Example> own;
+    if (!py::isinstance<std::vector<Example>>(a0)) own = to_examples(a0);
+    const std::vector<Example>& exs = py::isinstance<std::vector<Example>>(a0) ? a0.cast<const std::vector<Example>&>() : own;
+    py::object grid = arg_or(a, 1, kw, {"grid"});
+    Arg o(grid, "grid", 5, true);
     float rt = arg_or(a, 2, kw, {"random_translation"}, py::float_(0.0)).cast<float>();
     bool rr = arg_or(a, 3, kw, {"random_rotation"}, py::bool_(false)).cast<bool>();
     {
       Grid<float, 5, true> og = o.g5();
-      gm.forward(exs, og, rt, rr);
+      gm.forward(exs, og, rt, rr, o.cuda() ? stream_for(grid) : nullptr);
     }
     o.finish();
     return;
@@ -524,7 +633,7 @@ void bind_objects(py::module_& m, py::class_<GridMaker>& gm, py::class_<Transfor
       .def("center", &CoordinateSet::center)
       .def("clone", &CoordinateSet::clone)
       .def("togpu", &CoordinateSet::togpu, py::arg("copy") = true)
-      .def("tocpu", &CoordinateSet::tocpu, py::arg("copy") = true)
+      .def("tocpu", [](const CoordinateSet& s, bool copy) { s.tocpu(copy); }, py::arg("copy") = true)
       .def("copyTo",
            [](const CoordinateSet& s, const py::object& c, const py::object& t, const py::object& r) {
              py::object self = py::cast(s);
@@ -576,7 +685,7 @@ void bind_objects(py::module_& m, py::class_<GridMaker>& gm, py::class_<Transfor
              ViewInfo o = view_info(out, "out");
              if (o.is_double || o.shape.size() != 2 || o.shape[0] != v.size() || o.shape[1] != nl)
                throw std::out_of_range("Incorrect output grid shape for labels");
-             detail::copy_bytes(o.ptr, host.data(), host.size() * sizeof(float), false, o.cuda);
+             copy_out(out, o, host);
            })
       .def("extract_label",
            [](const std::vector<Example>& v, int labelpos, const py::object& out) {
@@ -589,7 +698,7 @@ void bind_objects(py::module_& m, py::class_<GridMaker>& gm, py::class_<Transfor
              ViewInfo o = view_info(out, "out");
              if (o.is_double || o.shape.size() != 1 || o.shape[0] != v.size())
                throw std::out_of_range("Incorrect output grid shape for label");
-             detail::copy_bytes(o.ptr, host.data(), host.size() * sizeof(float), false, o.cuda);
+             copy_out(out, o, host);
            })
       .def("sum_types",
            [](const std::vector<Example>& v, const py::object& sum, bool unique_types) {
@@ -604,6 +713,10 @@ void bind_objects(py::module_& m, py::class_<GridMaker>& gm, py::class_<Transfor
              }
            },
            py::arg("sum"), py::arg("unique_types") = true);
+
+  py::class_<RecordExample>(m, "_RecordExample")
+      .def(py::init<const py::list&, const py::list&, const py::list&, const std::vector<unsigned>&, std::vector<float>, int>());
+  m.def("_make_examples", &make_examples);
 
   gm.def("forward", [](GridMaker& g, const py::args& a, const py::kwargs& kw) { gm_forward_objects(g, a, kw); });
   // the overloads with typed object arguments are tried before the array overloads bound earlier

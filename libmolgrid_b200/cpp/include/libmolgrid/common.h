@@ -5,9 +5,13 @@
 
 #include <cuda_runtime.h>
 
+#include <condition_variable>
 #include <cstddef>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "lmg_b200.h"
 
@@ -41,13 +45,39 @@ inline void check(int rc) {
   throw std::runtime_error(msg);
 }
 
-// Scratch memory handed to the C ABI: one buffer per host thread and device, grown on demand.
-inline void* workspace(size_t bytes) {
-  struct Slot { void* p = nullptr; size_t cap = 0; };
-  thread_local Slot slots[64];
+// Scratch memory handed to the C ABI: one buffer per host thread, device and stream (calls on one
+// stream follow one another), grown on demand.  The eight used last are kept.
+struct WorkspaceSlot {
+  void* p = nullptr;
+  size_t cap = 0;
+  int device = -1;
+  cudaStream_t stream = nullptr;
+};
+inline std::vector<WorkspaceSlot>& workspaces() {
+  thread_local std::vector<WorkspaceSlot> w;  // the one used last in front
+  return w;
+}
+inline const WorkspaceSlot* last_workspace() { return workspaces().empty() ? nullptr : &workspaces().front(); }
+
+inline void* workspace(size_t bytes, cudaStream_t stream = nullptr) {
+  std::vector<WorkspaceSlot>& w = workspaces();
   int dev = 0;
   LMG_CUDA_CHECK(cudaGetDevice(&dev));
-  Slot& s = slots[dev & 63];
+  size_t i = 0;
+  while (i < w.size() && !(w[i].device == dev && w[i].stream == stream)) i++;
+  if (i == w.size()) {
+    if (i >= 8) {
+      cudaFree(w.back().p);  // waits for the work that uses it
+      w.pop_back();
+      i--;
+    }
+    WorkspaceSlot n;
+    n.device = dev;
+    n.stream = stream;
+    w.push_back(n);
+  }
+  if (i != 0) std::swap(w[0], w[i]);
+  WorkspaceSlot& s = w[0];
   if (bytes > s.cap) {
     if (s.p) cudaFree(s.p);
     s.p = nullptr;
@@ -84,6 +114,128 @@ class Staged {
   size_t n_;
   bool out_;
 };
+
+// Pinned host memory (and, for whole batches, device memory of the same size) through which host
+// arrays travel to the GPU without stopping the calling thread.  A slot belongs to one call at a
+// time; it is written again only after the copy out of it, and its device side only after the
+// kernels that read it, as its two events tell.  At most `slots` of them per device are kept, and a
+// slot above 64 MB gives its memory back as soon as its call is over.
+class Staging {
+ public:
+  struct Slot {
+    int device = -1;
+    char* host = nullptr;
+    char* dev = nullptr;
+    size_t cap = 0;
+    bool busy = false, used = false;
+    unsigned long long turn = 0;
+    cudaEvent_t copied = nullptr, done = nullptr;
+  };
+
+  Staging(int slots, bool device_side) : max_(slots), device_side_(device_side) {}
+
+  // a slot of at least `bytes` on the current device, exclusively the caller's until release()
+  Slot* acquire(size_t bytes) {
+    int dev = 0;
+    LMG_CUDA_CHECK(cudaGetDevice(&dev));
+    Slot* s = nullptr;
+    {
+      std::unique_lock<std::mutex> lock(mutex_);
+      for (;;) {
+        int mine = 0;
+        for (Slot* k : slots_) {
+          if (k->device != dev) continue;
+          mine++;
+          // in turn, so that the slot taken is the one whose work was issued first
+          if (!k->busy && (s == nullptr || k->turn < s->turn)) s = k;
+        }
+        if (mine < max_) {
+          s = new Slot();
+          s->device = dev;
+          slots_.push_back(s);
+        }
+        if (s != nullptr) break;
+        freed_.wait(lock);
+      }
+      s->busy = true;
+      s->turn = ++turns_;
+    }
+    try {
+      if (s->copied == nullptr) {
+        LMG_CUDA_CHECK(cudaEventCreateWithFlags(&s->copied, cudaEventDisableTiming));
+        LMG_CUDA_CHECK(cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming));
+      }
+      if (s->used) LMG_CUDA_CHECK(cudaEventSynchronize(s->copied));
+      if (s->cap < bytes) {
+        drop(s);
+        size_t cap = bytes + bytes / 2;
+        LMG_CUDA_CHECK(cudaMallocHost(&s->host, cap));
+        if (device_side_) LMG_CUDA_CHECK(cudaMalloc(&s->dev, cap));
+        s->cap = cap;
+      }
+    } catch (...) {
+      give(s);
+      throw;
+    }
+    return s;
+  }
+
+  // the caller has recorded the slot's events behind its work
+  void release(Slot* s) {
+    s->used = true;
+    if (s->cap > ((size_t)64 << 20)) drop(s);
+    give(s);
+  }
+  // the caller failed before it issued anything
+  void abandon(Slot* s) { give(s); }
+
+  // the stream on which batches travel beside the kernels of the batch before them
+  cudaStream_t copy_stream() {
+    int dev = 0;
+    LMG_CUDA_CHECK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mutex_);
+    if ((int)streams_.size() <= dev) streams_.resize(dev + 1, nullptr);
+    if (streams_[dev] == nullptr) LMG_CUDA_CHECK(cudaStreamCreateWithFlags(&streams_[dev], cudaStreamNonBlocking));
+    return streams_[dev];
+  }
+
+ private:
+  void drop(Slot* s) {
+    if (s->used) {
+      cudaEventSynchronize(s->copied);
+      if (device_side_) cudaEventSynchronize(s->done);
+    }
+    if (s->host) cudaFreeHost(s->host);
+    if (s->dev) cudaFree(s->dev);
+    s->host = s->dev = nullptr;
+    s->cap = 0;
+    s->used = false;
+  }
+  void give(Slot* s) {
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      s->busy = false;
+    }
+    freed_.notify_one();
+  }
+
+  int max_;
+  bool device_side_;
+  std::mutex mutex_;
+  std::condition_variable freed_;
+  std::vector<Slot*> slots_;
+  std::vector<cudaStream_t> streams_;
+  unsigned long long turns_ = 0;
+};
+
+inline Staging& batch_staging() {
+  static Staging* s = new Staging(3, true);  // lives as long as the process, like the CUDA context
+  return *s;
+}
+inline Staging& small_staging() {
+  static Staging* s = new Staging(8, false);
+  return *s;
+}
 
 }  // namespace detail
 }  // namespace libmolgrid

@@ -6,6 +6,8 @@
 #ifndef LMGB200_COORDINATESET_H_
 #define LMGB200_COORDINATESET_H_
 
+#include <cstring>
+#include <utility>
 #include <vector>
 
 #include "libmolgrid/managed_grid.h"
@@ -65,6 +67,10 @@ struct CoordinateSet {
     coords.copyFrom(c); type_vector.copyFrom(t); radii.copyFrom(r);
   }
 
+  // index types, from arrays that are taken over as they are
+  CoordinateSet(MGrid2f c, MGrid1f t, MGrid1f r, unsigned maxt)
+      : coords(std::move(c)), type_index(std::move(t)), radii(std::move(r)), max_type(maxt) {}
+
   // as in the reference, an empty set counts as having both kinds of types
   bool has_indexed_types() const { return type_index.size() > 0 || coords.size() == 0; }
   bool has_vector_types() const { return type_vector.size() > 0 || coords.size() == 0; }
@@ -84,7 +90,7 @@ struct CoordinateSet {
   }
 
   void togpu(bool copy = true) { coords.togpu(copy); type_index.togpu(copy); type_vector.togpu(copy); radii.togpu(copy); }
-  void tocpu(bool copy = true) { coords.tocpu(copy); type_index.tocpu(copy); type_vector.tocpu(copy); radii.tocpu(copy); }
+  void tocpu(bool copy = true) const { coords.tocpu(copy); type_index.tocpu(copy); type_vector.tocpu(copy); radii.tocpu(copy); }
 
   CoordinateSet clone() const {
     CoordinateSet r(*this);
@@ -122,6 +128,29 @@ struct Example {
     for (size_t i = start; i < sets.size(); i++)
       if (sets[i].size() > 0 && !sets[i].has_indexed_types()) return false;
     return true;
+  }
+
+  // The atoms of merge_coordinates() for index types, written to the caller's arrays (room for
+  // num_coordinates() atoms): a single set as it is, the types of further sets shifted past those
+  // of the non-empty sets before them.  Returns the number of atoms.
+  size_t pack_indexed(float* c, float* t, float* r) const {
+    size_t at = 0;
+    unsigned shift = 0;
+    for (const CoordinateSet& cs : sets) {
+      size_t n = cs.size();
+      if (n == 0) continue;
+      if (cs.type_index.size() != n || cs.radii.size() != n)
+        throw std::invalid_argument("Types/radii and coordinates are of different sizes");
+      std::memcpy(c + 3 * at, cs.coords.cpu().data(), n * 3 * sizeof(float));
+      const float* ti = cs.type_index.cpu().data();
+      const float fs = (float)shift;
+      if (shift == 0) std::memcpy(t + at, ti, n * sizeof(float));
+      else for (size_t i = 0; i < n; i++) t[at + i] = ti[i] + fs;
+      std::memcpy(r + at, cs.radii.cpu().data(), n * sizeof(float));
+      at += n;
+      shift += cs.max_type;
+    }
+    return at;
   }
 
   // Concatenation of the sets from `start` on (reference: src/example.cpp:80-110, 147-228): empty

@@ -13,6 +13,7 @@
 
 #include "libmolgrid/coordinateset.h"
 #include "libmolgrid/transform.h"
+#include "libmolgrid/workers.h"
 
 namespace libmolgrid {
 
@@ -172,51 +173,82 @@ class GridMaker {
     forward(in, t, out);
   }
 
-  // whole batch of examples in one pass: merged atoms are padded to the longest example on the
-  // host, copied once, and gridded with one Transform per example
+  // Whole batch of examples in one pass, ordered on `stream` like the array overloads.  The atoms of
+  // every example's sets go straight into one pinned block, merged and padded to the longest example,
+  // and to the GPU in one copy on a stream of its own, so that a batch travels while the kernels of
+  // the batch before it run; they are gridded with one Transform per example.
   void forward(const std::vector<Example>& in, Grid<float, 5, true>& out, float random_translation = 0.0,
-               bool random_rotation = false) const {
+               bool random_rotation = false, cudaStream_t stream = nullptr) const {
     if (in.size() != out.dimension(0)) throw std::out_of_range("output grid dimension does not match size of example vector");
-    size_t B = in.size(), T = out.dimension(1), nmax = 0;
-    std::vector<CoordinateSet> merged(B);
+    size_t B = in.size(), T = out.dimension(1), nmax = 1;
+    bool vec = false;
     for (size_t b = 0; b < B; b++) {
-      merged[b] = in[b].merge_coordinates();
-      if (merged[b].max_type != T)
-        throw std::out_of_range("Incorrect number of channels in output grid: " + itoa(merged[b].max_type) + " vs " + itoa(T));
-      nmax = std::max<size_t>(nmax, merged[b].size());
+      const Example& ex = in[b];
+      const bool v = ex.has_vector_types() && ex.num_coordinates() > 0;
+      if (!v && !ex.has_index_types()) throw std::invalid_argument("Inconsistent typing schemes in merge_coordinates");
+      vec = vec || v;
+      if (ex.num_types() != T)
+        throw std::out_of_range("Incorrect number of channels in output grid: " + itoa(ex.num_types()) + " vs " + itoa(T));
+      nmax = std::max(nmax, ex.num_coordinates());
     }
-    if (nmax == 0) nmax = 1;
-    std::vector<float> hc(B * nmax * 3, 0.f), ht(B * nmax, -1.f), hr(B * nmax, 0.f), hcen(B * 3);
-    std::vector<lmg_transform> htr(B);
-    std::vector<int> hn(B);
-    const float3 inf3 = make_float3(std::numeric_limits<float>::infinity(), 0, 0);
-    for (size_t b = 0; b < B; b++) {
-      Transform t(default_center(in[b], inf3), random_translation, random_rotation);
-      htr[b] = t.c_struct();
-      float3 c = t.get_rotation_center();
-      hcen[3 * b] = c.x; hcen[3 * b + 1] = c.y; hcen[3 * b + 2] = c.z;
-      unsigned n = merged[b].size();
-      hn[b] = (int)n;
-      if (n) {
-        Grid2f cc = merged[b].coords.cpu();
-        Grid1f tt = merged[b].type_index.cpu(), rr = merged[b].radii.cpu();
-        std::memcpy(&hc[b * nmax * 3], cc.data(), n * 3 * sizeof(float));
-        std::memcpy(&ht[b * nmax], tt.data(), n * sizeof(float));
-        std::memcpy(&hr[b * nmax], rr.data(), n * sizeof(float));
-      }
-    }
-    detail::Staged<float> dc(hc.data(), hc.size(), true, false), dt(ht.data(), ht.size(), true, false),
-        dr(hr.data(), hr.size(), true, false), dcen(hcen.data(), hcen.size(), true, false);
-    detail::Staged<lmg_transform> dtr(htr.data(), B, true, false);
-    detail::Staged<int> dn(hn.data(), B, true, false);
-    lmg_atoms a = {};
-    a.batch = (int)B; a.max_atoms = (int)nmax; a.ntypes = (int)T;
-    a.coords = dc.get(); a.type_index = dt.get(); a.radii = dr.get(); a.centers = dcen.get();
-    a.transforms = dtr.get(); a.n_atoms = dn.get();
     for (int i = 2; i <= 4; i++)
       if (out.dimension(i) != s_.dim) throw std::out_of_range("Output grid dimension incorrect: " + itoa(s_.dim) + " vs " + itoa(out.dimension(i)));
-    run_forward(a, out.data(), 0);
-    LMG_CUDA_CHECK(cudaStreamSynchronize(nullptr));  // staged inputs are released on return
+    if (B == 0) return;
+    const float3 inf3 = make_float3(std::numeric_limits<float>::infinity(), 0, 0);
+    if (vec) {  // type vectors: example by example
+      for (size_t b = 0; b < B; b++) {
+        Grid<float, 4, true> og = out[b];
+        forward(in[b], Transform(default_center(in[b], inf3), random_translation, random_rotation), og);
+      }
+      LMG_CUDA_CHECK(cudaStreamSynchronize(nullptr));
+      return;
+    }
+    // coords [B][nmax][3] | types [B][nmax] | radii [B][nmax] | centers [B][3] | transforms [B] | counts [B]
+    auto up = [](size_t n) { return (n + 15) / 16 * 16; };
+    const size_t oc = 0, ot = oc + up(B * nmax * 12), orad = ot + up(B * nmax * 4), ocen = orad + up(B * nmax * 4),
+                 otr = ocen + up(B * 12), on = otr + up(B * sizeof(lmg_transform)), total = on + up(B * 4);
+    detail::Staging& pool = detail::batch_staging();
+    detail::Staging::Slot* slot = pool.acquire(total);
+    try {
+      float *hc = reinterpret_cast<float*>(slot->host + oc), *ht = reinterpret_cast<float*>(slot->host + ot),
+            *hr = reinterpret_cast<float*>(slot->host + orad), *hcen = reinterpret_cast<float*>(slot->host + ocen);
+      lmg_transform* htr = reinterpret_cast<lmg_transform*>(slot->host + otr);
+      int* hn = reinterpret_cast<int*>(slot->host + on);
+      for (size_t b = 0; b < B; b++) {
+        Transform t(default_center(in[b], inf3), random_translation, random_rotation);
+        htr[b] = t.c_struct();
+        float3 c = t.get_rotation_center();
+        hcen[3 * b] = c.x; hcen[3 * b + 1] = c.y; hcen[3 * b + 2] = c.z;
+        for (const CoordinateSet& cs : in[b].sets) cs.tocpu();
+      }
+      // a batch of some 100 kB and more is laid out by several threads
+      auto pack = [&](size_t b) { hn[b] = (int)in[b].pack_indexed(hc + b * nmax * 3, ht + b * nmax, hr + b * nmax); };
+      if (B * nmax >= 8192) detail::Workers::run(B, pack);
+      else for (size_t b = 0; b < B; b++) pack(b);
+      cudaStream_t cs = pool.copy_stream();
+      if (slot->used) LMG_CUDA_CHECK(cudaStreamWaitEvent(cs, slot->done, 0));
+      LMG_CUDA_CHECK(cudaMemcpyAsync(slot->dev, slot->host, total, cudaMemcpyHostToDevice, cs));
+      LMG_CUDA_CHECK(cudaEventRecord(slot->copied, cs));
+      LMG_CUDA_CHECK(cudaStreamWaitEvent(stream, slot->copied, 0));
+    } catch (...) {
+      pool.abandon(slot);
+      throw;
+    }
+    lmg_atoms a = {};
+    a.batch = (int)B; a.max_atoms = (int)nmax; a.ntypes = (int)T;
+    a.coords = reinterpret_cast<float*>(slot->dev + oc); a.type_index = reinterpret_cast<float*>(slot->dev + ot);
+    a.radii = reinterpret_cast<float*>(slot->dev + orad); a.centers = reinterpret_cast<float*>(slot->dev + ocen);
+    a.transforms = reinterpret_cast<lmg_transform*>(slot->dev + otr); a.n_atoms = reinterpret_cast<int*>(slot->dev + on);
+    try {
+      run_forward(a, out.data(), 0, stream);
+    } catch (...) {
+      cudaEventRecord(slot->done, stream);
+      pool.release(slot);
+      throw;
+    }
+    cudaError_t e = cudaEventRecord(slot->done, stream);
+    pool.release(slot);
+    LMG_CUDA_CHECK(e);
   }
 
   // ------------------------------------------------------------------ forward, host grids
@@ -417,7 +449,8 @@ class GridMaker {
   // thread met a type index >= the number of channels (the reference checks this while looping
   // over atoms on the host, src/grid_maker.cpp:172,458-460).
   void check_types() const {
-    detail::check(lmg_check_status(detail::workspace(256), nullptr));
+    const detail::WorkspaceSlot* w = detail::last_workspace();
+    if (w != nullptr) detail::check(lmg_check_status(w->p, w->stream));
   }
 
  private:
@@ -468,9 +501,9 @@ class GridMaker {
     if (tr) { tr_ = tr->c_struct(); a.transform_host = &tr_; }
     return a;
   }
-  void run_forward(const lmg_atoms& a, float* out, int vec) const {
+  void run_forward(const lmg_atoms& a, float* out, int vec, cudaStream_t stream = nullptr) const {
     size_t bytes = lmg_workspace_bytes(&s_, LMG_OP_FORWARD, a.batch, a.max_atoms, a.ntypes, vec);
-    detail::check(lmg_forward(&s_, &a, out, detail::workspace(bytes), bytes, nullptr));
+    detail::check(lmg_forward(&s_, &a, out, detail::workspace(bytes, stream), bytes, stream));
   }
   mutable lmg_transform tr_;  // keeps the by-value transform alive for the duration of a call
 };

@@ -7,24 +7,72 @@
 
 #include <cstdlib>
 #include <memory>
+#include <mutex>
+#include <vector>
 
 #include "libmolgrid/grid.h"
 
 namespace libmolgrid {
 
 namespace detail {
+// Host memory for the arrays of one example, taken from and given back to a pool of at most 64 MB.
+// Batches of examples come and go once per training step; through malloc their few megabytes go
+// back to the operating system each time and every page of the next batch is faulted in again.
+class HostBlocks {
+ public:
+  static std::shared_ptr<char> get(size_t bytes) {
+    size_t cls = 12;  // blocks of a power of two, 4 kB and up
+    while (((size_t)1 << cls) < bytes) cls++;
+    char* p = nullptr;
+    {
+      std::lock_guard<std::mutex> lock(self().mutex_);
+      auto& f = self().free_[cls];
+      if (!f.empty()) {
+        p = f.back();
+        f.pop_back();
+        self().held_ -= (size_t)1 << cls;
+      }
+    }
+    if (p == nullptr) p = static_cast<char*>(std::malloc((size_t)1 << cls));
+    if (p == nullptr) throw std::bad_alloc();
+    return std::shared_ptr<char>(p, [cls](char* q) { put(q, cls); });
+  }
+
+ private:
+  std::mutex mutex_;
+  std::vector<char*> free_[64];
+  size_t held_ = 0;
+  static HostBlocks& self() {
+    static HostBlocks* pool = new HostBlocks();  // outlives every array, whatever the order of destruction
+    return *pool;
+  }
+  static void put(char* q, size_t cls) {
+    {
+      std::lock_guard<std::mutex> lock(self().mutex_);
+      if (self().held_ + ((size_t)1 << cls) <= (size_t)64 << 20) {
+        self().free_[cls].push_back(q);
+        self().held_ += (size_t)1 << cls;
+        return;
+      }
+    }
+    std::free(q);
+  }
+};
+
 template <typename Dtype>
 struct Storage {
   Dtype* host = nullptr;
   Dtype* dev = nullptr;
   size_t capacity = 0;   // elements
   bool on_gpu = false;   // the device copy is the valid one
+  std::shared_ptr<char> block;  // what `host` lies in when it is part of a larger allocation
   explicit Storage(size_t n) : capacity(n) {
     host = static_cast<Dtype*>(std::calloc(n ? n : 1, sizeof(Dtype)));
     if (!host) throw std::bad_alloc();
   }
+  Storage(size_t n, Dtype* h, std::shared_ptr<char> b) : host(h), capacity(n), block(std::move(b)) {}
   ~Storage() {
-    std::free(host);
+    if (!block) std::free(host);
     if (dev) cudaFree(dev);
   }
   Storage(const Storage&) = delete;
@@ -76,6 +124,17 @@ class ManagedGrid {
   explicit ManagedGrid(I... sizes) : dims_{static_cast<size_t>(sizes)...} {
     static_assert(NumDims == sizeof...(sizes), "Incorrect number of grid dimensions");
     store_ = std::make_shared<detail::Storage<Dtype>>(size());
+  }
+
+  // a grid whose host side is the memory at `host`, part of `block`
+  template <typename... I>
+  static ManagedGrid within(const std::shared_ptr<char>& block, Dtype* host, I... sizes) {
+    static_assert(NumDims == sizeof...(sizes), "Incorrect number of grid dimensions");
+    ManagedGrid g;
+    const size_t d[NumDims] = {static_cast<size_t>(sizes)...};
+    for (size_t i = 0; i < NumDims; i++) g.dims_[i] = d[i];
+    g.store_ = std::make_shared<detail::Storage<Dtype>>(g.size(), host, block);
+    return g;
   }
 
   size_t dimension(size_t i) const {

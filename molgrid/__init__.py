@@ -142,8 +142,32 @@ def _native_set(cs):
     return native.CoordinateSet(coords, cs.type_index.tonumpy(), radii, cs.max_type)
 
 
+# typers whose mapping is a table over the record types (a user's own typer may be anything)
+_TABLE_TYPERS = (_py.GninaIndexTyper, _py.FileMappedGninaTyper, _py.NullIndexTyper)
+
+
 class ExampleProvider(_py.ExampleProvider):
     """The example provider handing out the compiled Example / ExampleVec types."""
+
+    def _native_line(self, i):
+        """Line i as the compiled module turns it into Examples (its records, the tables of its
+        typers, its labels), made at the line's first use; None where the Python layer has to type
+        the atoms."""
+        lines = self.__dict__.setdefault("_lines", {})
+        if i in lines:
+            return lines[i]
+        ref, line = self.refs[i], None
+        files = self._files(ref)
+        if not self.settings.make_vector_types and all(type(self.caches[c].typer) in _TABLE_TYPERS for _, c in files):
+            recs = [self.caches[c].records(f) for f, c in files]
+            if all(len(r) == 0 or int(r["type"].min()) >= 0 for r in recs):
+                tables = [self.caches[c].tables() for _, c in files]
+                line = native._RecordExample(recs, [t for t, _ in tables], [r for _, r in tables],
+                                             [self.caches[c].num_types() for _, c in files],
+                                             [float(v) for v in ref.labels],
+                                             int(ref.group) if ref.group is not None else -1)
+        lines[i] = line
+        return line
 
     def _make(self, ref):
         pex = _py.ExampleProvider._make(self, ref)
@@ -158,6 +182,14 @@ class ExampleProvider(_py.ExampleProvider):
         B = int(batch_size) or int(self.settings.default_batch_size)
         if hasattr(self._order, "check_batch_size"):
             self._order.check_batch_size(B)
+        if not self._grouped and self.refs:
+            take = self._order.nextref
+            idx = [take() for _ in range(B)]
+            known = self.__dict__.setdefault("_lines", {})
+            lines = [known.get(i) or self._native_line(i) for i in idx]
+            if None not in lines:
+                return native._make_examples(lines)
+            return native.ExampleVec([self._make(self.refs[i]) for i in idx])
         return native.ExampleVec([self.next() for _ in range(B)])
 
 
