@@ -7,6 +7,7 @@ Arrays are torch tensors.  CUDA float32 tensors are used in place; CPU tensors a
 are staged through device memory around the call (every result is computed on the GPU).
 """
 import ctypes
+import os
 
 import numpy as np
 import torch
@@ -165,6 +166,22 @@ class _Arg(object):
     def finish(self):
         if self.output and self.host is not None:
             self.host.copy_(self.t)
+
+
+_native = None     # the compiled module (False: calls stay with ctypes)
+
+
+def _fast():
+    """The compiled module, whose ``_fast_*`` functions take the calls on resident tensors (the atoms,
+    grids and gradients of a training loop) to the C ABI without a line of Python."""
+    global _native
+    if _native is None:
+        if os.environ.get("LMG_B200_LIB"):   # another build of the library than the one the module links
+            _native = False
+        else:
+            from . import molgrid_native
+            _native = molgrid_native
+    return _native
 
 
 _have_cuda = []   # filled on the first successful check
@@ -431,6 +448,18 @@ class GridMaker(object):
         elif nr != N:
             raise exc("radii does not match number of atoms: %d vs %d" % (nr, N))
 
+    def _resident(self, name, args, kw):
+        """The call ``name`` by the compiled module when every array is a float32 CUDA tensor of the
+        right shape; False: the general route takes it (and raises what there is to raise)."""
+        m = _fast()
+        if not m:
+            return False
+        ws = getattr(m, name)(ctypes.addressof(self.s), args, kw or None, _workspaces)
+        if ws is None:
+            return False
+        self._last_ws = ws
+        return True
+
     def _ws(self, dev, op, B, N, T, vec):
         # the size depends on the shapes and the settings: asked once per combination
         key = (op, B, N, T, vec, self.s.radii_type_indexed, self.s.binary, self.s.dim)
@@ -451,6 +480,8 @@ class GridMaker(object):
         * ``forward(center, coords, types, radii, grid)`` - index or vector types, single or batched
           (plus the ``transforms=`` / ``n_atoms=`` extensions of :meth:`forward_arrays`).
         """
+        if len(args) == 5 and self._resident("_fast_forward", args, kw):
+            return
         from .coordinates import CoordinateSet, Example
         from .coord_cache import DeviceBatch
         a0 = args[0] if args else kw.get("example", kw.get("examples", kw.get("examplevec")))
@@ -459,8 +490,10 @@ class GridMaker(object):
             grid = rest[0] if rest else kw["grid"]
             rt = rest[1] if len(rest) > 1 else kw.get("random_translation", 0.0)
             rr = rest[2] if len(rest) > 2 else kw.get("random_rotation", False)
-            return self.forward_arrays(a0.centers, a0.coords, a0.type_index, a0.radii, grid,
-                                       transforms=self.batch_transforms(a0, rt, rr), n_atoms=a0.n_atoms)
+            more = dict(transforms=self.batch_transforms(a0, rt, rr), n_atoms=a0.n_atoms)
+            if self._resident("_fast_forward", (a0.centers, a0.coords, a0.type_index, a0.radii, grid), more):
+                return
+            return self.forward_arrays(a0.centers, a0.coords, a0.type_index, a0.radii, grid, **more)
         if isinstance(a0, Example):
             rest = list(args[1:])
             if rest and isinstance(rest[0], Transform):
@@ -578,6 +611,9 @@ class GridMaker(object):
         gridding kernels - the fused form of forward(Example, Transform, grid)
         (src/grid_maker.cpp:109-116).  ``n_atoms`` marks padded batches.
         """
+        if self._resident("_fast_forward", (center, coords, types, radii, out),
+                          dict(transforms=transforms, n_atoms=n_atoms)):
+            return
         dev, A, keep, batched, vec, B, N, nr = self._atoms(center, coords, types, radii, transforms, n_atoms)
         o = _Arg(out, dev, 5 if batched else 4, "out", output=True)
         oshape = tuple(o.t.shape[1:] if batched else o.t.shape)
@@ -612,6 +648,8 @@ class GridMaker(object):
         """The reference's backward overload set (python/bindings.in.cpp:869-896):
         ``backward(center, coordinate_set, diff, atom_gradients[, type_gradients])`` or
         ``backward(center, coords, types, radii, diff, atom_gradients[, type_gradients])``."""
+        if len(args) in (6, 7) and self._resident("_fast_backward", args, kw):
+            return
         from .coordinates import CoordinateSet
         from .coord_cache import DeviceBatch
         if args and isinstance(args[0], DeviceBatch):
@@ -637,6 +675,9 @@ class GridMaker(object):
         """Atom (and, for vector types, type) gradients from grid gradients ``diff``.
         ``want_type_gradients=False`` (vector types only) skips the type gradients, which lets the
         kernels read just the channels in which an atom carries weight."""
+        if self._resident("_fast_backward", (center, coords, types, radii, diff, atom_gradients, type_gradients),
+                          dict(transforms=transforms, n_atoms=n_atoms, want_type_gradients=bool(want_type_gradients))):
+            return
         dev, A, keep, batched, vec, B, N, nr = self._atoms(center, coords, types, radii, transforms, n_atoms)
         df = _Arg(diff, dev, 5 if batched else 4, "diff")
         ag = _Arg(atom_gradients, dev, 3 if batched else 2, "atom_gradients", output=True)
@@ -678,6 +719,8 @@ class GridMaker(object):
     def backward_relevance(self, *args, **kw):
         """``backward_relevance(center, coordinate_set, density, diff, relevance)`` or the array form
         of :meth:`backward_relevance_arrays` (include/libmolgrid/grid_maker.h:558-618)."""
+        if len(args) == 7 and self._resident("_fast_relevance", args, kw):
+            return
         from .coordinates import CoordinateSet
         if len(args) >= 2 and isinstance(args[1], CoordinateSet):
             center, cs, density, diff, rel = args[:5]

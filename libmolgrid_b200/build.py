@@ -17,7 +17,7 @@ NVCC_FLAGS = [
     "-lineinfo", "-O3", "-std=c++17",
     # no fused multiply-add in host code either: the host computes GridMaker's constants
     "-Xcompiler", "-fPIC,-ffp-contract=off,-fvisibility=default",
-    "--shared",
+    "--shared", "--threads", "8",
 ]
 
 
@@ -48,7 +48,7 @@ def build_library(force=False, verbose=False):
     return LIB
 
 
-NATIVE_SRCS = [os.path.join(HERE, "cpp", "bindings.cpp"), os.path.join(HERE, "cpp", "bindings_objects.cpp")]
+NATIVE_SRCS = [os.path.join(HERE, "cpp", f) for f in ("bindings.cpp", "bindings_objects.cpp", "bindings_fast.cpp")]
 
 
 def native_module_path():
@@ -58,23 +58,40 @@ def native_module_path():
 
 def build_native_module(force=False):
     """Compile the pybind11 module over the C++ host layer (g++; links liblmg_b200.so by $ORIGIN)."""
+    import concurrent.futures
     import pybind11
     import sysconfig
+    import tempfile
+    import torch
     out = native_module_path()
-    deps = NATIVE_SRCS + [os.path.join(HERE, "cpp", "bindings_common.h"), LIB] + [os.path.join(HERE, "cpp", "include", "libmolgrid", f)
-                                for f in os.listdir(os.path.join(HERE, "cpp", "include", "libmolgrid"))]
+    headers = os.path.join(HERE, "cpp", "include", "libmolgrid")
+    deps = NATIVE_SRCS + [LIB] + [os.path.join(HERE, "cpp", f) for f in ("bindings_common.h", "bindings_fast.h")] + \
+        [os.path.join(headers, f) for f in os.listdir(headers)]
     if not force and os.path.exists(out) and all(os.path.getmtime(d) <= os.path.getmtime(out) for d in deps):
         return out
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           "-I" + pybind11.get_include(), "-I" + sysconfig.get_paths()["include"],
-           "-I" + os.path.join(HERE, "cpp", "include"), "-I" + os.path.join(HERE, "..", "include"),
-           "-I" + os.path.join(cuda, "include")] + NATIVE_SRCS + ["-o", out,
-           "-L" + HERE, "-llmg_b200", "-L" + os.path.join(cuda, "lib64"), "-lcudart",
-           "-Wl,-rpath,$ORIGIN", "-pthread", "-Wl,-rpath," + os.path.join(cuda, "lib64")]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+    troot = os.path.dirname(torch.__file__)
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-pthread",
+             "-I" + pybind11.get_include(), "-I" + sysconfig.get_paths()["include"],
+             "-I" + os.path.join(HERE, "cpp", "include"), "-I" + os.path.join(HERE, "..", "include"),
+             "-I" + os.path.join(cuda, "include")]
+    # torch's headers come with their own pybind11: only the file that reads tensors sees them
+    torch_flags = ["-isystem", os.path.join(troot, "include"),
+                   "-isystem", os.path.join(troot, "include", "torch", "csrc", "api", "include")]
+
+    def run(cmd):
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+
+    with tempfile.TemporaryDirectory() as tmp, concurrent.futures.ThreadPoolExecutor() as pool:
+        objs = [os.path.join(tmp, os.path.basename(s) + ".o") for s in NATIVE_SRCS]
+        list(pool.map(lambda so: run(["g++", "-c"] + flags + (torch_flags if "fast" in so[0] else []) + [so[0], "-o", so[1]]),
+                      zip(NATIVE_SRCS, objs)))
+        run(["g++", "-shared", "-pthread"] + objs + ["-o", out, "-L" + HERE, "-llmg_b200",
+             "-L" + os.path.join(cuda, "lib64"), "-lcudart", "-L" + os.path.join(troot, "lib"), "-ltorch_python",
+             "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + os.path.join(cuda, "lib64"),
+             "-Wl,-rpath," + os.path.join(troot, "lib")])
     return out
 
 

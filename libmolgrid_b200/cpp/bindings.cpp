@@ -337,5 +337,7 @@ PYBIND11_MODULE(molgrid_native, m) {
              o.finish();
            });
 
+  gm_class.def_property_readonly("_settings", [](const GridMaker& g) { return (size_t)&g.settings(); });
   bind_objects(m, gm_class, tr_class);
+  if (add_fast_calls(m.ptr()) != 0) throw py::error_already_set();
 }

@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "bindings_fast.h"
 #include "libmolgrid/libmolgrid.h"
 
 namespace lmgpy {
@@ -42,63 +43,31 @@ struct ViewInfo {
   py::object keep;
 };
 
-// torch's tensor type, dtypes and current-stream query, looked up once (null when torch is not
-// importable)
-struct TorchNames {
-  PyTypeObject* tensor = nullptr;
-  py::object f32, f64, i32, stream;
-};
-inline const TorchNames& torch_names() {
-  static TorchNames* names = [] {
-    auto* n = new TorchNames();  // lives as long as the interpreter
-    try {
-      py::module_ torch = py::module_::import("torch");
-      n->f32 = torch.attr("float32");
-      n->f64 = torch.attr("float64");
-      n->i32 = torch.attr("int32");
-      n->stream = torch.attr("_C").attr("_cuda_getCurrentRawStream");
-      n->tensor = reinterpret_cast<PyTypeObject*>(torch.attr("Tensor").ptr());
-    } catch (py::error_already_set&) {
-      n->tensor = nullptr;
-    }
-    return n;
-  }();
-  return *names;
-}
-
 // The stream on which an asynchronous call that writes `o` is issued: torch's current one for a
 // tensor, the default stream for other arrays.
 inline cudaStream_t stream_for(const py::handle& o) {
-  const TorchNames& tn = torch_names();
-  if (tn.tensor == nullptr || !PyObject_TypeCheck(o.ptr(), tn.tensor)) return nullptr;
-  int dev = 0;
-  LMG_CUDA_CHECK(cudaGetDevice(&dev));
-  return reinterpret_cast<cudaStream_t>(tn.stream(dev).cast<size_t>());
+  TorchView t;
+  if (!torch_view(o.ptr(), t) || t.device < 0) return nullptr;
+  return torch_stream(t.device);
 }
 
-// The common case of a training loop, a plain contiguous torch tensor, read with as few attribute
-// look-ups as its checks need.  False: not such a tensor, take the general route.
+// A torch tensor, read through torch's C++ interface.  False: not one, take the general route.
 inline bool tensor_view(const py::object& o, const std::string& name, ViewInfo& v) {
-  const TorchNames& tn = torch_names();
-  if (tn.tensor == nullptr || Py_TYPE(o.ptr()) != tn.tensor) return false;
-  py::object dt = o.attr("dtype");
-  if (dt.is(tn.f32)) v.is_double = false;
-  else if (dt.is(tn.f64)) v.is_double = true;
-  else throw py::value_error(name + ": tensors must be float32 or float64");
-  if (!o.attr("is_contiguous")().cast<bool>()) throw py::value_error("Attempt to use non-contiguous tensor as grid");
-  int dev = o.attr("get_device")().cast<int>();  // -1 for a host tensor
-  v.cuda = dev >= 0;
+  TorchView t;
+  if (!torch_view(o.ptr(), t)) return false;
+  if (t.dtype != 'f' && t.dtype != 'd') throw py::value_error(name + ": tensors must be float32 or float64");
+  v.is_double = t.dtype == 'd';
+  if (!t.contiguous) throw py::value_error("Attempt to use non-contiguous tensor as grid");
+  v.cuda = t.device >= 0;
   if (v.cuda) {
     int cur = 0;
     LMG_CUDA_CHECK(cudaGetDevice(&cur));
-    if (dev != cur)
-      throw py::value_error("Tensor on different device than current: " + std::to_string(dev) + " vs " +
+    if (t.device != cur)
+      throw py::value_error("Tensor on different device than current: " + std::to_string(t.device) + " vs " +
                             std::to_string(cur));
   }
-  v.ptr = reinterpret_cast<void*>(o.attr("data_ptr")().cast<size_t>());
-  py::tuple shape = py::reinterpret_borrow<py::tuple>(o.attr("shape"));  // torch.Size is a tuple
-  v.shape.reserve(shape.size());
-  for (auto d : shape) v.shape.push_back(d.cast<size_t>());
+  v.ptr = t.ptr;
+  v.shape.assign(t.shape, t.shape + t.ndim);
   v.keep = o;
   return true;
 }
@@ -106,14 +75,14 @@ inline bool tensor_view(const py::object& o, const std::string& name, ViewInfo& 
 // A resident int32 tensor with one entry per example (valid atoms of a padded batch), or a
 // resident float32 (B,10) tensor of transforms: the device address, after the checks.
 inline const int* device_counts(const py::object& o, size_t batch) {
-  const TorchNames& tn = torch_names();
-  if (tn.tensor == nullptr || !py::isinstance(o, py::reinterpret_borrow<py::object>((PyObject*)tn.tensor)))
-    throw py::type_error("n_atoms: expected an int32 CUDA tensor");
-  py::object dt = o.attr("dtype");
-  if (!dt.is(tn.i32) || o.attr("get_device")().cast<int>() < 0 || !o.attr("is_contiguous")().cast<bool>())
+  TorchView t;
+  if (!torch_view(o.ptr(), t)) throw py::type_error("n_atoms: expected an int32 CUDA tensor");
+  if (t.dtype != 'i' || t.device < 0 || !t.contiguous)
     throw py::type_error("n_atoms: expected a contiguous int32 CUDA tensor");
-  if (o.attr("numel")().cast<size_t>() != batch) throw py::value_error("n_atoms must have one entry per example");
-  return reinterpret_cast<const int*>(o.attr("data_ptr")().cast<size_t>());
+  size_t n = 1;
+  for (int i = 0; i < t.ndim; i++) n *= t.shape[i];
+  if (n != batch) throw py::value_error("n_atoms must have one entry per example");
+  return static_cast<const int*>(t.ptr);
 }
 
 inline ViewInfo view_info(const py::handle& h, const std::string& name) {
@@ -207,6 +176,8 @@ class Arg {
 };
 
 inline int ndim_of(const py::handle& h) {
+  TorchView t;
+  if (torch_view(h.ptr(), t)) return t.ndim;
   py::object o = py::reinterpret_borrow<py::object>(h);
   if (py::hasattr(o, "shape")) return (int)py::len(o.attr("shape"));
   throw py::type_error("expected an array");

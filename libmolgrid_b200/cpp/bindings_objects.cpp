@@ -409,8 +409,8 @@ std::vector<Example> make_examples(const py::list& lines) {
 // on torch's current stream
 void copy_out(const py::object& dest, const ViewInfo& v, const std::vector<float>& host) {
   const size_t bytes = host.size() * sizeof(float);
-  if (!v.cuda || bytes == 0 || bytes > ((size_t)1 << 20) || torch_names().tensor == nullptr ||
-      !PyObject_TypeCheck(dest.ptr(), torch_names().tensor)) {
+  TorchView t;
+  if (!v.cuda || bytes == 0 || bytes > ((size_t)1 << 20) || !torch_view(dest.ptr(), t)) {
     detail::copy_bytes(v.ptr, host.data(), bytes, false, v.cuda);
     return;
   }

@@ -15,6 +15,7 @@ lists of Transform objects, ``DeviceBatch`` arguments).
 import numpy as np
 
 import libmolgrid_b200 as _py
+from libmolgrid_b200 import api as _api
 from libmolgrid_b200 import build as _build
 
 _build.build_library()
@@ -63,6 +64,12 @@ class GridMaker(native.GridMaker):
         native.GridMaker.__init__(self, resolution, dimension, binary, radius_type_indexed, radius_scale,
                                   gaussian_radius_multiple)
         self._radius_scale, self._grm = radius_scale, gaussian_radius_multiple
+        self._sp = self._settings   # address of the settings, fixed for the life of the object
+
+    def _shared(self, call, args, kw):
+        """A call that the Python layer serves (one centre for a whole batch, batched second
+        derivatives), on resident tensors: through the compiled module on torch's current stream."""
+        return call(self._sp, args, kw or None, _api._workspaces) is not None
 
     @staticmethod
     def _extension(args, kw):
@@ -85,6 +92,9 @@ class GridMaker(native.GridMaker):
         return na is None or (type(na) is torch.Tensor and na.is_cuda and na.dtype is torch.int32)
 
     def forward(self, *args, **kw):
+        if len(args) == 5 and (native._fast_forward(self._sp, args, kw or None, None)
+                               or self._shared(native._fast_forward, args, kw)):
+            return None
         if self._resident_batch(args, kw):
             return native.GridMaker.forward(self, *args, **kw)
         # a batch of arrays about one common centre given as a tuple is this library's shorthand
@@ -94,6 +104,9 @@ class GridMaker(native.GridMaker):
         return native.GridMaker.forward(self, *args, **kw)
 
     def backward(self, *args, **kw):
+        if len(args) in (6, 7) and (native._fast_backward(self._sp, args, kw or None, None)
+                                    or self._shared(native._fast_backward, args, kw)):
+            return None
         if self._resident_batch(args, kw):
             return native.GridMaker.backward(self, *args, **kw)
         batched = len(args) > 1 and _ndim(args[1]) == 3
@@ -107,7 +120,15 @@ class GridMaker(native.GridMaker):
     def forward_arrays(self, *args, **kw):
         return self._twin().forward_arrays(*args, **kw)
 
+    def backward_relevance(self, *args, **kw):
+        if len(args) == 7 and native._fast_relevance(self._sp, args, kw or None, None):
+            return None
+        return native.GridMaker.backward_relevance(self, *args, **kw)
+
     def backward_gradients(self, *args, **kw):
+        if len(args) == 10 and (native._fast_gradients(self._sp, args, kw or None, None)
+                                or self._shared(native._fast_gradients, args, kw)):
+            return None
         batched = len(args) > 1 and _ndim(args[1]) == 3
         if batched or self._extension(args, kw):
             return self._twin().backward_gradients(*args, **kw)
