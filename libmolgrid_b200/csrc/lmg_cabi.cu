@@ -165,6 +165,25 @@ void fill_emit(EmitArgs& E, const lmg_gridmaker* g, const lmg_atoms* a) {
 
 int quads_setting() { return g_quads; }
 
+// No atoms were prepared: nothing to report.
+cudaError_t clear_status(void* ws, cudaStream_t st) { return cudaMemsetAsync(ws, 0, sizeof(StatusHeader), st); }
+
+cudaError_t read_status(const void* ws, int* code, cudaStream_t st) {
+  StatusHeader h;
+  *code = 0;
+  h.count = 0;
+  cudaError_t e = cudaMemcpyAsync(&h, ws, sizeof h, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess || h.magic != STATUS_MAGIC || h.count == 0) return e;
+  std::vector<unsigned char> flags(h.count);
+  e = cudaMemcpyAsync(flags.data(), static_cast<const char*>(ws) + h.offset, h.count, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess)
+    for (unsigned char f : flags)
+      if (f) *code = h.code;
+  return e;
+}
+
 }  // namespace lmg
 
 namespace {
@@ -175,7 +194,7 @@ using lmg::to_xform;
 
 // Scratch layout of one pass over nb examples.
 struct Layout {
-  size_t status, recs, chanp, partial, total;
+  size_t flags, recs, chanp, partial, total;
   size_t per_example;
 };
 
@@ -188,9 +207,10 @@ Layout layout(const lmg_gridmaker* g, int op, int nb, int N, int T, int vec) {
   size_t chanp = (vec && g->radii_type_indexed) ? align_up((size_t)T * sizeof(lmg::ChanParam)) : 0;
   size_t partial = (vec && (op == LMG_OP_BACKWARD || op == LMG_OP_BACKWARD_GRADIENTS))
                        ? align_up((size_t)N * T * 3 * 4) : 0;
-  L.per_example = recs + chanp + partial;
+  size_t flags = align_up((size_t)N / 256 + 1);  // one byte per block of k_emit
+  L.per_example = flags + recs + chanp + partial;
   size_t o = STATUS_BYTES;
-  L.status = 0;
+  L.flags = o; o += flags * nb;
   L.recs = o; o += recs * nb;
   L.chanp = o; o += chanp * nb;
   L.partial = o; o += partial * nb;
@@ -216,7 +236,9 @@ int check_common(const lmg_gridmaker* g, const lmg_atoms* a, const void* ws) {
 }
 
 void carve(lmg::EmitArgs& E, const Layout& L, char* ws) {
-  E.status = reinterpret_cast<int*>(ws + L.status);
+  E.ws = ws;
+  E.flags = L.flags;
+  E.later_pass = E.b0 > 0;
   E.recs = reinterpret_cast<lmg::Rec*>(ws + L.recs);
   E.chanp = reinterpret_cast<lmg::ChanParam*>(ws + L.chanp);
 }
@@ -362,8 +384,7 @@ size_t lmg_workspace_bytes(const lmg_gridmaker* g, int op, int batch, int max_at
 int lmg_check_status(void* workspace, void* stream) {
   if (workspace == nullptr) return fail(LMG_ERR_WORKSPACE, "workspace missing");
   int st = 0;
-  cudaError_t e = cudaMemcpyAsync(&st, workspace, sizeof st, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+  cudaError_t e = lmg::read_status(workspace, &st, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "reading status");
   if (st == 1) return fail(LMG_ERR_OUT_OF_RANGE, "Type index larger than allowed");
   if (st == 2) return fail(LMG_ERR_INVALID_ARGUMENT, "Incorrect channel size for diff");
@@ -380,9 +401,10 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
   char* ws = (char*)workspace;
   int vec = a->type_vector != nullptr;
   size_t grid_elems = (size_t)a->ntypes * g->dim * g->dim * g->dim;
-  cudaError_t e = cudaMemsetAsync(ws, 0, STATUS_BYTES, st);
-  if (e != cudaSuccess) return cuda_fail(e, "clearing status");
+  cudaError_t e;
   if (a->max_atoms == 0 || g->dim == 0) {
+    e = lmg::clear_status(ws, st);
+    if (e != cudaSuccess) return cuda_fail(e, "clearing status");
     e = cudaMemsetAsync(out, 0, grid_elems * a->batch * sizeof(float), st);
     return e == cudaSuccess ? LMG_OK : cuda_fail(e, "zeroing output");
   }
@@ -404,19 +426,15 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
   }
   prof_end(pr_fill, st);
   if (e != cudaSuccess) return cuda_fail(e, "zeroing output");
+  bool self = false;  // the same for every pass of the call
   for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
     int nb = std::min(per_pass, a->batch - b0);
     Layout L = layout(g, LMG_OP_FORWARD, nb, a->max_atoms, a->ntypes, vec);
     lmg::EmitArgs E;
     fill_emit(E, g, a);
-    carve(E, L, ws);
     E.b0 = b0; E.nb = nb;
+    carve(E, L, ws);
     E.round_types = 0;
-    {
-      Range r("emit");
-      e = lmg::launch_emit(E, st);
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "emit");
     lmg::BwdArgs S;
     std::memset(&S, 0, sizeof S);
     S.gm = E.gm; S.b0 = b0; S.nb = nb; S.N = E.N; S.T = E.T;
@@ -427,6 +445,20 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
     S.out_grid = out;
     S.precise = use_precise(g);
     S.quads = g_quads;
+    if (b0 == 0) self = lmg::forward_self_serves(E, S);
+    if (self) {  // its flags, one per atom, run on into the records it does not need
+      ProfRec* pr = prof_begin(0, st);
+      e = lmg::launch_forward_self(E, S, st);
+      prof_end(pr, st);
+      g_launches += 1;
+      if (e != cudaSuccess) return cuda_fail(e, "forward scatter");
+      continue;
+    }
+    {
+      Range r("emit");
+      e = lmg::launch_emit(E, st);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "emit");
     ProfRec* pr = prof_begin(0, st);
     {
       Range r("forward scatter");
@@ -446,27 +478,25 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
   cudaStream_t st = (cudaStream_t)stream;
   char* ws = (char*)workspace;
   int vec = a->type_vector != nullptr;
-  cudaError_t e = cudaMemsetAsync(ws, 0, STATUS_BYTES, st);
-  if (e != cudaSuccess) return cuda_fail(e, "clearing status");
-  if (a->max_atoms == 0) return LMG_OK;
+  cudaError_t e;
+  if (a->max_atoms == 0) {
+    e = lmg::clear_status(ws, st);
+    return e == cudaSuccess ? LMG_OK : cuda_fail(e, "clearing status");
+  }
   Layout one = layout(g, op, 1, a->max_atoms, a->ntypes, vec);
   int per_pass = examples_per_pass(one, workspace_bytes, a->batch);
   if (per_pass == 0)
     return fail(LMG_ERR_WORKSPACE, "workspace too small for one example: need " +
                                        std::to_string(STATUS_BYTES + one.per_example) + " bytes");
+  bool self = false;  // the same for every pass of the call
   for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
     int nb = std::min(per_pass, a->batch - b0);
     Layout L = layout(g, op, nb, a->max_atoms, a->ntypes, vec);
     lmg::EmitArgs E;
     fill_emit(E, g, a);
-    carve(E, L, ws);
     E.b0 = b0; E.nb = nb;
+    carve(E, L, ws);
     E.round_types = 1;
-    {
-      Range r("emit");
-      e = lmg::launch_emit(E, st);
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "emit");
     lmg::BwdArgs B;
     std::memset(&B, 0, sizeof B);
     B.gm = E.gm; B.b0 = b0; B.nb = nb; B.N = E.N; B.T = E.T;
@@ -478,6 +508,20 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
     B.atom_gradients = atom_gradients; B.type_gradients = type_gradients; B.relevance = relevance;
     B.partial = reinterpret_cast<float*>(ws + L.partial);
     B.quads = g_quads;
+    if (b0 == 0) self = lmg::backward_self_serves(E, B, mode);
+    if (self) {  // its flags, one per atom, run on into the records it does not need
+      ProfRec* pr = prof_begin(1, st);
+      e = lmg::launch_backward_self(E, B, mode, st);
+      prof_end(pr, st);
+      g_launches += 1;
+      if (e != cudaSuccess) return cuda_fail(e, "backward");
+      continue;
+    }
+    {
+      Range r("emit");
+      e = lmg::launch_emit(E, st);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "emit");
     g_launches += 1 + ((vec && g->radii_type_indexed) ? 1 : 0);
     ProfRec* pr = prof_begin(1, st);
     {
@@ -543,12 +587,13 @@ int lmg_backward_gradients(const lmg_gridmaker* g, const lmg_atoms* a, const flo
   cudaStream_t st = (cudaStream_t)stream;
   char* ws = (char*)workspace;
   size_t grid_elems = (size_t)a->ntypes * g->dim * g->dim * g->dim;
-  cudaError_t e = cudaMemsetAsync(ws, 0, STATUS_BYTES, st);
-  if (e != cudaSuccess) return cuda_fail(e, "clearing status");
+  cudaError_t e;
   // type_diffdiff is identically zero: the density is linear in the type weights
   e = cudaMemsetAsync(type_diffdiff, 0, (size_t)a->batch * a->max_atoms * a->ntypes * sizeof(float), st);
   if (e != cudaSuccess) return cuda_fail(e, "zeroing type_diffdiff");
   if (a->max_atoms == 0 || g->dim == 0) {
+    e = lmg::clear_status(ws, st);
+    if (e != cudaSuccess) return cuda_fail(e, "clearing status");
     e = cudaMemsetAsync(diffdiff, 0, grid_elems * a->batch * sizeof(float), st);
     return e == cudaSuccess ? LMG_OK : cuda_fail(e, "zeroing output");
   }
@@ -564,8 +609,8 @@ int lmg_backward_gradients(const lmg_gridmaker* g, const lmg_atoms* a, const flo
     Layout L = layout(g, LMG_OP_BACKWARD_GRADIENTS, nb, a->max_atoms, a->ntypes, 1);
     lmg::EmitArgs E;
     fill_emit(E, g, a);
-    carve(E, L, ws);
     E.b0 = b0; E.nb = nb;
+    carve(E, L, ws);
     E.round_types = 0;
     // atom part (atom_diffdiff) and, by scatter, the grid part (diffdiff)
     lmg::BwdArgs B;

@@ -147,8 +147,11 @@ __device__ __forceinline__ void bounds_1d(float origin, float coord, float densi
   }
 }
 
+// (float)i for i < 2^23 without the conversion instruction, which runs on the special-function pipe
+__device__ __forceinline__ float small_float(unsigned i) { return __uint_as_float(i | 0x4b000000u) - 8388608.f; }
+
 __device__ __forceinline__ float voxel_coord(float origin, unsigned i, float res) {
-  return __fadd_rn(origin, __fmul_rn((float)i, res));
+  return __fadd_rn(origin, __fmul_rn(small_float(i), res));
 }
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -165,6 +168,42 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Two floats in a register pair: additions, products and fused multiply-adds of both in one issue slot
+// (each rounded like the single operation).
+struct Pair {
+  unsigned long long v;
+};
+__device__ __forceinline__ Pair pair(float a, float b) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
+  return p;
+}
+__device__ __forceinline__ Pair pair(float a) { return pair(a, a); }
+__device__ __forceinline__ void split(Pair p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+  Pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
 }
 
 constexpr float NEG2_LOG2E = -2.8853900817779268f;  // -2*log2(e)
@@ -194,6 +233,37 @@ __device__ __forceinline__ float density_precise(float rsq, float ar, float Tg, 
   float dr = __fdiv_rn(dist, ar);
   float q = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(A, dr), B), dr), C);
   return q > 0.f ? q : 0.f;
+}
+
+// n / d, correctly rounded, for a divisor whose correctly rounded reciprocal `rd` is at hand: quotient,
+// exact remainder, correction (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990, theorem on division; no overflow or underflow
+// on the way, which distances and radii do not cause).
+__device__ __forceinline__ float divide_by(float n, float d, float rd) {
+  const float q = __fmul_rn(n, rd);
+  return fmaf(fmaf(-q, d, n), rd, q);
+}
+
+// n / d through an approximate reciprocal and the same correction: off by less than one unit in the
+// last place.  Where the correction has no meaning (an infinite quotient) the quotient stands.
+__device__ __forceinline__ float divide_near(float n, float d) {
+  const float r = rcp_approx(d), q = __fmul_rn(n, r), c = fmaf(fmaf(-q, d, n), r, q);
+  return c == c ? c : q;
+}
+
+// sqrt(x), correctly rounded for normal x: root, exact remainder, correction (Markstein, the same
+// paper).  Zero gives NaN.
+__device__ __forceinline__ float root(float x) {
+  const float y = rsqrt_approx(x), s = __fmul_rn(x, y);
+  return fmaf(fmaf(-s, s, x), 0.5f * y, s);
+}
+
+// The tail of calc_point<false> where a quotient of two densities is wanted: near the cut-off it is a
+// small difference of 32-bit numbers, and only the reference's own operation order on the correctly
+// rounded distance over radius gives the reference's quotient.
+__device__ __forceinline__ float tail_quotient(float rsq, float ar, float inv_ar, float A, float B, float C) {
+  const float dr = divide_by(root(rsq), ar, inv_ar);
+  return fmaxf(__fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(A, dr), B), dr), C), 0.f);
 }
 
 __device__ __forceinline__ unsigned lo16(unsigned v) { return v & 0xffffu; }

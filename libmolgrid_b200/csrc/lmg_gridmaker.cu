@@ -8,6 +8,7 @@
 // the density into the grid with red.global.add (k_forward_quads*, k_forward_scatter).
 // Backward passes: one warp per atom reads the grid gradient under the footprint and reduces with
 // shuffles, so no global atomics are needed (k_backward_quads*, k_backward_warp).
+#include "lmg_atoms.cuh"
 #include "lmg_device.cuh"
 #include "lmg_launch.h"
 
@@ -16,21 +17,6 @@ namespace lmg {
 // ---------------------------------------------------------------------------------------------
 // emit
 // ---------------------------------------------------------------------------------------------
-
-// Type-indexed radii: constants of channel t of example b.
-__device__ __forceinline__ void make_chan_param(const GMParams& gm, float radius, ChanParam& cp) {
-  float ar = __fmul_rn(radius, gm.rscale);
-  float densityrad = __fmul_rn(ar, gm.finalm);
-  float Tcut = sqrt_threshold(densityrad);
-  float Tg = sqrt_threshold(__fmul_rn(ar, gm.G));
-  float Tbin = __fmul_rn(ar, ar);
-  bool ok = ar > 0.f;
-  float inv_ar = ok ? 1.f / ar : 0.f;
-  float inv_ar2 = ok ? 1.f / Tbin : 0.f;
-  if (!ok) { Tcut = -1.f; Tg = -1.f; Tbin = -1.f; }
-  cp.p = make_float4(inv_ar2, Tg, inv_ar, Tcut);
-  cp.q = make_float4(Tbin, ar, densityrad, fmaxf(Tcut, gm.binary ? Tbin : -1.f));
-}
 
 __global__ void __launch_bounds__(256) k_chan_params(EmitArgs A) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -44,79 +30,15 @@ __global__ void __launch_bounds__(256) k_chan_params(EmitArgs A) {
 // One thread per atom slot of the pass.
 __global__ void __launch_bounds__(256) k_emit(EmitArgs A) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.nb * A.N) return;
-  int bl = i / A.N, a = i - bl * A.N;
-  int b = A.b0 + bl;
-  const GMParams& gm = A.gm;
-
-  Rec r;
-  r.a = make_float4(0.f, 0.f, 0.f, -1.f);
-  r.b = make_float4(0.f, 0.f, -1.f, 0.f);
-  r.c = make_uint4(0u, 0u, 0u, 0u);
-  r.d = make_float4(-1.f, -1.f, 0.f, 0.f);
-
-  bool valid = A.n_atoms == nullptr || a < A.n_atoms[b];
-  int chan = 0;
-  float ox = 0.f, oy = 0.f, oz = 0.f;
-  if (valid && !A.vec) {
-    float tf = A.type_index[(size_t)b * A.N + a];
-    // forward takes floor (src/grid_maker.cpp:171), the backward passes round (:456, :698)
-    float tc = A.round_types ? roundf(tf) : floorf(tf);
-    if (!(tc >= 0.f)) {
-      valid = false;
-    } else if (tc >= (float)A.T) {
-      valid = false;
-      if (A.check_types) atomicMax(A.status, A.round_types ? 2 : 1);
-    } else {
-      chan = (int)tc;
-    }
+  bool bad = false;
+  if (i < A.nb * A.N) {
+    int bl = i / A.N, a = i - bl * A.N;
+    Rec r;
+    bad = make_rec(A, A.b0 + bl, a, r);
+    A.recs[i] = r;
   }
-  if (valid) {
-    size_t ci = ((size_t)b * A.N + a) * 3;
-    float x = A.coords[ci], y = A.coords[ci + 1], z = A.coords[ci + 2];
-    if (A.transforms != nullptr || A.has_xform_host) {
-      Xform X = A.transforms != nullptr ? A.transforms[b] : A.xform_host;
-      float cn[4];
-      quat_conj_over_norm(X.q, cn);
-      xform_apply(X, cn, x, y, z, true);
-    }
-    float cx, cy, cz;
-    if (A.centers != nullptr) {
-      cx = A.centers[b * 3]; cy = A.centers[b * 3 + 1]; cz = A.centers[b * 3 + 2];
-    } else {
-      cx = A.center_host[0]; cy = A.center_host[1]; cz = A.center_host[2];
-    }
-    ox = __fsub_rn(cx, gm.half); oy = __fsub_rn(cy, gm.half); oz = __fsub_rn(cz, gm.half);
-
-    float radius;
-    if (gm.rti) {
-      // footprint for binning = the largest channel radius of this example
-      radius = -CUDART_INF_F;
-      for (int t = 0; t < A.T; t++) radius = fmaxf(radius, A.radii[(size_t)b * A.T + t]);
-    } else {
-      radius = A.radii[(size_t)b * A.N + a];
-    }
-    ChanParam cp;
-    make_chan_param(gm, radius, cp);
-    float densityrad = cp.q.z;
-    // binary occupancy extends to ar, which exceeds densityrad only when final_radius_multiple < 1;
-    // the reference still clips it to the densityrad footprint, and so do the bounds below
-    unsigned lox, hix, loy, hiy, loz, hiz;
-    bounds_1d(ox, x, densityrad, gm.res, gm.dim, lox, hix);
-    bounds_1d(oy, y, densityrad, gm.res, gm.dim, loy, hiy);
-    bounds_1d(oz, z, densityrad, gm.res, gm.dim, loz, hiz);
-    bool any = cp.q.y > 0.f && hix > lox && hiy > loy && hiz > loz;
-    if (any) {
-      r.a = make_float4(x, y, z, cp.q.w);
-      r.b = make_float4(1.f, cp.p.x, cp.p.y, cp.p.z);
-      r.c = make_uint4(lox | (loy << 16), hix | (hiy << 16), loz | (hiz << 16),
-                       (unsigned)chan | (REC_VALID << 16));
-      r.d = make_float4(cp.p.w, cp.q.x, cp.q.y, cp.q.z);
-    }
-    valid = any;
-  }
-
-  A.recs[i] = r;
+  bad = __syncthreads_or(bad) != 0;
+  if (threadIdx.x == 0) put_flag(A, blockIdx.x, gridDim.x, bad);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -130,6 +52,19 @@ struct ItemParams {
   int chan;
   bool valid;
 };
+
+// The constants of an index-typed atom from its record.
+__device__ __forceinline__ ItemParams item_of(const Rec& r) {
+  ItemParams P;
+  P.valid = ((r.c.w >> 16) & REC_VALID) != 0;
+  P.x = r.a.x; P.y = r.a.y; P.z = r.a.z;
+  P.chan = (int)(r.c.w & 0xffffu);
+  P.w = 1.f;
+  P.inv_ar2 = r.b.y; P.Tg = r.b.z; P.inv_ar = r.b.w; P.Tcut = r.d.x; P.Tbin = r.d.y; P.ar = r.d.z;
+  P.lox = lo16(r.c.x); P.loy = hi16(r.c.x); P.hix = lo16(r.c.y); P.hiy = hi16(r.c.y);
+  P.loz = lo16(r.c.z); P.hiz = hi16(r.c.z);
+  return P;
+}
 
 // Loads the constants of work item `item` (an atom, or an (atom, channel) pair with VEC).
 template <bool VEC>
@@ -191,6 +126,19 @@ constexpr int SCAT_WARPS = LMG_SCAT_WARPS;   // the same for the scatter kernels
 #define LMG_QS_WARPS 1
 #endif
 constexpr int QS_WARPS = LMG_QS_WARPS;
+#ifndef LMG_SELF_ATOMS
+#define LMG_SELF_ATOMS 8192
+#endif
+#ifndef LMG_SELF_SPLIT
+#define LMG_SELF_SPLIT 1200
+#endif
+constexpr int SELF_SPLIT = LMG_SELF_SPLIT;   // most of them that four warps each take
+constexpr int SELF_ATOMS = LMG_SELF_ATOMS;   // most atom slots of a backward pass without k_emit
+#ifndef LMG_FWD_SELF_ATOMS
+#define LMG_FWD_SELF_ATOMS 32768
+#endif
+constexpr int FWD_SELF_ATOMS = LMG_FWD_SELF_ATOMS;  // the same for the forward pass (densities)
+constexpr int REL_SELF_ATOMS = 2560;                // ... and for relevance, whose kernel is the heaviest
 constexpr int BWD2_COLS = 256;  // compacted columns held per warp at a time
 constexpr int ZSTEPS = 4;       // z positions per lane and chunk; a chunk covers 4*ZSTEPS voxels
 
@@ -211,44 +159,70 @@ struct ColBufDT {
 typedef ColBufT<BWD2_COLS> ColBuf;
 typedef ColBufDT<BWD2_COLS> ColBufD;
 
-// Appends the columns of [cbase, ncols) whose squared distance in the xy plane is <= Tcull to the
-// buffer until it is (nearly) full; returns how many it holds and advances cbase.
-template <class BUF, bool WITH_D>
-__device__ __forceinline__ unsigned compact_columns(BUF& buf, const ItemParams& P, unsigned& cbase,
-                                                    unsigned ncols, unsigned ny, float inv_ny, float Tcull,
-                                                    float ox, float oy, float res, unsigned dim, int lane) {
-  unsigned nkept = 0;
-  while (cbase < ncols && nkept + 32 <= BUF::CAP) {
-    unsigned c = cbase + lane;
-    bool keep = false;
-    unsigned x = 0, y = 0;
-    float dx = 0.f, dy = 0.f, dxy2 = 0.f;
-    if (c < ncols) {
-      // c / ny through a float reciprocal (exact for the footprint sizes that fit a grid)
-      unsigned xi = ncols < (1u << 20) ? (unsigned)(((float)c + 0.5f) * inv_ny) : c / ny;
-      unsigned yi = c - xi * ny;
-      x = P.lox + xi;
-      y = P.loy + yi;
-      dx = __fsub_rn(voxel_coord(ox, x, res), P.x);
-      dy = __fsub_rn(voxel_coord(oy, y, res), P.y);
-      dxy2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-      keep = dxy2 <= Tcull;
+// Walk over the columns (x, y) of an item's footprint, a candidate per lane and 32 further on per round.
+// Within a stretch the coordinates are carried along as floats (whole numbers, exact) and the row as an
+// integer, so a round has no division and no conversion: those run on the special-function pipe, which
+// the sweeps need for themselves (occupancy: 34 % of the pipe before).  Between stretches - most
+// footprints are one - only the position is kept.  Of `parts` warps that share an item each walks its
+// share of whole rounds.
+struct Columns {
+  unsigned next, end;
+
+  __device__ __forceinline__ Columns(const ItemParams& P, unsigned part = 0, unsigned parts = 1) {
+    next = 0;
+    end = (P.hix - P.lox) * (P.hiy - P.loy);
+    if (parts > 1) {
+      const unsigned rounds = (end + 31) / 32, per = (rounds + parts - 1) / parts * 32;
+      next = part * per;
+      end = min(end, next + per);
     }
-    unsigned m = __ballot_sync(0xffffffffu, keep);
-    if (keep) {
-      unsigned slot = nkept + __popc(m & ((1u << lane) - 1u));
-      buf.row[slot] = x * dim + y;
-      buf.dxy2[slot] = dxy2;
-      if constexpr (WITH_D) {
-        buf.dx[slot] = dx;
-        buf.dy[slot] = dy;
-      }
-    }
-    nkept += __popc(m);
-    cbase += 32;
   }
-  return nkept;
-}
+  __device__ __forceinline__ bool more() const { return next < end; }
+
+  // Appends the columns whose squared distance in the xy plane is <= Tcull to the buffer until it is
+  // (nearly) full or the walk is over; returns how many it holds.
+  template <bool WITH_D, class BUF>
+  __device__ __forceinline__ unsigned compact(BUF& buf, const ItemParams& P, float Tcull, float ox, float oy, float res,
+                                              unsigned dim, int lane) {
+    const unsigned ny = P.hiy - P.loy;
+    const float nyf = small_float(ny), inv_ny = __fdividef(1.f, nyf);
+    unsigned c = next + lane;
+    // small quotients through the reciprocal: off by less than the half that is added
+    const unsigned xi = next != 0 ? c / ny : (unsigned)((small_float(c) + 0.5f) * inv_ny), yi = c - xi * ny;
+    const unsigned q = (unsigned)(32.5f * inv_ny), r = 32u - q * ny;
+    float xf = small_float(P.lox + xi), yf = small_float(P.loy + yi);
+    const float yend = small_float(P.hiy), qf = small_float(q), rf = small_float(r);
+    unsigned row = (P.lox + xi) * dim + P.loy + yi;
+    unsigned nkept = 0;
+    do {
+      const float dx = __fsub_rn(__fadd_rn(ox, __fmul_rn(xf, res)), P.x), dy = __fsub_rn(__fadd_rn(oy, __fmul_rn(yf, res)), P.y);
+      const float dxy2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+      const bool keep = c < end && dxy2 <= Tcull;
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const unsigned slot = nkept + __popc(m & ((1u << lane) - 1u));
+        buf.row[slot] = row;
+        buf.dxy2[slot] = dxy2;
+        if constexpr (WITH_D) {
+          buf.dx[slot] = dx;
+          buf.dy[slot] = dy;
+        }
+      }
+      nkept += __popc(m);
+      next += 32;
+      c += 32;
+      yf += rf;
+      xf += qf;
+      row += q * dim + r;
+      if (yf >= yend) {
+        yf -= nyf;
+        xf += 1.f;
+        row += dim - ny;
+      }
+    } while (next < end && nkept + 32 <= BUF::CAP);
+    return nkept;
+  }
+};
 
 // MODE 0: atom gradient (index types)          -> atom_gradients[b][a][3]
 // MODE 1: atom + type gradient (vector types)  -> partial[b][a][t][3], type_gradients[b][a][t]
@@ -300,13 +274,9 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
   const float k4 = 4.f * P.inv_ar2, kD = -gm.D * P.inv_ar2, kE = -gm.E * P.inv_ar;  // sign of -(s*dv) folded in
 
   if (P.valid) {
-    unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-    unsigned ncols = nx * ny;
-    float inv_ny = 1.f / (float)ny;
     int grp = lane >> 2, sub = lane & 3;
-    for (unsigned cbase = 0; cbase < ncols;) {
-      unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, Tcull, ox, oy,
-                                                      gm.res, gm.dim, lane);
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
       __syncwarp();
       for (unsigned zc = P.loz; zc < P.hiz; zc += 4 * ZSTEPS) {
         // this lane's z positions of the chunk; positions past the footprint get NaN, which fails
@@ -379,7 +349,8 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
               if (BINARY) {
                 v = rsq < P.Tbin ? 1.f : 0.f;
               } else if (MODE == 2) {
-                v = density_precise(rsq, P.ar, P.Tg, P.Tcut, gm.A, gm.B, gm.C);
+                v = rsq <= P.Tg ? g : tail_quotient(rsq, P.ar, P.inv_ar, gm.A, gm.B, gm.C);
+                v = rsq <= P.Tcut ? v : 0.f;
               } else {
                 float sq = sqrt_approx(rsq * P.inv_ar2);
                 float q = fmaxf(fmaf(fmaf(gm.A, sq, gm.B), sq, gm.C), 0.f);
@@ -390,7 +361,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
                 tg = fmaf(v, dv, tg);
               } else if (v > 0.f) {
                 float de = __ldg(dens + rowoff + 4 * k);
-                if (de > 0.f) tg += __fdiv_rn(__fmul_rn(dv, v), de);
+                if (de > 0.f) tg += divide_near(__fmul_rn(dv, v), de);
               }
             }
           }  // k
@@ -434,10 +405,9 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
 // forward by scatter: the grid is zero-filled first, then one warp per atom (or per (atom, channel)
 // pair with vector types) sweeps the atom's footprint exactly as the backward kernel does and adds
 // its density into the grid with fire-and-forget reductions (red.global.add.f32), which resolve in
-// L2.  No lists, no per-region work: the cost is proportional to the atoms' footprints.  Binary
-// occupancy with index types needs no reduction at all (every writer stores the same 1.0).
+// L2.  No lists, no per-region work: the cost is proportional to the atoms' footprints.
 // ---------------------------------------------------------------------------------------------
-template <bool BINARY, bool PRECISE, bool VEC>
+template <bool BINARY, bool PRECISE, bool VEC>  // not <true, *, false>: k_forward_binary
 __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_scatter(BwdArgs G) {
   __shared__ ColBuf bufs[SCAT_WARPS];
   const GMParams& gm = G.gm;
@@ -469,13 +439,9 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_scatter(BwdArgs G) 
   const float Tcull = BINARY ? P.Tbin : P.Tcut;
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
 
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
   int grp = lane >> 2, sub = lane & 3;
-  for (unsigned cbase = 0; cbase < ncols;) {
-    unsigned nkept = compact_columns<ColBuf, false>(buf, P, cbase, ncols, ny, inv_ny, Tcull, ox, oy,
-                                                    gm.res, gm.dim, lane);
+  for (Columns cols(P); cols.more();) {
+    const unsigned nkept = cols.compact<false>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
     __syncwarp();
     for (unsigned zc = P.loz; zc < P.hiz; zc += 4 * ZSTEPS) {
       unsigned z0 = zc + sub;
@@ -495,10 +461,7 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_scatter(BwdArgs G) 
         for (int k = 0; k < ZSTEPS; k++) {
           float rsq = __fadd_rn(dxy2, dz2t[k]);
           if (BINARY) {
-            if (rsq < P.Tbin) {
-              if (VEC) atomicAdd(row + 4 * k, P.w);
-              else row[4 * k] = 1.f;
-            }
+            if (rsq < P.Tbin) atomicAdd(row + 4 * k, P.w);  // type vectors: weights add up
           } else {
             if (!(rsq <= P.Tcut)) continue;
             float v;
@@ -557,13 +520,9 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_gradgrad_scatter(BwdArgs G)
   // -w * (d density/d dist)/dist: Gaussian 4 w g / ar^2; tail -w (D/ar^2 + E/(ar dist))
   const float k4 = 4.f * P.inv_ar2 * P.w, kD = -gm.D * P.inv_ar2 * P.w, kE = -gm.E * P.inv_ar * P.w;
 
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
   int grp = lane >> 2, sub = lane & 3;
-  for (unsigned cbase = 0; cbase < ncols;) {
-    unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, P.Tcut, ox, oy,
-                                                    gm.res, gm.dim, lane);
+  for (Columns cols(P); cols.more();) {
+    const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
     __syncwarp();
     for (unsigned zc = P.loz; zc < P.hiz; zc += 4 * ZSTEPS) {
       unsigned z0 = zc + sub;
@@ -705,38 +664,20 @@ __device__ __forceinline__ void qlane_sweep_span(unsigned span, const ItemParams
 // number of aligned quads between the first and the last z of a footprint
 __device__ __forceinline__ unsigned quad_span(const ItemParams& P) { return (P.hiz - (P.loz & ~3u) + 3) >> 2; }
 
-// One work item (an atom, or an (atom, channel) pair with VEC) of the forward pass on aligned quads.
+// The sweep of one work item of the forward pass on aligned quads, whose constants are in P.  Of
+// `parts` warps that share an item, this one takes the `part`-th share of its columns.
 template <bool VEC>
-__device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, int bl, ColBuf& buf, int lane) {
+__device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemParams& P, int b, float ox, float oy,
+                                                   float oz, ColBuf& buf, int lane, unsigned part = 0,
+                                                   unsigned parts = 1) {
   const GMParams& gm = G.gm;
-  int b = G.b0 + bl;
-  if (VEC) {
-    // an (atom, channel) pair without weight contributes nothing: leave before any other load
-    int ea = item / G.T;
-    if (G.type_vector[((size_t)b * G.N + ea) * G.T + (item - ea * G.T)] == 0.f) return;
-  }
-
-  float cx, cy, cz;
-  if (G.centers != nullptr) {
-    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
-  } else {
-    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
-  }
-  float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
-  ItemParams P = load_item<VEC>(G, bl, b, item, ox, oy, oz);
-  if (!P.valid || (VEC && P.w == 0.f)) return;  // zero weights add nothing (src/grid_maker.cpp:229)
-
   size_t dim = gm.dim;
   float* out = G.out_grid + ((size_t)b * G.T + P.chan) * dim * dim * dim;
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
   const float ta = gm.ta, ntb = -gm.tb;
 
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
-  for (unsigned cbase = 0; cbase < ncols;) {
-    unsigned nkept = compact_columns<ColBuf, false>(buf, P, cbase, ncols, ny, inv_ny, P.Tcut, ox, oy,
-                                                    gm.res, gm.dim, lane);
+  for (Columns cols(P, part, parts); cols.more();) {
+    const unsigned nkept = cols.compact<false>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
     __syncwarp();
     // With a tail the density is continuous in the distance, and the squared distances may be taken
     // in units of ar^2 (s = rsq / ar^2: one multiplication per column and z position instead of one per
@@ -749,12 +690,21 @@ __device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, i
       auto quad = [&](unsigned, float dxy2, float exy, const float (&d2v)[4], const float (&ev)[4],
                       const float (&)[4], size_t off) {
         float v[4];
+        const Pair xy = pair(dxy2), e2 = pair(exy), ta2 = pair(ta), ntb2 = pair(ntb);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          float sq = dxy2 + d2v[j];
-          float tq = fminf(fmaf(ta, sqrt_approx(sq), ntb), 0.f);  // a NaN gives zero too
-          float val = sq <= sg ? exy * ev[j] : tq * tq;
-          v[j] = VEC ? val * P.w : val;
+        for (int j = 0; j < 4; j += 2) {
+          float s0, s1, g0, g1, t0, t1;
+          split(add2(xy, pair(d2v[j], d2v[j + 1])), s0, s1);
+          split(mul2(e2, pair(ev[j], ev[j + 1])), g0, g1);
+          split(fma2(ta2, pair(sqrt_approx(s0), sqrt_approx(s1)), ntb2), t0, t1);
+          const Pair tq = pair(fminf(t0, 0.f), fminf(t1, 0.f));  // a NaN gives zero too
+          split(mul2(tq, tq), t0, t1);
+          v[j] = s0 <= sg ? g0 : t0;
+          v[j + 1] = s1 <= sg ? g1 : t1;
+          if (VEC) {
+            v[j] *= P.w;
+            v[j + 1] *= P.w;
+          }
         }
         red_add_v4(out + off, v[0], v[1], v[2], v[3]);
       };
@@ -779,6 +729,29 @@ __device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, i
   }
 }
 
+// One work item (an atom, or an (atom, channel) pair with VEC) of the forward pass on aligned quads.
+template <bool VEC>
+__device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, int bl, ColBuf& buf, int lane) {
+  const GMParams& gm = G.gm;
+  int b = G.b0 + bl;
+  if (VEC) {
+    // an (atom, channel) pair without weight contributes nothing: leave before any other load
+    int ea = item / G.T;
+    if (G.type_vector[((size_t)b * G.N + ea) * G.T + (item - ea * G.T)] == 0.f) return;
+  }
+
+  float cx, cy, cz;
+  if (G.centers != nullptr) {
+    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
+  } else {
+    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
+  }
+  float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
+  ItemParams P = load_item<VEC>(G, bl, b, item, ox, oy, oz);
+  if (!P.valid || (VEC && P.w == 0.f)) return;  // zero weights add nothing (src/grid_maker.cpp:229)
+  forward_quads_core<VEC>(G, P, b, ox, oy, oz, buf, lane);
+}
+
 template <bool VEC>
 __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads(BwdArgs G) {
   __shared__ ColBuf bufs[QS_WARPS];
@@ -786,6 +759,99 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads(BwdArgs G) {
   int item = blockIdx.x * QS_WARPS + wid;
   if (item >= (VEC ? G.N * G.T : G.N)) return;
   forward_quads_item<VEC>(G, item, blockIdx.y, bufs[wid], lane);
+}
+
+// Occupancy of index types: every writer stores the same 1.0, so nothing is reduced and any alignment
+// will do.  A sphere of one radius lies in a third of the columns of the density's footprint (1.5 radii):
+// the candidates are cut down to it, and the z steps to its height.  The lanes are eight columns of four.
+template <int STEPS>
+__device__ __forceinline__ void occupancy_sweep(const ItemParams& P, const ColBuf& buf, unsigned nkept, unsigned zlo,
+                                                unsigned zhi, float oz, const GMParams& gm, float* out, int lane) {
+  const int grp = lane >> 2, sub = lane & 3;
+  for (unsigned zc = zlo; zc < zhi; zc += 4 * STEPS) {
+    const unsigned z0 = zc + sub;
+    float dz2[STEPS];
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+      const unsigned zz = z0 + 4 * k;
+      const float dz = __fsub_rn(voxel_coord(oz, zz, gm.res), P.z);
+      dz2[k] = zz < zhi ? __fmul_rn(dz, dz) : CUDART_NAN_F;
+    }
+    for (unsigned i = grp; i < nkept; i += 8) {
+      const float dxy2 = buf.dxy2[i];
+      float* row = out + (size_t)buf.row[i] * gm.dim + z0;
+#pragma unroll
+      for (int k = 0; k < STEPS; k++)
+        if (__fadd_rn(dxy2, dz2[k]) < P.Tbin) row[4 * k] = 1.f;
+    }
+  }
+}
+
+// [lo, hi) within the voxels less than `ar` from the atom along an axis, and one more at either end
+__device__ __forceinline__ void within(float origin, float at, float ar, float res, unsigned& lo, unsigned& hi) {
+  const float inv = __fdividef(1.f, res), c = (at - origin) * inv, r = ar * inv;
+  const float l = floorf(c - r) - 1.f, h = ceilf(c + r) + 1.f;
+  if (l > (float)lo) lo = (unsigned)l;
+  if (h < (float)hi) hi = h > 0.f ? (unsigned)h : 0u;
+}
+
+__device__ __forceinline__ void forward_binary_core(const BwdArgs& G, ItemParams P, int b, float ox, float oy, float oz,
+                                                    ColBuf& buf, int lane, unsigned part = 0, unsigned parts = 1) {
+  const GMParams& gm = G.gm;
+  const size_t dim = gm.dim;
+  float* out = G.out_grid + ((size_t)b * G.T + P.chan) * dim * dim * dim;
+  within(ox, P.x, P.ar, gm.res, P.lox, P.hix);
+  within(oy, P.y, P.ar, gm.res, P.loy, P.hiy);
+  within(oz, P.z, P.ar, gm.res, P.loz, P.hiz);
+  if (P.hix <= P.lox || P.hiy <= P.loy || P.hiz <= P.loz) return;
+  for (Columns cols(P, part, parts); cols.more();) {
+    const unsigned nkept = cols.compact<false>(buf, P, P.Tbin, ox, oy, gm.res, gm.dim, lane);
+    __syncwarp();
+    const unsigned nz = P.hiz - P.loz;
+    if (nz <= 8) occupancy_sweep<2>(P, buf, nkept, P.loz, P.hiz, oz, gm, out, lane);
+    else if (nz <= 12) occupancy_sweep<3>(P, buf, nkept, P.loz, P.hiz, oz, gm, out, lane);
+    else occupancy_sweep<4>(P, buf, nkept, P.loz, P.hiz, oz, gm, out, lane);
+    __syncwarp();
+  }
+}
+
+#ifndef LMG_BIN_WARPS
+#define LMG_BIN_WARPS 4
+#endif
+constexpr int BIN_WARPS = LMG_BIN_WARPS;
+__global__ void __launch_bounds__(BIN_WARPS * 32) k_forward_binary(BwdArgs G) {
+  __shared__ ColBuf bufs[BIN_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, item = blockIdx.x * BIN_WARPS + wid;
+  if (item >= G.N) return;
+  const int bl = blockIdx.y, b = G.b0 + bl;
+  float cx, cy, cz;
+  if (G.centers != nullptr) {
+    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
+  } else {
+    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
+  }
+  const float ox = __fsub_rn(cx, G.gm.half), oy = __fsub_rn(cy, G.gm.half), oz = __fsub_rn(cz, G.gm.half);
+  const ItemParams P = load_item<false>(G, bl, b, item, ox, oy, oz);
+  if (P.valid) forward_binary_core(G, P, b, ox, oy, oz, bufs[wid], lane);
+}
+
+// Index types without k_emit: every warp prepares its atom itself, and WARPS warps share an atom's columns
+// while the atoms alone would leave most of the chip idle.  With the zero fill, 300 atoms into 28x48^3:
+// 11.6 -> 7.3 us; 64 x 1000 atoms: 234.9 -> 229.7 us; 50 x 3000: 264 -> 285 us, so densities of more than
+// FWD_SELF_ATOMS slots keep k_emit.  Occupancy, whose sweeps are a third as long, gains at every size
+// (50 x 3000: 250 -> 228 us).
+template <bool BINARY, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_forward_self(EmitArgs A, BwdArgs G) {
+  __shared__ ColBuf bufs[WARPS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, a = blockIdx.x, bl = blockIdx.y, b = A.b0 + bl;
+  Rec r;
+  float ox, oy, oz;
+  const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
+  if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
+  const ItemParams P = item_of(r);
+  if (!P.valid) return;
+  if (BINARY) forward_binary_core(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
+  else forward_quads_core<false>(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
 }
 
 // Vector types whose radii differ by channel: one warp takes a group of NZ_GROUP consecutive channels
@@ -822,11 +888,12 @@ struct BwdSums {
 };
 
 // The sweep of one work item whose constants are in P: sums over the item's footprint, reduced
-// over the warp.  `item` and `b` only serve MODE 3 (its incoming gradients).
+// over the warp.  `item` and `b` only serve MODE 3 (its incoming gradients).  Of `parts` warps that
+// share an item, this one takes the `part`-th share of its columns.
 template <int MODE, bool BINARY, class BUF>
 __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemParams& P, int b, int item,
                                                        float ox, float oy, float oz, BUF& buf, ZTabs& zt,
-                                                       int lane) {
+                                                       int lane, unsigned part = 0, unsigned parts = 1) {
   const GMParams& gm = G.gm;
   size_t dim = gm.dim;
   size_t chan_off = ((size_t)b * G.T + P.chan) * dim * dim * dim;
@@ -853,14 +920,11 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
   const float ta = gm.ta, ntb = -gm.tb;
   const float g16 = 16.f * P.inv_ar2 * P.inv_ar2, gm4 = -4.f * P.inv_ar2;  // MODE 3, Gaussian part
   float sb = 0.f;                                                            // MODE 3: sum of diff*beta
+  Pair az2 = pair(0.f);                                                      // MODE 0: agz of even and odd voxels
 
   if (P.valid) {
-    unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-    unsigned ncols = nx * ny;
-    float inv_ny = 1.f / (float)ny;
-    for (unsigned cbase = 0; cbase < ncols;) {
-      unsigned nkept = compact_columns<BUF, true>(buf, P, cbase, ncols, ny, inv_ny, Tcull, ox, oy,
-                                                  gm.res, gm.dim, lane);
+    for (Columns cols(P, part, parts); cols.more();) {
+      const unsigned nkept = cols.compact<true>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
       for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
         fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
@@ -877,6 +941,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
           float exy4 = k4 * exy;
           float fsum = 0.f;
           float dotxy = MODE == 3 ? fmaf(dx, inx, dy * iny) : 0.f;
+          Pair fs2 = pair(0.f);                // MODE 0: fsum of even and odd voxels
           float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // MODE 3: sums over the column of diff*alpha*{1, dz, dz^2}
           for (unsigned q0 = 0; q0 < nq; q0 += 4) {
             // up to four quads of the column are requested together, then used
@@ -901,11 +966,26 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
                     dev[0] = de.x; dev[1] = de.y; dev[2] = de.z; dev[3] = de.w;
                   }
                 }
+                if (MODE == 0) {
+                  // the arithmetic of the branch below on two voxels at a time
+                  const Pair xy = pair(dxy2), e4 = pair(exy4), kE2 = pair(kE), kD2 = pair(kD);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
+                  for (int j = 0; j < 4; j += 2) {
+                    float r0, r1, g0, g1, t0, t1;
+                    split(add2(xy, pair(d2v[j], d2v[j + 1])), r0, r1);
+                    split(mul2(e4, pair(ev[j], ev[j + 1])), g0, g1);
+                    split(fma2(kE2, pair(rsqrt_approx(r0), rsqrt_approx(r1)), kD2), t0, t1);
+                    const Pair f = mul2(pair(r0 <= P.Tg ? g0 : fmaxf(t0, 0.f), r1 <= P.Tg ? g1 : fmaxf(t1, 0.f)),
+                                        pair(dvv[j], dvv[j + 1]));
+                    fs2 = add2(fs2, f);
+                    az2 = fma2(f, pair(dzv[j], dzv[j + 1]), az2);
+                  }
+                }
+#pragma unroll
+                for (int j = 0; j < (MODE == 0 ? 0 : 4); j++) {
                   float rsq = __fadd_rn(dxy2, d2v[j]);
                   float g = exy * ev[j];  // exp(-2 rsq / ar^2)
-                  if (MODE == 0 || MODE == 1) {
+                  if (MODE == 1) {
                     // -(d density / d dist) / dist * dv, src/grid_maker.cu:881-919; rsq == 0
                     // contributes nothing because dx = dy = dz = 0 there
                     // a NaN rsq (z outside the footprint) takes the second branch and clamps to zero
@@ -925,9 +1005,15 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
                     tg = fmaf(v, dvv[j], tg);
                   }
                   if (MODE == 2) {
-                    float v = BINARY ? (rsq < P.Tbin ? 1.f : 0.f)
-                                     : density_precise(rsq, P.ar, P.Tg, P.Tcut, gm.A, gm.B, gm.C);
-                    if (v > 0.f && dev[j] > 0.f) tg += __fdiv_rn(__fmul_rn(dvv[j], v), dev[j]);
+                    float v;
+                    if (BINARY) {
+                      v = rsq < P.Tbin ? 1.f : 0.f;
+                    } else {
+                      v = rsq <= P.Tg ? g : tail_quotient(rsq, P.ar, P.inv_ar, gm.A, gm.B, gm.C);
+                      v = rsq <= P.Tcut ? v : 0.f;  // also for a NaN
+                    }
+                    const float t = divide_near(__fmul_rn(dvv[j], v), dev[j]);
+                    if (v > 0.f && dev[j] > 0.f) tg += t;
                   }
                   if (MODE == 3) {
                     // second derivatives H_ab = alpha*delta_a*delta_b + [a==b]*beta of the density
@@ -958,6 +1044,11 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
               }
             }
           }
+          if (MODE == 0) {
+            float f0, f1;
+            split(fs2, f0, f1);
+            fsum = f0 + f1;
+          }
           if (MODE == 0 || MODE == 1) {
             agx = fmaf(fsum, dx, agx);
             agy = fmaf(fsum, dy, agy);
@@ -973,6 +1064,11 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
       }
       __syncwarp();
     }
+  }
+  if (MODE == 0) {
+    float z0, z1;
+    split(az2, z0, z1);
+    agz = z0 + z1;
   }
   if (MODE == 3) {
     // the isotropic part: diff*beta*(w*in_c + intg), the same factor for every voxel of the item
@@ -1047,6 +1143,41 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads(BwdArgs G) {
   backward_quads_item<MODE, BINARY>(G, item, blockIdx.y, bufs[wid], ztabs[wid], lane);
 }
 
+// Atom gradients (MODE 0) and relevance (MODE 2) of index types for inputs of at most SELF_ATOMS slots:
+// every warp prepares its atom itself, so the pass is one launch, and WARPS warps share an atom's
+// columns, because so few atoms leave most of the chip idle and the pass lasts as long as one atom.
+// Larger inputs notice that every warp repeats the preparation (with 200 000 slots 0.230-0.316 ms
+// against 0.225 ms for k_emit and the kernel above).
+template <int MODE, bool BINARY, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, BwdArgs G) {
+  __shared__ ColBufD bufs[WARPS];
+  __shared__ ZTabs zts[WARPS];
+  __shared__ float4 sums[WARPS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, a = blockIdx.x, bl = blockIdx.y, b = A.b0 + bl;
+  Rec r;
+  float ox, oy, oz;
+  const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
+  if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
+  ItemParams P = item_of(r);
+  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, a, ox, oy, oz, bufs[w], zts[w], lane, w, WARPS);
+  if (WARPS > 1) {
+    if (lane == 0) sums[w] = make_float4(R.agx, R.agy, R.agz, R.tg);
+    __syncthreads();
+    if (w != 0) return;
+    R.agx = R.agy = R.agz = R.tg = 0.f;
+#pragma unroll
+    for (int k = 0; k < WARPS; k++) {
+      R.agx += sums[k].x; R.agy += sums[k].y; R.agz += sums[k].z; R.tg += sums[k].w;
+    }
+  }
+  const size_t ai = (size_t)b * A.N + a;
+  if (MODE == 0) {
+    if (lane < 3) G.atom_gradients[ai * 3 + lane] = lane == 0 ? R.agx : lane == 1 ? R.agy : R.agz;
+  } else if (lane == 0) {
+    G.relevance[ai] = R.tg;
+  }
+}
+
 // The (atom, channel) items of the weighted channels of one atom, by one warp: modes that need
 // nothing from channels without weight (MODE 1 when no type gradients are wanted, MODE 3).
 template <int MODE, bool BINARY>
@@ -1093,12 +1224,8 @@ __device__ __forceinline__ void gradgrad_quads_item(const BwdArgs& G, int item, 
   const float k4 = 4.f * P.inv_ar2 * P.w, kD = -gm.D * P.inv_ar2 * P.w, kE = -gm.E * P.inv_ar * P.w;
   const float ta = gm.ta, ntb = -gm.tb;
 
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
-  for (unsigned cbase = 0; cbase < ncols;) {
-    unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, P.Tcut, ox, oy,
-                                                    gm.res, gm.dim, lane);
+  for (Columns cols(P); cols.more();) {
+    const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
     for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
       __syncwarp();
       fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
@@ -1193,9 +1320,6 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
   const float ta = gm.ta, ntb = -gm.tb;
 
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
   for (int tb = 0; tb < G.T; tb += VA_CH) {
     // channels of this round that carry weight (zero weights add nothing, src/grid_maker.cpp:229)
     int t = tb + lane;
@@ -1210,9 +1334,8 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
       nz_w[wid][slot] = w;
     }
     __syncwarp();
-    for (unsigned cbase = 0; cbase < ncols;) {
-      unsigned nkept = compact_columns<ColBuf, false>(buf, P, cbase, ncols, ny, inv_ny, Tcull, ox, oy,
-                                                      gm.res, gm.dim, lane);
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<false>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
       if (!BINARY && !PRECISE && nnz <= VA_SPARSE) {
         // few weighted channels (one-hot types): one sweep per channel in the lane layout of the
         // index-typed forward, whose reductions touch a quarter of the rows
@@ -1335,12 +1458,8 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
   const float ta = gm.ta, ntb = -gm.tb;
   const unsigned span = quad_span(P);
   ColBufD& buf = sh.buf;
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
-  for (unsigned cbase = 0; cbase < ncols;) {
-    unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, Tcull, ox, oy, gm.res,
-                                                    gm.dim, lane);
+  for (Columns cols(P); cols.more();) {
+    const unsigned nkept = cols.compact<true>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
     __syncwarp();
     auto quad = [&](unsigned i, float dxy2, float exy, const float (&d2v)[4], const float (&ev)[4],
                     const float (&dzv)[4], size_t off) {
@@ -1525,12 +1644,8 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_ag(BwdA
       nz_w[wid][slot] = w;
     }
     __syncwarp();
-    unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-    unsigned ncols = nx * ny;
-    float inv_ny = 1.f / (float)ny;
-    for (unsigned cbase = 0; cbase < ncols;) {
-      unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, P.Tcut, ox, oy,
-                                                      gm.res, gm.dim, lane);
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
       for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
         fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
@@ -1627,9 +1742,6 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_gradgrad_quads_atom(BwdArgs G
   const float k4 = 4.f * P.inv_ar2, kD = -gm.D * P.inv_ar2, kE = -gm.E * P.inv_ar;
   const float ta = gm.ta, ntb = -gm.tb;
 
-  unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-  unsigned ncols = nx * ny;
-  float inv_ny = 1.f / (float)ny;
   for (int tb = 0; tb < G.T; tb += VA_CH) {
     int t = tb + lane;
     float w = t < G.T ? wrow[t] : 0.f;
@@ -1644,9 +1756,8 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_gradgrad_quads_atom(BwdArgs G
       nz_g[wid][slot] = grow[t];
     }
     __syncwarp();
-    for (unsigned cbase = 0; cbase < ncols;) {
-      unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, P.Tcut, ox, oy,
-                                                      gm.res, gm.dim, lane);
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
       for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
         fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
@@ -1743,12 +1854,8 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_gg(BwdA
       nz_g[wid][slot] = grow[t];
     }
     __syncwarp();
-    unsigned nx = P.hix - P.lox, ny = P.hiy - P.loy;
-    unsigned ncols = nx * ny;
-    float inv_ny = 1.f / (float)ny;
-    for (unsigned cbase = 0; cbase < ncols;) {
-      unsigned nkept = compact_columns<ColBufD, true>(buf, P, cbase, ncols, ny, inv_ny, P.Tcut, ox, oy,
-                                                      gm.res, gm.dim, lane);
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
       for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
         fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
@@ -1856,6 +1963,46 @@ cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode) {
+  return (mode == 0 || mode == 2) && !A.vec && (long)A.nb * A.N <= (mode == 0 ? SELF_ATOMS : REL_SELF_ATOMS) && G.quads && A.gm.dim % 4 == 0 &&
+         (uintptr_t)G.diff % 16 == 0 && (mode == 0 || (uintptr_t)G.density % 16 == 0);
+}
+
+bool forward_self_serves(const EmitArgs& A, const BwdArgs& G) {
+  if (A.vec || (long)A.nb * A.N > FWD_SELF_ATOMS) return false;
+  return A.gm.binary || (G.quads && !G.precise && A.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0);
+}
+
+template <int WARPS>
+static void forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_t st) {
+  const dim3 grid(A.N, A.nb);
+  if (A.gm.binary) k_forward_self<true, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  else k_forward_self<false, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+}
+
+cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_t st) {
+  if (A.N == 0 || A.nb == 0) return cudaSuccess;
+  if ((long)A.nb * A.N <= SELF_SPLIT) forward_self<4>(A, G, st);
+  else forward_self<1>(A, G, st);
+  return cudaGetLastError();
+}
+
+template <int WARPS>
+static void backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
+  const dim3 grid(A.N, A.nb);
+  if (mode == 0) k_backward_quads_self<0, false, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  else if (A.gm.binary) k_backward_quads_self<2, true, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  else k_backward_quads_self<2, false, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+}
+
+cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
+  if (A.N == 0 || A.nb == 0) return cudaSuccess;
+  // up to one atom's warps per scheduler and a bit: shared columns, beyond that a warp per atom
+  if ((long)A.nb * A.N <= SELF_SPLIT) backward_self<4>(A, G, mode, st);
+  else backward_self<1>(A, G, mode, st);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
   long items = (long)G.N * ((mode == 1 || mode == 3) ? G.T : 1);
   if (items == 0 || G.nb == 0) return cudaSuccess;
@@ -1952,13 +2099,10 @@ cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st) 
     else if (G.precise) k_forward_scatter<false, true, true><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
     else k_forward_scatter<false, false, true><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
   } else {
-    if (bin) k_forward_scatter<true, false, false><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
+    if (bin) k_forward_binary<<<dim3((G.N + BIN_WARPS - 1) / BIN_WARPS, G.nb), BIN_WARPS * 32, 0, st>>>(G);
     else if (G.precise) k_forward_scatter<false, true, false><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
     else k_forward_scatter<false, false, false><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
   }
   return cudaGetLastError();
 }
-
-// Slab height: about 110 KB of one channel per block, so that the slabs being worked on together
-// (a few per SM) stay in L2 between their clearing and their last reduction.
 }  // namespace lmg

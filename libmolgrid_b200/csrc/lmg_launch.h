@@ -8,6 +8,17 @@ namespace lmg {
 
 // A pass covers examples [b0, b0+nb) of the caller's batch; scratch arrays are indexed by the
 // example's position in the pass (bl = b - b0), caller arrays by b.
+// Front of the workspace: where the pass left its flags (one byte per block or warp that prepared
+// atoms: 1 = it met a type index >= T) and what such an atom means for the call.  Every call writes
+// its flags and this header anew, so nothing has to be cleared before it.
+constexpr unsigned long long STATUS_MAGIC = 0x6c6d675f737461ull;  // tells a header from a fresh buffer's contents
+struct StatusHeader {
+  unsigned long long magic;
+  unsigned long long offset;  // bytes from the start of the workspace
+  unsigned count;
+  int code;                   // 1: out of range, 2: invalid argument
+};
+
 struct EmitArgs {
   GMParams gm;
   int b0, nb, N, T;
@@ -27,7 +38,9 @@ struct EmitArgs {
   // scratch
   Rec* recs;          // [nb][N]
   ChanParam* chanp;   // [nb][T], type-indexed radii only
-  int* status;
+  char* ws;                   // workspace: StatusHeader in front
+  unsigned long long flags;   // offset of the flags in it
+  int later_pass;             // flags of earlier passes of the same call are kept
 };
 
 struct BwdArgs {
@@ -55,6 +68,13 @@ struct BwdArgs {
 
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st);
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st);
+// the forward pass of index types without k_emit: every warp prepares its own atom (density on aligned
+// grids, or occupancy; the output is zero-filled before)
+bool forward_self_serves(const EmitArgs& A, const BwdArgs& G);
+cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_t st);
+// the same for the backward passes (modes 0 and 2, aligned grids)
+bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode);
+cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st);
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st);
 cudaError_t launch_gradgrad_scatter(const BwdArgs& G, cudaStream_t st);
 
@@ -69,5 +89,7 @@ GMParams to_params(const lmg_gridmaker* g);
 Xform to_xform(const lmg_transform* t);
 // input side of a pass: settings, sizes, the caller's arrays, per-example or single transform
 void fill_emit(EmitArgs& E, const lmg_gridmaker* g, const lmg_atoms* a);
+cudaError_t clear_status(void* ws, cudaStream_t st);
+cudaError_t read_status(const void* ws, int* code, cudaStream_t st);
 int quads_setting();  // current value of the aligned-quad kernel switch
 }  // namespace lmg

@@ -13,7 +13,7 @@
 //   * batch * max_atoms may not exceed LMG_STATIC_MAX_ATOMS; larger requests are refused with
 //     LMG_ERR_WORKSPACE and nothing is launched.
 //   * All calls on a device share the one array and it keeps whatever the previous call left.
-//     The status word is cleared and every record slot is rewritten at the start of each call, so
+//     The status flags and every record slot is rewritten at the start of each call, so
 //     calls issued one after another on the same stream are independent; calls that can overlap on
 //     the GPU (different streams, different host threads) race on it and must be serialised by the
 //     caller.
@@ -34,7 +34,8 @@ extern "C" void lmg_internal_set_error(const char* msg);
 
 namespace {
 
-constexpr size_t STATIC_STATUS_BYTES = 256;
+constexpr size_t STATIC_STATUS_BYTES = 256;   // header, then the flags (up to 64 bytes, or one per atom over unused records)
+constexpr size_t STATIC_FLAGS = 64;
 constexpr size_t STATIC_MAX_ATOMS = 16384;
 constexpr size_t STATIC_BYTES = STATIC_STATUS_BYTES + STATIC_MAX_ATOMS * sizeof(lmg::Rec);
 
@@ -99,20 +100,16 @@ int lmg_backward_static(const lmg_gridmaker* g, const lmg_atoms* a, const float*
   int rc = scratch_for_current_device(&ws);
   if (rc != LMG_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  // the status word must start at zero; the record slots are all rewritten by the first kernel
-  cudaError_t e = cudaMemsetAsync(ws, 0, STATIC_STATUS_BYTES, st);
-  if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: ") + cudaGetErrorString(e));
-
+  // the status flags and the record slots are all rewritten by the first kernel
   lmg::EmitArgs E;
   lmg::fill_emit(E, g, a);
   E.gm.rti = 0;
   E.b0 = 0; E.nb = a->batch;
   E.round_types = 1;
-  E.status = reinterpret_cast<int*>(ws);
+  E.ws = ws;
+  E.flags = STATIC_FLAGS;
+  E.later_pass = 0;
   E.recs = reinterpret_cast<lmg::Rec*>(ws + STATIC_STATUS_BYTES);
-  e = lmg::launch_emit(E, st);
-  if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: emit: ") + cudaGetErrorString(e));
-
   lmg::BwdArgs B;
   std::memset(&B, 0, sizeof B);
   B.gm = E.gm;
@@ -123,7 +120,14 @@ int lmg_backward_static(const lmg_gridmaker* g, const lmg_atoms* a, const float*
   B.diff = diff;
   B.atom_gradients = atom_gradients;
   B.quads = lmg::quads_setting();  // the aligned-quad kernel where the grid allows it (the launcher checks)
-  e = lmg::launch_backward(B, 0, st);
+  cudaError_t e;
+  if (lmg::backward_self_serves(E, B, 0)) {  // the split of lmg_backward, whose results these are
+    e = lmg::launch_backward_self(E, B, 0, st);
+  } else {
+    e = lmg::launch_emit(E, st);
+    if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: emit: ") + cudaGetErrorString(e));
+    e = lmg::launch_backward(B, 0, st);
+  }
   if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: backward: ") + cudaGetErrorString(e));
   return LMG_OK;
 }
@@ -136,8 +140,7 @@ int lmg_static_check_status(void* stream) {
   int rc = scratch_for_current_device(&ws);
   if (rc != LMG_OK) return rc;
   int st = 0;
-  cudaError_t e = cudaMemcpyAsync(&st, ws, sizeof st, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+  cudaError_t e = lmg::read_status(ws, &st, (cudaStream_t)stream);
   if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: reading status: ") + cudaGetErrorString(e));
   if (st == 1) return fail(LMG_ERR_OUT_OF_RANGE, "Type index larger than allowed");
   if (st == 2) return fail(LMG_ERR_INVALID_ARGUMENT, "Incorrect channel size for diff");

@@ -1,0 +1,89 @@
+"""Passes whose warps prepare their own atoms, and the status flags they leave: sizes on both sides of
+the limits between the kernels, against the CPU checker or the same input in a larger batch."""
+import numpy as np
+import pytest
+import torch
+
+import libmolgrid_b200 as lmg
+from libmolgrid_b200 import synthetic as cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def port():
+    from oracle.oracle import CpuOracle
+    return CpuOracle("port")
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+# one atom; four warps an atom up to 1200 slots, one beyond; relevance changes at 2560, gradients at 8192
+@pytest.mark.parametrize("B,N", [(1, 1), (3, 5), (1, 1200), (1, 1201), (8, 320), (8, 321), (8, 1024), (8, 1025)])
+@pytest.mark.parametrize("binary", [False, True])
+def test_every_size_against_the_checker(port, B, N, binary):
+    T, P = 4, 12
+    g, og = lmg.GridMaker(0.5, (P - 1) * 0.5, binary), port.gm(0.5, (P - 1) * 0.5, binary)
+    ex = [cases.index_case(100 + b, N, T, 4.0) for b in range(B)]
+    coords, types, radii = (np.stack([e[k] for e in ex]) for k in range(3))
+    out = torch.full((B,) + g.grid_dimensions(T), 7.0, device="cuda")
+    cen = torch.zeros((B, 3), device="cuda")
+    g.forward(cen, dev(coords), dev(types), dev(radii), out)
+    rng = np.random.default_rng(N)
+    diff = rng.normal(size=out.shape).astype(np.float32)
+    ag, rel = torch.full((B, N, 3), 7.0, device="cuda"), torch.full((B, N), 7.0, device="cuda")
+    g.backward(cen, dev(coords), dev(types), dev(radii), dev(diff), ag)
+    g.backward_relevance(cen, dev(coords), dev(types), dev(radii), out, dev(diff), rel)
+    g.check_types()
+    for b in (0, B - 1):
+        want = port.forward_index(og, (0, 0, 0), coords[b], types[b], radii[b], T)
+        got = out[b].cpu().numpy()
+        if binary:
+            np.testing.assert_array_equal(got, want)
+        else:
+            # up to N / T terms a voxel in any order: a rounding of the running sum each
+            np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-6 * max(1.0, N / T / 50))
+        wag = port.backward_index(og, (0, 0, 0), coords[b], types[b], radii[b], diff[b])
+        np.testing.assert_allclose(ag[b].cpu().numpy(), wag, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wag).max())))
+        wrel = port.backward_relevance(og, (0, 0, 0), coords[b], types[b], radii[b], got, diff[b])
+        np.testing.assert_allclose(rel[b].cpu().numpy(), wrel, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wrel).max())))
+
+
+@pytest.mark.parametrize("N", [3, 1300, 9000])
+@pytest.mark.parametrize("at", [0, 1, -1])
+def test_status_of_every_pass(N, at):
+    """A type beyond the channels is reported wherever it is, by the call that met it and by no later
+    one, also when a workspace makes the call run in passes of unequal size."""
+    import libmolgrid_b200.api as api
+    B, T = 5, 3
+    g = lmg.GridMaker(0.5, 5.5)
+    coords = torch.zeros((B, N, 3), device="cuda")
+    good = torch.ones((B, N), device="cuda")
+    radii = torch.ones((B, N), device="cuda")
+    cen = torch.zeros((B, 3), device="cuda")
+    out = torch.empty((B,) + g.grid_dimensions(T), device="cuda")
+    ag = torch.empty((B, N, 3), device="cuda")
+    old = api.MAX_WORKSPACE_BYTES
+    one = api._cabi.lib().lmg_workspace_bytes(g.s, 0, 1, N, T, 0)
+    try:
+        for limit in (old, 2 * one):
+            api.MAX_WORKSPACE_BYTES = limit
+            api._workspaces.clear()
+            for b in (0, B - 1):
+                bad = good.clone()
+                bad[b, at] = T
+                g.forward(cen, coords, bad, radii, out)
+                with pytest.raises(IndexError):
+                    g.check_types()
+                g.forward(cen, coords, good, radii, out)
+                g.check_types()
+                g.backward(cen, coords, bad, radii, out, ag)
+                with pytest.raises(ValueError):
+                    g.check_types()
+                g.backward(cen, coords, good, radii, out, ag)
+                g.check_types()
+    finally:
+        api.MAX_WORKSPACE_BYTES = old
+        api._workspaces.clear()
