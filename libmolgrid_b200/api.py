@@ -876,17 +876,20 @@ class GridInterpolater(object):
         if osh[1:] != (self.s.out_dim,) * 3:
             raise ValueError("Output grid wrong dimension. Should be %d along all axes but is %d,%d,%d"
                              % ((self.s.out_dim,) + osh[1:]))
-        T = (_cabi.TransformStruct * B)(*[t.struct() for t in trs])
+        T, rotation = (_cabi.TransformStruct * B)(), (ctypes.c_float * (3 * B))()
+        if _fast() and all(type(t) is Transform for t in trs):
+            _native._pack_transforms(trs, ctypes.addressof(T), ctypes.addressof(rotation))
+        else:
+            for b, t in enumerate(trs):
+                T[b] = t.struct()
+                rotation[3 * b:3 * b + 3] = [float(v) for v in t.get_rotation_center()]
 
         def centers(c):
+            if c is None:
+                return rotation
             arr = (ctypes.c_float * (3 * B))()
             for b in range(B):
-                if c is None:
-                    v = trs[b].get_rotation_center()
-                elif batched:
-                    v = c[b]
-                else:
-                    v = c
+                v = c[b] if batched else c
                 arr[3 * b:3 * b + 3] = [float(v[0]), float(v[1]), float(v[2])]
             return arr
 

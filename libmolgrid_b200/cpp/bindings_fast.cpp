@@ -283,7 +283,47 @@ PyObject* fast_gradients(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return finish(rc, ret);
 }
 
+// A float attribute (any Python or numpy number) of an object; false with an exception set.
+bool number_of(PyObject* o, PyObject* name, float* f) {
+  PyObject* v = PyObject_GetAttr(o, name);
+  if (v == nullptr) return false;
+  *f = (float)PyFloat_AsDouble(v);
+  Py_DECREF(v);
+  return !(*f == -1.f && PyErr_Occurred());
+}
+
+// (list of Transform objects of the Python layer, address of as many lmg_transform, address of as many
+// rotation centres): their numbers in one go instead of a ctypes object each
+PyObject* pack_transforms(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  static PyObject *Q = PyUnicode_InternFromString("Q"), *center = PyUnicode_InternFromString("center"),
+                  *translate = PyUnicode_InternFromString("translate");
+  static PyObject* part[4] = {PyUnicode_InternFromString("a"), PyUnicode_InternFromString("b"), PyUnicode_InternFromString("c"),
+                              PyUnicode_InternFromString("d")};
+  static PyObject* xyz[3] = {PyUnicode_InternFromString("x"), PyUnicode_InternFromString("y"), PyUnicode_InternFromString("z")};
+  if (nargs != 3 || !PyList_Check(a[0])) {
+    PyErr_SetString(PyExc_TypeError, "a list and two addresses are needed");
+    return nullptr;
+  }
+  lmg_transform* t = static_cast<lmg_transform*>(PyLong_AsVoidPtr(a[1]));
+  float* ce = static_cast<float*>(PyLong_AsVoidPtr(a[2]));
+  if (PyErr_Occurred()) return nullptr;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[0]); i++) {
+    PyObject* o = PyList_GET_ITEM(a[0], i);
+    PyObject *q = PyObject_GetAttr(o, Q), *c = q ? PyObject_GetAttr(o, center) : nullptr, *r = c ? PyObject_GetAttr(o, translate) : nullptr;
+    bool ok = r != nullptr;
+    for (int k = 0; ok && k < 4; k++) ok = number_of(q, part[k], &t[i].q[k]);
+    for (int k = 0; ok && k < 3; k++) ok = number_of(c, xyz[k], &t[i].center[k]) && number_of(r, xyz[k], &t[i].translate[k]);
+    for (int k = 0; ok && k < 3; k++) ce[3 * i + k] = t[i].center[k];
+    Py_XDECREF(q);
+    Py_XDECREF(c);
+    Py_XDECREF(r);
+    if (!ok) return nullptr;
+  }
+  Py_RETURN_NONE;
+}
+
 PyMethodDef methods[] = {
+    {"_pack_transforms", (PyCFunction)(void (*)(void))pack_transforms, METH_FASTCALL, nullptr},
     {"_fast_forward", (PyCFunction)(void (*)(void))fast_forward, METH_FASTCALL, nullptr},
     {"_fast_backward", (PyCFunction)(void (*)(void))fast_backward, METH_FASTCALL, nullptr},
     {"_fast_relevance", (PyCFunction)(void (*)(void))fast_relevance, METH_FASTCALL, nullptr},

@@ -192,6 +192,74 @@ using lmg::fill_emit;
 using lmg::to_params;
 using lmg::to_xform;
 
+// The frame of one example, operation by operation as the reference forms it (src/grid_interpolater.cpp:
+// 31-45, quaternion.h:145-166; the host code of this file is compiled without fused multiply-add).
+lmg::InterpFrame interp_frame(const lmg_interpolater* gi, const lmg_transform& t, const float* in_center,
+                              const float* out_center) {
+  lmg::InterpFrame F;
+  const float in_half = (float)(gi->in_dimension / 2.0), out_half = (float)(gi->out_dimension / 2.0);
+  F.iox = in_center[0] - in_half; F.ioy = in_center[1] - in_half; F.ioz = in_center[2] - in_half;
+  F.oox = out_center[0] - out_half; F.ooy = out_center[1] - out_half; F.ooz = out_center[2] - out_half;
+  auto conj_over_norm = [](const float* q, float* o) {
+    const float n = ((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3];
+    o[0] = q[0] / n; o[1] = -q[1] / n; o[2] = -q[2] / n; o[3] = -q[3] / n;
+  };
+  conj_over_norm(t.q, F.inv);
+  conj_over_norm(F.inv, F.cn);
+  F.ux = -t.translate[0] - t.center[0];
+  F.uy = -t.translate[1] - t.center[1];
+  F.uz = -t.translate[2] - t.center[2];
+  F.cx = t.center[0]; F.cy = t.center[1]; F.cz = t.center[2];
+  return F;
+}
+
+// The affine map of a frame from output to input indices and its inverse, in double and rounded once.
+lmg::GatherFrame gather_frame(const lmg_interpolater* gi, const lmg::InterpFrame& F) {
+  lmg::GatherFrame W;
+  const double a = F.inv[0], b = F.inv[1], c = F.inv[2], d = F.inv[3], s = 2.0 / (a * a + b * b + c * c + d * d);
+  const double f = (double)gi->out_resolution / gi->in_resolution;
+  const double r[3][3] = {{1 - s * (c * c + d * d), s * (b * c - a * d), s * (b * d + a * c)},
+                          {s * (b * c + a * d), 1 - s * (b * b + d * d), s * (c * d - a * b)},
+                          {s * (b * d - a * c), s * (c * d + a * b), 1 - s * (b * b + c * c)}};
+  const double p[3] = {(double)F.oox + F.ux, (double)F.ooy + F.uy, (double)F.ooz + F.uz};
+  const double o[3] = {(double)F.cx - F.iox, (double)F.cy - F.ioy, (double)F.cz - F.ioz};
+  double size = gi->out_dim * f;
+  for (float v : {F.iox, F.ioy, F.ioz, F.oox, F.ooy, F.ooz, F.ux, F.uy, F.uz, F.cx, F.cy, F.cz})
+    size = std::max(size, std::fabs((double)v) / gi->in_resolution);
+  bool sane = f > 0;
+  for (int i = 0; i < 3; i++) {
+    const double g0 = (r[i][0] * p[0] + r[i][1] * p[1] + r[i][2] * p[2] + o[i]) / gi->in_resolution;
+    double reach = 0;
+    for (int j = 0; j < 3; j++) {
+      W.a[i][j] = (float)(r[i][j] * f);
+      W.ai[i][j] = (float)(r[j][i] / f);
+      reach += std::fabs(r[j][i] / f);
+    }
+    W.g0[i] = (float)g0;
+    W.reach[i] = (float)reach;
+    sane = sane && std::fabs(g0) < 1e6 && reach < 1e6;  // also false for NaN
+  }
+  W.slack = (float)(0.01 + 4e-6 * size);
+  W.sane = sane && size < 1e6;
+  return W;
+}
+
+// What all launches of an interpolation share.
+lmg::InterpArgs interp_args(const lmg_interpolater* gi, int nchannels, const float* in, float* out) {
+  lmg::InterpArgs I;
+  I.in_res = gi->in_resolution;
+  I.out_res = gi->out_resolution;
+  int e;
+  I.inv_in_res = std::frexp(I.in_res, &e) == 0.5f && e > -100 && e < 100 ? 1.f / I.in_res : 0.f;
+  I.minus_zero = -0.f;
+  I.in_dim = gi->in_dim;
+  I.out_dim = gi->out_dim;
+  I.K = nchannels;
+  I.in = in;
+  I.out = out;
+  return I;
+}
+
 // Scratch layout of one pass over nb examples.
 struct Layout {
   size_t flags, recs, chanp, partial, total;
@@ -678,16 +746,7 @@ int lmg_interpolate(const lmg_interpolater* gi, int batch, int nchannels, const 
     return fail(LMG_ERR_INVALID_ARGUMENT, "Input and output grid can not be the same in GridInterpolator.");
   if (in == nullptr) return fail(LMG_ERR_INVALID_ARGUMENT, "Input grid not allocated");
   if (out == nullptr) return fail(LMG_ERR_INVALID_ARGUMENT, "Output grid not allocated");
-  lmg::InterpArgs I;
-  I.in_res = gi->in_resolution;
-  I.out_res = gi->out_resolution;
-  I.in_half = (float)(gi->in_dimension / 2.0);
-  I.out_half = (float)(gi->out_dimension / 2.0);
-  I.in_dim = gi->in_dim;
-  I.out_dim = gi->out_dim;
-  I.K = nchannels;
-  I.in = in;
-  I.out = out;
+  lmg::InterpArgs I = interp_args(gi, nchannels, in, out);
   // The tiled kernel stages boxes of the input through tensor copies: rows of the input must start
   // on 16-byte boundaries, and an 8^3 output tile must map into a 16x16x20 box of input voxels under
   // any rotation (8*sqrt(3)*out_res/in_res + 2 <= 16).
@@ -700,13 +759,8 @@ int lmg_interpolate(const lmg_interpolater* gi, int batch, int nchannels, const 
   for (int b0 = 0; b0 < batch; b0 += lmg::INTERP_MAX_EX) {
     int nb = std::min(lmg::INTERP_MAX_EX, batch - b0);
     I.b0 = b0;
-    for (int i = 0; i < nb; i++) {
-      I.ex[i].X = to_xform(&transforms[b0 + i]);
-      for (int k = 0; k < 3; k++) {
-        I.ex[i].in_center[k] = in_centers[(size_t)(b0 + i) * 3 + k];
-        I.ex[i].out_center[k] = out_centers[(size_t)(b0 + i) * 3 + k];
-      }
-    }
+    for (int i = 0; i < nb; i++)
+      I.ex[i] = interp_frame(gi, transforms[b0 + i], in_centers + (size_t)(b0 + i) * 3, out_centers + (size_t)(b0 + i) * 3);
     cudaError_t e = tiled ? lmg::launch_interpolate_tiled(maps, I, nb, (cudaStream_t)stream)
                           : lmg::launch_interpolate(I, nb, (cudaStream_t)stream);
     g_launches += 1;
@@ -726,30 +780,16 @@ int lmg_interpolate_backward(const lmg_interpolater* gi, int batch, int nchannel
   if (grad_out == nullptr) return fail(LMG_ERR_INVALID_ARGUMENT, "Output gradient grid not allocated");
   if (grad_in == nullptr) return fail(LMG_ERR_INVALID_ARGUMENT, "Input gradient grid not allocated");
   cudaStream_t st = (cudaStream_t)stream;
-  size_t in_elems = (size_t)nchannels * gi->in_dim * gi->in_dim * gi->in_dim;
-  cudaError_t e = cudaMemsetAsync(grad_in, 0, in_elems * batch * sizeof(float), st);
-  if (e != cudaSuccess) return cuda_fail(e, "zeroing the input gradient");
-  lmg::InterpArgs I;
-  I.in_res = gi->in_resolution;
-  I.out_res = gi->out_resolution;
-  I.in_half = (float)(gi->in_dimension / 2.0);
-  I.out_half = (float)(gi->out_dimension / 2.0);
-  I.in_dim = gi->in_dim;
-  I.out_dim = gi->out_dim;
-  I.K = nchannels;
-  I.in = grad_out;
-  I.out = grad_in;
+  lmg::InterpArgs I = interp_args(gi, nchannels, grad_out, grad_in);
+  lmg::GatherFrames W;
   for (int b0 = 0; b0 < batch; b0 += lmg::INTERP_MAX_EX) {
     int nb = std::min(lmg::INTERP_MAX_EX, batch - b0);
     I.b0 = b0;
     for (int i = 0; i < nb; i++) {
-      I.ex[i].X = to_xform(&transforms[b0 + i]);
-      for (int k = 0; k < 3; k++) {
-        I.ex[i].in_center[k] = in_centers[(size_t)(b0 + i) * 3 + k];
-        I.ex[i].out_center[k] = out_centers[(size_t)(b0 + i) * 3 + k];
-      }
+      I.ex[i] = interp_frame(gi, transforms[b0 + i], in_centers + (size_t)(b0 + i) * 3, out_centers + (size_t)(b0 + i) * 3);
+      W.ex[i] = gather_frame(gi, I.ex[i]);
     }
-    e = lmg::launch_interpolate_backward(I, nb, st);
+    cudaError_t e = lmg::launch_interpolate_backward(I, W, nb, st);
     g_launches += 1;
     if (e != cudaSuccess) return cuda_fail(e, "interpolate backward");
   }

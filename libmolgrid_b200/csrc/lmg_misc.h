@@ -7,30 +7,47 @@
 
 namespace lmg {
 
-struct InterpExample {
-  Xform X;
-  float in_center[3];
-  float out_center[3];
+// What is the same for every output voxel of an example: grid origins and the inverse rotation, computed
+// once on the host with the roundings of the reference.
+struct InterpFrame {
+  float iox, ioy, ioz, oox, ooy, ooz;
+  float inv[4], cn[4];
+  float ux, uy, uz, cx, cy, cz;
 };
 
-// examples per launch whose transforms travel inside the kernel parameter block
+// examples per launch whose frames travel inside the kernel parameter block
 constexpr int INTERP_MAX_EX = 48;
 
 struct InterpArgs {
-  float in_res, out_res, in_half, out_half;
+  float in_res, out_res;
+  float inv_in_res;  // 1 / in_res where that is exact (a power of two), 0 otherwise
+  float minus_zero;  // see interp_blend
   unsigned in_dim, out_dim;
   int K;
   int b0;
   const float* in;
   float* out;
-  InterpExample ex[INTERP_MAX_EX];
+  InterpFrame ex[INTERP_MAX_EX];
+};
+
+// The same map, approximately, as a matrix and its inverse: where the backward pass looks.
+struct GatherFrame {
+  float a[3][3];   // d(input index) / d(output index)
+  float ai[3][3];  // its inverse
+  float g0[3];     // position of output voxel (0, 0, 0)
+  float reach[3];  // half extent of the box about an input voxel's image that its output voxels lie in
+  float slack;     // allowance for the roundings of the positions, in cells
+  int sane;        // 0: the map has no use (an infinite or enormous transform), every voxel is looked at
+};
+struct GatherFrames {
+  GatherFrame ex[INTERP_MAX_EX];
 };
 
 cudaError_t launch_transform(const Xform& X, int n, const float* in, float* out, int dotranslate,
                              bool forward, cudaStream_t st);
 cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st);
-// adjoint: I.in = gradient of the output grid (read), I.out = gradient of the input grid (accumulated)
-cudaError_t launch_interpolate_backward(const InterpArgs& I, int nb, cudaStream_t st);
+// adjoint: I.in = gradient of the output grid (read), I.out = gradient of the input grid (written)
+cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames& W, int nb, cudaStream_t st);
 
 // Tiled kernel: output tiles of ITILE^3 voxels read a staged box of the input (z is the contiguous
 // axis; the box starts on a multiple of four in z).  A rotated tile needs (ITILE - 1) * (|r1| + |r2| +
