@@ -697,11 +697,9 @@ int lmg_backward_gradients(const lmg_gridmaker* g, const lmg_atoms* a, const flo
     B.quads = g_quads;
     e = lmg::launch_emit(E, st);
     if (e != cudaSuccess) return cuda_fail(e, "emit");
-    e = lmg::launch_gradgrad_scatter(B, st);
-    if (e != cudaSuccess) return cuda_fail(e, "backward_gradients grid");
-    e = lmg::launch_backward(B, 3, st);
-    if (e != cudaSuccess) return cuda_fail(e, "backward_gradients atoms");
-    g_launches += 4 + (g->radii_type_indexed ? 1 : 0);
+    e = lmg::launch_second_order(B, st);
+    if (e != cudaSuccess) return cuda_fail(e, "backward_gradients");
+    g_launches += 2 + (g->radii_type_indexed ? 2 : 0);
   }
   return LMG_OK;
 }

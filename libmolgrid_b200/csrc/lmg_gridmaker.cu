@@ -888,10 +888,9 @@ struct BwdSums {
 };
 
 // The sweep of one work item whose constants are in P: sums over the item's footprint, reduced
-// over the warp.  `item` and `b` only serve MODE 3 (its incoming gradients).  Of `parts` warps that
-// share an item, this one takes the `part`-th share of its columns.
+// over the warp.  Of `parts` warps that share an item, this one takes the `part`-th share of its columns.
 template <int MODE, bool BINARY, class BUF>
-__device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemParams& P, int b, int item,
+__device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const ItemParams& P, int b,
                                                        float ox, float oy, float oz, BUF& buf, ZTabs& zt,
                                                        int lane, unsigned part = 0, unsigned parts = 1) {
   const GMParams& gm = G.gm;
@@ -900,15 +899,8 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
   const float* diff = G.diff + chan_off;
   const float* dens = MODE == 2 ? G.density + chan_off : nullptr;
   float agx = 0.f, agy = 0.f, agz = 0.f, tg = 0.f;
-  bool want_ag = MODE == 0 || ((MODE == 1 || MODE == 3) && P.w != 0.f);
-  const float Tcull = (MODE == 0 || MODE == 3) ? P.Tcut : fmaxf(P.Tcut, BINARY ? P.Tbin : -1.f);
-  float inx = 0.f, iny = 0.f, inz = 0.f, intg = 0.f;  // MODE 3: incoming gradients of this item
-  if (MODE == 3) {
-    size_t gi = (size_t)b * G.N + item / G.T;
-    inx = G.ag_in[gi * 3]; iny = G.ag_in[gi * 3 + 1]; inz = G.ag_in[gi * 3 + 2];
-    intg = G.tg_in[gi * G.T + P.chan];
-    if (!want_ag) P.valid = false;  // zero-weight channels contribute nothing (src/grid_maker.cpp:573)
-  }
+  const bool want_ag = MODE == 0 || (MODE == 1 && P.w != 0.f);
+  const float Tcull = MODE == 0 ? P.Tcut : fmaxf(P.Tcut, BINARY ? P.Tbin : -1.f);
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
   // The gradient's radial factor beyond the Gaussian part is kE/d + kD: positive inside the cut-off,
   // zero at it (the tail polynomial has a double root there) and negative beyond, so a clamp at zero
@@ -918,9 +910,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
   const float k4 = want_ag ? 4.f * P.inv_ar2 : 0.f;
   const float kD = (want_ag && tail) ? -gm.D * P.inv_ar2 : 0.f, kE = (want_ag && tail) ? -gm.E * P.inv_ar : 0.f;
   const float ta = gm.ta, ntb = -gm.tb;
-  const float g16 = 16.f * P.inv_ar2 * P.inv_ar2, gm4 = -4.f * P.inv_ar2;  // MODE 3, Gaussian part
-  float sb = 0.f;                                                            // MODE 3: sum of diff*beta
-  Pair az2 = pair(0.f);                                                      // MODE 0: agz of even and odd voxels
+  Pair az2 = pair(0.f), tg2 = pair(0.f);  // agz and tg of even and odd voxels
 
   if (P.valid) {
     for (Columns cols(P, part, parts); cols.more();) {
@@ -939,10 +929,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
           const float4* row = reinterpret_cast<const float4*>(diff + rowoff);
           float exy = ex2_approx(dxy2 * kexp);
           float exy4 = k4 * exy;
-          float fsum = 0.f;
-          float dotxy = MODE == 3 ? fmaf(dx, inx, dy * iny) : 0.f;
-          Pair fs2 = pair(0.f);                // MODE 0: fsum of even and odd voxels
-          float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // MODE 3: sums over the column of diff*alpha*{1, dz, dz^2}
+          Pair fs2 = pair(0.f);  // sum over the column of -(d density / d dist) / dist * dv, even and odd voxels
           for (unsigned q0 = 0; q0 < nq; q0 += 4) {
             // up to four quads of the column are requested together, then used
             float4 dv[4];
@@ -966,44 +953,45 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
                     dev[0] = de.x; dev[1] = de.y; dev[2] = de.z; dev[3] = de.w;
                   }
                 }
-                if (MODE == 0) {
-                  // the arithmetic of the branch below on two voxels at a time
+                if (MODE == 0 || MODE == 1) {
+                  // -(d density / d dist) / dist * dv, src/grid_maker.cu:881-919, two voxels at a time; rsq == 0
+                  // contributes nothing because dx = dy = dz = 0 there, a NaN rsq (z outside the footprint)
+                  // takes the tail, which the clamp makes zero
                   const Pair xy = pair(dxy2), e4 = pair(exy4), kE2 = pair(kE), kD2 = pair(kD);
 #pragma unroll
                   for (int j = 0; j < 4; j += 2) {
                     float r0, r1, g0, g1, t0, t1;
-                    split(add2(xy, pair(d2v[j], d2v[j + 1])), r0, r1);
-                    split(mul2(e4, pair(ev[j], ev[j + 1])), g0, g1);
-                    split(fma2(kE2, pair(rsqrt_approx(r0), rsqrt_approx(r1)), kD2), t0, t1);
-                    const Pair f = mul2(pair(r0 <= P.Tg ? g0 : fmaxf(t0, 0.f), r1 <= P.Tg ? g1 : fmaxf(t1, 0.f)),
-                                        pair(dvv[j], dvv[j + 1]));
+                    const Pair r = add2(xy, pair(d2v[j], d2v[j + 1])), e2 = pair(ev[j], ev[j + 1]);
+                    split(r, r0, r1);
+                    split(mul2(e4, e2), g0, g1);
+                    const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1)), d2 = pair(dvv[j], dvv[j + 1]);
+                    split(fma2(kE2, id, kD2), t0, t1);
+                    const Pair f = mul2(pair(r0 <= P.Tg ? g0 : fmaxf(t0, 0.f), r1 <= P.Tg ? g1 : fmaxf(t1, 0.f)), d2);
                     fs2 = add2(fs2, f);
                     az2 = fma2(f, pair(dzv[j], dzv[j + 1]), az2);
+                    if (MODE == 1) {
+                      float v0, v1;
+                      if (BINARY) {
+                        v0 = r0 < P.Tbin ? 1.f : 0.f;
+                        v1 = r1 < P.Tbin ? 1.f : 0.f;
+                      } else {
+                        // the distance in radii from the reciprocal root that the gradient needs
+                        float q0, q1;
+                        split(fma2(pair(ta), mul2(mul2(r, id), pair(P.inv_ar)), pair(ntb)), q0, q1);
+                        const Pair tq = pair(fminf(q0, 0.f), fminf(q1, 0.f));  // zero beyond the cut-off and for a NaN
+                        split(mul2(tq, tq), q0, q1);
+                        split(mul2(pair(exy), e2), g0, g1);
+                        v0 = r0 <= P.Tg ? g0 : q0;
+                        v1 = r1 <= P.Tg ? g1 : q1;
+                      }
+                      tg2 = fma2(pair(v0, v1), d2, tg2);
+                    }
                   }
                 }
 #pragma unroll
-                for (int j = 0; j < (MODE == 0 ? 0 : 4); j++) {
+                for (int j = 0; j < (MODE == 2 ? 4 : 0); j++) {
                   float rsq = __fadd_rn(dxy2, d2v[j]);
                   float g = exy * ev[j];  // exp(-2 rsq / ar^2)
-                  if (MODE == 1) {
-                    // -(d density / d dist) / dist * dv, src/grid_maker.cu:881-919; rsq == 0
-                    // contributes nothing because dx = dy = dz = 0 there
-                    // a NaN rsq (z outside the footprint) takes the second branch and clamps to zero
-                    float sg = rsq <= P.Tg ? exy4 * ev[j] : fmaxf(fmaf(kE, rsqrt_approx(rsq), kD), 0.f);
-                    float f = sg * dvv[j];
-                    fsum += f;
-                    agz = fmaf(f, dzv[j], agz);
-                  }
-                  if (MODE == 1) {
-                    float v;
-                    if (BINARY) {
-                      v = rsq < P.Tbin ? 1.f : 0.f;
-                    } else {
-                      float tq = fminf(fmaf(ta, sqrt_approx(rsq * P.inv_ar2), ntb), 0.f);
-                      v = rsq <= P.Tg ? g : tq * tq;  // tq is zero beyond the cut-off and for a NaN rsq
-                    }
-                    tg = fmaf(v, dvv[j], tg);
-                  }
                   if (MODE == 2) {
                     float v;
                     if (BINARY) {
@@ -1015,66 +1003,29 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
                     const float t = divide_near(__fmul_rn(dvv[j], v), dev[j]);
                     if (v > 0.f && dev[j] > 0.f) tg += t;
                   }
-                  if (MODE == 3) {
-                    // second derivatives H_ab = alpha*delta_a*delta_b + [a==b]*beta of the density
-                    // (src/grid_maker.cu:812-878); delta = atom - grid point.  Per voxel only the
-                    // moments of diff*alpha in dz and the sum of diff*beta are taken; what is the same
-                    // for a whole column (dx, dy, the incoming gradients) is applied after it.
-                    float alpha, beta;
-                    if (rsq <= P.Tg) {
-                      alpha = g16 * g;
-                      beta = gm4 * g;
-                    } else {
-                      float id = rsqrt_approx(rsq);
-                      float S = fmaf(gm.D * P.inv_ar, rsq * id, gm.E);
-                      beta = S * id * P.inv_ar;
-                      alpha = fmaf(gm.D * P.inv_ar2, id * id, -beta * id * id);
-                    }
-                    // nothing beyond the cut-off, nor for a NaN rsq (z outside the footprint), whose
-                    // alpha and beta are NaN as well: the products are selected, not multiplied by zero
-                    const bool inside = rsq <= P.Tcut;
-                    float t0 = inside ? dvv[j] * alpha : 0.f, tb = inside ? dvv[j] * beta : 0.f;
-                    float t1 = t0 * dzv[j];
-                    a0 += t0;
-                    a1 += t1;
-                    a2 = fmaf(t1, dzv[j], a2);
-                    sb += tb;
-                  }
                 }
               }
             }
           }
-          if (MODE == 0) {
+          if (MODE != 2) {
             float f0, f1;
             split(fs2, f0, f1);
-            fsum = f0 + f1;
-          }
-          if (MODE == 0 || MODE == 1) {
-            agx = fmaf(fsum, dx, agx);
-            agy = fmaf(fsum, dy, agy);
-          }
-          if (MODE == 3) {
-            // sum over the column of diff * (w*alpha*dot*delta_c + intg*alpha*delta_c^2), dot = dotxy + dz*inz
-            float wd = P.w * fmaf(dotxy, a0, inz * a1);
-            agx = fmaf(dx, fmaf(intg * dx, a0, wd), agx);
-            agy = fmaf(dy, fmaf(intg * dy, a0, wd), agy);
-            agz += fmaf(P.w, fmaf(dotxy, a1, inz * a2), intg * a2);
+            agx = fmaf(f0 + f1, dx, agx);
+            agy = fmaf(f0 + f1, dy, agy);
           }
         }
       }
       __syncwarp();
     }
   }
-  if (MODE == 0) {
+  if (MODE != 2) {
     float z0, z1;
     split(az2, z0, z1);
     agz = z0 + z1;
-  }
-  if (MODE == 3) {
-    // the isotropic part: diff*beta*(w*in_c + intg), the same factor for every voxel of the item
-    agx = fmaf(sb, fmaf(P.w, inx, intg), agx);
-    agy = fmaf(sb, fmaf(P.w, iny, intg), agy);
-    agz = fmaf(sb, fmaf(P.w, inz, intg), agz);
+    if (MODE == 1) {
+      split(tg2, z0, z1);
+      tg = z0 + z1;
+    }
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
@@ -1095,10 +1046,10 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, ItemPar
 template <int MODE, bool BINARY>
 __device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, int bl, ColBufD& buf, ZTabs& zt,
                                                     int lane) {
-  constexpr bool VEC = MODE == 1 || MODE == 3;
+  constexpr bool VEC = MODE == 1;
   const GMParams& gm = G.gm;
   int b = G.b0 + bl;
-  if (MODE == 3 || (MODE == 1 && G.type_gradients == nullptr)) {
+  if (MODE == 1 && G.type_gradients == nullptr) {
     // an (atom, channel) pair without weight contributes nothing: leave before any other load
     int ea = item / G.T;
     if (G.type_vector[((size_t)b * G.N + ea) * G.T + (item - ea * G.T)] == 0.f) return;
@@ -1112,7 +1063,7 @@ __device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, 
   }
   float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
   ItemParams P = load_item<VEC>(G, bl, b, item, ox, oy, oz);
-  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, item, ox, oy, oz, buf, zt, lane);
+  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, ox, oy, oz, buf, zt, lane);
   float agx = R.agx, agy = R.agy, agz = R.agz, tg = R.tg;
   if (lane == 0) {
     size_t ai = (size_t)b * G.N + (VEC ? item / G.T : item);
@@ -1120,21 +1071,23 @@ __device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, 
       G.atom_gradients[ai * 3] = agx;
       G.atom_gradients[ai * 3 + 1] = agy;
       G.atom_gradients[ai * 3 + 2] = agz;
-    } else if (MODE == 1 || MODE == 3) {
+    } else if (MODE == 1) {
       size_t pi = (size_t)bl * G.N * G.T + item;
       G.partial[pi * 3] = agx;
       G.partial[pi * 3 + 1] = agy;
       G.partial[pi * 3 + 2] = agz;
-      if (MODE == 1 && G.type_gradients != nullptr) G.type_gradients[ai * G.T + P.chan] = tg;
+      if (G.type_gradients != nullptr) G.type_gradients[ai * G.T + P.chan] = tg;
     } else {
       G.relevance[ai] = tg;
     }
   }
 }
 
+// 64 registers: the most of the blocks of one warp that an SM takes.  MODE 1 waits on the L1 (89 % of its throughput: a lane per column touches 32 lines a load): 64 registers and
+// 32 resident warps instead of 72 and 28, 2.67 -> 2.58 ms at 28x96^3 (4 x 3000 atoms, 28 channels).
 template <int MODE, bool BINARY>
-__global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads(BwdArgs G) {
-  constexpr bool VEC = MODE == 1 || MODE == 3;
+__global__ void __launch_bounds__(BWD2_WARPS * 32, 32) k_backward_quads(BwdArgs G) {
+  constexpr bool VEC = MODE == 1;
   __shared__ ColBufD bufs[BWD2_WARPS];
   __shared__ ZTabs ztabs[BWD2_WARPS];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1159,7 +1112,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, 
   const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
   if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
   ItemParams P = item_of(r);
-  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, a, ox, oy, oz, bufs[w], zts[w], lane, w, WARPS);
+  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, ox, oy, oz, bufs[w], zts[w], lane, w, WARPS);
   if (WARPS > 1) {
     if (lane == 0) sums[w] = make_float4(R.agx, R.agy, R.agz, R.tg);
     __syncthreads();
@@ -1179,7 +1132,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, 
 }
 
 // The (atom, channel) items of the weighted channels of one atom, by one warp: modes that need
-// nothing from channels without weight (MODE 1 when no type gradients are wanted, MODE 3).
+// nothing from channels without weight (MODE 1 when no type gradients are wanted).
 template <int MODE, bool BINARY>
 __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_nz(BwdArgs G) {
   __shared__ ColBufD bufs[BWD2_WARPS];
@@ -1194,85 +1147,173 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_nz(BwdArgs G
   }
 }
 
-// Grid term of backward_gradients on aligned quads (see k_gradgrad_scatter).
-__device__ __forceinline__ void gradgrad_quads_item(const BwdArgs& G, int item, int bl, ColBufD& buf, ZTabs& zt,
-                                                    int lane) {
-  const GMParams& gm = G.gm;
-  int b = G.b0 + bl;
-  if (true) {
-    // an (atom, channel) pair without weight contributes nothing: leave before any other load
-    int ea = item / G.T;
-    if (G.type_vector[((size_t)b * G.N + ea) * G.T + (item - ea * G.T)] == 0.f) return;
-  }
+// ---------------------------------------------------------------------------------------------
+// backward_gradients on aligned quads: the grid term and the atom term in one sweep of the footprint, which
+// share the distance, the Gaussian and its two derivatives.  With s = -(d density / d dist) / dist and the
+// second derivatives H_ab = alpha delta_a delta_b - [a == b] s of the density (src/grid_maker.cu:812-878;
+// delta = grid point - atom up to a sign that cancels):
+//   Gaussian  g = exp(-2 d^2 / ar^2):   s = 4 g / ar^2,    alpha = 4 s / ar^2
+//   tail      (D and E of the reference): s = kE / d + kD,   alpha = kE / d^3,   kE = -E / ar, kD = -D / ar^2
+// the grid receives  density * type_gradient + w * s * (delta . atom_gradient)  (src/grid_maker.cpp:618-634),
+// the atom needs, per column, the sums of diff * alpha * {1, dz, dz^2} and of diff * s (:636-662).
+// Bound by instruction issue: 28x96^3 at 0.25 A, 4 x 3000 atoms of 28 weighted channels each: 6.70 ms as
+// two sweeps with scalar arithmetic, 4.17 ms now (issue 68 %, L1 75 %).
+// ---------------------------------------------------------------------------------------------
+constexpr int SO_WARPS = 1;
+// Two lanes share a column, each taking every other quad: a load or reduction of a warp touches 16 lines
+// instead of 32 (4.54 -> 4.17 ms; the sweeps without reductions lose more to their column terms).
+constexpr int SO_ZL = 2;
+constexpr int SO_MINB = 16, SO_ATOM_MINB = 26;  // resident blocks: 114 and 72 registers
 
+struct SecondConst {
+  Pair k4, c4, kE, kD, ta, ntb, inv_ar;
+  __device__ __forceinline__ SecondConst(const GMParams& gm, const ItemParams& P) {
+    const bool tail = gm.ta != 0.f || gm.tb != 0.f;
+    k4 = c4 = pair(4.f * P.inv_ar2);
+    kE = pair(tail ? -gm.E * P.inv_ar : 0.f);
+    kD = pair(tail ? -gm.D * P.inv_ar2 : 0.f);
+    ta = pair(gm.ta);
+    ntb = pair(-gm.tb);
+    inv_ar = pair(P.inv_ar);
+  }
+};
+
+// density, s and alpha at two voxels; all zero beyond the cut-off and for a NaN distance (z outside the
+// footprint)
+__device__ __forceinline__ void second_factors(const SecondConst& K, const ItemParams& P, Pair rsq, Pair g, Pair& val, Pair& s,
+                                               Pair& alpha) {
+  float r0, r1, a0, a1, b0, b1;
+  split(rsq, r0, r1);
+  const bool gauss0 = r0 <= P.Tg, gauss1 = r1 <= P.Tg, in0 = r0 <= P.Tcut, in1 = r1 <= P.Tcut;
+  const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1));
+  float g0, g1;
+  split(g, g0, g1);
+  split(fma2(K.ta, mul2(mul2(rsq, id), K.inv_ar), K.ntb), a0, a1);
+  const Pair tq = pair(fminf(a0, 0.f), fminf(a1, 0.f));
+  split(mul2(tq, tq), a0, a1);
+  val = pair(gauss0 ? g0 : a0, gauss1 ? g1 : a1);
+  const Pair sg = mul2(K.k4, g), kid = mul2(K.kE, id);
+  split(sg, g0, g1);
+  split(add2(kid, K.kD), a0, a1);
+  s = pair(gauss0 ? g0 : fmaxf(a0, 0.f), gauss1 ? g1 : fmaxf(a1, 0.f));
+  split(mul2(K.c4, sg), g0, g1);
+  split(mul2(kid, mul2(id, id)), b0, b1);
+  alpha = pair(gauss0 ? g0 : in0 ? b0 : 0.f, gauss1 ? g1 : in1 ? b1 : 0.f);
+}
+
+// What the atom term keeps over an item's voxels: sums over pairs of voxels of one column, then over columns.
+struct SecondColumn {
+  Pair a0, a1, a2;  // diff * alpha * {1, dz, dz^2}
+};
+
+__device__ __forceinline__ void second_quads_item(const BwdArgs& G, int item, int bl, ColBufD& buf, ZTabs& zt, int lane) {
+  const GMParams& gm = G.gm;
+  const int b = G.b0 + bl;
   float cx, cy, cz;
   if (G.centers != nullptr) {
     cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
   } else {
     cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
   }
-  float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
-  ItemParams P = load_item<true>(G, bl, b, item, ox, oy, oz);
-  if (!P.valid || P.w == 0.f) return;
-
-  size_t dim = gm.dim;
-  float* out = G.out_grid + ((size_t)b * G.T + P.chan) * dim * dim * dim;
-  size_t gi = (size_t)b * G.N + item / G.T;
-  const float inx = G.ag_in[gi * 3], iny = G.ag_in[gi * 3 + 1], inz = G.ag_in[gi * 3 + 2];
-  const float intg = G.tg_in[gi * G.T + P.chan];
-  const float kexp = P.inv_ar2 * NEG2_LOG2E;
-  const float k4 = 4.f * P.inv_ar2 * P.w, kD = -gm.D * P.inv_ar2 * P.w, kE = -gm.E * P.inv_ar * P.w;
-  const float ta = gm.ta, ntb = -gm.tb;
-
-  for (Columns cols(P); cols.more();) {
-    const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
-    for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
-      __syncwarp();
-      fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
-      __syncwarp();
-      unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
-      for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
-        unsigned i = c0 + lane;
-        bool have = i < nkept;
-        float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F;
-        float dotxy = have ? fmaf(buf.dx[i], inx, buf.dy[i] * iny) : 0.f;
-        float* row = out + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
-        float exy = ex2_approx(dxy2 * kexp);
-        for (unsigned q = 0; q < nq; q++) {
-          float4 d2 = zt.dz2[q], e = zt.ez[q], dz = zt.dz[q];
-          float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w};
-          float dzv[4] = {dz.x, dz.y, dz.z, dz.w}, v[4];
+  const float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
+  const ItemParams P = load_item<true>(G, bl, b, item, ox, oy, oz);
+  float agx = 0.f, agy = 0.f, agz = 0.f;
+  if (P.valid) {
+    const size_t dim = gm.dim, chan = ((size_t)b * G.T + P.chan) * dim * dim * dim, gi = (size_t)b * G.N + item / G.T;
+    const float inx = G.ag_in[gi * 3], iny = G.ag_in[gi * 3 + 1], inz = G.ag_in[gi * 3 + 2];
+    const float intg = G.tg_in[gi * G.T + P.chan];
+    const float kexp = P.inv_ar2 * NEG2_LOG2E;
+    const SecondConst K(gm, P);
+    const Pair winz = pair(P.w * inz), tg2 = pair(intg);
+    Pair sb = pair(0.f);  // sum of diff * s
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
+      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+        __syncwarp();
+        fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
+        __syncwarp();
+        const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+        for (unsigned c0 = 0; c0 < nkept; c0 += 32 / SO_ZL) {
+          const unsigned i = c0 + lane / SO_ZL;
+          const bool have = i < nkept;
+          const float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F, dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
+          const size_t off = chan + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
+          const float4* row = reinterpret_cast<const float4*>(G.diff + off);
+          float* out = G.out_grid + off;
+          const Pair xy = pair(dxy2), exy = pair(ex2_approx(dxy2 * kexp));
+          const float dotxy = fmaf(dx, inx, dy * iny);
+          const Pair wdot = pair(P.w * dotxy);
+          SecondColumn C = {pair(0.f), pair(0.f), pair(0.f)};
+          for (unsigned q0 = lane % SO_ZL; q0 < nq; q0 += 4 * SO_ZL) {
+            float4 dv[4];
+            unsigned live = 0;
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            float rsq = __fadd_rn(dxy2, d2v[j]);
-            float g = exy * ev[j];
-            float tq = fminf(fmaf(ta, sqrt_approx(rsq * P.inv_ar2), ntb), 0.f);
-            bool gauss = rsq <= P.Tg;
-            float val = gauss ? g : tq * tq;
-            float sg = gauss ? k4 * g : fmaf(kE, rsqrt_approx(rsq), kD);
-            float dot = rsq > 0.f ? fmaf(dzv[j], inz, dotxy) : 0.f;
-            float gval = fmaf(val, intg, sg * dot);
-            v[j] = rsq <= P.Tcut ? gval : 0.f;
+            for (int u = 0; u < 4; u++) {
+              dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (q0 + SO_ZL * u < nq && __fadd_rn(dxy2, zt.lo[q0 + SO_ZL * u]) <= P.Tcut) {
+                live |= 1u << u;
+                dv[u] = __ldg(row + q0 + SO_ZL * u);
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              if (!(live >> u & 1u)) continue;
+              const float4 d2 = zt.dz2[q0 + SO_ZL * u], e = zt.ez[q0 + SO_ZL * u], dz = zt.dz[q0 + SO_ZL * u];
+              const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
+                         dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)}, dvp[2] = {pair(dv[u].x, dv[u].y), pair(dv[u].z, dv[u].w)};
+              float v[4];
+#pragma unroll
+              for (int j = 0; j < 2; j++) {
+                Pair val, s, alpha;
+                second_factors(K, P, add2(xy, d2p[j]), mul2(exy, ep[j]), val, s, alpha);
+                split(fma2(val, tg2, mul2(s, fma2(dzp[j], winz, wdot))), v[2 * j], v[2 * j + 1]);
+                const Pair t0 = mul2(dvp[j], alpha), t1 = mul2(t0, dzp[j]);
+                C.a0 = add2(C.a0, t0);
+                C.a1 = add2(C.a1, t1);
+                C.a2 = fma2(t1, dzp[j], C.a2);
+                sb = fma2(dvp[j], s, sb);
+              }
+              red_add_v4(out + 4 * (q0 + SO_ZL * u), v[0], v[1], v[2], v[3]);
+            }
           }
-          unsigned any = __float_as_uint(v[0]) | __float_as_uint(v[1]) | __float_as_uint(v[2]) |
-                         __float_as_uint(v[3]);
-          if (any != 0u) red_add_v4(row + 4 * q, v[0], v[1], v[2], v[3]);
+          // sum over the column of diff * (w*alpha*dot*delta_c + intg*alpha*delta_c^2), dot = dotxy + dz*inz
+          float a0, a1, a2, t;
+          split(C.a0, a0, t); a0 += t;
+          split(C.a1, a1, t); a1 += t;
+          split(C.a2, a2, t); a2 += t;
+          const float wd = P.w * fmaf(dotxy, a0, inz * a1);
+          agx = fmaf(dx, fmaf(intg * dx, a0, wd), agx);
+          agy = fmaf(dy, fmaf(intg * dy, a0, wd), agy);
+          agz += fmaf(P.w, fmaf(dotxy, a1, inz * a2), intg * a2);
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
+    // the isotropic part: -diff * s * (w*in_c + intg), the same factor for every voxel of the item
+    float s0, s1;
+    split(sb, s0, s1);
+    s0 = -(s0 + s1);
+    agx = fmaf(s0, fmaf(P.w, inx, intg), agx);
+    agy = fmaf(s0, fmaf(P.w, iny, intg), agy);
+    agz = fmaf(s0, fmaf(P.w, inz, intg), agz);
   }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    agx += __shfl_xor_sync(0xffffffffu, agx, o);
+    agy += __shfl_xor_sync(0xffffffffu, agy, o);
+    agz += __shfl_xor_sync(0xffffffffu, agz, o);
+  }
+  if (lane < 3) G.partial[((size_t)bl * G.N * G.T + item) * 3 + lane] = lane == 0 ? agx : lane == 1 ? agy : agz;
 }
 
-__global__ void __launch_bounds__(SCAT_WARPS * 32) k_gradgrad_quads_nz(BwdArgs G) {
-  __shared__ ColBufD bufs[SCAT_WARPS];
-  __shared__ ZTabs ztabs[SCAT_WARPS];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int unit = blockIdx.x * SCAT_WARPS + wid;
+__global__ void __launch_bounds__(SO_WARPS * 32, SO_MINB) k_second_quads_nz(BwdArgs G) {
+  __shared__ ColBufD bufs[SO_WARPS];
+  __shared__ ZTabs ztabs[SO_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, unit = blockIdx.x * SO_WARPS + wid;
   if (unit >= G.N * nz_groups(G.T)) return;
-  int b = G.b0 + blockIdx.y;
+  const int b = G.b0 + blockIdx.y;
   LMG_FOR_EACH_WEIGHTED_CHANNEL(G, b, unit, lane, atom, t) {
-    gradgrad_quads_item(G, atom * G.T + t, blockIdx.y, bufs[wid], ztabs[wid], lane);
+    second_quads_item(G, atom * G.T + t, blockIdx.y, bufs[wid], ztabs[wid], lane);
     __syncwarp();
   }
 }
@@ -1703,20 +1744,19 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_ag(BwdA
   }
 }
 
-// backward_gradients for the same layout (vector types, per-atom radii), one warp per atom.  Only
-// channels in which the atom carries weight take part (src/grid_maker.cpp:573).
-// Grid term, per voxel and such channel t:  density * tgrad_t  -  w_t * s * (delta . agrad), with
-// s = (d density/d dist)/dist: the two voxel-dependent factors are shared by the channels.
-__global__ void __launch_bounds__(QS_WARPS * 32) k_gradgrad_quads_atom(BwdArgs G) {
-  __shared__ ColBufD bufs[QS_WARPS];
-  __shared__ ZTabs ztabs[QS_WARPS];
-  __shared__ int nz_t[QS_WARPS][VA_CH];
-  __shared__ float nz_w[QS_WARPS][VA_CH], nz_g[QS_WARPS][VA_CH];
+// backward_gradients for the same layout (vector types, per-atom radii), one warp per atom, both terms in
+// one sweep as above.  Only channels in which the atom carries weight take part (src/grid_maker.cpp:573); the
+// voxel-dependent factors are shared by them.  Grid term of channel t: density * tgrad_t + w_t * s * (delta .
+// agrad); atom term: (alpha (delta.agrad) delta_a - s agrad_a) S1 + (alpha delta_a^2 - s) S2 with
+// S1 = sum_t w_t diff_t and S2 = sum_t tgrad_t diff_t.
+__global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_atom(BwdArgs G) {
+  __shared__ ColBufD bufs[SO_WARPS];
+  __shared__ ZTabs ztabs[SO_WARPS];
+  __shared__ int nz_t[SO_WARPS][VA_CH];
+  __shared__ float2 nz_wg[SO_WARPS][VA_CH];  // weight and incoming type gradient
   const GMParams& gm = G.gm;
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int item = blockIdx.x * QS_WARPS + wid;
-  int bl = blockIdx.y;
-  int b = G.b0 + bl;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, item = blockIdx.x * SO_WARPS + wid;
+  const int bl = blockIdx.y, b = G.b0 + bl;
   if (item >= G.N) return;
   ColBufD& buf = bufs[wid];
   ZTabs& zt = ztabs[wid];
@@ -1727,189 +1767,107 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_gradgrad_quads_atom(BwdArgs G
   } else {
     cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
   }
-  float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
-  ItemParams P = load_item<false>(G, bl, b, item, ox, oy, oz);
-  if (!P.valid) return;
+  const float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
+  const ItemParams P = load_item<false>(G, bl, b, item, ox, oy, oz);
 
-  size_t dim = gm.dim;
-  const size_t chan_stride = dim * dim * dim;
-  float* outb = G.out_grid + (size_t)b * G.T * chan_stride;
-  const size_t ai = (size_t)b * G.N + item;
+  const size_t dim = gm.dim, cs = dim * dim * dim, base = (size_t)b * G.T * cs, ai = (size_t)b * G.N + item;
   const float* wrow = G.type_vector + ai * G.T;
   const float* grow = G.tg_in + ai * G.T;
   const float inx = G.ag_in[ai * 3], iny = G.ag_in[ai * 3 + 1], inz = G.ag_in[ai * 3 + 2];
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
-  const float k4 = 4.f * P.inv_ar2, kD = -gm.D * P.inv_ar2, kE = -gm.E * P.inv_ar;
-  const float ta = gm.ta, ntb = -gm.tb;
-
-  for (int tb = 0; tb < G.T; tb += VA_CH) {
-    int t = tb + lane;
-    float w = t < G.T ? wrow[t] : 0.f;
-    unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
-    int nnz = __popc(m);
-    if (nnz == 0) continue;
-    __syncwarp();
-    if (w != 0.f) {
-      int slot = __popc(m & ((1u << lane) - 1u));
-      nz_t[wid][slot] = t;
-      nz_w[wid][slot] = w;
-      nz_g[wid][slot] = grow[t];
-    }
-    __syncwarp();
-    for (Columns cols(P); cols.more();) {
-      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
-      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
-        __syncwarp();
-        fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
-        __syncwarp();
-        unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
-        for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
-          unsigned i = c0 + lane;
-          bool have = i < nkept;
-          float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F;
-          float dotxy = have ? fmaf(buf.dx[i], inx, buf.dy[i] * iny) : 0.f;
-          float* row = outb + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
-          float exy = ex2_approx(dxy2 * kexp);
-          for (unsigned q = 0; q < nq; q++) {
-            float4 d2 = zt.dz2[q], e = zt.ez[q], dz = zt.dz[q];
-            float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w};
-            float dzv[4] = {dz.x, dz.y, dz.z, dz.w}, val[4], sd[4];
-            bool any = false;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              float rsq = __fadd_rn(dxy2, d2v[j]);
-              float g = exy * ev[j];
-              float tq = fminf(fmaf(ta, sqrt_approx(rsq * P.inv_ar2), ntb), 0.f);
-              bool gauss = rsq <= P.Tg, in = rsq <= P.Tcut;
-              float sg = gauss ? k4 * g : fmaf(kE, rsqrt_approx(rsq), kD);
-              float dot = rsq > 0.f ? fmaf(dzv[j], inz, dotxy) : 0.f;
-              val[j] = in ? (gauss ? g : tq * tq) : 0.f;
-              sd[j] = in ? sg * dot : 0.f;
-              any = any || in;
-            }
-            if (any) {
-              for (int k = 0; k < nnz; k++) {
-                float wk = nz_w[wid][k], gk = nz_g[wid][k];
-                red_add_v4(row + (size_t)nz_t[wid][k] * chan_stride + 4 * q, fmaf(val[0], gk, sd[0] * wk),
-                           fmaf(val[1], gk, sd[1] * wk), fmaf(val[2], gk, sd[2] * wk),
-                           fmaf(val[3], gk, sd[3] * wk));
-              }
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
-// Atom term (src/grid_maker.cpp:636-662, second derivatives of src/grid_maker.cu:812-878): per voxel
-//   sum_t dv_t [ w_t (alpha (delta.agrad) delta_a + beta agrad_a) + tgrad_t (alpha delta_a^2 + beta) ]
-// = (alpha (delta.agrad) delta_a + beta agrad_a) S1 + (alpha delta_a^2 + beta) S2
-// with S1 = sum_t w_t dv_t and S2 = sum_t tgrad_t dv_t over the weighted channels.
-__global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_gg(BwdArgs G) {
-  __shared__ ColBufD bufs[BWD2_WARPS];
-  __shared__ ZTabs ztabs[BWD2_WARPS];
-  __shared__ int nz_t[BWD2_WARPS][VA_CH];
-  __shared__ float nz_w[BWD2_WARPS][VA_CH], nz_g[BWD2_WARPS][VA_CH];
-  const GMParams& gm = G.gm;
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int item = blockIdx.x * BWD2_WARPS + wid;
-  int bl = blockIdx.y;
-  int b = G.b0 + bl;
-  if (item >= G.N) return;
-  ColBufD& buf = bufs[wid];
-  ZTabs& zt = ztabs[wid];
-
-  float cx, cy, cz;
-  if (G.centers != nullptr) {
-    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
-  } else {
-    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
-  }
-  float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
-  ItemParams P = load_item<false>(G, bl, b, item, ox, oy, oz);
-
-  size_t dim = gm.dim;
-  const size_t chan_stride = dim * dim * dim;
-  const float* diffb = G.diff + (size_t)b * G.T * chan_stride;
-  const size_t ai = (size_t)b * G.N + item;
-  const float* wrow = G.type_vector + ai * G.T;
-  const float* grow = G.tg_in + ai * G.T;
-  const float inx = G.ag_in[ai * 3], iny = G.ag_in[ai * 3 + 1], inz = G.ag_in[ai * 3 + 2];
-  const float kexp = P.inv_ar2 * NEG2_LOG2E;
+  const SecondConst K(gm, P);
   float agx = 0.f, agy = 0.f, agz = 0.f;
 
   for (int tb = 0; P.valid && tb < G.T; tb += VA_CH) {
-    int t = tb + lane;
-    float w = t < G.T ? wrow[t] : 0.f;
-    unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
-    int nnz = __popc(m);
+    const int t = tb + lane;
+    const float w = t < G.T ? wrow[t] : 0.f;
+    const unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
+    const int nnz = __popc(m);
     if (nnz == 0) continue;
     __syncwarp();
     if (w != 0.f) {
-      int slot = __popc(m & ((1u << lane) - 1u));
+      const int slot = __popc(m & ((1u << lane) - 1u));
       nz_t[wid][slot] = t;
-      nz_w[wid][slot] = w;
-      nz_g[wid][slot] = grow[t];
+      nz_wg[wid][slot] = make_float2(w, grow[t]);
     }
     __syncwarp();
+    Pair sb1 = pair(0.f), sb2 = pair(0.f);  // sums of s * S1 and s * S2
     for (Columns cols(P); cols.more();) {
       const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
       for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
         fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
         __syncwarp();
-        unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+        const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
         for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
-          unsigned i = c0 + lane;
-          bool have = i < nkept;
-          float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F;
-          float dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
-          const float4* row = reinterpret_cast<const float4*>(diffb + (size_t)(have ? buf.row[i] : 0u) * dim + zc);
-          float exy = ex2_approx(dxy2 * kexp);
-          float dotxy = fmaf(dx, inx, dy * iny);
+          const unsigned i = c0 + lane;
+          const bool have = i < nkept;
+          const float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F, dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
+          const size_t off = base + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
+          const Pair xy = pair(dxy2), exy = pair(ex2_approx(dxy2 * kexp));
+          const float dotxy = fmaf(dx, inx, dy * iny);
+          // sums over the column: alpha * S2 * {1, dz^2}, alpha * (delta . agrad) * S1 * {1, dz}
+          Pair p0 = pair(0.f), p2 = pair(0.f), u0 = pair(0.f), u1 = pair(0.f);
           for (unsigned q = 0; q < nq; q++) {
-            float4 d2 = zt.dz2[q], e = zt.ez[q], dz = zt.dz[q];
-            float lo = zt.lo[q];
-            if (!(__fadd_rn(dxy2, lo) <= P.Tcut)) continue;
-            float s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int k = 0; k < nnz; k++) {
-              float wk = nz_w[wid][k], gk = nz_g[wid][k];
-              float4 dv = __ldg(row + q + (size_t)nz_t[wid][k] * (chan_stride / 4));
-              s1[0] = fmaf(wk, dv.x, s1[0]); s1[1] = fmaf(wk, dv.y, s1[1]);
-              s1[2] = fmaf(wk, dv.z, s1[2]); s1[3] = fmaf(wk, dv.w, s1[3]);
-              s2[0] = fmaf(gk, dv.x, s2[0]); s2[1] = fmaf(gk, dv.y, s2[1]);
-              s2[2] = fmaf(gk, dv.z, s2[2]); s2[3] = fmaf(gk, dv.w, s2[3]);
-            }
-            float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w}, dzv[4] = {dz.x, dz.y, dz.z, dz.w};
+            if (!(__fadd_rn(dxy2, zt.lo[q]) <= P.Tcut)) continue;
+            const float4 d2 = zt.dz2[q], e = zt.ez[q], dz = zt.dz[q];
+            const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
+                       dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)};
+            Pair val[2], s[2], sd[2], alpha[2], dot[2], s1[2], s2[2];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              float rsq = __fadd_rn(dxy2, d2v[j]);
-              if (rsq <= P.Tcut) {
-                float alpha, beta;
-                if (rsq <= P.Tg) {
-                  float g = exy * ev[j];
-                  alpha = 16.f * g * P.inv_ar2 * P.inv_ar2;
-                  beta = -4.f * g * P.inv_ar2;
-                } else {
-                  float id = rsqrt_approx(rsq);
-                  float S = fmaf(gm.D * P.inv_ar, rsq * id, gm.E);
-                  beta = S * id * P.inv_ar;
-                  alpha = fmaf(gm.D * P.inv_ar2, id * id, -beta * id * id);
-                }
-                float dzj = dzv[j];
-                float ad = alpha * fmaf(dzj, inz, dotxy);
-                agx += fmaf(ad, dx, beta * inx) * s1[j] + fmaf(alpha, dx * dx, beta) * s2[j];
-                agy += fmaf(ad, dy, beta * iny) * s1[j] + fmaf(alpha, dy * dy, beta) * s2[j];
-                agz += fmaf(ad, dzj, beta * inz) * s1[j] + fmaf(alpha, dzj * dzj, beta) * s2[j];
+            for (int j = 0; j < 2; j++) {
+              second_factors(K, P, add2(xy, d2p[j]), mul2(exy, ep[j]), val[j], s[j], alpha[j]);
+              dot[j] = fma2(dzp[j], pair(inz), pair(dotxy));
+              sd[j] = mul2(s[j], dot[j]);
+              s1[j] = s2[j] = pair(0.f);
+            }
+            const float* src = G.diff + off + 4 * q;
+            float* dst = G.out_grid + off + 4 * q;
+            for (int k = 0; k < nnz; k++) {
+              const float2 wg = nz_wg[wid][k];
+              const size_t co = (size_t)nz_t[wid][k] * cs;
+              const float4 dv = __ldg(reinterpret_cast<const float4*>(src + co));
+              const Pair dvp[2] = {pair(dv.x, dv.y), pair(dv.z, dv.w)}, wk = pair(wg.x), gk = pair(wg.y);
+              float v[4];
+#pragma unroll
+              for (int j = 0; j < 2; j++) {
+                s1[j] = fma2(wk, dvp[j], s1[j]);
+                s2[j] = fma2(gk, dvp[j], s2[j]);
+                split(fma2(val[j], gk, mul2(sd[j], wk)), v[2 * j], v[2 * j + 1]);
               }
+              red_add_v4(dst + co, v[0], v[1], v[2], v[3]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+              const Pair a2 = mul2(alpha[j], s2[j]), a1 = mul2(mul2(alpha[j], dot[j]), s1[j]);
+              p0 = add2(p0, a2);
+              p2 = fma2(a2, mul2(dzp[j], dzp[j]), p2);
+              u0 = add2(u0, a1);
+              u1 = fma2(a1, dzp[j], u1);
+              sb1 = fma2(s[j], s1[j], sb1);
+              sb2 = fma2(s[j], s2[j], sb2);
             }
           }
+          float a, b0, c, d, t0;
+          split(p0, a, t0); a += t0;
+          split(p2, b0, t0); b0 += t0;
+          split(u0, c, t0); c += t0;
+          split(u1, d, t0); d += t0;
+          agx = fmaf(dx, fmaf(a, dx, c), agx);
+          agy = fmaf(dy, fmaf(a, dy, c), agy);
+          agz += b0 + d;
         }
       }
       __syncwarp();
     }
+    float x0, x1, y0, y1;
+    split(sb1, x0, x1);
+    split(sb2, y0, y1);
+    x0 += x1;
+    y0 += y1;
+    agx -= fmaf(x0, inx, y0);
+    agy -= fmaf(x0, iny, y0);
+    agz -= fmaf(x0, inz, y0);
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
@@ -1917,11 +1875,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_gg(BwdA
     agy += __shfl_xor_sync(0xffffffffu, agy, o);
     agz += __shfl_xor_sync(0xffffffffu, agz, o);
   }
-  if (lane == 0) {
-    G.atom_gradients[ai * 3] = agx;
-    G.atom_gradients[ai * 3 + 1] = agy;
-    G.atom_gradients[ai * 3 + 2] = agz;
-  }
+  if (lane < 3) G.atom_gradients[ai * 3 + lane] = lane == 0 ? agx : lane == 1 ? agy : agz;
 }
 
 // atom_gradients[a] = sum over channels in ascending order of partial[a][t] * w[a][t] for w != 0
@@ -2004,7 +1958,7 @@ cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, 
 }
 
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
-  long items = (long)G.N * ((mode == 1 || mode == 3) ? G.T : 1);
+  long items = (long)G.N * (mode == 1 ? G.T : 1);
   if (items == 0 || G.nb == 0) return cudaSuccess;
   dim3 grid((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
   bool bin = G.gm.binary != 0;
@@ -2035,15 +1989,6 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
     else k_backward_warp<1, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
     int n = G.nb * G.N;
     k_reduce_types<<<(n + 255) / 256, 256, 0, st>>>(G);
-  } else if (mode == 3 && quads && !G.gm.rti) {
-    dim3 ga((unsigned)((G.N + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
-    k_backward_quads_atom_gg<<<ga, BWD2_WARPS * 32, 0, st>>>(G);
-  } else if (mode == 3) {
-    dim3 ga((unsigned)(((long)G.N * nz_groups(G.T) + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
-    if (quads) k_backward_quads_nz<3, false><<<ga, BWD2_WARPS * 32, 0, st>>>(G);
-    else k_backward_warp<3, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    int n = G.nb * G.N;
-    k_reduce_types<<<(n + 255) / 256, 256, 0, st>>>(G);
   } else {
     if (quads && bin) k_backward_quads<2, true><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
     else if (quads) k_backward_quads<2, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
@@ -2053,19 +1998,23 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_gradgrad_scatter(const BwdArgs& G, cudaStream_t st) {
-  long items = (long)G.N * G.T;
+cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
+  const long items = (long)G.N * G.T;
   if (items == 0 || G.nb == 0) return cudaSuccess;
-  dim3 grid((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb);
-  if (G.quads && !G.gm.rti && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0) {
-    dim3 ga((unsigned)((G.N + QS_WARPS - 1) / QS_WARPS), G.nb);
-    k_gradgrad_quads_atom<<<ga, QS_WARPS * 32, 0, st>>>(G);
-  } else if (G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0) {
-    dim3 ga((unsigned)(((long)G.N * nz_groups(G.T) + SCAT_WARPS - 1) / SCAT_WARPS), G.nb);
-    k_gradgrad_quads_nz<<<ga, SCAT_WARPS * 32, 0, st>>>(G);
+  const bool quads = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0 && (uintptr_t)G.diff % 16 == 0;
+  if (quads && !G.gm.rti) {
+    k_second_quads_atom<<<dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st>>>(G);
+    return cudaGetLastError();
   }
-  else
-    k_gradgrad_scatter<<<grid, SCAT_WARPS * 32, 0, st>>>(G);
+  if (quads) {
+    const long units = (long)G.N * nz_groups(G.T);
+    k_second_quads_nz<<<dim3((unsigned)((units + SO_WARPS - 1) / SO_WARPS), G.nb), SO_WARPS * 32, 0, st>>>(G);
+  } else {
+    k_gradgrad_scatter<<<dim3((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb), SCAT_WARPS * 32, 0, st>>>(G);
+    k_backward_warp<3, false><<<dim3((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb), BWD2_WARPS * 32, 0, st>>>(G);
+  }
+  const int n = G.nb * G.N;
+  k_reduce_types<<<(n + 255) / 256, 256, 0, st>>>(G);
   return cudaGetLastError();
 }
 

@@ -76,7 +76,8 @@ cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_
 bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode);
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st);
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st);
-cudaError_t launch_gradgrad_scatter(const BwdArgs& G, cudaStream_t st);
+// both terms of backward_gradients: out_grid (zero-filled before) and atom_gradients
+cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st);
 
 }  // namespace lmg
 
