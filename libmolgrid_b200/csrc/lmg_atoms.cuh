@@ -164,4 +164,12 @@ __device__ __forceinline__ void put_flag(const EmitArgs& A, unsigned i, unsigned
   }
 }
 
+// [lo, hi) cut down to the voxels less than `ar` from the atom along an axis, with an allowance for roundings
+__device__ __forceinline__ void within(float origin, float at, float ar, float res, unsigned& lo, unsigned& hi) {
+  const float inv = __fdividef(1.f, res), c = (at - origin) * inv, r = ar * inv + 0.01f + (fabsf(at) + fabsf(origin)) * inv * 2e-6f;
+  const float l = ceilf(c - r), h = floorf(c + r) + 1.f;
+  if (l > (float)lo) lo = l < 65535.f ? (unsigned)l : 65535u;
+  if (h < (float)hi) hi = h > 0.f ? (unsigned)h : 0u;
+}
+
 }  // namespace lmg

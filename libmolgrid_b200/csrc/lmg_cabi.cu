@@ -481,6 +481,25 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
   if (per_pass == 0)
     return fail(LMG_ERR_WORKSPACE, "workspace too small for one example: need " +
                                        std::to_string(STATUS_BYTES + one.per_example) + " bytes");
+  if (vec == 0 && g->binary) {
+    lmg::EmitArgs E;
+    fill_emit(E, g, a);
+    E.nb = std::min(per_pass, a->batch);
+    if (lmg::occupancy_serves(E)) {
+      Range whole("lmg_forward");
+      for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
+        E.b0 = b0; E.nb = std::min(per_pass, a->batch - b0);
+        carve(E, layout(g, LMG_OP_FORWARD, E.nb, a->max_atoms, a->ntypes, vec), ws);
+        E.round_types = 0;
+        ProfRec* pr = prof_begin(0, st);
+        e = lmg::launch_occupancy(E, out, st);
+        prof_end(pr, st);
+        g_launches += 1;
+        if (e != cudaSuccess) return cuda_fail(e, "occupancy");
+      }
+      return LMG_OK;
+    }
+  }
   // One zero fill of the whole output, then per pass one emit and one scatter launch.  (Measured
   // and dropped: filling on an auxiliary stream one chunk ahead of the scatter - the library's fill
   // kernels occupy every SM, so the scatter blocks merely queue behind them; and letting each

@@ -787,14 +787,6 @@ __device__ __forceinline__ void occupancy_sweep(const ItemParams& P, const ColBu
   }
 }
 
-// [lo, hi) within the voxels less than `ar` from the atom along an axis, and one more at either end
-__device__ __forceinline__ void within(float origin, float at, float ar, float res, unsigned& lo, unsigned& hi) {
-  const float inv = __fdividef(1.f, res), c = (at - origin) * inv, r = ar * inv;
-  const float l = floorf(c - r) - 1.f, h = ceilf(c + r) + 1.f;
-  if (l > (float)lo) lo = (unsigned)l;
-  if (h < (float)hi) hi = h > 0.f ? (unsigned)h : 0u;
-}
-
 __device__ __forceinline__ void forward_binary_core(const BwdArgs& G, ItemParams P, int b, float ox, float oy, float oz,
                                                     ColBuf& buf, int lane, unsigned part = 0, unsigned parts = 1) {
   const GMParams& gm = G.gm;

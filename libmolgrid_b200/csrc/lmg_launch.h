@@ -68,6 +68,9 @@ struct BwdArgs {
 
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st);
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st);
+// occupancy of index types in one launch that writes every voxel once (lmg_occupancy.cu)
+bool occupancy_serves(const EmitArgs& A);
+cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st);
 // the forward pass of index types without k_emit: every warp prepares its own atom (density on aligned
 // grids, or occupancy; the output is zero-filled before)
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G);

@@ -87,3 +87,26 @@ def test_status_of_every_pass(N, at):
     finally:
         api.MAX_WORKSPACE_BYTES = old
         api._workspaces.clear()
+
+
+# whole channels, parts of channels and single planes per block; runs of more than one and two words of the mask;
+# rows that start anywhere; atoms of one channel in several chunks of the search
+@pytest.mark.parametrize("B,N,T,points,res", [(1, 40, 3, 24, 1.0), (3, 100, 50, 13, 0.5), (30, 9, 5, 11, 0.5), (1, 128, 2, 65, 0.0625),
+                                              (75, 2100, 2, 10, 0.5), (1, 20, 2, 200, 0.1)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_occupancy_in_one_launch(port, B, N, T, points, res, shift):
+    side = (points - 1) * res
+    g, og = lmg.GridMaker(res, side, True), port.gm(res, side, True)
+    ex = [cases.index_case(7 * b + N, N, T, 0.6 * side) for b in range(B)]
+    coords, types, radii = (np.stack([e[k] for e in ex]) for k in range(3))
+    if N > 2000:
+        types[:] = 1.0                      # every atom in one channel
+    ns = np.full(B, N, np.int32)
+    ns[-1] = N - 1
+    buf = torch.full((B * T * points ** 3 + shift,), 7.0, device="cuda")
+    out = buf[shift:].view((B,) + g.grid_dimensions(T))
+    g.forward(torch.zeros((B, 3), device="cuda"), dev(coords), dev(types), dev(radii), out, n_atoms=dev(ns))
+    for b in {0, B - 1}:
+        want = port.forward_index(og, (0, 0, 0), coords[b][:ns[b]], types[b][:ns[b]], radii[b][:ns[b]], T)
+        np.testing.assert_array_equal(out[b].cpu().numpy(), want)
+    assert shift == 0 or float(buf[0]) == 7.0
