@@ -28,7 +28,7 @@ struct ProfRec { cudaEvent_t e0, e1; int kind; };
 std::vector<ProfRec> g_prof;
 size_t g_prof_used = 0;
 bool g_prof_on = false;
-long g_launches = 0;  // kernels launched by this library since load (memsets not counted)
+long g_launches = 0;  // kernels launched by this library since load (clears of outputs not counted)
 
 ProfRec* prof_begin(int kind, cudaStream_t st) {
   if (!g_prof_on || g_prof_used >= g_prof.size()) return nullptr;
@@ -506,13 +506,6 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
   // scatter launch clear the next chunk of examples - ten small launches lose more in ramp-up and
   // tail than the overlap gains.)
   Range whole("lmg_forward");
-  ProfRec* pr_fill = prof_begin(2, st);
-  {
-    Range r("zero fill");
-    e = cudaMemsetAsync(out, 0, grid_elems * a->batch * sizeof(float), st);
-  }
-  prof_end(pr_fill, st);
-  if (e != cudaSuccess) return cuda_fail(e, "zeroing output");
   bool self = false;  // the same for every pass of the call
   for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
     int nb = std::min(per_pass, a->batch - b0);
@@ -532,10 +525,23 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
     S.out_grid = out;
     S.precise = use_precise(g);
     S.quads = g_quads;
+    const size_t n = grid_elems * a->batch;
+    // our own zeros where they can be written in quads: they overlap with the kernels around them
+    const bool zeros = b0 == 0 && n % 4 == 0 && (uintptr_t)out % 16 == 0;
+    auto clear = [&](bool beside) {
+      Range r("zero fill");
+      ProfRec* pr = prof_begin(2, st);
+      cudaError_t z = zeros ? lmg::launch_zero(out, n, beside, st) : cudaMemsetAsync(out, 0, n * sizeof(float), st);
+      prof_end(pr, st);
+      return z;
+    };
     if (b0 == 0) self = lmg::forward_self_serves(E, S);
+    const bool after_emit = zeros && !self;
+    if (b0 == 0 && !after_emit) e = clear(false);
+    if (b0 == 0 && !after_emit && e != cudaSuccess) return cuda_fail(e, "zeroing output");
     if (self) {  // its flags, one per atom, run on into the records it does not need
       ProfRec* pr = prof_begin(0, st);
-      e = lmg::launch_forward_self(E, S, st);
+      e = lmg::launch_forward_self(E, S, zeros, st);
       prof_end(pr, st);
       g_launches += 1;
       if (e != cudaSuccess) return cuda_fail(e, "forward scatter");
@@ -546,6 +552,10 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
       e = lmg::launch_emit(E, st);
     }
     if (e != cudaSuccess) return cuda_fail(e, "emit");
+    if (after_emit) {
+      e = clear(true);
+      if (e != cudaSuccess) return cuda_fail(e, "zeroing output");
+    }
     ProfRec* pr = prof_begin(0, st);
     {
       Range r("forward scatter");

@@ -19,6 +19,7 @@ namespace lmg {
 // ---------------------------------------------------------------------------------------------
 
 __global__ void __launch_bounds__(256) k_chan_params(EmitArgs A) {
+  wait_for_stream();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= A.nb * A.T) return;
   int b = A.b0 + i / A.T, t = i % A.T;
@@ -29,6 +30,8 @@ __global__ void __launch_bounds__(256) k_chan_params(EmitArgs A) {
 
 // One thread per atom slot of the pass.
 __global__ void __launch_bounds__(256) k_emit(EmitArgs A) {
+  wait_for_stream();
+  let_next_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool bad = false;
   if (i < A.nb * A.N) {
@@ -230,6 +233,7 @@ struct Columns {
 // MODE 3: backward_gradients' atom term        -> partial[b][a][t][3]  (src/grid_maker.cpp:636-662)
 template <int MODE, bool BINARY>
 __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
+  wait_for_stream();
   constexpr bool VEC = MODE == 1 || MODE == 3;
   __shared__ ColBufD bufs[BWD2_WARPS];
   const GMParams& gm = G.gm;
@@ -409,6 +413,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
 // ---------------------------------------------------------------------------------------------
 template <bool BINARY, bool PRECISE, bool VEC>  // not <true, *, false>: k_forward_binary
 __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_scatter(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBuf bufs[SCAT_WARPS];
   const GMParams& gm = G.gm;
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -487,6 +492,7 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_scatter(BwdArgs G) 
 //   density * type_gradient  -  w * ((d density/d dist)/dist) * (delta . atom_gradient),
 // delta = grid point - atom.  The output is zero-filled before the launch.
 __global__ void __launch_bounds__(SCAT_WARPS * 32) k_gradgrad_scatter(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBufD bufs[SCAT_WARPS];
   const GMParams& gm = G.gm;
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -754,6 +760,7 @@ __device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, i
 
 template <bool VEC>
 __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBuf bufs[QS_WARPS];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int item = blockIdx.x * QS_WARPS + wid;
@@ -812,6 +819,7 @@ __device__ __forceinline__ void forward_binary_core(const BwdArgs& G, ItemParams
 #endif
 constexpr int BIN_WARPS = LMG_BIN_WARPS;
 __global__ void __launch_bounds__(BIN_WARPS * 32) k_forward_binary(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBuf bufs[BIN_WARPS];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, item = blockIdx.x * BIN_WARPS + wid;
   if (item >= G.N) return;
@@ -832,13 +840,14 @@ __global__ void __launch_bounds__(BIN_WARPS * 32) k_forward_binary(BwdArgs G) {
 // 11.6 -> 7.3 us; 64 x 1000 atoms: 234.9 -> 229.7 us; 50 x 3000: 264 -> 285 us, so densities of more than
 // FWD_SELF_ATOMS slots keep k_emit.  Occupancy, whose sweeps are a third as long, gains at every size
 // (50 x 3000: 250 -> 228 us).
-template <bool BINARY, int WARPS>
+template <bool BINARY, int WARPS, bool ZEROED_BEFORE>
 __global__ void __launch_bounds__(32 * WARPS) k_forward_self(EmitArgs A, BwdArgs G) {
   __shared__ ColBuf bufs[WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, a = blockIdx.x, bl = blockIdx.y, b = A.b0 + bl;
   Rec r;
   float ox, oy, oz;
   const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
+  if (ZEROED_BEFORE) wait_for_stream();  // the output is zero
   if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
   const ItemParams P = item_of(r);
   if (!P.valid) return;
@@ -863,6 +872,7 @@ __host__ __device__ inline int nz_groups(int T) { return (T + NZ_GROUP - 1) / NZ
         if (int t = t0_ + __ffs(m_) - 1; true)
 
 __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_quads_nz(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBuf bufs[SCAT_WARPS];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int unit = blockIdx.x * SCAT_WARPS + wid;
@@ -1079,6 +1089,7 @@ __device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, 
 // 32 resident warps instead of 72 and 28, 2.67 -> 2.58 ms at 28x96^3 (4 x 3000 atoms, 28 channels).
 template <int MODE, bool BINARY>
 __global__ void __launch_bounds__(BWD2_WARPS * 32, 32) k_backward_quads(BwdArgs G) {
+  wait_for_stream();
   constexpr bool VEC = MODE == 1;
   __shared__ ColBufD bufs[BWD2_WARPS];
   __shared__ ZTabs ztabs[BWD2_WARPS];
@@ -1099,6 +1110,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, 
   __shared__ ZTabs zts[WARPS];
   __shared__ float4 sums[WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, a = blockIdx.x, bl = blockIdx.y, b = A.b0 + bl;
+  wait_for_stream();
   Rec r;
   float ox, oy, oz;
   const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
@@ -1127,6 +1139,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, 
 // nothing from channels without weight (MODE 1 when no type gradients are wanted).
 template <int MODE, bool BINARY>
 __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_nz(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBufD bufs[BWD2_WARPS];
   __shared__ ZTabs ztabs[BWD2_WARPS];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1299,6 +1312,7 @@ __device__ __forceinline__ void second_quads_item(const BwdArgs& G, int item, in
 }
 
 __global__ void __launch_bounds__(SO_WARPS * 32, SO_MINB) k_second_quads_nz(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBufD bufs[SO_WARPS];
   __shared__ ZTabs ztabs[SO_WARPS];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, unit = blockIdx.x * SO_WARPS + wid;
@@ -1322,6 +1336,7 @@ constexpr int VA_SPARSE = 2;  // rounds with at most this many weighted channels
 
 template <bool BINARY, bool PRECISE>
 __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBuf bufs[QS_WARPS];
   __shared__ ZTabs ztabs[QS_WARPS];
   __shared__ int nz_t[QS_WARPS][VA_CH];
@@ -1563,6 +1578,7 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
 
 template <bool BINARY>
 __global__ void __launch_bounds__(VA_WARPS * 32) k_backward_quads_atom(BwdArgs G) {
+  wait_for_stream();
   __shared__ VaShared shs[VA_WARPS];
   const GMParams& gm = G.gm;
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1633,6 +1649,7 @@ __global__ void __launch_bounds__(VA_WARPS * 32) k_backward_quads_atom(BwdArgs G
 // The same without type gradients (the caller passed none: types that are inputs, not parameters):
 // only the channels that carry weight are read.
 __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_ag(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBufD bufs[BWD2_WARPS];
   __shared__ ZTabs ztabs[BWD2_WARPS];
   __shared__ int nz_t[BWD2_WARPS][VA_CH];
@@ -1742,6 +1759,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_ag(BwdA
 // agrad); atom term: (alpha (delta.agrad) delta_a - s agrad_a) S1 + (alpha delta_a^2 - s) S2 with
 // S1 = sum_t w_t diff_t and S2 = sum_t tgrad_t diff_t.
 __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_atom(BwdArgs G) {
+  wait_for_stream();
   __shared__ ColBufD bufs[SO_WARPS];
   __shared__ ZTabs ztabs[SO_WARPS];
   __shared__ int nz_t[SO_WARPS][VA_CH];
@@ -1873,6 +1891,7 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
 // atom_gradients[a] = sum over channels in ascending order of partial[a][t] * w[a][t] for w != 0
 // (src/grid_maker.cpp:508-515)
 __global__ void __launch_bounds__(256) k_reduce_types(BwdArgs G) {
+  wait_for_stream();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= G.nb * G.N) return;
   int bl = i / G.N, a = i - bl * G.N;
@@ -1902,10 +1921,10 @@ __global__ void __launch_bounds__(256) k_reduce_types(BwdArgs G) {
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st) {
   if (A.gm.rti && A.vec) {
     int n = A.nb * A.T;
-    k_chan_params<<<(n + 255) / 256, 256, 0, st>>>(A);
+    launch_early(k_chan_params, dim3((n + 255) / 256), 256, 0, st, A);
   }
   int n = A.nb * A.N;
-  k_emit<<<(n + 255) / 256, 256, 0, st>>>(A);
+  launch_early(k_emit, dim3((n + 255) / 256), 256, 0, st, A);
   return cudaGetLastError();
 }
 
@@ -1920,25 +1939,50 @@ bool forward_self_serves(const EmitArgs& A, const BwdArgs& G) {
 }
 
 template <int WARPS>
-static void forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_t st) {
+static cudaError_t forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st) {
   const dim3 grid(A.N, A.nb);
-  if (A.gm.binary) k_forward_self<true, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
-  else k_forward_self<false, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  if (early) {
+    return A.gm.binary ? launch_early(k_forward_self<true, WARPS, true>, grid, 32 * WARPS, 0, st, A, G)
+                       : launch_early(k_forward_self<false, WARPS, true>, grid, 32 * WARPS, 0, st, A, G);
+  }
+  if (A.gm.binary) k_forward_self<true, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  else k_forward_self<false, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  return cudaGetLastError();
 }
 
-cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_t st) {
+// `early`: the launch before this one is launch_zero() of this call's output
+cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st) {
   if (A.N == 0 || A.nb == 0) return cudaSuccess;
-  if ((long)A.nb * A.N <= SELF_SPLIT) forward_self<4>(A, G, st);
-  else forward_self<1>(A, G, st);
-  return cudaGetLastError();
+  return (long)A.nb * A.N <= SELF_SPLIT ? forward_self<4>(A, G, early, st) : forward_self<1>(A, G, early, st);
+}
+
+// Bound by its stores.  Two of 16 bytes a thread: with more per thread small outputs take longer (12.4 MB: 7 us of zeros and
+// reductions instead of 5.5).
+constexpr int ZERO_THREADS = 256, ZERO_QUADS = 2;
+// BESIDE: runs beside the kernel before it, which began once all earlier work was done.
+template <bool BESIDE>
+__global__ void __launch_bounds__(ZERO_THREADS) k_zero(float4* p, size_t quads) {
+  if (!BESIDE) wait_for_stream();
+  let_next_begin();  // earlier work is done: the next kernel may read what this one does not write
+  const size_t i0 = (size_t)blockIdx.x * (ZERO_THREADS * ZERO_QUADS) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < ZERO_QUADS; k++)
+    if (i0 + ZERO_THREADS * k < quads) p[i0 + ZERO_THREADS * k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (BESIDE) wait_for_stream();  // this kernel is not done before the one before it
+}
+
+cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st) {
+  const size_t per = (size_t)ZERO_THREADS * ZERO_QUADS;
+  const dim3 grid((unsigned)((n / 4 + per - 1) / per));
+  return launch_early(beside ? k_zero<true> : k_zero<false>, grid, ZERO_THREADS, 0, st, reinterpret_cast<float4*>(p), n / 4);
 }
 
 template <int WARPS>
 static void backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
   const dim3 grid(A.N, A.nb);
-  if (mode == 0) k_backward_quads_self<0, false, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
-  else if (A.gm.binary) k_backward_quads_self<2, true, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
-  else k_backward_quads_self<2, false, WARPS><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  if (mode == 0) launch_early(k_backward_quads_self<0, false, WARPS>, grid, 32 * WARPS, 0, st, A, G);
+  else if (A.gm.binary) launch_early(k_backward_quads_self<2, true, WARPS>, grid, 32 * WARPS, 0, st, A, G);
+  else launch_early(k_backward_quads_self<2, false, WARPS>, grid, 32 * WARPS, 0, st, A, G);
 }
 
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
@@ -1958,34 +2002,34 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
   bool quads = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.diff % 16 == 0 &&
                (mode != 2 || (uintptr_t)G.density % 16 == 0);
   if (mode == 0) {
-    if (quads) k_backward_quads<0, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else k_backward_warp<0, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
+    if (quads) launch_early(k_backward_quads<0, false>, grid, BWD2_WARPS * 32, 0, st, G);
+    else launch_early(k_backward_warp<0, false>, grid, BWD2_WARPS * 32, 0, st, G);
   } else if (mode == 1 && quads && !G.gm.rti) {
     // per-atom radii: one work item per atom writes both gradients, no reduction over channels after it
     dim3 ga((unsigned)((G.N + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
     dim3 gv((unsigned)((G.N + VA_WARPS - 1) / VA_WARPS), G.nb);
-    if (G.type_gradients == nullptr) k_backward_quads_atom_ag<<<ga, BWD2_WARPS * 32, 0, st>>>(G);
-    else if (bin) k_backward_quads_atom<true><<<gv, VA_WARPS * 32, 0, st>>>(G);
-    else k_backward_quads_atom<false><<<gv, VA_WARPS * 32, 0, st>>>(G);
+    if (G.type_gradients == nullptr) launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
+    else if (bin) launch_early(k_backward_quads_atom<true>, gv, VA_WARPS * 32, 0, st, G);
+    else launch_early(k_backward_quads_atom<false>, gv, VA_WARPS * 32, 0, st, G);
   } else if (mode == 1 && quads && G.type_gradients == nullptr) {
     // radii by channel, no type gradients wanted: only the weighted channels of each atom
     dim3 ga((unsigned)(((long)G.N * nz_groups(G.T) + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
-    if (bin) k_backward_quads_nz<1, true><<<ga, BWD2_WARPS * 32, 0, st>>>(G);
-    else k_backward_quads_nz<1, false><<<ga, BWD2_WARPS * 32, 0, st>>>(G);
+    if (bin) launch_early(k_backward_quads_nz<1, true>, ga, BWD2_WARPS * 32, 0, st, G);
+    else launch_early(k_backward_quads_nz<1, false>, ga, BWD2_WARPS * 32, 0, st, G);
     int n = G.nb * G.N;
-    k_reduce_types<<<(n + 255) / 256, 256, 0, st>>>(G);
+    launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
   } else if (mode == 1) {
-    if (quads && bin) k_backward_quads<1, true><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else if (quads) k_backward_quads<1, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else if (bin) k_backward_warp<1, true><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else k_backward_warp<1, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
+    if (quads && bin) launch_early(k_backward_quads<1, true>, grid, BWD2_WARPS * 32, 0, st, G);
+    else if (quads) launch_early(k_backward_quads<1, false>, grid, BWD2_WARPS * 32, 0, st, G);
+    else if (bin) launch_early(k_backward_warp<1, true>, grid, BWD2_WARPS * 32, 0, st, G);
+    else launch_early(k_backward_warp<1, false>, grid, BWD2_WARPS * 32, 0, st, G);
     int n = G.nb * G.N;
-    k_reduce_types<<<(n + 255) / 256, 256, 0, st>>>(G);
+    launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
   } else {
-    if (quads && bin) k_backward_quads<2, true><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else if (quads) k_backward_quads<2, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else if (bin) k_backward_warp<2, true><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
-    else k_backward_warp<2, false><<<grid, BWD2_WARPS * 32, 0, st>>>(G);
+    if (quads && bin) launch_early(k_backward_quads<2, true>, grid, BWD2_WARPS * 32, 0, st, G);
+    else if (quads) launch_early(k_backward_quads<2, false>, grid, BWD2_WARPS * 32, 0, st, G);
+    else if (bin) launch_early(k_backward_warp<2, true>, grid, BWD2_WARPS * 32, 0, st, G);
+    else launch_early(k_backward_warp<2, false>, grid, BWD2_WARPS * 32, 0, st, G);
   }
   return cudaGetLastError();
 }
@@ -1995,18 +2039,18 @@ cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
   if (items == 0 || G.nb == 0) return cudaSuccess;
   const bool quads = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0 && (uintptr_t)G.diff % 16 == 0;
   if (quads && !G.gm.rti) {
-    k_second_quads_atom<<<dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st>>>(G);
+    launch_early(k_second_quads_atom, dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st, G);
     return cudaGetLastError();
   }
   if (quads) {
     const long units = (long)G.N * nz_groups(G.T);
-    k_second_quads_nz<<<dim3((unsigned)((units + SO_WARPS - 1) / SO_WARPS), G.nb), SO_WARPS * 32, 0, st>>>(G);
+    launch_early(k_second_quads_nz, dim3((unsigned)((units + SO_WARPS - 1) / SO_WARPS), G.nb), SO_WARPS * 32, 0, st, G);
   } else {
-    k_gradgrad_scatter<<<dim3((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb), SCAT_WARPS * 32, 0, st>>>(G);
-    k_backward_warp<3, false><<<dim3((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb), BWD2_WARPS * 32, 0, st>>>(G);
+    launch_early(k_gradgrad_scatter, dim3((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb), SCAT_WARPS * 32, 0, st, G);
+    launch_early(k_backward_warp<3, false>, dim3((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb), BWD2_WARPS * 32, 0, st, G);
   }
   const int n = G.nb * G.N;
-  k_reduce_types<<<(n + 255) / 256, 256, 0, st>>>(G);
+  launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
   return cudaGetLastError();
 }
 
@@ -2019,30 +2063,30 @@ cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st) 
   if (vec && !G.gm.rti && aligned) {
     // per-atom radii: one work item per atom, channels inside
     dim3 ga((unsigned)((G.N + QS_WARPS - 1) / QS_WARPS), G.nb);
-    if (bin) k_forward_quads_atom<true, false><<<ga, QS_WARPS * 32, 0, st>>>(G);
-    else if (G.precise) k_forward_quads_atom<false, true><<<ga, QS_WARPS * 32, 0, st>>>(G);
-    else k_forward_quads_atom<false, false><<<ga, QS_WARPS * 32, 0, st>>>(G);
+    if (bin) launch_early(k_forward_quads_atom<true, false>, ga, QS_WARPS * 32, 0, st, G);
+    else if (G.precise) launch_early(k_forward_quads_atom<false, true>, ga, QS_WARPS * 32, 0, st, G);
+    else launch_early(k_forward_quads_atom<false, false>, ga, QS_WARPS * 32, 0, st, G);
     return cudaGetLastError();
   }
   if (G.quads && !bin && !G.precise && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0) {
     if (vec) {
       // radii by channel: one warp per atom runs the items of its weighted channels
       dim3 ga((unsigned)(((long)G.N * nz_groups(G.T) + SCAT_WARPS - 1) / SCAT_WARPS), G.nb);
-      k_forward_quads_nz<<<ga, SCAT_WARPS * 32, 0, st>>>(G);
+      launch_early(k_forward_quads_nz, ga, SCAT_WARPS * 32, 0, st, G);
       return cudaGetLastError();
     }
     dim3 gq((unsigned)((items + QS_WARPS - 1) / QS_WARPS), G.nb);
-    k_forward_quads<false><<<gq, QS_WARPS * 32, 0, st>>>(G);
+    launch_early(k_forward_quads<false>, gq, QS_WARPS * 32, 0, st, G);
     return cudaGetLastError();
   }
   if (vec) {
-    if (bin) k_forward_scatter<true, false, true><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
-    else if (G.precise) k_forward_scatter<false, true, true><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
-    else k_forward_scatter<false, false, true><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
+    if (bin) launch_early(k_forward_scatter<true, false, true>, grid, SCAT_WARPS * 32, 0, st, G);
+    else if (G.precise) launch_early(k_forward_scatter<false, true, true>, grid, SCAT_WARPS * 32, 0, st, G);
+    else launch_early(k_forward_scatter<false, false, true>, grid, SCAT_WARPS * 32, 0, st, G);
   } else {
-    if (bin) k_forward_binary<<<dim3((G.N + BIN_WARPS - 1) / BIN_WARPS, G.nb), BIN_WARPS * 32, 0, st>>>(G);
-    else if (G.precise) k_forward_scatter<false, true, false><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
-    else k_forward_scatter<false, false, false><<<grid, SCAT_WARPS * 32, 0, st>>>(G);
+    if (bin) launch_early(k_forward_binary, dim3((G.N + BIN_WARPS - 1) / BIN_WARPS, G.nb), BIN_WARPS * 32, 0, st, G);
+    else if (G.precise) launch_early(k_forward_scatter<false, true, false>, grid, SCAT_WARPS * 32, 0, st, G);
+    else launch_early(k_forward_scatter<false, false, false>, grid, SCAT_WARPS * 32, 0, st, G);
   }
   return cudaGetLastError();
 }

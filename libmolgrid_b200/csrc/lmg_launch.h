@@ -6,6 +6,31 @@
 
 namespace lmg {
 
+// Launch that may begin while the kernel before it on the stream drains: what it does before wait_for_stream()
+// overlaps with that kernel, the rest finds all earlier work done.  Every kernel launched this way calls
+// wait_for_stream() before it touches memory that others write, so that a kernel's end still means the end of all
+// before it.  Zeros, then sums, of 300 atoms in 28x48^3: 6.85 -> 5.45 us; 40 atoms in 14x24^3: 3.8 -> 3.0 us; records,
+// zeros and sums of 50 x 3000 atoms: 254 -> 248 us.
+template <class... P, class... Q>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, Q... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// lets the next launch_early() kernel of the stream begin
+__device__ __forceinline__ void let_next_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // A pass covers examples [b0, b0+nb) of the caller's batch; scratch arrays are indexed by the
 // example's position in the pass (bl = b - b0), caller arrays by b.
 // Front of the workspace: where the pass left its flags (one byte per block or warp that prepared
@@ -66,6 +91,9 @@ struct BwdArgs {
   int quads;           // rows are walked in aligned quads of four voxels when the grid allows it
 };
 
+// zeroes n floats (a multiple of four, 16-byte aligned); the next kernel may begin meanwhile.  `beside`: while the
+// kernel before it, whose results the zeros do not touch, is still at work
+cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st);
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st);
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st);
 // occupancy of index types in one launch that writes every voxel once (lmg_occupancy.cu)
@@ -74,7 +102,7 @@ cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st);
 // the forward pass of index types without k_emit: every warp prepares its own atom (density on aligned
 // grids, or occupancy; the output is zero-filled before)
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G);
-cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, cudaStream_t st);
+cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st);
 // the same for the backward passes (modes 0 and 2, aligned grids)
 bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode);
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st);

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "lmg_device.cuh"
+#include "lmg_launch.h"
 #include "lmg_misc.h"
 
 namespace lmg {
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(256) k_interpolate(InterpArgs I) {
   float* out = I.out + b * I.K * ochan + ((size_t)i * od + j) * od + k;
   const ChannelRange R(I.K);
   const InterpReads Q(C, id);
+  wait_for_stream();
 #pragma unroll 2
   for (int c = R.c0; c < R.c1; c++) __stcs(out + c * ochan, interp_direct(C, Q, I.minus_zero, in + c * ichan));
 }
@@ -398,6 +400,7 @@ __global__ void __launch_bounds__(INT + 32, LMG_INTERP_MINBLOCKS) k_interpolate_
     V[u].base = (V[u].base & 1023u) * sx + (V[u].base >> 10 & 1023u) * sy + (V[u].base >> 20);
 
   int c = R.c0;
+  wait_for_stream();
   if (tiled) {
     const int slot = (BX * BY * BZ + 31) & ~31;  // floats from box to box: 128-byte boundaries
     const int nst = min(IMAXST, IRING / slot);
@@ -518,8 +521,7 @@ cudaError_t launch_interpolate_tiled(const InterpMaps& maps, const InterpArgs& I
       if (dev >= 0 && dev < 64) opted[dev] = true;
     }
   }
-  k_interpolate_tiled<<<grid, INT + 32, smem, st>>>(maps, I);
-  return cudaGetLastError();
+  return launch_early(k_interpolate_tiled, grid, INT + 32, smem, st, maps, I);
 }
 
 cudaError_t read_tma_timeouts(unsigned* count) {
@@ -583,6 +585,7 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
       if (w != 0.f) list[m++][tid] = make_uint2(__float_as_uint(w), (i * od + j) * od + k);
     }
     n = 0;
+    wait_for_stream();
     for (int e = 0; e < m; e++) {
       const uint2 t = list[e][tid];
       const float w = __uint_as_float(t.x);
@@ -642,10 +645,8 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
   const int per = (I.K + (int)shares - 1) / (int)shares;
   const int ch = per > 16 ? 32 : per > 8 ? 16 : 8;
   const dim3 grid(tiles, nb, (I.K + ch - 1) / ch);
-  if (ch == 32) k_interpolate_gather<32><<<grid, IG_THREADS, 0, st>>>(I, W);
-  else if (ch == 16) k_interpolate_gather<16><<<grid, IG_THREADS, 0, st>>>(I, W);
-  else k_interpolate_gather<8><<<grid, IG_THREADS, 0, st>>>(I, W);
-  return cudaGetLastError();
+  return launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>, grid,
+                      IG_THREADS, 0, st, I, W);
 }
 
 cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st) {
@@ -653,8 +654,7 @@ cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st) {
   if (nv == 0 || nb == 0 || I.K == 0) return cudaSuccess;
   const unsigned od = I.out_dim, nblk = ((od + 3) / 4) * ((od + 7) / 8) * ((od + 7) / 8);
   dim3 grid(nblk, nb, channel_shares((unsigned long)nblk * nb, I.K, LMG_ID_BLOCKS));
-  k_interpolate<<<grid, 256, 0, st>>>(I);
-  return cudaGetLastError();
+  return launch_early(k_interpolate, grid, 256, 0, st, I);
 }
 
 }  // namespace lmg

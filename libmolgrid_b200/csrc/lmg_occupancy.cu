@@ -60,9 +60,10 @@ __global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float*
   const int chan = blockIdx.y, bl = blockIdx.z, b = A.b0 + bl;
   const unsigned dim = gm.dim, x0 = blockIdx.x * planes, x1 = min(x0 + planes, dim);
   const unsigned total = (x1 - x0) * dim * dim, words = (total + 31) / 32;
+  for (unsigned i = tid; i <= words; i += OCC_THREADS) bits[i] = 0;  // and one word to read beyond the last
+  wait_for_stream();
   const int n = A.n_atoms != nullptr ? min(A.N, A.n_atoms[b]) : A.N;
   const float* types = A.type_index + (size_t)b * A.N;
-  for (unsigned i = tid; i <= words; i += OCC_THREADS) bits[i] = 0;  // and one word to read beyond the last
 
   bool bad = false;
   for (int base = 0; base < n; base += OCC_CHUNK) {
@@ -190,8 +191,7 @@ cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st) {
   unsigned planes = (dim + slabs - 1) / slabs;
   if ((size_t)planes * per_plane > (size_t)OCC_WORDS * 32) planes = OCC_WORDS * 32 / per_plane;
   const size_t smem = ((size_t)planes * per_plane + 31) / 32 * 4 + 4;
-  k_occupancy<<<dim3((dim + planes - 1) / planes, A.T, A.nb), OCC_THREADS, smem, st>>>(A, out, planes);
-  return cudaGetLastError();
+  return launch_early(k_occupancy, dim3((dim + planes - 1) / planes, A.T, A.nb), OCC_THREADS, smem, st, A, out, planes);
 }
 
 }  // namespace lmg
