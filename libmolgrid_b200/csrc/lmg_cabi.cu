@@ -527,7 +527,7 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
     S.quads = g_quads;
     const size_t n = grid_elems * a->batch;
     // our own zeros where they can be written in quads: they overlap with the kernels around them
-    const bool zeros = b0 == 0 && n % 4 == 0 && (uintptr_t)out % 16 == 0;
+    const bool zeros = b0 == 0 && (uintptr_t)out % 16 == 0;
     auto clear = [&](bool beside) {
       Range r("zero fill");
       ProfRec* pr = prof_begin(2, st);

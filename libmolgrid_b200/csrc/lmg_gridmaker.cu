@@ -12,6 +12,8 @@
 #include "lmg_device.cuh"
 #include "lmg_launch.h"
 
+#include <type_traits>
+
 namespace lmg {
 
 // ---------------------------------------------------------------------------------------------
@@ -137,6 +139,9 @@ constexpr int QS_WARPS = LMG_QS_WARPS;
 #endif
 constexpr int SELF_SPLIT = LMG_SELF_SPLIT;   // most of them that four warps each take
 constexpr int SELF_ATOMS = LMG_SELF_ATOMS;   // most atom slots of a backward pass without k_emit
+// Gradients on loose rows, whose quads take longer than single voxels do: 2380 slots 12.2 -> 10.3 us, 4760 slots
+// 15.0 and 15.1, 7650 slots 20.0 and 21.5.
+constexpr int LOOSE_SELF_ATOMS = 4096;
 #ifndef LMG_FWD_SELF_ATOMS
 #define LMG_FWD_SELF_ATOMS 32768
 #endif
@@ -601,6 +606,53 @@ __device__ __forceinline__ void fill_ztabs(ZTabs& zt, unsigned zc, const ItemPar
   if ((lane & 3) == 0) zt.lo[lane >> 2] = lo;
 }
 
+// Rows of any alignment (a side that is no multiple of four, on an aligned tensor).  A column starts 0 to 3 floats
+// beyond a 16-byte boundary; its quads are the aligned ones of memory all the same, and reach up to three voxels
+// into the rows beside it, where they add zero or are not looked at.  What depends on z is tabulated once for each
+// of the four shifts.  Against lanes of one voxel, 17 x 700 atoms on 22x41^3: forward
+// 44.9 -> 39.3 us; 300 atoms on 28x41^3, forward and gradients in launches of their own: 25.9 -> 11.4.
+__device__ __forceinline__ unsigned quad_shift(unsigned chan_low, unsigned row, unsigned dim, unsigned zc) {
+  return (chan_low + row * dim + zc) & 3u;
+}
+
+struct __align__(16) LooseForward {
+  float4 dz2[QPASS], ez[QPASS];
+  float lo[QPASS], pad[8];  // 80 words: two shifts' quads lie in different banks
+};
+struct __align__(16) LooseBackward {
+  float4 dz2[QPASS], ez[QPASS], dz[QPASS];
+  float lo[QPASS], pad[8];  // 112 words
+};
+typedef LooseBackward LooseZTabs[4];
+
+// squared distances times `scale`
+template <bool SCALED, class TAB>
+__device__ __forceinline__ void fill_loose(TAB (&f)[4], unsigned zc, const ItemParams& P, float oz, float res, float kexp,
+                                           float scale, int lane) {
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+    const unsigned zz = zc - t + lane;
+    const bool in = zz >= P.loz && zz < P.hiz;  // not the places before zero either, which voxel_coord() does not take
+    const float dz = in ? __fsub_rn(voxel_coord(oz, zz, res), P.z) : 0.f;
+    float d2 = in ? __fmul_rn(dz, dz) : CUDART_NAN_F;
+    if (SCALED) d2 *= scale;
+    reinterpret_cast<float*>(f[t].dz2)[lane] = d2;
+    reinterpret_cast<float*>(f[t].ez)[lane] = ex2_approx(d2 * kexp);
+    if constexpr (std::is_same<TAB, LooseBackward>::value) reinterpret_cast<float*>(f[t].dz)[lane] = dz;
+    float lo = fminf(d2, __shfl_xor_sync(0xffffffffu, d2, 1));
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, 2));
+    if ((lane & 3) == 0) f[t].lo[lane >> 2] = lo;
+  }
+}
+
+// quads along z that a footprint spans with the widest shift
+__device__ __forceinline__ unsigned loose_span(const ItemParams& P) { return (P.hiz - P.loz + 6) >> 2; }
+
+// where the pass's examples end, counted from an example's channel
+__device__ __forceinline__ long floats_left(const BwdArgs& G, size_t chan_off, size_t dim) {
+  return (long)((size_t)(G.b0 + G.nb) * G.T * dim * dim * dim - chan_off);
+}
+
 __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
                : "memory");
@@ -649,6 +701,43 @@ __device__ __forceinline__ void qlane_sweep(const ItemParams& P, const BUF& buf,
 // SCALED: squared distances are handed to `quad` (and compared with Tcull) in units of the squared
 // atom radius, `scale` = 1 / ar^2 and `kexp` = -2 log2(e): one multiplication per column instead of
 // one per voxel for callers that want rsq / ar^2 (density only: the binary test keeps rsq itself).
+// The sweep on rows of any alignment; off may be up to three floats before the row.  (The lanes along z as a
+// variable instead of a template argument: 39.3 -> 41.4 us at the size above.)
+template <int ZQ, bool SCALED, class BUF, class QuadFn>
+__device__ __forceinline__ void loose_sweep(const BUF& buf, unsigned nkept, unsigned dim, unsigned chan_low,
+                                            const LooseForward (&tabs)[4], unsigned zc, float kexp, float Tcull, float scale,
+                                            int lane, QuadFn quad) {
+  constexpr int CPI = 32 / ZQ;
+  const int zq = lane % ZQ, cl = lane / ZQ;
+  for (unsigned c0 = 0; c0 < nkept; c0 += CPI) {
+    const unsigned i = c0 + cl;
+    if (cl >= CPI || i >= nkept) continue;
+    float dxy2 = buf.dxy2[i];
+    if (SCALED) dxy2 *= scale;
+    const unsigned row = buf.row[i], t = quad_shift(chan_low, row, dim, zc);
+    if (!(__fadd_rn(dxy2, tabs[t].lo[zq]) <= Tcull)) continue;
+    const float4 d2 = tabs[t].dz2[zq], e = tabs[t].ez[zq];
+    const float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w};
+    quad(i, dxy2, ex2_approx(dxy2 * kexp), d2v, ev, d2v, (long)((size_t)row * dim + zc + 4 * zq) - (long)t);
+  }
+}
+template <bool SCALED, class BUF, class QuadFn>
+__device__ __forceinline__ void loose_sweep_span(const ItemParams& P, const BUF& buf, unsigned nkept, unsigned dim,
+                                                 unsigned chan_low, LooseForward (&tabs)[4], float oz, float res, float kexp,
+                                                 float Tcull, float scale, int lane, QuadFn quad) {
+  const unsigned span = loose_span(P);
+  for (unsigned zc = P.loz; zc < P.hiz + 3; zc += 4 * QPASS) {
+    fill_loose<SCALED>(tabs, zc, P, oz, res, kexp, scale, lane);
+    __syncwarp();
+    if (span <= 2) loose_sweep<2, SCALED>(buf, nkept, dim, chan_low, tabs, zc, kexp, Tcull, scale, lane, quad);
+    else if (span == 3) loose_sweep<3, SCALED>(buf, nkept, dim, chan_low, tabs, zc, kexp, Tcull, scale, lane, quad);
+    else if (span == 4) loose_sweep<4, SCALED>(buf, nkept, dim, chan_low, tabs, zc, kexp, Tcull, scale, lane, quad);
+    else if (span == 5) loose_sweep<5, SCALED>(buf, nkept, dim, chan_low, tabs, zc, kexp, Tcull, scale, lane, quad);
+    else loose_sweep<8, SCALED>(buf, nkept, dim, chan_low, tabs, zc, kexp, Tcull, scale, lane, quad);
+    __syncwarp();
+  }
+}
+
 template <bool SCALED, class BUF, class QuadFn>
 __device__ __forceinline__ void qlane_sweep_span_t(unsigned span, const ItemParams& P, const BUF& buf, unsigned nkept,
                                                    size_t dim, float oz, float res, float kexp, float Tcull,
@@ -672,13 +761,24 @@ __device__ __forceinline__ unsigned quad_span(const ItemParams& P) { return (P.h
 
 // The sweep of one work item of the forward pass on aligned quads, whose constants are in P.  Of
 // `parts` warps that share an item, this one takes the `part`-th share of its columns.
-template <bool VEC>
+template <bool VEC, bool LOOSE>
 __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemParams& P, int b, float ox, float oy,
-                                                   float oz, ColBuf& buf, int lane, unsigned part = 0,
-                                                   unsigned parts = 1) {
+                                                   float oz, ColBuf& buf, LooseForward (&tabs)[4], int lane,
+                                                   unsigned part = 0, unsigned parts = 1) {
   const GMParams& gm = G.gm;
   size_t dim = gm.dim;
-  float* out = G.out_grid + ((size_t)b * G.T + P.chan) * dim * dim * dim;
+  const size_t chan_off = ((size_t)b * G.T + P.chan) * dim * dim * dim;
+  float* out = G.out_grid + chan_off;
+  const long whole = LOOSE ? floats_left(G, chan_off, dim) - 4 : 0;  // the last place of a quad
+  auto add = [&](auto off, const float (&v)[4]) {
+    if (!LOOSE || (long)off <= whole) {
+      red_add_v4(out + off, v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if ((long)off + j < whole + 4) atomicAdd(out + off + j, v[j]);
+    }
+  };
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
   const float ta = gm.ta, ntb = -gm.tb;
 
@@ -694,7 +794,7 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
     if (tail) {
       const float sg = P.Tg * P.inv_ar2, scut = P.Tcut * P.inv_ar2;
       auto quad = [&](unsigned, float dxy2, float exy, const float (&d2v)[4], const float (&ev)[4],
-                      const float (&)[4], size_t off) {
+                      const float (&)[4], auto off) {
         float v[4];
         const Pair xy = pair(dxy2), e2 = pair(exy), ta2 = pair(ta), ntb2 = pair(ntb);
 #pragma unroll
@@ -712,12 +812,15 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
             v[j + 1] *= P.w;
           }
         }
-        red_add_v4(out + off, v[0], v[1], v[2], v[3]);
+        add(off, v);
       };
-      qlane_sweep_span_t<true>(quad_span(P), P, buf, nkept, dim, oz, gm.res, NEG2_LOG2E, scut, P.inv_ar2, lane, quad);
+      if constexpr (LOOSE)
+        loose_sweep_span<true>(P, buf, nkept, gm.dim, (unsigned)chan_off, tabs, oz, gm.res, NEG2_LOG2E, scut, P.inv_ar2, lane, quad);
+      else
+        qlane_sweep_span_t<true>(quad_span(P), P, buf, nkept, dim, oz, gm.res, NEG2_LOG2E, scut, P.inv_ar2, lane, quad);
     } else {
       auto quad = [&](unsigned, float dxy2, float exy, const float (&d2v)[4], const float (&ev)[4],
-                      const float (&)[4], size_t off) {
+                      const float (&)[4], auto off) {
         float v[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -727,17 +830,21 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
           float val = rsq <= P.Tg ? exy * ev[j] : tq * tq;
           v[j] = VEC ? val * P.w : val;
         }
-        red_add_v4(out + off, v[0], v[1], v[2], v[3]);
+        add(off, v);
       };
-      qlane_sweep_span(quad_span(P), P, buf, nkept, dim, oz, gm.res, kexp, P.Tcut, lane, quad);
+      if constexpr (LOOSE)
+        loose_sweep_span<false>(P, buf, nkept, gm.dim, (unsigned)chan_off, tabs, oz, gm.res, kexp, P.Tcut, 1.f, lane, quad);
+      else
+        qlane_sweep_span(quad_span(P), P, buf, nkept, dim, oz, gm.res, kexp, P.Tcut, lane, quad);
     }
     __syncwarp();
   }
 }
 
 // One work item (an atom, or an (atom, channel) pair with VEC) of the forward pass on aligned quads.
-template <bool VEC>
-__device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, int bl, ColBuf& buf, int lane) {
+template <bool VEC, bool LOOSE>
+__device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, int bl, ColBuf& buf,
+                                                   LooseForward (&tabs)[4], int lane) {
   const GMParams& gm = G.gm;
   int b = G.b0 + bl;
   if (VEC) {
@@ -755,17 +862,18 @@ __device__ __forceinline__ void forward_quads_item(const BwdArgs& G, int item, i
   float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
   ItemParams P = load_item<VEC>(G, bl, b, item, ox, oy, oz);
   if (!P.valid || (VEC && P.w == 0.f)) return;  // zero weights add nothing (src/grid_maker.cpp:229)
-  forward_quads_core<VEC>(G, P, b, ox, oy, oz, buf, lane);
+  forward_quads_core<VEC, LOOSE>(G, P, b, ox, oy, oz, buf, tabs, lane);
 }
 
-template <bool VEC>
+template <bool VEC, bool LOOSE>
 __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads(BwdArgs G) {
   wait_for_stream();
   __shared__ ColBuf bufs[QS_WARPS];
+  __shared__ LooseForward tabs[QS_WARPS][4];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int item = blockIdx.x * QS_WARPS + wid;
   if (item >= (VEC ? G.N * G.T : G.N)) return;
-  forward_quads_item<VEC>(G, item, blockIdx.y, bufs[wid], lane);
+  forward_quads_item<VEC, LOOSE>(G, item, blockIdx.y, bufs[wid], tabs[wid], lane);
 }
 
 // Occupancy of index types: every writer stores the same 1.0, so nothing is reduced and any alignment
@@ -840,9 +948,10 @@ __global__ void __launch_bounds__(BIN_WARPS * 32) k_forward_binary(BwdArgs G) {
 // 11.6 -> 7.3 us; 64 x 1000 atoms: 234.9 -> 229.7 us; 50 x 3000: 264 -> 285 us, so densities of more than
 // FWD_SELF_ATOMS slots keep k_emit.  Occupancy, whose sweeps are a third as long, gains at every size
 // (50 x 3000: 250 -> 228 us).
-template <bool BINARY, int WARPS, bool ZEROED_BEFORE>
+template <bool BINARY, int WARPS, bool ZEROED_BEFORE, bool LOOSE>
 __global__ void __launch_bounds__(32 * WARPS) k_forward_self(EmitArgs A, BwdArgs G) {
   __shared__ ColBuf bufs[WARPS];
+  __shared__ LooseForward tabs[WARPS][4];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, a = blockIdx.x, bl = blockIdx.y, b = A.b0 + bl;
   Rec r;
   float ox, oy, oz;
@@ -852,7 +961,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_forward_self(EmitArgs A, BwdArgs
   const ItemParams P = item_of(r);
   if (!P.valid) return;
   if (BINARY) forward_binary_core(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
-  else forward_quads_core<false>(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
+  else forward_quads_core<false, LOOSE>(G, P, b, ox, oy, oz, bufs[w], tabs[w], lane, w, WARPS);
 }
 
 // Vector types whose radii differ by channel: one warp takes a group of NZ_GROUP consecutive channels
@@ -874,12 +983,13 @@ __host__ __device__ inline int nz_groups(int T) { return (T + NZ_GROUP - 1) / NZ
 __global__ void __launch_bounds__(SCAT_WARPS * 32) k_forward_quads_nz(BwdArgs G) {
   wait_for_stream();
   __shared__ ColBuf bufs[SCAT_WARPS];
+  __shared__ LooseForward tabs[SCAT_WARPS][4];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int unit = blockIdx.x * SCAT_WARPS + wid;
   if (unit >= G.N * nz_groups(G.T)) return;
   int b = G.b0 + blockIdx.y;
   LMG_FOR_EACH_WEIGHTED_CHANNEL(G, b, unit, lane, atom, t) {
-    forward_quads_item<true>(G, atom * G.T + t, blockIdx.y, bufs[wid], lane);
+    forward_quads_item<true, false>(G, atom * G.T + t, blockIdx.y, bufs[wid], tabs[wid], lane);
     __syncwarp();
   }
 }
@@ -889,12 +999,18 @@ struct BwdSums {
   float agx, agy, agz, tg;  // reduced over the warp: every lane holds the totals
 };
 
+// The quad at the end of the grids, of which `n` floats are left.
+__device__ __forceinline__ float4 last_quad(const float* p, long n) {
+  return make_float4(n > 0 ? __ldg(p) : 0.f, n > 1 ? __ldg(p + 1) : 0.f, n > 2 ? __ldg(p + 2) : 0.f, n > 3 ? __ldg(p + 3) : 0.f);
+}
+
 // The sweep of one work item whose constants are in P: sums over the item's footprint, reduced
 // over the warp.  Of `parts` warps that share an item, this one takes the `part`-th share of its columns.
-template <int MODE, bool BINARY, class BUF>
+template <int MODE, bool BINARY, class BUF, class TABS>
 __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const ItemParams& P, int b,
-                                                       float ox, float oy, float oz, BUF& buf, ZTabs& zt,
+                                                       float ox, float oy, float oz, BUF& buf, TABS& zt,
                                                        int lane, unsigned part = 0, unsigned parts = 1) {
+  constexpr bool LOOSE = !std::is_same<TABS, ZTabs>::value;
   const GMParams& gm = G.gm;
   size_t dim = gm.dim;
   size_t chan_off = ((size_t)b * G.T + P.chan) * dim * dim * dim;
@@ -914,10 +1030,118 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
   const float ta = gm.ta, ntb = -gm.tb;
   Pair az2 = pair(0.f), tg2 = pair(0.f);  // agz and tg of even and odd voxels
 
+  // one quad of a column
+  auto voxels = [&](float dxy2, float exy, float exy4, const float (&d2v)[4], const float (&ev)[4], const float (&dzv)[4],
+                    const float (&dvv)[4], const float (&dev)[4], Pair& fs2) {
+    if (MODE == 0 || MODE == 1) {
+      // -(d density / d dist) / dist * dv, src/grid_maker.cu:881-919, two voxels at a time; rsq == 0
+      // contributes nothing because dx = dy = dz = 0 there, a NaN rsq (z outside the footprint)
+      // takes the tail, which the clamp makes zero
+      const Pair xy = pair(dxy2), e4 = pair(exy4), kE2 = pair(kE), kD2 = pair(kD);
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        float r0, r1, g0, g1, t0, t1;
+        const Pair r = add2(xy, pair(d2v[j], d2v[j + 1])), e2 = pair(ev[j], ev[j + 1]);
+        split(r, r0, r1);
+        split(mul2(e4, e2), g0, g1);
+        // a neighbouring row's values, whatever they are, are not looked at
+        const float v0_ = !LOOSE || r0 <= Tcull ? dvv[j] : 0.f, v1_ = !LOOSE || r1 <= Tcull ? dvv[j + 1] : 0.f;
+        const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1)), d2 = pair(v0_, v1_);
+        split(fma2(kE2, id, kD2), t0, t1);
+        const Pair f = mul2(pair(r0 <= P.Tg ? g0 : fmaxf(t0, 0.f), r1 <= P.Tg ? g1 : fmaxf(t1, 0.f)), d2);
+        fs2 = add2(fs2, f);
+        az2 = fma2(f, pair(dzv[j], dzv[j + 1]), az2);
+        if (MODE == 1) {
+          float v0, v1;
+          if (BINARY) {
+            v0 = r0 < P.Tbin ? 1.f : 0.f;
+            v1 = r1 < P.Tbin ? 1.f : 0.f;
+          } else {
+            // the distance in radii from the reciprocal root that the gradient needs
+            float q0, q1;
+            split(fma2(pair(ta), mul2(mul2(r, id), pair(P.inv_ar)), pair(ntb)), q0, q1);
+            const Pair tq = pair(fminf(q0, 0.f), fminf(q1, 0.f));  // zero beyond the cut-off and for a NaN
+            split(mul2(tq, tq), q0, q1);
+            split(mul2(pair(exy), e2), g0, g1);
+            v0 = r0 <= P.Tg ? g0 : q0;
+            v1 = r1 <= P.Tg ? g1 : q1;
+          }
+          tg2 = fma2(pair(v0, v1), d2, tg2);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < (MODE == 2 ? 4 : 0); j++) {
+      float rsq = __fadd_rn(dxy2, d2v[j]);
+      float g = exy * ev[j];  // exp(-2 rsq / ar^2)
+      if (MODE == 2) {
+        float v;
+        if (BINARY) {
+          v = rsq < P.Tbin ? 1.f : 0.f;
+        } else {
+          v = rsq <= P.Tg ? g : tail_quotient(rsq, P.ar, P.inv_ar, gm.A, gm.B, gm.C);
+          v = rsq <= P.Tcut ? v : 0.f;  // also for a NaN
+        }
+        const float t = divide_near(__fmul_rn(dvv[j], v), dev[j]);
+        if (v > 0.f && dev[j] > 0.f) tg += t;
+      }
+    }
+  };
+
   if (P.valid) {
     for (Columns cols(P, part, parts); cols.more();) {
       const unsigned nkept = cols.compact<true>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
-      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+      if constexpr (LOOSE) {
+        // The lanes are (column, z quad), the quads of COLS columns requested at a time: a lane per column, as below,
+        // would read four different tables at a time (17 x 700 atoms on 22x41^3, relevance: 90 against 60 us).
+        constexpr int COLS = MODE == 2 ? 2 : 4;
+        const unsigned nz = min(loose_span(P), (unsigned)QPASS), cpi = 32u / nz, cl = lane / nz, zq = lane - cl * nz;
+        const long whole = floats_left(G, chan_off, dim) - 4;  // the last place of a quad
+        for (unsigned zc = P.loz; zc < P.hiz + 3; zc += 4 * QPASS) {
+          __syncwarp();
+          fill_loose<false>(zt, zc, P, oz, gm.res, kexp, 1.f, lane);
+          __syncwarp();
+          for (unsigned c0 = 0; c0 < nkept; c0 += COLS * cpi) {
+            float dxy2[COLS];
+            unsigned t[COLS];
+            float4 dv[COLS], de[COLS];
+            bool in[COLS];
+#pragma unroll
+            for (int u = 0; u < COLS; u++) {
+              const unsigned i = c0 + u * cpi + cl;
+              const bool have = cl < cpi && i < nkept;
+              const unsigned cell = have ? buf.row[i] : 0u;
+              dxy2[u] = have ? buf.dxy2[i] : CUDART_NAN_F;
+              t[u] = quad_shift((unsigned)chan_off, cell, gm.dim, zc);
+              in[u] = __fadd_rn(dxy2[u], zt[t[u]].lo[zq]) <= Tcull;  // false for a NaN
+              dv[u] = de[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              const long off = (long)((size_t)cell * dim + zc + 4 * zq) - (long)t[u];
+              if (in[u]) {
+                dv[u] = off <= whole ? __ldg(reinterpret_cast<const float4*>(diff + off)) : last_quad(diff + off, whole + 4 - off);
+                if (MODE == 2)
+                  de[u] = off <= whole ? __ldg(reinterpret_cast<const float4*>(dens + off)) : last_quad(dens + off, whole + 4 - off);
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < COLS; u++) {
+              if (!in[u]) continue;
+              const float4 d2 = zt[t[u]].dz2[zq], e = zt[t[u]].ez[zq], dz = zt[t[u]].dz[zq];
+              const float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w}, dzv[4] = {dz.x, dz.y, dz.z, dz.w};
+              const float dvv[4] = {dv[u].x, dv[u].y, dv[u].z, dv[u].w}, dev[4] = {de[u].x, de[u].y, de[u].z, de[u].w};
+              const float exy = ex2_approx(dxy2[u] * kexp);
+              Pair fs2 = pair(0.f);
+              voxels(dxy2[u], exy, k4 * exy, d2v, ev, dzv, dvv, dev, fs2);
+              if (MODE != 2) {
+                float f0, f1;
+                split(fs2, f0, f1);
+                const unsigned i = c0 + u * cpi + cl;
+                agx = fmaf(f0 + f1, buf.dx[i], agx);
+                agy = fmaf(f0 + f1, buf.dy[i], agy);
+              }
+            }
+          }
+        }
+      } else for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
         fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
         __syncwarp();
@@ -939,7 +1163,8 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
             for (int u = 0; u < 4; u++) {
               dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
               // no load where no voxel of the quad can lie inside the cut-off (false for a NaN too)
-              if (q0 + u < nq && __fadd_rn(dxy2, zt.lo[q0 + u]) <= Tcull) dv[u] = __ldg(row + q0 + u);
+              if (q0 + u < nq && __fadd_rn(dxy2, zt.lo[q0 + u]) <= Tcull)
+                dv[u] = __ldg(row + q0 + u);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -955,57 +1180,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
                     dev[0] = de.x; dev[1] = de.y; dev[2] = de.z; dev[3] = de.w;
                   }
                 }
-                if (MODE == 0 || MODE == 1) {
-                  // -(d density / d dist) / dist * dv, src/grid_maker.cu:881-919, two voxels at a time; rsq == 0
-                  // contributes nothing because dx = dy = dz = 0 there, a NaN rsq (z outside the footprint)
-                  // takes the tail, which the clamp makes zero
-                  const Pair xy = pair(dxy2), e4 = pair(exy4), kE2 = pair(kE), kD2 = pair(kD);
-#pragma unroll
-                  for (int j = 0; j < 4; j += 2) {
-                    float r0, r1, g0, g1, t0, t1;
-                    const Pair r = add2(xy, pair(d2v[j], d2v[j + 1])), e2 = pair(ev[j], ev[j + 1]);
-                    split(r, r0, r1);
-                    split(mul2(e4, e2), g0, g1);
-                    const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1)), d2 = pair(dvv[j], dvv[j + 1]);
-                    split(fma2(kE2, id, kD2), t0, t1);
-                    const Pair f = mul2(pair(r0 <= P.Tg ? g0 : fmaxf(t0, 0.f), r1 <= P.Tg ? g1 : fmaxf(t1, 0.f)), d2);
-                    fs2 = add2(fs2, f);
-                    az2 = fma2(f, pair(dzv[j], dzv[j + 1]), az2);
-                    if (MODE == 1) {
-                      float v0, v1;
-                      if (BINARY) {
-                        v0 = r0 < P.Tbin ? 1.f : 0.f;
-                        v1 = r1 < P.Tbin ? 1.f : 0.f;
-                      } else {
-                        // the distance in radii from the reciprocal root that the gradient needs
-                        float q0, q1;
-                        split(fma2(pair(ta), mul2(mul2(r, id), pair(P.inv_ar)), pair(ntb)), q0, q1);
-                        const Pair tq = pair(fminf(q0, 0.f), fminf(q1, 0.f));  // zero beyond the cut-off and for a NaN
-                        split(mul2(tq, tq), q0, q1);
-                        split(mul2(pair(exy), e2), g0, g1);
-                        v0 = r0 <= P.Tg ? g0 : q0;
-                        v1 = r1 <= P.Tg ? g1 : q1;
-                      }
-                      tg2 = fma2(pair(v0, v1), d2, tg2);
-                    }
-                  }
-                }
-#pragma unroll
-                for (int j = 0; j < (MODE == 2 ? 4 : 0); j++) {
-                  float rsq = __fadd_rn(dxy2, d2v[j]);
-                  float g = exy * ev[j];  // exp(-2 rsq / ar^2)
-                  if (MODE == 2) {
-                    float v;
-                    if (BINARY) {
-                      v = rsq < P.Tbin ? 1.f : 0.f;
-                    } else {
-                      v = rsq <= P.Tg ? g : tail_quotient(rsq, P.ar, P.inv_ar, gm.A, gm.B, gm.C);
-                      v = rsq <= P.Tcut ? v : 0.f;  // also for a NaN
-                    }
-                    const float t = divide_near(__fmul_rn(dvv[j], v), dev[j]);
-                    if (v > 0.f && dev[j] > 0.f) tg += t;
-                  }
-                }
+                voxels(dxy2, exy, exy4, d2v, ev, dzv, dvv, dev, fs2);
               }
             }
           }
@@ -1045,8 +1220,8 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
 
 // One work item (an atom, or an (atom, channel) pair for the vector modes) from its record in the
 // workspace.
-template <int MODE, bool BINARY>
-__device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, int bl, ColBufD& buf, ZTabs& zt,
+template <int MODE, bool BINARY, class TABS>
+__device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, int bl, ColBufD& buf, TABS& zt,
                                                     int lane) {
   constexpr bool VEC = MODE == 1;
   const GMParams& gm = G.gm;
@@ -1065,7 +1240,7 @@ __device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, 
   }
   float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
   ItemParams P = load_item<VEC>(G, bl, b, item, ox, oy, oz);
-  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, ox, oy, oz, buf, zt, lane);
+  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD, TABS>(G, P, b, ox, oy, oz, buf, zt, lane);
   float agx = R.agx, agy = R.agy, agz = R.agz, tg = R.tg;
   if (lane == 0) {
     size_t ai = (size_t)b * G.N + (VEC ? item / G.T : item);
@@ -1087,16 +1262,16 @@ __device__ __forceinline__ void backward_quads_item(const BwdArgs& G, int item, 
 
 // 64 registers: the most of the blocks of one warp that an SM takes.  MODE 1 waits on the L1 (89 % of its throughput: a lane per column touches 32 lines a load): 64 registers and
 // 32 resident warps instead of 72 and 28, 2.67 -> 2.58 ms at 28x96^3 (4 x 3000 atoms, 28 channels).
-template <int MODE, bool BINARY>
+template <int MODE, bool BINARY, class TABS>
 __global__ void __launch_bounds__(BWD2_WARPS * 32, 32) k_backward_quads(BwdArgs G) {
   wait_for_stream();
   constexpr bool VEC = MODE == 1;
   __shared__ ColBufD bufs[BWD2_WARPS];
-  __shared__ ZTabs ztabs[BWD2_WARPS];
+  __shared__ TABS ztabs[BWD2_WARPS];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int item = blockIdx.x * BWD2_WARPS + wid;
   if (item >= (VEC ? G.N * G.T : G.N)) return;
-  backward_quads_item<MODE, BINARY>(G, item, blockIdx.y, bufs[wid], ztabs[wid], lane);
+  backward_quads_item<MODE, BINARY, TABS>(G, item, blockIdx.y, bufs[wid], ztabs[wid], lane);
 }
 
 // Atom gradients (MODE 0) and relevance (MODE 2) of index types for inputs of at most SELF_ATOMS slots:
@@ -1104,10 +1279,10 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32, 32) k_backward_quads(BwdArgs 
 // columns, because so few atoms leave most of the chip idle and the pass lasts as long as one atom.
 // Larger inputs notice that every warp repeats the preparation (with 200 000 slots 0.230-0.316 ms
 // against 0.225 ms for k_emit and the kernel above).
-template <int MODE, bool BINARY, int WARPS>
+template <int MODE, bool BINARY, int WARPS, class TABS>
 __global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, BwdArgs G) {
   __shared__ ColBufD bufs[WARPS];
-  __shared__ ZTabs zts[WARPS];
+  __shared__ TABS zts[WARPS];
   __shared__ float4 sums[WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, a = blockIdx.x, bl = blockIdx.y, b = A.b0 + bl;
   wait_for_stream();
@@ -1116,7 +1291,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, 
   const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
   if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
   ItemParams P = item_of(r);
-  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD>(G, P, b, ox, oy, oz, bufs[w], zts[w], lane, w, WARPS);
+  BwdSums R = backward_quads_core<MODE, BINARY, ColBufD, TABS>(G, P, b, ox, oy, oz, bufs[w], zts[w], lane, w, WARPS);
   if (WARPS > 1) {
     if (lane == 0) sums[w] = make_float4(R.agx, R.agy, R.agz, R.tg);
     __syncthreads();
@@ -1147,7 +1322,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_nz(BwdArgs G
   if (unit >= G.N * nz_groups(G.T)) return;
   int b = G.b0 + blockIdx.y;
   LMG_FOR_EACH_WEIGHTED_CHANNEL(G, b, unit, lane, atom, t) {
-    backward_quads_item<MODE, BINARY>(G, atom * G.T + t, blockIdx.y, bufs[wid], ztabs[wid], lane);
+    backward_quads_item<MODE, BINARY, ZTabs>(G, atom * G.T + t, blockIdx.y, bufs[wid], ztabs[wid], lane);
     __syncwarp();
   }
 }
@@ -1928,26 +2103,35 @@ cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// tensors that quads are taken from: on 16-byte boundaries
+static bool quads_of(const BwdArgs& G, const void* p, const void* q = nullptr) {
+  return G.quads && (uintptr_t)p % 16 == 0 && (uintptr_t)q % 16 == 0;
+}
+static bool loose_rows(const BwdArgs& G) { return G.gm.dim % 4 != 0; }  // else every row is on one as well
+
 bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode) {
-  return (mode == 0 || mode == 2) && !A.vec && (long)A.nb * A.N <= (mode == 0 ? SELF_ATOMS : REL_SELF_ATOMS) && G.quads && A.gm.dim % 4 == 0 &&
-         (uintptr_t)G.diff % 16 == 0 && (mode == 0 || (uintptr_t)G.density % 16 == 0);
+  const long most = mode == 2 ? REL_SELF_ATOMS : loose_rows(G) ? LOOSE_SELF_ATOMS : SELF_ATOMS;
+  return (mode == 0 || mode == 2) && !A.vec && (long)A.nb * A.N <= most &&
+         quads_of(G, G.diff, mode == 2 ? G.density : nullptr);
 }
 
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G) {
   if (A.vec || (long)A.nb * A.N > FWD_SELF_ATOMS) return false;
-  return A.gm.binary || (G.quads && !G.precise && A.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0);
+  return A.gm.binary || (!G.precise && quads_of(G, G.out_grid));
+}
+
+template <bool BINARY, int WARPS, bool LOOSE>
+static cudaError_t forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st) {
+  const dim3 grid(A.N, A.nb);
+  if (early) return launch_early(k_forward_self<BINARY, WARPS, true, LOOSE>, grid, 32 * WARPS, 0, st, A, G);
+  k_forward_self<BINARY, WARPS, false, LOOSE><<<grid, 32 * WARPS, 0, st>>>(A, G);
+  return cudaGetLastError();
 }
 
 template <int WARPS>
 static cudaError_t forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st) {
-  const dim3 grid(A.N, A.nb);
-  if (early) {
-    return A.gm.binary ? launch_early(k_forward_self<true, WARPS, true>, grid, 32 * WARPS, 0, st, A, G)
-                       : launch_early(k_forward_self<false, WARPS, true>, grid, 32 * WARPS, 0, st, A, G);
-  }
-  if (A.gm.binary) k_forward_self<true, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(A, G);
-  else k_forward_self<false, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(A, G);
-  return cudaGetLastError();
+  if (A.gm.binary) return forward_self<true, WARPS, false>(A, G, early, st);
+  return loose_rows(G) ? forward_self<false, WARPS, true>(A, G, early, st) : forward_self<false, WARPS, false>(A, G, early, st);
 }
 
 // `early`: the launch before this one is launch_zero() of this call's output
@@ -1961,28 +2145,35 @@ cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, bool early,
 constexpr int ZERO_THREADS = 256, ZERO_QUADS = 2;
 // BESIDE: runs beside the kernel before it, which began once all earlier work was done.
 template <bool BESIDE>
-__global__ void __launch_bounds__(ZERO_THREADS) k_zero(float4* p, size_t quads) {
+__global__ void __launch_bounds__(ZERO_THREADS) k_zero(float4* p, size_t n) {
   if (!BESIDE) wait_for_stream();
   let_next_begin();  // earlier work is done: the next kernel may read what this one does not write
   const size_t i0 = (size_t)blockIdx.x * (ZERO_THREADS * ZERO_QUADS) + threadIdx.x;
 #pragma unroll
   for (int k = 0; k < ZERO_QUADS; k++)
-    if (i0 + ZERO_THREADS * k < quads) p[i0 + ZERO_THREADS * k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i0 + ZERO_THREADS * k < n / 4) p[i0 + ZERO_THREADS * k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (blockIdx.x == 0 && threadIdx.x < n % 4) reinterpret_cast<float*>(p)[n - 1 - threadIdx.x] = 0.f;
   if (BESIDE) wait_for_stream();  // this kernel is not done before the one before it
 }
 
 cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st) {
   const size_t per = (size_t)ZERO_THREADS * ZERO_QUADS;
-  const dim3 grid((unsigned)((n / 4 + per - 1) / per));
-  return launch_early(beside ? k_zero<true> : k_zero<false>, grid, ZERO_THREADS, 0, st, reinterpret_cast<float4*>(p), n / 4);
+  const dim3 grid((unsigned)(n / 4 / per + 1));
+  return launch_early(beside ? k_zero<true> : k_zero<false>, grid, ZERO_THREADS, 0, st, reinterpret_cast<float4*>(p), n);
+}
+
+template <int WARPS, class TABS>
+static void backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
+  const dim3 grid(A.N, A.nb);
+  if (mode == 0) launch_early(k_backward_quads_self<0, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
+  else if (A.gm.binary) launch_early(k_backward_quads_self<2, true, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
+  else launch_early(k_backward_quads_self<2, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
 }
 
 template <int WARPS>
 static void backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
-  const dim3 grid(A.N, A.nb);
-  if (mode == 0) launch_early(k_backward_quads_self<0, false, WARPS>, grid, 32 * WARPS, 0, st, A, G);
-  else if (A.gm.binary) launch_early(k_backward_quads_self<2, true, WARPS>, grid, 32 * WARPS, 0, st, A, G);
-  else launch_early(k_backward_quads_self<2, false, WARPS>, grid, 32 * WARPS, 0, st, A, G);
+  if (loose_rows(G)) backward_self<WARPS, LooseZTabs>(A, G, mode, st);
+  else backward_self<WARPS, ZTabs>(A, G, mode, st);
 }
 
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
@@ -1993,45 +2184,49 @@ cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, 
   return cudaGetLastError();
 }
 
+// `quads`: rows of diff (and of the density, for relevance) start on 16-byte boundaries
+template <int MODE, bool BINARY>
+static cudaError_t backward_items(const BwdArgs& G, bool quads, dim3 grid, cudaStream_t st) {
+  if (!quads) return launch_early(k_backward_warp<MODE, BINARY>, grid, BWD2_WARPS * 32, 0, st, G);
+  return launch_early(k_backward_quads<MODE, BINARY, ZTabs>, grid, BWD2_WARPS * 32, 0, st, G);
+}
+
+// Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:
+// 72.5 -> 59.8 us; 50 x 3000 on 28x41^3: 525 -> 501).  Gradients with records do not (26.9 us by single voxels, 30.0
+// by quads), nor do type vectors (4 x 1000 atoms, 28 channels of 41^3: 212 and 251 us).
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
   long items = (long)G.N * (mode == 1 ? G.T : 1);
   if (items == 0 || G.nb == 0) return cudaSuccess;
   dim3 grid((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
-  bool bin = G.gm.binary != 0;
-  // rows of diff (and of the density, for relevance) start on 16-byte boundaries
-  bool quads = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.diff % 16 == 0 &&
-               (mode != 2 || (uintptr_t)G.density % 16 == 0);
-  if (mode == 0) {
-    if (quads) launch_early(k_backward_quads<0, false>, grid, BWD2_WARPS * 32, 0, st, G);
-    else launch_early(k_backward_warp<0, false>, grid, BWD2_WARPS * 32, 0, st, G);
-  } else if (mode == 1 && quads && !G.gm.rti) {
+  const bool bin = G.gm.binary != 0, any = quads_of(G, G.diff, mode == 2 ? G.density : nullptr), loose = any && loose_rows(G);
+  const bool quads = any && !loose;
+  if (mode == 0) return backward_items<0, false>(G, quads, grid, st);
+  if (mode == 2) {
+    if (loose)
+      return bin ? launch_early(k_backward_quads<2, true, LooseZTabs>, grid, BWD2_WARPS * 32, 0, st, G)
+                 : launch_early(k_backward_quads<2, false, LooseZTabs>, grid, BWD2_WARPS * 32, 0, st, G);
+    return bin ? backward_items<2, true>(G, quads, grid, st) : backward_items<2, false>(G, quads, grid, st);
+  }
+  if (quads && !G.gm.rti) {
     // per-atom radii: one work item per atom writes both gradients, no reduction over channels after it
     dim3 ga((unsigned)((G.N + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
     dim3 gv((unsigned)((G.N + VA_WARPS - 1) / VA_WARPS), G.nb);
-    if (G.type_gradients == nullptr) launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
-    else if (bin) launch_early(k_backward_quads_atom<true>, gv, VA_WARPS * 32, 0, st, G);
-    else launch_early(k_backward_quads_atom<false>, gv, VA_WARPS * 32, 0, st, G);
-  } else if (mode == 1 && quads && G.type_gradients == nullptr) {
+    if (G.type_gradients == nullptr) return launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
+    return bin ? launch_early(k_backward_quads_atom<true>, gv, VA_WARPS * 32, 0, st, G)
+               : launch_early(k_backward_quads_atom<false>, gv, VA_WARPS * 32, 0, st, G);
+  }
+  cudaError_t e;
+  if (quads && G.type_gradients == nullptr) {
     // radii by channel, no type gradients wanted: only the weighted channels of each atom
     dim3 ga((unsigned)(((long)G.N * nz_groups(G.T) + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
-    if (bin) launch_early(k_backward_quads_nz<1, true>, ga, BWD2_WARPS * 32, 0, st, G);
-    else launch_early(k_backward_quads_nz<1, false>, ga, BWD2_WARPS * 32, 0, st, G);
-    int n = G.nb * G.N;
-    launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
-  } else if (mode == 1) {
-    if (quads && bin) launch_early(k_backward_quads<1, true>, grid, BWD2_WARPS * 32, 0, st, G);
-    else if (quads) launch_early(k_backward_quads<1, false>, grid, BWD2_WARPS * 32, 0, st, G);
-    else if (bin) launch_early(k_backward_warp<1, true>, grid, BWD2_WARPS * 32, 0, st, G);
-    else launch_early(k_backward_warp<1, false>, grid, BWD2_WARPS * 32, 0, st, G);
-    int n = G.nb * G.N;
-    launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
+    e = bin ? launch_early(k_backward_quads_nz<1, true>, ga, BWD2_WARPS * 32, 0, st, G)
+            : launch_early(k_backward_quads_nz<1, false>, ga, BWD2_WARPS * 32, 0, st, G);
   } else {
-    if (quads && bin) launch_early(k_backward_quads<2, true>, grid, BWD2_WARPS * 32, 0, st, G);
-    else if (quads) launch_early(k_backward_quads<2, false>, grid, BWD2_WARPS * 32, 0, st, G);
-    else if (bin) launch_early(k_backward_warp<2, true>, grid, BWD2_WARPS * 32, 0, st, G);
-    else launch_early(k_backward_warp<2, false>, grid, BWD2_WARPS * 32, 0, st, G);
+    e = bin ? backward_items<1, true>(G, quads, grid, st) : backward_items<1, false>(G, quads, grid, st);
   }
-  return cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int n = G.nb * G.N;
+  return launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
 }
 
 cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
@@ -2059,25 +2254,23 @@ cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st) 
   if (items == 0 || G.nb == 0) return cudaSuccess;
   dim3 grid((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb);
   bool bin = G.gm.binary != 0;
-  bool aligned = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0;
-  if (vec && !G.gm.rti && aligned) {
+  const bool quads = quads_of(G, G.out_grid), loose = loose_rows(G);
+  if (vec && !G.gm.rti && quads && !loose) {
     // per-atom radii: one work item per atom, channels inside
     dim3 ga((unsigned)((G.N + QS_WARPS - 1) / QS_WARPS), G.nb);
-    if (bin) launch_early(k_forward_quads_atom<true, false>, ga, QS_WARPS * 32, 0, st, G);
-    else if (G.precise) launch_early(k_forward_quads_atom<false, true>, ga, QS_WARPS * 32, 0, st, G);
-    else launch_early(k_forward_quads_atom<false, false>, ga, QS_WARPS * 32, 0, st, G);
-    return cudaGetLastError();
+    if (bin) return launch_early(k_forward_quads_atom<true, false>, ga, QS_WARPS * 32, 0, st, G);
+    if (G.precise) return launch_early(k_forward_quads_atom<false, true>, ga, QS_WARPS * 32, 0, st, G);
+    return launch_early(k_forward_quads_atom<false, false>, ga, QS_WARPS * 32, 0, st, G);
   }
-  if (G.quads && !bin && !G.precise && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0) {
+  if (quads && !bin && !G.precise && !(vec && loose)) {  // soft types on loose rows: 157 us by single voxels, 209 by quads
     if (vec) {
       // radii by channel: one warp per atom runs the items of its weighted channels
       dim3 ga((unsigned)(((long)G.N * nz_groups(G.T) + SCAT_WARPS - 1) / SCAT_WARPS), G.nb);
-      launch_early(k_forward_quads_nz, ga, SCAT_WARPS * 32, 0, st, G);
-      return cudaGetLastError();
+      return launch_early(k_forward_quads_nz, ga, SCAT_WARPS * 32, 0, st, G);
     }
     dim3 gq((unsigned)((items + QS_WARPS - 1) / QS_WARPS), G.nb);
-    launch_early(k_forward_quads<false>, gq, QS_WARPS * 32, 0, st, G);
-    return cudaGetLastError();
+    return loose ? launch_early(k_forward_quads<false, true>, gq, QS_WARPS * 32, 0, st, G)
+                 : launch_early(k_forward_quads<false, false>, gq, QS_WARPS * 32, 0, st, G);
   }
   if (vec) {
     if (bin) launch_early(k_forward_scatter<true, false, true>, grid, SCAT_WARPS * 32, 0, st, G);

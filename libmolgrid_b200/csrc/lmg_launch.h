@@ -91,7 +91,7 @@ struct BwdArgs {
   int quads;           // rows are walked in aligned quads of four voxels when the grid allows it
 };
 
-// zeroes n floats (a multiple of four, 16-byte aligned); the next kernel may begin meanwhile.  `beside`: while the
+// zeroes n floats (16-byte aligned); the next kernel may begin meanwhile.  `beside`: while the
 // kernel before it, whose results the zeros do not touch, is still at work
 cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st);
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st);
@@ -99,11 +99,11 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st);
 // occupancy of index types in one launch that writes every voxel once (lmg_occupancy.cu)
 bool occupancy_serves(const EmitArgs& A);
 cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st);
-// the forward pass of index types without k_emit: every warp prepares its own atom (density on aligned
-// grids, or occupancy; the output is zero-filled before)
+// the forward pass of index types without k_emit: every warp prepares its own atom (density on a 16-byte
+// aligned tensor, or occupancy; the output is zero-filled before)
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G);
 cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st);
-// the same for the backward passes (modes 0 and 2, aligned grids)
+// the same for the backward passes (modes 0 and 2, aligned tensors)
 bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode);
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st);
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st);
