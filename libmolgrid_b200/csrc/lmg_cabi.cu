@@ -260,7 +260,8 @@ lmg::InterpArgs interp_args(const lmg_interpolater* gi, int nchannels, const flo
   return I;
 }
 
-// Scratch layout of one pass over nb examples.
+// Scratch layout of a pass over at most nb examples.  All passes of a call share the layout of the first and largest:
+// its flags stay where its header says while later passes write their records.
 struct Layout {
   size_t flags, recs, chanp, partial, total;
   size_t per_example;
@@ -487,9 +488,10 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
     E.nb = std::min(per_pass, a->batch);
     if (lmg::occupancy_serves(E)) {
       Range whole("lmg_forward");
+      const Layout L = layout(g, LMG_OP_FORWARD, E.nb, a->max_atoms, a->ntypes, vec);
       for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
         E.b0 = b0; E.nb = std::min(per_pass, a->batch - b0);
-        carve(E, layout(g, LMG_OP_FORWARD, E.nb, a->max_atoms, a->ntypes, vec), ws);
+        carve(E, L, ws);
         E.round_types = 0;
         ProfRec* pr = prof_begin(0, st);
         e = lmg::launch_occupancy(E, out, st);
@@ -507,9 +509,9 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
   // tail than the overlap gains.)
   Range whole("lmg_forward");
   bool self = false;  // the same for every pass of the call
+  const Layout L = layout(g, LMG_OP_FORWARD, std::min(per_pass, a->batch), a->max_atoms, a->ntypes, vec);
   for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
     int nb = std::min(per_pass, a->batch - b0);
-    Layout L = layout(g, LMG_OP_FORWARD, nb, a->max_atoms, a->ntypes, vec);
     lmg::EmitArgs E;
     fill_emit(E, g, a);
     E.b0 = b0; E.nb = nb;
@@ -586,9 +588,9 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
     return fail(LMG_ERR_WORKSPACE, "workspace too small for one example: need " +
                                        std::to_string(STATUS_BYTES + one.per_example) + " bytes");
   bool self = false;  // the same for every pass of the call
+  const Layout L = layout(g, op, std::min(per_pass, a->batch), a->max_atoms, a->ntypes, vec);
   for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
     int nb = std::min(per_pass, a->batch - b0);
-    Layout L = layout(g, op, nb, a->max_atoms, a->ntypes, vec);
     lmg::EmitArgs E;
     fill_emit(E, g, a);
     E.b0 = b0; E.nb = nb;
@@ -701,9 +703,9 @@ int lmg_backward_gradients(const lmg_gridmaker* g, const lmg_atoms* a, const flo
                                        std::to_string(STATUS_BYTES + one.per_example) + " bytes");
   e = cudaMemsetAsync(diffdiff, 0, grid_elems * a->batch * sizeof(float), st);
   if (e != cudaSuccess) return cuda_fail(e, "zeroing output");
+  const Layout L = layout(g, LMG_OP_BACKWARD_GRADIENTS, std::min(per_pass, a->batch), a->max_atoms, a->ntypes, 1);
   for (int b0 = 0; b0 < a->batch; b0 += per_pass) {
     int nb = std::min(per_pass, a->batch - b0);
-    Layout L = layout(g, LMG_OP_BACKWARD_GRADIENTS, nb, a->max_atoms, a->ntypes, 1);
     lmg::EmitArgs E;
     fill_emit(E, g, a);
     E.b0 = b0; E.nb = nb;

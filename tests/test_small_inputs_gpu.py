@@ -146,3 +146,39 @@ def test_calls_of_one_stream_keep_their_order(B, N, P, binary):
         off = (a - b).abs() > 1e-4 * (1 + a.abs())
         assert float(off.float().mean()) <= (1e-4 if binary else 0.0)
     assert float((results[0][1] - results[1][1]).abs().max()) < 1e-4
+
+
+# flags of the first pass run past 256 bytes: 20 examples and 1, 500 and 24 of them to a pass
+@pytest.mark.parametrize("B,N,fit", [(21, 4000, 20), (524, 4000, 500)])
+def test_status_when_the_last_pass_is_small(B, N, fit):
+    """The records of a small last pass stay clear of the flags of the passes before it: valid types give no
+    error, and a bad one of the first pass is still reported after the last."""
+    import libmolgrid_b200.api as api
+    T = 2
+    g = lmg.GridMaker(1.0, 3.0)
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    coords = torch.rand((B, N, 3), device="cuda", generator=gen) * 3 - 1.5
+    good = torch.randint(T, (B, N), device="cuda", generator=gen).float()
+    radii = torch.ones((B, N), device="cuda")
+    cen = torch.zeros((B, 3), device="cuda")
+    out = torch.empty((B,) + g.grid_dimensions(T), device="cuda")
+    ag = torch.empty((B, N, 3), device="cuda")
+    old = api.MAX_WORKSPACE_BYTES
+    try:
+        api.MAX_WORKSPACE_BYTES = api._cabi.lib().lmg_workspace_bytes(g.s, 0, fit, N, T, 0)
+        api._workspaces.clear()
+        for b, a in ((None, None), (fit - 1, N - 1), (B - 1, 0)):
+            types = good.clone()
+            if b is not None:
+                types[b, a] = T
+            for call, error in ((lambda: g.forward(cen, coords, types, radii, out), IndexError),
+                                (lambda: g.backward(cen, coords, types, radii, out, ag), ValueError)):
+                call()
+                if b is None:
+                    g.check_types()
+                else:
+                    with pytest.raises(error):
+                        g.check_types()
+    finally:
+        api.MAX_WORKSPACE_BYTES = old
+        api._workspaces.clear()
