@@ -113,9 +113,24 @@ __global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float*
                        bz = __shfl_sync(0xffffffffu, O.zz, s);
         const unsigned lx = max(lo16(bxy), x0), ly = hi16(bxy), ny = hi16(hxy) - ly, ncols = (min(lo16(hxy), x1) - lx) * ny;
         const int lz = (int)lo16(bz), hz = (int)hi16(bz) - 1;
-        // what the positions of the run's ends may be off by, in voxels
-        const float eps = 1e-3f + fmaxf(fabsf(pz), fabsf(oz)) * inv * 2e-6f;
+        // What the ends of a run of half length h may be off by, in voxels: the roundings of the positions and of the
+        // root that gives them, and 1.2e-7 R^2 / h for a sphere of R voxels, because the exact test compares numbers
+        // near Tbin, each off by up to 2^-24 of it, whose difference is h^2.  Enough for h > 0.05.
+        const float eps = 1e-3f + fmaxf(fabsf(pz), fabsf(oz)) * inv * 4e-6f + Tbin * inv * inv * 3e-6f;
         const float zc = (pz - oz) * inv, inv_ny = __fdividef(1.f, small_float(ny));
+        if (!(eps < 0.25f)) {  // ends that may be off by half a voxel: voxel by voxel
+          for (unsigned c = lane; c < ncols; c += 32) {
+            const unsigned x = lx + c / ny, y = ly + c % ny;
+            const float dx = __fsub_rn(voxel_coord(ox, x, gm.res), px), dy = __fsub_rn(voxel_coord(oy, y, gm.res), py);
+            const float dxy2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+            for (int z = lz; z <= hz; z++) {
+              const float dz = __fsub_rn(voxel_coord(oz, (unsigned)z, gm.res), pz);
+              const unsigned p = ((x - x0) * dim + y) * dim + z;
+              if (__fadd_rn(dxy2, __fmul_rn(dz, dz)) < Tbin) atomicOr(&bits[p >> 5], 1u << (p & 31));
+            }
+          }
+          continue;
+        }
         for (unsigned c = lane; c < ncols; c += 32) {
           const unsigned xi = ncols < 4096u ? (unsigned)((small_float(c) + 0.5f) * inv_ny) : c / ny, x = lx + xi, y = ly + c - xi * ny;
           const float dx = __fsub_rn(voxel_coord(ox, x, gm.res), px), dy = __fsub_rn(voxel_coord(oy, y, gm.res), py);
@@ -126,7 +141,8 @@ __global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float*
             return __fadd_rn(dxy2, __fmul_rn(dz, dz)) < Tbin;
           };
           // |dz| grows away from the atom, so the voxels that pass are one run.  The root gives its ends; where
-          // one lies near a voxel, the exact test has the last word.
+          // one lies near a voxel, the exact test has the last word.  (With R left out of eps, ends are wrong from
+          // radii of 60 voxels on.)
           const float h = sqrt_approx(Tbin - dxy2) * inv, e0 = fmaxf(zc - h, -1e6f), e1 = fminf(zc + h, 1e6f);
           const float f0 = ceilf(e0), f1 = floorf(e1);
           int z0 = max(lz, (int)f0), z1 = min(hz, (int)f1);

@@ -182,3 +182,20 @@ def test_status_when_the_last_pass_is_small(B, N, fit):
     finally:
         api.MAX_WORKSPACE_BYTES = old
         api._workspaces.clear()
+
+
+def test_occupancy_of_large_spheres(port):
+    """Radii of 155 to 192 voxels, where the exact test's roundings reach further along a grazed column than the
+    positions' do: these four atoms have a column each that ends within that reach of a voxel."""
+    P, res = 401, 0.1
+    g, og = lmg.GridMaker(res, (P - 1) * res, True), port.gm(res, (P - 1) * res, True)
+    assert g.grid_dimensions(1)[1] == P
+    atoms = np.array([[-2.6152842044830322, -1.7248189449310303, 2.2062289714813232, 15.479239463806152],
+                      [0.5863897800445557, 2.7818641662597656, 1.3268423080444336, 16.368009567260742],
+                      [2.0464634895324707, -2.813606023788452, 1.333905577659607, 19.232105255126953],
+                      [-2.0822806358337402, 1.2371628284454346, 2.695906639099121, 18.976465225219727]], np.float32)
+    for a in atoms:
+        coords, types, radii = a[None, :3], np.zeros(1, np.float32), a[3:]
+        out = torch.empty(g.grid_dimensions(1), device="cuda")
+        g.forward((0.0, 0.0, 0.0), dev(coords), dev(types), dev(radii), out)
+        np.testing.assert_array_equal(out.cpu().numpy(), port.forward_index(og, (0, 0, 0), coords, types, radii, 1))
