@@ -494,9 +494,8 @@ int lmg_forward(const lmg_gridmaker* g, const lmg_atoms* a, float* out, void* wo
         carve(E, L, ws);
         E.round_types = 0;
         ProfRec* pr = prof_begin(0, st);
-        e = lmg::launch_occupancy(E, out, st);
+        e = lmg::launch_occupancy(E, out, &g_launches, st);
         prof_end(pr, st);
-        g_launches += 1;
         if (e != cudaSuccess) return cuda_fail(e, "occupancy");
       }
       return LMG_OK;

@@ -12,6 +12,7 @@
 #include "lmg_device.cuh"
 #include "lmg_launch.h"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace lmg {
@@ -952,6 +953,42 @@ __global__ void __launch_bounds__(BIN_WARPS * 32) k_forward_binary(BwdArgs G) {
   const float ox = __fsub_rn(cx, G.gm.half), oy = __fsub_rn(cy, G.gm.half), oz = __fsub_rn(cz, G.gm.half);
   const ItemParams P = load_item<false>(G, bl, b, item, ox, oy, oz);
   if (P.valid) forward_binary_core(G, P, b, ox, oy, oz, bufs[wid], lane);
+}
+
+// The listed atoms of a pass of k_occupancy, whose output is zero in their channels: a warp prepares 32 atoms, one a
+// lane, and stores their ones together (each atom prepared by the whole warp: 150 x 4000 atoms in one channel 482 us,
+// like this 298).
+__global__ void __launch_bounds__(BIN_WARPS * 32) k_occupancy_listed(EmitArgs A, BwdArgs G, OccList L) {
+  wait_for_stream();
+  __shared__ ColBuf bufs[BIN_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, bl = blockIdx.y, b = A.b0 + bl;
+  const unsigned n = L.n[bl], warps = gridDim.x * BIN_WARPS;
+  float cx, cy, cz;
+  if (A.centers != nullptr) {
+    cx = A.centers[b * 3]; cy = A.centers[b * 3 + 1]; cz = A.centers[b * 3 + 2];
+  } else {
+    cx = A.center_host[0]; cy = A.center_host[1]; cz = A.center_host[2];
+  }
+  const float ox = __fsub_rn(cx, A.gm.half), oy = __fsub_rn(cy, A.gm.half), oz = __fsub_rn(cz, A.gm.half);
+  for (unsigned i0 = blockIdx.x * BIN_WARPS + wid; i0 < n; i0 += 32 * warps) {
+    Rec own = empty_rec();
+    if (i0 + lane * warps < n) make_rec(A, b, (int)L.atom[(size_t)bl * A.N + i0 + lane * warps], own);
+    for (unsigned m = __ballot_sync(0xffffffffu, own.c.w >> 16 & REC_VALID); m != 0u; m &= m - 1u) {
+      const int k = __ffs(m) - 1;
+      Rec r = empty_rec();
+      r.a.x = __shfl_sync(0xffffffffu, own.a.x, k);
+      r.a.y = __shfl_sync(0xffffffffu, own.a.y, k);
+      r.a.z = __shfl_sync(0xffffffffu, own.a.z, k);
+      r.c.x = __shfl_sync(0xffffffffu, own.c.x, k);
+      r.c.y = __shfl_sync(0xffffffffu, own.c.y, k);
+      r.c.z = __shfl_sync(0xffffffffu, own.c.z, k);
+      r.c.w = __shfl_sync(0xffffffffu, own.c.w, k);
+      r.d.y = __shfl_sync(0xffffffffu, own.d.y, k);
+      r.d.z = __shfl_sync(0xffffffffu, own.d.z, k);
+      forward_binary_core(G, item_of(r), b, ox, oy, oz, bufs[wid], lane);
+      __syncwarp();
+    }
+  }
 }
 
 // Index types without k_emit: every warp prepares its atom itself, and WARPS warps share an atom's columns
@@ -2150,6 +2187,16 @@ static cudaError_t forward_self(const EmitArgs& A, const BwdArgs& G, bool early,
 cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, bool early, cudaStream_t st) {
   if (A.N == 0 || A.nb == 0) return cudaSuccess;
   return (long)A.nb * A.N <= SELF_SPLIT ? forward_self<4>(A, G, early, st) : forward_self<1>(A, G, early, st);
+}
+
+cudaError_t launch_occupancy_listed(const EmitArgs& A, const OccList& L, float* out, cudaStream_t st) {
+  BwdArgs G = {};
+  G.gm = A.gm;
+  G.T = A.T;
+  G.out_grid = out;
+  // what the chip holds at a time, and a few per example at least: how many atoms there are is not known here
+  const unsigned blocks = std::min((unsigned)(A.N + BIN_WARPS - 1) / BIN_WARPS, std::max(8u, (16 * 148 + (unsigned)A.nb - 1) / A.nb));
+  return launch_early(k_occupancy_listed, dim3(blocks, A.nb), BIN_WARPS * 32, 0, st, A, G, L);
 }
 
 // Bound by its stores.  Two of 16 bytes a thread: with more per thread small outputs take longer (12.4 MB: 7 us of zeros and

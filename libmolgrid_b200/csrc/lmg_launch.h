@@ -96,9 +96,17 @@ struct BwdArgs {
 cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st);
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st);
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st);
-// occupancy of index types in one launch that writes every voxel once (lmg_occupancy.cu)
+// occupancy of index types that writes every voxel once, but for channels that hold many atoms (lmg_occupancy.cu);
+// counts its launches
 bool occupancy_serves(const EmitArgs& A);
-cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st);
+cudaError_t launch_occupancy(const EmitArgs& A, float* out, long* launches, cudaStream_t st);
+// the atoms of those channels, listed by example, into a grid that is zero there (lmg_gridmaker.cu)
+struct OccList {
+  unsigned* atom;       // [nb][N]
+  unsigned* n;          // [nb]
+  unsigned char* mark;  // [nb][T]
+};
+cudaError_t launch_occupancy_listed(const EmitArgs& A, const OccList& L, float* out, cudaStream_t st);
 // the forward pass of index types without k_emit: every warp prepares its own atom (density on a 16-byte
 // aligned tensor, or occupancy; the output is zero-filled before)
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G);

@@ -3,6 +3,8 @@
 #include "lmg_device.cuh"
 #include "lmg_launch.h"
 
+#include <algorithm>
+
 namespace lmg {
 
 // ---------------------------------------------------------------------------------------------
@@ -51,7 +53,50 @@ __device__ __forceinline__ OccAtom make_occ(const EmitArgs& A, int b, int a) {
   return O;
 }
 
-__global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float* __restrict__ out, unsigned planes) {
+// Real structures put a third and more of their atoms into two or three channels, and the blocks of a channel last
+// as long as its atoms take eight warps.  Channels of more than `most` atoms in an example are marked by this kernel
+// and their atoms listed: k_occupancy writes zeros there, and the atoms are stored afterwards (launch_occupancy_listed).
+// 50 x 3000 atoms in 28 channels, evenly / a third in one / all in one: 126/213/396 us without, 132/157/181 with.
+constexpr int FULL_THREADS = 1024;  // 256: 3 us more
+__global__ void __launch_bounds__(FULL_THREADS) k_occupancy_full(EmitArgs A, OccList L, unsigned most) {
+  extern __shared__ unsigned count[];
+  __shared__ unsigned listed;
+  const int tid = threadIdx.x, bl = blockIdx.x, b = A.b0 + bl;
+  for (int t = tid; t < A.T; t += FULL_THREADS) count[t] = 0;
+  if (tid == 0) listed = 0;
+  __syncthreads();
+  wait_for_stream();
+  let_next_begin();
+  const int n = A.n_atoms != nullptr ? min(A.N, A.n_atoms[b]) : A.N;
+  const float* types = A.type_index + (size_t)b * A.N;
+  bool bad = false;
+#pragma unroll 4
+  for (int i = tid; i < n; i += FULL_THREADS) {
+    const float tc = floorf(types[i]);
+    if (tc >= (float)A.T) bad = true;
+    else if (tc >= 0.f) atomicAdd(&count[(int)tc], 1u);
+  }
+  bad = __syncthreads_or(bad && A.check_types) != 0;
+  if (tid == 0) put_flag(A, bl, A.nb, bad);
+  bool any = false;
+  for (int t = tid; t < A.T; t += FULL_THREADS) {
+    L.mark[(size_t)bl * A.T + t] = count[t] > most;
+    any = any || count[t] > most;
+  }
+  if (__syncthreads_or(any)) {
+    for (int i = tid; i < n; i += FULL_THREADS) {
+      const float tc = floorf(types[i]);
+      if (tc >= 0.f && tc < (float)A.T && count[(int)tc] > most) L.atom[(size_t)bl * A.N + atomicAdd(&listed, 1u)] = (unsigned)i;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) L.n[bl] = listed;
+}
+
+// MARKED: k_occupancy_full went before.
+template <bool MARKED>
+__global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float* __restrict__ out, unsigned planes,
+                                                              const unsigned char* mark) {
   extern __shared__ unsigned bits[];
   __shared__ unsigned short list[OCC_CHUNK];
   __shared__ unsigned listed;
@@ -62,7 +107,8 @@ __global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float*
   const unsigned total = (x1 - x0) * dim * dim, words = (total + 31) / 32;
   for (unsigned i = tid; i <= words; i += OCC_THREADS) bits[i] = 0;  // and one word to read beyond the last
   wait_for_stream();
-  const int n = A.n_atoms != nullptr ? min(A.N, A.n_atoms[b]) : A.N;
+  int n = A.n_atoms != nullptr ? min(A.N, A.n_atoms[b]) : A.N;
+  if (MARKED && mark[(size_t)bl * A.T + chan]) n = 0;
   const float* types = A.type_index + (size_t)b * A.N;
 
   bool bad = false;
@@ -170,7 +216,7 @@ __global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float*
     }
     __syncthreads();
   }
-  if (chan == 0 && blockIdx.x == 0) {  // one block per example reports types beyond the channels
+  if (!MARKED && chan == 0 && blockIdx.x == 0) {  // one block per example reports types beyond the channels
     bad = __syncthreads_or(bad) != 0;
     if (tid == 0) put_flag(A, bl, A.nb, bad);
   }
@@ -189,16 +235,25 @@ __global__ void __launch_bounds__(OCC_THREADS, 6) k_occupancy(EmitArgs A, float*
   }
 }
 
+// Most atoms of a channel that its blocks take: four times a block's share of the pass when six blocks an SM share it
+// evenly (a larger share outlasts the others), or as few as cost next to nothing.
+static long occupancy_most(const EmitArgs& A) { return std::max(128L, (long)A.nb * A.N / 222); }
+
 // Whether the pass is this kernel's.  A block looks through all of its example's types and marks its atoms
-// with eight warps, so it wants a channel per block and a chip full of such blocks (4 examples of 28 channels
-// and 4000 atoms: 26 us against 22 us for clearing and storing; 8 examples: 37 against 41), or hardly any atoms
-// (40 atoms, 28 channels: 5.2 against 5.9 us; 300 atoms: 6.4 against 6.2).
+// with eight warps, so it wants a channel per block and a chip full of such blocks, or hardly any atoms (40 atoms, 28
+// channels: 5.2 against 5.9 us; 300 atoms: 6.4 against 6.2).  Against clearing and storing, us for types spread
+// evenly / a third in one channel / all in one (channels x examples x atoms, 48^3): 28x50x3000 132/157/181 and
+// 251/223/165; 28x24x3000 81/93/98 and 128/114/83; 28x16x3000 64/73/75 and 83/73/60; 4x100x3000 149/185/179 and
+// 183/185/177; 14x50x2000 87/100/112 and 147/134/99; 14x16x3000 83/75/63 and 46; 2x100x4000 216/376/218 and 212;
+// 28x8x3000 50/54/50 and 38; and where no channel can be too full, 1x256x1000 123 and 155; 4x256x300 95/96/109 and
+// 161/157/124.
 bool occupancy_serves(const EmitArgs& A) {
-  const bool pays = (long)A.T * A.nb >= 148 || A.N <= 128;
+  const long blocks = (long)A.T * A.nb;
+  const bool pays = A.N <= 128 || blocks >= 400 || (blocks >= 222 && A.N <= occupancy_most(A));
   return pays && !A.vec && A.gm.binary && A.gm.dim * A.gm.dim <= OCC_WORDS * 32 && A.T <= 65535 && A.nb <= 65535;
 }
 
-cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st) {
+cudaError_t launch_occupancy(const EmitArgs& A, float* out, long* launches, cudaStream_t st) {
   const unsigned dim = A.gm.dim, per_plane = dim * dim;
   const long per = (long)A.T * A.nb;
   // whole channels per block for large batches, parts of them while that leaves SMs idle
@@ -207,7 +262,20 @@ cudaError_t launch_occupancy(const EmitArgs& A, float* out, cudaStream_t st) {
   unsigned planes = (dim + slabs - 1) / slabs;
   if ((size_t)planes * per_plane > (size_t)OCC_WORDS * 32) planes = OCC_WORDS * 32 / per_plane;
   const size_t smem = ((size_t)planes * per_plane + 31) / 32 * 4 + 4;
-  return launch_early(k_occupancy, dim3((dim + planes - 1) / planes, A.T, A.nb), OCC_THREADS, smem, st, A, out, planes);
+  const dim3 grid((dim + planes - 1) / planes, A.T, A.nb);
+  const long most = occupancy_most(A);
+  // marks and lists lie where other passes keep their records
+  const bool marked = A.N > most + most / 4 && A.T <= 8192 && 4 + 4 * (size_t)A.N + A.T <= A.N * sizeof(Rec);
+  *launches += marked ? 3 : 1;
+  if (!marked) return launch_early(k_occupancy<false>, grid, OCC_THREADS, smem, st, A, out, planes, (const unsigned char*)nullptr);
+  OccList L;
+  L.atom = reinterpret_cast<unsigned*>(A.recs);
+  L.n = L.atom + (size_t)A.nb * A.N;
+  L.mark = reinterpret_cast<unsigned char*>(L.n + A.nb);
+  cudaError_t e = launch_early(k_occupancy_full, dim3(A.nb), FULL_THREADS, A.T * sizeof(unsigned), st, A, L, (unsigned)most);
+  if (e != cudaSuccess) return e;
+  e = launch_early(k_occupancy<true>, grid, OCC_THREADS, smem, st, A, out, planes, (const unsigned char*)L.mark);
+  return e != cudaSuccess ? e : launch_occupancy_listed(A, L, out, st);
 }
 
 }  // namespace lmg

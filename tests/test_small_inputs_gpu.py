@@ -199,3 +199,42 @@ def test_occupancy_of_large_spheres(port):
         out = torch.empty(g.grid_dimensions(1), device="cuda")
         g.forward((0.0, 0.0, 0.0), dev(coords), dev(types), dev(radii), out)
         np.testing.assert_array_equal(out.cpu().numpy(), port.forward_index(og, (0, 0, 0), coords, types, radii, 1))
+
+
+@pytest.mark.parametrize("full", [127, 128, 129, 400])
+@pytest.mark.parametrize("passes", [False, True])
+def test_occupancy_with_full_channels(port, full, passes):
+    """Channels with more atoms than their blocks take (128 for passes this small), beside others that have few or
+    none, in batches that run at once or in passes, with types beyond the channels and below them."""
+    import libmolgrid_b200.api as api
+    B, N, T, P = 40, 420, 9, 12
+    g, og = lmg.GridMaker(0.5, (P - 1) * 0.5, True), port.gm(0.5, (P - 1) * 0.5, True)
+    ex = [cases.index_case(31 * b + full, N, T, 4.0) for b in range(B)]
+    coords, types, radii = (np.stack([e[k] for e in ex]) for k in range(3))
+    types = np.where(types == 3, 4, types)
+    for b in range(0, B, 3):
+        where = np.random.default_rng(b).permutation(N - 15)
+        types[b] = np.where(types[b] == 7, 8, types[b])
+        types[b, where[:full]] = 7
+    types[:, N - 15] = -1.0
+    ns = np.full(B, N, np.int32)
+    ns[1:] -= np.arange(B - 1, dtype=np.int32) % 5
+    out = torch.full((B,) + g.grid_dimensions(T), 7.0, device="cuda")
+    old = api.MAX_WORKSPACE_BYTES
+    try:
+        if passes:
+            api.MAX_WORKSPACE_BYTES = api._cabi.lib().lmg_workspace_bytes(g.s, 0, 17, N, T, 0)
+            api._workspaces.clear()
+        args = (torch.zeros((B, 3), device="cuda"), dev(coords), dev(types), dev(radii), out)
+        g.forward(*args, n_atoms=dev(ns))
+        g.check_types()
+        for b in range(B):
+            want = port.forward_index(og, (0, 0, 0), coords[b][:ns[b]], types[b][:ns[b]], radii[b][:ns[b]], T)
+            np.testing.assert_array_equal(out[b].cpu().numpy(), want)
+        types[B - 1, 0] = T
+        g.forward(args[0], args[1], dev(types), args[3], out, n_atoms=dev(ns))
+        with pytest.raises(IndexError):
+            g.check_types()
+    finally:
+        api.MAX_WORKSPACE_BYTES = old
+        api._workspaces.clear()
