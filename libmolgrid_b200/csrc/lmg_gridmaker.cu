@@ -1418,12 +1418,14 @@ struct SecondConst {
 };
 
 // density, s and alpha at two voxels; all zero beyond the cut-off and for a NaN distance (z outside the
-// footprint)
+// footprint), which `in0` and `in1` tell for products with values that need not be finite
 __device__ __forceinline__ void second_factors(const SecondConst& K, const ItemParams& P, Pair rsq, Pair g, Pair& val, Pair& s,
-                                               Pair& alpha) {
+                                               Pair& alpha, bool& in0, bool& in1) {
   float r0, r1, a0, a1, b0, b1;
   split(rsq, r0, r1);
-  const bool gauss0 = r0 <= P.Tg, gauss1 = r1 <= P.Tg, in0 = r0 <= P.Tcut, in1 = r1 <= P.Tcut;
+  const bool gauss0 = r0 <= P.Tg, gauss1 = r1 <= P.Tg;
+  in0 = r0 <= P.Tcut;
+  in1 = r1 <= P.Tcut;
   const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1));
   float g0, g1;
   split(g, g0, g1);
@@ -1438,6 +1440,23 @@ __device__ __forceinline__ void second_factors(const SecondConst& K, const ItemP
   split(mul2(K.c4, sg), g0, g1);
   split(mul2(kid, mul2(id, id)), b0, b1);
   alpha = pair(gauss0 ? g0 : in0 ? b0 : 0.f, gauss1 ? g1 : in1 ? b1 : 0.f);
+}
+
+// The values at two voxels, zero where `in0`, `in1` are false.
+__device__ __forceinline__ Pair only(Pair v, bool in0, bool in1) {
+  float a, b;
+  split(v, a, b);
+  return pair(in0 ? a : 0.f, in1 ? b : 0.f);
+}
+// s * (delta . atom_gradient) at two voxels for an atom gradient that is not finite: nothing beyond the cut-off
+// nor on the atom itself.
+__device__ __forceinline__ Pair only_off_atom(Pair sd, Pair rsq, bool in0, bool in1) {
+  float r0, r1;
+  split(rsq, r0, r1);
+  return only(sd, in0 && r0 > 0.f, in1 && r1 > 0.f);
+}
+__device__ __forceinline__ bool finite3(float x, float y, float z) {
+  return fabsf(x) < CUDART_INF_F && fabsf(y) < CUDART_INF_F && fabsf(z) < CUDART_INF_F;
 }
 
 // What the atom term keeps over an item's voxels: sums over pairs of voxels of one column, then over columns.
@@ -1464,70 +1483,83 @@ __device__ __forceinline__ void second_quads_item(const BwdArgs& G, int item, in
     const float kexp = P.inv_ar2 * NEG2_LOG2E;
     const SecondConst K(gm, P);
     const Pair winz = pair(P.w * inz), tg2 = pair(intg);
+    const bool odd = !finite3(P.w * inx, P.w * iny, P.w * inz) || !finite3(intg, 0.f, 0.f);  // the same for every lane
     Pair sb = pair(0.f);  // sum of diff * s
-    for (Columns cols(P); cols.more();) {
-      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
-      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
-        __syncwarp();
-        fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
-        __syncwarp();
-        const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
-        for (unsigned c0 = 0; c0 < nkept; c0 += 32 / SO_ZL) {
-          const unsigned i = c0 + lane / SO_ZL;
-          const bool have = i < nkept;
-          const float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F, dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
-          const size_t off = chan + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
-          const float4* row = reinterpret_cast<const float4*>(G.diff + off);
-          float* out = G.out_grid + off;
-          const Pair xy = pair(dxy2), exy = pair(ex2_approx(dxy2 * kexp));
-          const float dotxy = fmaf(dx, inx, dy * iny);
-          const Pair wdot = pair(P.w * dotxy);
-          SecondColumn C = {pair(0.f), pair(0.f), pair(0.f)};
-          for (unsigned q0 = lane % SO_ZL; q0 < nq; q0 += 4 * SO_ZL) {
-            float4 dv[4];
-            unsigned live = 0;
+    auto sweep = [&](auto odd) {
+      for (Columns cols(P); cols.more();) {
+        const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
+        for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+          __syncwarp();
+          fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
+          __syncwarp();
+          const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+          for (unsigned c0 = 0; c0 < nkept; c0 += 32 / SO_ZL) {
+            const unsigned i = c0 + lane / SO_ZL;
+            const bool have = i < nkept;
+            const float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F, dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
+            const size_t off = chan + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
+            const float4* row = reinterpret_cast<const float4*>(G.diff + off);
+            float* out = G.out_grid + off;
+            const Pair xy = pair(dxy2), exy = pair(ex2_approx(dxy2 * kexp));
+            const float dotxy = fmaf(dx, inx, dy * iny);
+            const Pair wdot = pair(P.w * dotxy);
+            SecondColumn C = {pair(0.f), pair(0.f), pair(0.f)};
+            for (unsigned q0 = lane % SO_ZL; q0 < nq; q0 += 4 * SO_ZL) {
+              float4 dv[4];
+              unsigned live = 0;
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-              dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (q0 + SO_ZL * u < nq && __fadd_rn(dxy2, zt.lo[q0 + SO_ZL * u]) <= P.Tcut) {
-                live |= 1u << u;
-                dv[u] = __ldg(row + q0 + SO_ZL * u);
+              for (int u = 0; u < 4; u++) {
+                dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (q0 + SO_ZL * u < nq && __fadd_rn(dxy2, zt.lo[q0 + SO_ZL * u]) <= P.Tcut) {
+                  live |= 1u << u;
+                  dv[u] = __ldg(row + q0 + SO_ZL * u);
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                if (!(live >> u & 1u)) continue;
+                const float4 d2 = zt.dz2[q0 + SO_ZL * u], e = zt.ez[q0 + SO_ZL * u], dz = zt.dz[q0 + SO_ZL * u];
+                const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
+                           dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)};
+                Pair dvp[2] = {pair(dv[u].x, dv[u].y), pair(dv[u].z, dv[u].w)};
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                  Pair val, s, alpha;
+                  bool in0, in1;
+                  const Pair rsq = add2(xy, d2p[j]);
+                  second_factors(K, P, rsq, mul2(exy, ep[j]), val, s, alpha, in0, in1);
+                  Pair sd = mul2(s, fma2(dzp[j], winz, wdot));
+                  if constexpr (odd.value) sd = only_off_atom(sd, rsq, in0, in1);
+                  Pair out2 = fma2(val, tg2, sd);
+                  if constexpr (odd.value) out2 = only(out2, in0, in1);
+                  split(out2, v[2 * j], v[2 * j + 1]);
+                  dvp[j] = only(dvp[j], in0, in1);  // a neighbour's value may be anything
+                  const Pair t0 = mul2(dvp[j], alpha), t1 = mul2(t0, dzp[j]);
+                  C.a0 = add2(C.a0, t0);
+                  C.a1 = add2(C.a1, t1);
+                  C.a2 = fma2(t1, dzp[j], C.a2);
+                  sb = fma2(dvp[j], s, sb);
+                }
+                red_add_v4(out + 4 * (q0 + SO_ZL * u), v[0], v[1], v[2], v[3]);
               }
             }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-              if (!(live >> u & 1u)) continue;
-              const float4 d2 = zt.dz2[q0 + SO_ZL * u], e = zt.ez[q0 + SO_ZL * u], dz = zt.dz[q0 + SO_ZL * u];
-              const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
-                         dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)}, dvp[2] = {pair(dv[u].x, dv[u].y), pair(dv[u].z, dv[u].w)};
-              float v[4];
-#pragma unroll
-              for (int j = 0; j < 2; j++) {
-                Pair val, s, alpha;
-                second_factors(K, P, add2(xy, d2p[j]), mul2(exy, ep[j]), val, s, alpha);
-                split(fma2(val, tg2, mul2(s, fma2(dzp[j], winz, wdot))), v[2 * j], v[2 * j + 1]);
-                const Pair t0 = mul2(dvp[j], alpha), t1 = mul2(t0, dzp[j]);
-                C.a0 = add2(C.a0, t0);
-                C.a1 = add2(C.a1, t1);
-                C.a2 = fma2(t1, dzp[j], C.a2);
-                sb = fma2(dvp[j], s, sb);
-              }
-              red_add_v4(out + 4 * (q0 + SO_ZL * u), v[0], v[1], v[2], v[3]);
-            }
+            // sum over the column of diff * (w*alpha*dot*delta_c + intg*alpha*delta_c^2), dot = dotxy + dz*inz
+            float a0, a1, a2, t;
+            split(C.a0, a0, t); a0 += t;
+            split(C.a1, a1, t); a1 += t;
+            split(C.a2, a2, t); a2 += t;
+            const float wd = P.w * fmaf(dotxy, a0, inz * a1);
+            agx = fmaf(dx, fmaf(intg * dx, a0, wd), agx);
+            agy = fmaf(dy, fmaf(intg * dy, a0, wd), agy);
+            agz += fmaf(P.w, fmaf(dotxy, a1, inz * a2), intg * a2);
           }
-          // sum over the column of diff * (w*alpha*dot*delta_c + intg*alpha*delta_c^2), dot = dotxy + dz*inz
-          float a0, a1, a2, t;
-          split(C.a0, a0, t); a0 += t;
-          split(C.a1, a1, t); a1 += t;
-          split(C.a2, a2, t); a2 += t;
-          const float wd = P.w * fmaf(dotxy, a0, inz * a1);
-          agx = fmaf(dx, fmaf(intg * dx, a0, wd), agx);
-          agy = fmaf(dy, fmaf(intg * dy, a0, wd), agy);
-          agz += fmaf(P.w, fmaf(dotxy, a1, inz * a2), intg * a2);
         }
+        __syncwarp();
       }
-      __syncwarp();
-    }
+    };
+    if (odd) sweep(std::true_type());
+    else sweep(std::false_type());
     // the isotropic part: -diff * s * (w*in_c + intg), the same factor for every voxel of the item
     float s0, s1;
     split(sb, s0, s1);
@@ -2019,6 +2051,7 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
   const float* wrow = G.type_vector + ai * G.T;
   const float* grow = G.tg_in + ai * G.T;
   const float inx = G.ag_in[ai * 3], iny = G.ag_in[ai * 3 + 1], inz = G.ag_in[ai * 3 + 2];
+  const bool odd = !finite3(inx, iny, inz);  // the same for every lane
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
   const SecondConst K(gm, P);
   float agx = 0.f, agy = 0.f, agz = 0.f;
@@ -2037,74 +2070,86 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
     }
     __syncwarp();
     Pair sb1 = pair(0.f), sb2 = pair(0.f);  // sums of s * S1 and s * S2
-    for (Columns cols(P); cols.more();) {
-      const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
-      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
-        __syncwarp();
-        fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
-        __syncwarp();
-        const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
-        for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
-          const unsigned i = c0 + lane;
-          const bool have = i < nkept;
-          const float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F, dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
-          const size_t off = base + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
-          const Pair xy = pair(dxy2), exy = pair(ex2_approx(dxy2 * kexp));
-          const float dotxy = fmaf(dx, inx, dy * iny);
-          // sums over the column: alpha * S2 * {1, dz^2}, alpha * (delta . agrad) * S1 * {1, dz}
-          Pair p0 = pair(0.f), p2 = pair(0.f), u0 = pair(0.f), u1 = pair(0.f);
-          for (unsigned q = 0; q < nq; q++) {
-            if (!(__fadd_rn(dxy2, zt.lo[q]) <= P.Tcut)) continue;
-            const float4 d2 = zt.dz2[q], e = zt.ez[q], dz = zt.dz[q];
-            const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
-                       dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)};
-            Pair val[2], s[2], sd[2], alpha[2], dot[2], s1[2], s2[2];
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-              second_factors(K, P, add2(xy, d2p[j]), mul2(exy, ep[j]), val[j], s[j], alpha[j]);
-              dot[j] = fma2(dzp[j], pair(inz), pair(dotxy));
-              sd[j] = mul2(s[j], dot[j]);
-              s1[j] = s2[j] = pair(0.f);
-            }
-            const float* src = G.diff + off + 4 * q;
-            float* dst = G.out_grid + off + 4 * q;
-            for (int k = 0; k < nnz; k++) {
-              const float2 wg = nz_wg[wid][k];
-              const size_t co = (size_t)nz_t[wid][k] * cs;
-              const float4 dv = __ldg(reinterpret_cast<const float4*>(src + co));
-              const Pair dvp[2] = {pair(dv.x, dv.y), pair(dv.z, dv.w)}, wk = pair(wg.x), gk = pair(wg.y);
-              float v[4];
+    auto sweep = [&](auto odd) {
+      for (Columns cols(P); cols.more();) {
+        const unsigned nkept = cols.compact<true>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
+        for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+          __syncwarp();
+          fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
+          __syncwarp();
+          const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+          for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
+            const unsigned i = c0 + lane;
+            const bool have = i < nkept;
+            const float dxy2 = have ? buf.dxy2[i] : CUDART_NAN_F, dx = have ? buf.dx[i] : 0.f, dy = have ? buf.dy[i] : 0.f;
+            const size_t off = base + (size_t)(have ? buf.row[i] : 0u) * dim + zc;
+            const Pair xy = pair(dxy2), exy = pair(ex2_approx(dxy2 * kexp));
+            const float dotxy = fmaf(dx, inx, dy * iny);
+            // sums over the column: alpha * S2 * {1, dz^2}, alpha * (delta . agrad) * S1 * {1, dz}
+            Pair p0 = pair(0.f), p2 = pair(0.f), u0 = pair(0.f), u1 = pair(0.f);
+            for (unsigned q = 0; q < nq; q++) {
+              if (!(__fadd_rn(dxy2, zt.lo[q]) <= P.Tcut)) continue;
+              const float4 d2 = zt.dz2[q], e = zt.ez[q], dz = zt.dz[q];
+              const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
+                         dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)};
+              Pair val[2], s[2], sd[2], alpha[2], dot[2], s1[2], s2[2];
+              bool in[4];
 #pragma unroll
               for (int j = 0; j < 2; j++) {
-                s1[j] = fma2(wk, dvp[j], s1[j]);
-                s2[j] = fma2(gk, dvp[j], s2[j]);
-                split(fma2(val[j], gk, mul2(sd[j], wk)), v[2 * j], v[2 * j + 1]);
+                const Pair rsq = add2(xy, d2p[j]);
+                second_factors(K, P, rsq, mul2(exy, ep[j]), val[j], s[j], alpha[j], in[2 * j], in[2 * j + 1]);
+                dot[j] = fma2(dzp[j], pair(inz), pair(dotxy));
+                sd[j] = mul2(s[j], dot[j]);
+                if constexpr (odd.value) {
+                  sd[j] = only_off_atom(sd[j], rsq, in[2 * j], in[2 * j + 1]);
+                  dot[j] = only(dot[j], in[2 * j], in[2 * j + 1]);
+                }
+                s1[j] = s2[j] = pair(0.f);
               }
-              red_add_v4(dst + co, v[0], v[1], v[2], v[3]);
-            }
+              const float* src = G.diff + off + 4 * q;
+              float* dst = G.out_grid + off + 4 * q;
+              for (int k = 0; k < nnz; k++) {
+                const float2 wg = nz_wg[wid][k];
+                const size_t co = (size_t)nz_t[wid][k] * cs;
+                const float4 dv = __ldg(reinterpret_cast<const float4*>(src + co));
+                const Pair dvp[2] = {pair(dv.x, dv.y), pair(dv.z, dv.w)}, wk = pair(wg.x), gk = pair(wg.y);
+                float v[4];
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-              const Pair a2 = mul2(alpha[j], s2[j]), a1 = mul2(mul2(alpha[j], dot[j]), s1[j]);
-              p0 = add2(p0, a2);
-              p2 = fma2(a2, mul2(dzp[j], dzp[j]), p2);
-              u0 = add2(u0, a1);
-              u1 = fma2(a1, dzp[j], u1);
-              sb1 = fma2(s[j], s1[j], sb1);
-              sb2 = fma2(s[j], s2[j], sb2);
+                for (int j = 0; j < 2; j++) {
+                  s1[j] = fma2(wk, dvp[j], s1[j]);
+                  s2[j] = fma2(gk, dvp[j], s2[j]);
+                  split(fma2(val[j], gk, mul2(sd[j], wk)), v[2 * j], v[2 * j + 1]);
+                }
+                red_add_v4(dst + co, v[0], v[1], v[2], v[3]);
+              }
+#pragma unroll
+              for (int j = 0; j < 2; j++) {
+                s1[j] = only(s1[j], in[2 * j], in[2 * j + 1]);  // a neighbour's values may be anything
+                s2[j] = only(s2[j], in[2 * j], in[2 * j + 1]);
+                const Pair a2 = mul2(alpha[j], s2[j]), a1 = mul2(mul2(alpha[j], dot[j]), s1[j]);
+                p0 = add2(p0, a2);
+                p2 = fma2(a2, mul2(dzp[j], dzp[j]), p2);
+                u0 = add2(u0, a1);
+                u1 = fma2(a1, dzp[j], u1);
+                sb1 = fma2(s[j], s1[j], sb1);
+                sb2 = fma2(s[j], s2[j], sb2);
+              }
             }
+            float a, b0, c, d, t0;
+            split(p0, a, t0); a += t0;
+            split(p2, b0, t0); b0 += t0;
+            split(u0, c, t0); c += t0;
+            split(u1, d, t0); d += t0;
+            agx = fmaf(dx, fmaf(a, dx, c), agx);
+            agy = fmaf(dy, fmaf(a, dy, c), agy);
+            agz += b0 + d;
           }
-          float a, b0, c, d, t0;
-          split(p0, a, t0); a += t0;
-          split(p2, b0, t0); b0 += t0;
-          split(u0, c, t0); c += t0;
-          split(u1, d, t0); d += t0;
-          agx = fmaf(dx, fmaf(a, dx, c), agx);
-          agy = fmaf(dy, fmaf(a, dy, c), agy);
-          agz += b0 + d;
         }
+        __syncwarp();
       }
-      __syncwarp();
-    }
+    };
+    if (odd) sweep(std::true_type());
+    else sweep(std::false_type());
     float x0, x1, y0, y1;
     split(sb1, x0, x1);
     split(sb2, y0, y1);

@@ -38,3 +38,44 @@ def test_both_terms(port, res, points, T, rti):
     for got, w in zip((dd, add, tdd), want):
         scale = max(1.0, float(np.abs(w).max()))
         np.testing.assert_allclose(got.cpu().numpy(), w, rtol=1e-4, atol=1e-5 * scale)
+
+
+def beyond(coords, radii, res, points, channels):
+    """[atom, channel] voxels that the atom's density does not reach, of a multiple of 1 (cut-off 1.5 radii)."""
+    ax = torch.arange(points, dtype=torch.float64) * res - (points - 1) * res / 2
+    x = torch.stack(torch.meshgrid(ax, ax, ax, indexing="ij"), -1)
+    d = torch.stack([(x - torch.tensor(c, dtype=torch.float64)).norm(dim=-1) for c in coords])
+    if len(radii) == channels:   # by type
+        return torch.stack([(d > 1.5 * float(r) * 1.0001) for r in radii], 1)
+    return torch.stack([(d[a] > 1.5 * float(radii[a]) * 1.0001) for a in range(len(coords))])[:, None].expand(-1, channels, -1, -1, -1)
+
+
+# sweeps of quads per (atom, channel) and per atom, and single voxels; values that are not finite next to a footprint
+@pytest.mark.parametrize("points", [24, 13])
+@pytest.mark.parametrize("rti", [False, True])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_values_beyond_the_cut_off_do_not_matter(points, rti, bad):
+    N, T, res = 5, 7, 0.5
+    coords, tv, radii = cases.vector_case(points + rti, N, T, points * res / 4, rti=rti)
+    tv = np.maximum(tv, 0.05).astype(np.float32)
+    out = beyond(coords, radii, res, points, T)
+    g = lmg.GridMaker(res, (points - 1) * res, False, rti)
+    rng = np.random.default_rng(7)
+    diff = torch.from_numpy(rng.normal(size=(T,) + (points,) * 3).astype(np.float32))
+    ag, tg = (torch.from_numpy(rng.normal(size=s).astype(np.float32)).cuda() for s in ((N, 3), (N, T)))
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    def run(diff, ag):
+        dd, add, tdd = (torch.full(x.shape, 7.0, device="cuda") for x in (diff, ag, tg))
+        g.backward_gradients((0, 0, 0), d(coords), d(tv), d(radii), diff.cuda(), ag, tg, dd, add, tdd)
+        return dd.cpu(), add.cpu()
+
+    free = out.all(0)   # voxels that no atom reaches
+    assert bool(free.any()) and not bool(free.all())
+    ok, want = run(torch.where(free, 0.0, diff), ag)
+    _, got = run(torch.where(free, bad, diff), ag)
+    assert bool(torch.isfinite(got).all()) and torch.equal(got, want)
+    wild = ag.clone()
+    wild[2] = bad       # and an atom's gradient where the atom does not reach
+    dd, _ = run(diff, wild)
+    assert bool(torch.isfinite(dd[out[2]]).all()) and torch.allclose(dd[out[2]], ok[out[2]], rtol=1e-5, atol=1e-5)
