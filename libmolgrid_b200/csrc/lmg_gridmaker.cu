@@ -1405,7 +1405,7 @@ constexpr int SO_ZL = 2;
 constexpr int SO_MINB = 16, SO_ATOM_MINB = 26;  // resident blocks: 114 and 72 registers
 
 struct SecondConst {
-  Pair k4, c4, kE, kD, ta, ntb, inv_ar;
+  Pair k4, c4, kE, kD, ta, ntb, inv_ar, inv_ar2;
   __device__ __forceinline__ SecondConst(const GMParams& gm, const ItemParams& P) {
     const bool tail = gm.ta != 0.f || gm.tb != 0.f;
     k4 = c4 = pair(4.f * P.inv_ar2);
@@ -1414,11 +1414,16 @@ struct SecondConst {
     ta = pair(gm.ta);
     ntb = pair(-gm.tb);
     inv_ar = pair(P.inv_ar);
+    inv_ar2 = pair(P.inv_ar2);
   }
 };
 
 // density, s and alpha at two voxels; all zero beyond the cut-off and for a NaN distance (z outside the
-// footprint), which `in0` and `in1` tell for products with values that need not be finite
+// footprint), which `in0` and `in1` tell for products with values that need not be finite.  OWN_ROOT: the density
+// from a root of its own and s in one rounding, instead of both from the reciprocal root and the product that alpha
+// needs.  With radii by atom the grid term is else 6 % further from 64 bits than it was as a sweep of its own (1.85e-7,
+// 1.75e-7 like this); with radii by type it is as near either way, and 2 % of the time less without.
+template <bool OWN_ROOT>
 __device__ __forceinline__ void second_factors(const SecondConst& K, const ItemParams& P, Pair rsq, Pair g, Pair& val, Pair& s,
                                                Pair& alpha, bool& in0, bool& in1) {
   float r0, r1, a0, a1, b0, b1;
@@ -1429,13 +1434,20 @@ __device__ __forceinline__ void second_factors(const SecondConst& K, const ItemP
   const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1));
   float g0, g1;
   split(g, g0, g1);
-  split(fma2(K.ta, mul2(mul2(rsq, id), K.inv_ar), K.ntb), a0, a1);
+  Pair dr;
+  if (OWN_ROOT) {
+    split(mul2(rsq, K.inv_ar2), a0, a1);
+    dr = pair(sqrt_approx(a0), sqrt_approx(a1));
+  } else {
+    dr = mul2(mul2(rsq, id), K.inv_ar);
+  }
+  split(fma2(K.ta, dr, K.ntb), a0, a1);
   const Pair tq = pair(fminf(a0, 0.f), fminf(a1, 0.f));
   split(mul2(tq, tq), a0, a1);
   val = pair(gauss0 ? g0 : a0, gauss1 ? g1 : a1);
   const Pair sg = mul2(K.k4, g), kid = mul2(K.kE, id);
   split(sg, g0, g1);
-  split(add2(kid, K.kD), a0, a1);
+  split(OWN_ROOT ? fma2(K.kE, id, K.kD) : add2(kid, K.kD), a0, a1);
   s = pair(gauss0 ? g0 : fmaxf(a0, 0.f), gauss1 ? g1 : fmaxf(a1, 0.f));
   split(mul2(K.c4, sg), g0, g1);
   split(mul2(kid, mul2(id, id)), b0, b1);
@@ -1528,7 +1540,7 @@ __device__ __forceinline__ void second_quads_item(const BwdArgs& G, int item, in
                   Pair val, s, alpha;
                   bool in0, in1;
                   const Pair rsq = add2(xy, d2p[j]);
-                  second_factors(K, P, rsq, mul2(exy, ep[j]), val, s, alpha, in0, in1);
+                  second_factors<false>(K, P, rsq, mul2(exy, ep[j]), val, s, alpha, in0, in1);
                   Pair sd = mul2(s, fma2(dzp[j], winz, wdot));
                   if constexpr (odd.value) sd = only_off_atom(sd, rsq, in0, in1);
                   Pair out2 = fma2(val, tg2, sd);
@@ -2097,7 +2109,7 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
 #pragma unroll
               for (int j = 0; j < 2; j++) {
                 const Pair rsq = add2(xy, d2p[j]);
-                second_factors(K, P, rsq, mul2(exy, ep[j]), val[j], s[j], alpha[j], in[2 * j], in[2 * j + 1]);
+                second_factors<true>(K, P, rsq, mul2(exy, ep[j]), val[j], s[j], alpha[j], in[2 * j], in[2 * j + 1]);
                 dot[j] = fma2(dzp[j], pair(inz), pair(dotxy));
                 sd[j] = mul2(s[j], dot[j]);
                 if constexpr (odd.value) {
