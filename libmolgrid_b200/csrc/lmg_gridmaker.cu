@@ -2213,11 +2213,11 @@ __global__ void __launch_bounds__(256) k_reduce_types(BwdArgs G) {
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st) {
   if (A.gm.rti && A.vec) {
     int n = A.nb * A.T;
-    launch_early(k_chan_params, dim3((n + 255) / 256), 256, 0, st, A);
+    const cudaError_t e = launch_early(k_chan_params, dim3((n + 255) / 256), 256, 0, st, A);
+    if (e != cudaSuccess) return e;
   }
   int n = A.nb * A.N;
-  launch_early(k_emit, dim3((n + 255) / 256), 256, 0, st, A);
-  return cudaGetLastError();
+  return launch_early(k_emit, dim3((n + 255) / 256), 256, 0, st, A);
 }
 
 // tensors that quads are taken from: on 16-byte boundaries
@@ -2290,25 +2290,22 @@ cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st) {
 }
 
 template <int WARPS, class TABS>
-static void backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
+static cudaError_t backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
   const dim3 grid(A.N, A.nb);
-  if (mode == 0) launch_early(k_backward_quads_self<0, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
-  else if (A.gm.binary) launch_early(k_backward_quads_self<2, true, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
-  else launch_early(k_backward_quads_self<2, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
+  if (mode == 0) return launch_early(k_backward_quads_self<0, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
+  if (A.gm.binary) return launch_early(k_backward_quads_self<2, true, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
+  return launch_early(k_backward_quads_self<2, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
 }
 
 template <int WARPS>
-static void backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
-  if (loose_rows(G)) backward_self<WARPS, LooseZTabs>(A, G, mode, st);
-  else backward_self<WARPS, ZTabs>(A, G, mode, st);
+static cudaError_t backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
+  return loose_rows(G) ? backward_self<WARPS, LooseZTabs>(A, G, mode, st) : backward_self<WARPS, ZTabs>(A, G, mode, st);
 }
 
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
   if (A.N == 0 || A.nb == 0) return cudaSuccess;
   // up to one atom's warps per scheduler and a bit: shared columns, beyond that a warp per atom
-  if ((long)A.nb * A.N <= SELF_SPLIT) backward_self<4>(A, G, mode, st);
-  else backward_self<1>(A, G, mode, st);
-  return cudaGetLastError();
+  return (long)A.nb * A.N <= SELF_SPLIT ? backward_self<4>(A, G, mode, st) : backward_self<1>(A, G, mode, st);
 }
 
 // `quads`: rows of diff (and of the density, for relevance) start on 16-byte boundaries
@@ -2361,19 +2358,20 @@ cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
   if (items == 0 || G.nb == 0) return cudaSuccess;
   const bool quads = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0 && (uintptr_t)G.diff % 16 == 0;
   if (quads && !G.gm.rti) {
-    launch_early(k_second_quads_atom, dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st, G);
-    return cudaGetLastError();
+    return launch_early(k_second_quads_atom, dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st, G);
   }
+  cudaError_t e;
   if (quads) {
     const long units = (long)G.N * nz_groups(G.T);
-    launch_early(k_second_quads_nz, dim3((unsigned)((units + SO_WARPS - 1) / SO_WARPS), G.nb), SO_WARPS * 32, 0, st, G);
+    e = launch_early(k_second_quads_nz, dim3((unsigned)((units + SO_WARPS - 1) / SO_WARPS), G.nb), SO_WARPS * 32, 0, st, G);
   } else {
-    launch_early(k_gradgrad_scatter, dim3((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb), SCAT_WARPS * 32, 0, st, G);
-    launch_early(k_backward_warp<3, false>, dim3((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb), BWD2_WARPS * 32, 0, st, G);
+    e = launch_early(k_gradgrad_scatter, dim3((unsigned)((items + SCAT_WARPS - 1) / SCAT_WARPS), G.nb), SCAT_WARPS * 32, 0, st, G);
+    if (e == cudaSuccess)
+      e = launch_early(k_backward_warp<3, false>, dim3((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb), BWD2_WARPS * 32, 0, st, G);
   }
+  if (e != cudaSuccess) return e;
   const int n = G.nb * G.N;
-  launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
-  return cudaGetLastError();
+  return launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
 }
 
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st) {
@@ -2400,14 +2398,12 @@ cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st) 
                  : launch_early(k_forward_quads<false, false>, gq, QS_WARPS * 32, 0, st, G);
   }
   if (vec) {
-    if (bin) launch_early(k_forward_scatter<true, false, true>, grid, SCAT_WARPS * 32, 0, st, G);
-    else if (G.precise) launch_early(k_forward_scatter<false, true, true>, grid, SCAT_WARPS * 32, 0, st, G);
-    else launch_early(k_forward_scatter<false, false, true>, grid, SCAT_WARPS * 32, 0, st, G);
-  } else {
-    if (bin) launch_early(k_forward_binary, dim3((G.N + BIN_WARPS - 1) / BIN_WARPS, G.nb), BIN_WARPS * 32, 0, st, G);
-    else if (G.precise) launch_early(k_forward_scatter<false, true, false>, grid, SCAT_WARPS * 32, 0, st, G);
-    else launch_early(k_forward_scatter<false, false, false>, grid, SCAT_WARPS * 32, 0, st, G);
+    if (bin) return launch_early(k_forward_scatter<true, false, true>, grid, SCAT_WARPS * 32, 0, st, G);
+    if (G.precise) return launch_early(k_forward_scatter<false, true, true>, grid, SCAT_WARPS * 32, 0, st, G);
+    return launch_early(k_forward_scatter<false, false, true>, grid, SCAT_WARPS * 32, 0, st, G);
   }
-  return cudaGetLastError();
+  if (bin) return launch_early(k_forward_binary, dim3((G.N + BIN_WARPS - 1) / BIN_WARPS, G.nb), BIN_WARPS * 32, 0, st, G);
+  if (G.precise) return launch_early(k_forward_scatter<false, true, false>, grid, SCAT_WARPS * 32, 0, st, G);
+  return launch_early(k_forward_scatter<false, false, false>, grid, SCAT_WARPS * 32, 0, st, G);
 }
 }  // namespace lmg

@@ -23,7 +23,9 @@ inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned thread
   c.stream = st;
   c.attrs = &attr;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, args...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // it is in `e`: not to be found again by a later launch
+  return e;
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
