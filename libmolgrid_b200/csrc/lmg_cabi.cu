@@ -255,6 +255,7 @@ lmg::InterpArgs interp_args(const lmg_interpolater* gi, int nchannels, const flo
   I.in_dim = gi->in_dim;
   I.out_dim = gi->out_dim;
   I.K = nchannels;
+  I.c0 = 0;
   I.in = in;
   I.out = out;
   return I;

@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
   const bool live = x < id && y < id && z < id;
   const size_t ichan = (size_t)id * id * id, ochan = (size_t)od * od * od;
   const size_t b = (size_t)I.b0 + bl;
-  const int c0 = blockIdx.z * CH, nch = min(CH, I.K - c0);
+  const int c0 = I.c0 + blockIdx.z * CH, nch = min(CH, I.K - c0);
   const float* gout = I.in + (b * I.K + c0) * ochan;
   float acc[CH];
 #pragma unroll
@@ -644,9 +644,12 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
   const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, LMG_IG_BLOCKS);
   const int per = (I.K + (int)shares - 1) / (int)shares;
   const int ch = per > 16 ? 32 : per > 8 ? 16 : 8;
-  const dim3 grid(tiles, nb, (I.K + ch - 1) / ch);
-  return launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>, grid,
-                      IG_THREADS, 0, st, I, W);
+  InterpArgs J = I;
+  cudaError_t e = cudaSuccess;
+  for (int left = (I.K + ch - 1) / ch; left > 0 && e == cudaSuccess; left -= 65535, J.c0 += 65535 * ch)
+    e = launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>,
+                     dim3(tiles, nb, left < 65535 ? left : 65535), IG_THREADS, 0, st, J, W);
+  return e;
 }
 
 cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st) {

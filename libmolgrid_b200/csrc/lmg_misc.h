@@ -25,6 +25,7 @@ struct InterpArgs {
   unsigned in_dim, out_dim;
   int K;
   int b0;
+  int c0;  // first channel of the launch (backward)
   const float* in;
   float* out;
   InterpFrame ex[INTERP_MAX_EX];

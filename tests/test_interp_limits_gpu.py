@@ -26,3 +26,14 @@ def test_a_refused_launch_is_not_found_again(lib):
     _cabi.check(lib.lmg_transform_forward(ctypes.byref(t), 10, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(y.data_ptr()), 1, None))
     torch.cuda.synchronize()
     assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("more", [-40, 0, 1, 40])
+def test_backward_of_many_channels(more):
+    """Channels beyond 65535 blocks of 32: all of them come through, with the identity unchanged."""
+    K = 65535 * 32 + more
+    gi = lmg.GridInterpolater(1.0, 1.0, 1.0, 1.0)
+    g = torch.rand((K, 2, 2, 2), device="cuda")
+    out = torch.full_like(g, 7.0)
+    gi.backward(g, lmg.Transform(), out)
+    assert torch.equal(g, out)
