@@ -596,10 +596,9 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
     }
   };
 
-  int lo[3] = {0, 0, 0}, hi[3] = {od - 1, od - 1, od - 1};
-  const bool sane = W.sane != 0;
-  float at[3];  // the voxel's image in output indices
-  if (sane) {
+  int lo[3] = {0, 0, 0}, hi[3] = {-1, -1, -1};  // zeros where the map has no use: k_interpolate_scatter adds to them
+  float at[3] = {0.f, 0.f, 0.f};                // the voxel's image in output indices
+  if (W.sane) {
     const float d[3] = {(float)x - W.g0[0], (float)y - W.g0[1], (float)z - W.g0[2]};
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -619,7 +618,7 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
               dy = fmaf(W.a[1][0], fi, fmaf(W.a[1][1], fj, W.a[1][2] * fk)),
               dz = fmaf(W.a[2][0], fi, fmaf(W.a[2][1], fj, W.a[2][2] * fk));
         for (int k = lo[2]; k <= hi[2]; k++) {
-          if (!sane || fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) < limit) {
+          if (fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) < limit) {
             list[n++][tid] = make_uint2((unsigned)i << 16 | (unsigned)j, (unsigned)k);
             if (n == IG_CAP) work_off();
           }
@@ -637,6 +636,33 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
   }
 }
 
+// The adjoint for the examples of `which`, whose maps have no use (a quaternion of length zero, an infinite or
+// enormous transform): every output voxel adds to the input voxels it was blended from, as far as there are any.  (A search of
+// all output voxels by every input voxel: 48^6 positions for two grids of 48^3.)
+__global__ void __launch_bounds__(256) k_interpolate_scatter(InterpArgs I, unsigned long long which) {
+  wait_for_stream();
+  const int bl = blockIdx.y, id = (int)I.in_dim;
+  if (!(which >> bl & 1ull)) return;
+  const InterpFrame& F = I.ex[bl];
+  const size_t od = I.out_dim, v = (size_t)blockIdx.x * blockDim.x + threadIdx.x, ichan = (size_t)id * id * id, ochan = od * od * od;
+  if (v >= ochan) return;
+  float gx, gy, gz;
+  interp_point(I, F, (unsigned)(v / (od * od)), (unsigned)(v / od % od), (unsigned)(v % od), gx, gy, gz);
+  const InterpCell C = interp_cell(gx, gy, gz);
+  const size_t b = (size_t)I.b0 + bl;
+  const float* gout = I.in + b * I.K * ochan + v;
+  float* gin = I.out + b * I.K * ichan;
+  const int xs[2] = {C.xl, C.xh}, ys[2] = {C.yl, C.yh}, zs[2] = {C.zl, C.zh};
+  const float wx[2] = {C.xm, C.xd}, wy[2] = {C.ym, C.yd}, wz[2] = {C.zm, C.zd};
+  for (int k = 0; k < 8; k++) {
+    const int x = xs[k >> 2], y = ys[k >> 1 & 1], z = zs[k & 1];
+    const float w = wx[k >> 2] * wy[k >> 1 & 1] * wz[k & 1];
+    if (w == 0.f || x < 0 || x >= id || y < 0 || y >= id || z < 0 || z >= id) continue;
+    float* p = gin + ((size_t)x * id + y) * id + z;
+    for (int c = 0; c < I.K; c++) atomicAdd(p + c * ichan, w * __ldg(gout + c * ochan));
+  }
+}
+
 cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames& W, int nb, cudaStream_t st) {
   const unsigned id = I.in_dim, tiles = ((id + IG_X - 1) / IG_X) * ((id + IG_Y - 1) / IG_Y) * ((id + IG_Z - 1) / IG_Z);
   if (tiles == 0 || nb == 0 || I.K == 0) return cudaSuccess;
@@ -649,7 +675,12 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
   for (int left = (I.K + ch - 1) / ch; left > 0 && e == cudaSuccess; left -= 65535, J.c0 += 65535 * ch)
     e = launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>,
                      dim3(tiles, nb, left < 65535 ? left : 65535), IG_THREADS, 0, st, J, W);
-  return e;
+  unsigned long long which = 0;
+  static_assert(INTERP_MAX_EX <= 64, "a bit per example");
+  for (int i = 0; i < nb; i++) which |= (unsigned long long)(W.ex[i].sane == 0) << i;
+  if (which == 0 || e != cudaSuccess || I.out_dim == 0) return e;
+  const size_t voxels = (size_t)I.out_dim * I.out_dim * I.out_dim;
+  return launch_early(k_interpolate_scatter, dim3((unsigned)((voxels + 255) / 256), nb), 256, 0, st, I, which);
 }
 
 cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st) {

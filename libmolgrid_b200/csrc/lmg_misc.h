@@ -38,7 +38,7 @@ struct GatherFrame {
   float g0[3];     // position of output voxel (0, 0, 0)
   float reach[3];  // half extent of the box about an input voxel's image that its output voxels lie in
   float slack;     // allowance for the roundings of the positions, in cells
-  int sane;        // 0: the map has no use (an infinite or enormous transform), every voxel is looked at
+  int sane;        // 0: the map has no use (an infinite or enormous transform)
 };
 struct GatherFrames {
   GatherFrame ex[INTERP_MAX_EX];

@@ -37,3 +37,33 @@ def test_backward_of_many_channels(more):
     out = torch.full_like(g, 7.0)
     gi.backward(g, lmg.Transform(), out)
     assert torch.equal(g, out)
+
+
+@pytest.mark.parametrize("odd", ["zero", "far", "infinite", "nan"])
+def test_backward_of_maps_without_use(odd):
+    """A quaternion of length zero, positions far beyond the numbers between voxels and none at all, beside an example as usual:
+    the adjoint of the forward pass, in milliseconds (a search of every pair of voxels takes seconds)."""
+    n, K = 96, 3
+    gi = lmg.GridInterpolater(0.5, (n - 1) * 0.5, 0.5, (n - 1) * 0.5)
+    t = {"zero": lmg.Transform(lmg.Quaternion(0, 0, 0, 0)), "far": lmg.Transform(lmg.Quaternion(1, 0, 0, 0), (0, 0, 0), (3e7, 0, 0)),
+         "infinite": lmg.Transform(lmg.Quaternion(1, 0, 0, 0), (0, 0, 0), (float("inf"), 0, 0)),
+         "nan": lmg.Transform(lmg.Quaternion(float("nan"), 0, 0, 0))}[odd]
+    trs = [lmg.Transform(lmg.Quaternion(0.6, 0, 0.8, 0)), t]
+    src = torch.rand((2, K, n, n, n), device="cuda") + 0.5
+    # sums of 96^3 small whole numbers in one voxel are exact
+    g = torch.randint(0, 8, src.shape, device="cuda").float()
+    out, back = torch.empty_like(src), torch.full_like(src, 7.0)
+    gi.forward(src, trs, out)
+    gi.backward(g, trs, back)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    start.record()
+    gi.backward(g, trs, back)
+    end.record()
+    end.synchronize()
+    assert start.elapsed_time(end) < 200.0
+    for b in range(2):
+        left, right = (out[b].double() * g[b].double()).sum(), (src[b].double() * back[b].double()).sum()
+        scale = float((out[b].double() * g[b].double()).abs().sum() + (src[b].double() * back[b].double()).abs().sum())
+        assert abs(float(left - right)) <= 16 * 2.0 ** -24 * scale
+    if odd == "far":
+        assert not out[1].any() and not back[1].any()
