@@ -8,6 +8,7 @@ are staged through device memory around the call (every result is computed on th
 """
 import ctypes
 import os
+import threading
 
 import numpy as np
 import torch
@@ -195,16 +196,36 @@ def _current_device():
     return torch.device("cuda", torch.cuda.current_device())
 
 
-_workspaces = {}
+class _Workspaces(threading.local):
+    """Scratch buffers reused across calls, a thread's own: ``by`` has them by stream and device.  Calls on one
+    stream follow one another; those of two streams, or of two threads on one, may be under way together."""
+
+    KEPT = 8   # streams
+
+    def __init__(self):
+        self.by = {}
+
+    def clear(self):
+        self.by.clear()
+
+
+_workspaces = _Workspaces()
 _transform_ring = {}   # (device, batch) -> pinned staging buffers of GridMaker.batch_transforms
 
 
 def _workspace(device, nbytes):
-    """Per-device scratch buffer reused across calls (grown on demand)."""
-    ws = _workspaces.get(device)
+    """Scratch buffer of the current stream, reused across calls (grown on demand).  Given up, it goes back to
+    torch's allocator for that stream, whose order keeps it from calls still under way.  A call that is being captured has
+    one of its own, in the memory of its graph."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+    by, key = _workspaces.by, torch._C._cuda_getCurrentRawStream(device.index) << 6 | device.index
+    ws = by.pop(key, None)
     if ws is None or ws.numel() < nbytes:
+        if len(by) >= _Workspaces.KEPT:
+            del by[next(iter(by))]
         ws = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
-        _workspaces[device] = ws
+    by[key] = ws
     return ws
 
 
@@ -454,7 +475,7 @@ class GridMaker(object):
         m = _fast()
         if not m:
             return False
-        ws = getattr(m, name)(ctypes.addressof(self.s), args, kw or None, _workspaces)
+        ws = getattr(m, name)(ctypes.addressof(self.s), args, kw or None, _workspaces.by)
         if ws is None:
             return False
         self._last_ws = ws

@@ -4,11 +4,12 @@
 //     (settings address, args, kwargs or None, workspaces or None)
 // and returns None when it does not serve the call (other kinds of arrays, objects, wrong shapes): the
 // caller then takes the general route, which also raises what there is to raise.  With `workspaces`
-// (a dict device -> uint8 tensor) the call runs on torch's current stream in the device's tensor,
-// which is returned; without, on the default stream in this thread's buffer, and True is returned.
-#include <torch/csrc/Device.h>
+// (a dict (stream << 6 | device) -> uint8 tensor) the call runs on torch's current stream in that
+// stream's tensor, which is held for the length of the call and returned; without, on the default stream in this thread's buffer, and True is returned.
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
+
+#include <cstdint>
 
 #include "bindings_fast.h"
 #include "libmolgrid/common.h"
@@ -143,7 +144,8 @@ bool per_atom(const Call& c, PyObject* o, const lmg_atoms& A, bool batched, size
          (last == 0 || x.shape[1 + batched] == last);
 }
 
-// where the call runs: false leaves it to the general route (no workspace of that size yet)
+// where the call runs, `ret` a new reference; false leaves it to the general route (no workspace of that size yet, or
+// a call that is being captured)
 bool place(const Call& c, size_t bytes, void** ws, size_t* ws_bytes, cudaStream_t* st, PyObject** ret) {
   if (c.workspaces == Py_None) {
     try {
@@ -153,28 +155,29 @@ bool place(const Call& c, size_t bytes, void** ws, size_t* ws_bytes, cudaStream_
     }
     *ws_bytes = bytes;
     *st = nullptr;
-    *ret = Py_True;
+    *ret = Py_NewRef(Py_True);
     return true;
   }
-  static PyObject* key[64] = {};
   if (c.device >= 64) return false;
-  if (key[c.device] == nullptr) {
-    const at::Tensor& t = THPVariable_Unpack(c.item[1]);
-    key[c.device] = THPDevice_New(t.device());
-  }
-  PyObject* w = key[c.device] ? PyDict_GetItem(c.workspaces, key[c.device]) : nullptr;
+  *st = torch_stream(c.device);
+  cudaStreamCaptureStatus capture;
+  if (cudaStreamIsCapturing(*st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+  PyObject* key = PyLong_FromUnsignedLongLong((unsigned long long)reinterpret_cast<uintptr_t>(*st) << 6 | (unsigned)c.device);
+  PyObject* w = key ? PyDict_GetItem(c.workspaces, key) : nullptr;
+  Py_XDECREF(key);
   if (w == nullptr || !THPVariable_Check(w)) return false;
   const at::Tensor& t = THPVariable_Unpack(w);
   if ((size_t)t.numel() < bytes) return false;
   *ws = t.data_ptr();
   *ws_bytes = (size_t)t.numel();
-  *st = torch_stream(c.device);
-  *ret = w;
+  *ret = Py_NewRef(w);
   return true;
 }
 
+// takes over the reference
 PyObject* finish(int rc, PyObject* ret) {
-  if (rc == LMG_OK) return Py_NewRef(ret);
+  if (rc == LMG_OK) return ret;
+  Py_DECREF(ret);
   PyErr_SetString(rc == LMG_ERR_OUT_OF_RANGE ? PyExc_IndexError : rc == LMG_ERR_INVALID_ARGUMENT ? PyExc_ValueError : PyExc_RuntimeError,
                   lmg_last_error());
   return nullptr;

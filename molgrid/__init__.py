@@ -69,7 +69,7 @@ class GridMaker(native.GridMaker):
     def _shared(self, call, args, kw):
         """A call that the Python layer serves (one centre for a whole batch, batched second
         derivatives), on resident tensors: through the compiled module on torch's current stream."""
-        return call(self._sp, args, kw or None, _api._workspaces) is not None
+        return call(self._sp, args, kw or None, _api._workspaces.by) is not None
 
     @staticmethod
     def _extension(args, kw):
