@@ -112,6 +112,7 @@ inline ViewInfo view_info(const py::handle& h, const std::string& name) {
     }
     v.ptr = reinterpret_cast<void*>(o.attr("data_ptr")().cast<size_t>());
     for (auto d : o.attr("shape")) v.shape.push_back(d.cast<size_t>());
+    if (v.ptr == nullptr && o.attr("numel")().cast<size_t>() > 0) throw py::value_error(name + ": tensor without memory");
   } else if (py::isinstance<py::array>(o)) {
     py::array a = py::reinterpret_borrow<py::array>(o);
     bool f32 = py::isinstance<py::array_t<float>>(a), f64 = py::isinstance<py::array_t<double>>(a);

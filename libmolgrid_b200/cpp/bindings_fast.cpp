@@ -16,9 +16,12 @@
 
 namespace lmgpy {
 
-bool torch_view(PyObject* o, TorchView& v) {
+// Tensors that have no memory of their own (of vmap and other transforms, fake and nested ones) throw at
+// one of these questions or answer with a null address: not ours.
+bool torch_view(PyObject* o, TorchView& v) try {
   if (!THPVariable_Check(o)) return false;
   const at::Tensor& t = THPVariable_Unpack(o);
+  if (t.is_nested()) return false;
   const at::ScalarType st = t.scalar_type();
   v.dtype = st == at::kFloat ? 'f' : st == at::kDouble ? 'd' : st == at::kInt ? 'i' : '?';
   v.ndim = (int)t.dim();
@@ -28,7 +31,9 @@ bool torch_view(PyObject* o, TorchView& v) {
   v.device = t.is_cuda() ? (int)t.get_device() : t.is_cpu() ? -1 : -2;
   if (v.device == -2) return false;
   v.ptr = t.numel() ? t.data_ptr() : nullptr;
-  return true;
+  return v.ptr != nullptr || t.numel() == 0;
+} catch (const std::exception&) {
+  return false;
 }
 
 cudaStream_t torch_stream(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
@@ -38,6 +43,12 @@ namespace {
 // A tensor argument of the fast route.
 struct Arr : TorchView {
   float* f() const { return static_cast<float*>(ptr); }
+};
+
+// The interpreter is others' while this lives.
+struct Released {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Released() { PyEval_RestoreThread(state); }
 };
 
 struct Call {
@@ -58,7 +69,9 @@ bool number(PyObject* o, float* f) {
   if (PyFloat_CheckExact(o)) *f = (float)PyFloat_AS_DOUBLE(o);
   else if (PyLong_CheckExact(o)) *f = (float)PyLong_AsDouble(o);
   else return false;
-  return true;
+  if (PyErr_Occurred() == nullptr) return true;
+  PyErr_Clear();  // a whole number beyond a double: the general route says so
+  return false;
 }
 
 // settings, arguments and keywords; false: not for the fast route
@@ -202,11 +215,10 @@ PyObject* fast_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   A.ntypes = (int)T;
   if (!radii_fit(c, vec, nr, A.max_atoms, T)) Py_RETURN_NONE;
   if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_FORWARD, A.batch, A.max_atoms, A.ntypes, vec), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = lmg_forward(c.g, &A, out.f(), ws, wb, st);
-  Py_END_ALLOW_THREADS
-  return finish(rc, ret);
+  return finish([&] {
+    Released r;
+    return lmg_forward(c.g, &A, out.f(), ws, wb, st);
+  }(), ret);
 }
 
 PyObject* fast_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -231,11 +243,10 @@ PyObject* fast_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   }
   if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_BACKWARD, A.batch, A.max_atoms, A.ntypes, vec), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = lmg_backward(c.g, &A, diff.f(), ag.f(), tg.f(), ws, wb, st);
-  Py_END_ALLOW_THREADS
-  return finish(rc, ret);
+  return finish([&] {
+    Released r;
+    return lmg_backward(c.g, &A, diff.f(), ag.f(), tg.f(), ws, wb, st);
+  }(), ret);
 }
 
 PyObject* fast_relevance(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -253,11 +264,10 @@ PyObject* fast_relevance(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   A.ntypes = (int)T;
   if (!per_atom(c, c.item[6], A, batched, 0, rel) || nr != (size_t)A.max_atoms) Py_RETURN_NONE;
   if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_RELEVANCE, A.batch, A.max_atoms, A.ntypes, 0), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = lmg_backward_relevance(c.g, &A, de.f(), diff.f(), rel.f(), ws, wb, st);
-  Py_END_ALLOW_THREADS
-  return finish(rc, ret);
+  return finish([&] {
+    Released r;
+    return lmg_backward_relevance(c.g, &A, de.f(), diff.f(), rel.f(), ws, wb, st);
+  }(), ret);
 }
 
 PyObject* fast_gradients(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -279,11 +289,10 @@ PyObject* fast_gradients(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !radii_fit(c, vec, nr, A.max_atoms, T))
     Py_RETURN_NONE;
   if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_GRADIENTS, A.batch, A.max_atoms, A.ntypes, 1), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = lmg_backward_gradients(c.g, &A, diff.f(), ag.f(), tg.f(), dd.f(), add.f(), tdd.f(), ws, wb, st);
-  Py_END_ALLOW_THREADS
-  return finish(rc, ret);
+  return finish([&] {
+    Released r;
+    return lmg_backward_gradients(c.g, &A, diff.f(), ag.f(), tg.f(), dd.f(), add.f(), tdd.f(), ws, wb, st);
+  }(), ret);
 }
 
 // A float attribute (any Python or numpy number) of an object; false with an exception set.
@@ -325,12 +334,26 @@ PyObject* pack_transforms(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   Py_RETURN_NONE;
 }
 
+// No C++ exception crosses into the interpreter, whose frames know none.
+typedef PyObject* (*Fast)(PyObject*, PyObject* const*, Py_ssize_t);
+template <Fast F>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  try {
+    return F(self, a, n);
+  } catch (const std::exception& e) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+template <Fast F>
+PyCFunction entry() { return (PyCFunction)(void (*)(void))guarded<F>; }
+
 PyMethodDef methods[] = {
-    {"_pack_transforms", (PyCFunction)(void (*)(void))pack_transforms, METH_FASTCALL, nullptr},
-    {"_fast_forward", (PyCFunction)(void (*)(void))fast_forward, METH_FASTCALL, nullptr},
-    {"_fast_backward", (PyCFunction)(void (*)(void))fast_backward, METH_FASTCALL, nullptr},
-    {"_fast_relevance", (PyCFunction)(void (*)(void))fast_relevance, METH_FASTCALL, nullptr},
-    {"_fast_gradients", (PyCFunction)(void (*)(void))fast_gradients, METH_FASTCALL, nullptr},
+    {"_pack_transforms", entry<pack_transforms>(), METH_FASTCALL, nullptr},
+    {"_fast_forward", entry<fast_forward>(), METH_FASTCALL, nullptr},
+    {"_fast_backward", entry<fast_backward>(), METH_FASTCALL, nullptr},
+    {"_fast_relevance", entry<fast_relevance>(), METH_FASTCALL, nullptr},
+    {"_fast_gradients", entry<fast_gradients>(), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace
