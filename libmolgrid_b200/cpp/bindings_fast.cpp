@@ -57,6 +57,7 @@ struct Call {
   Py_ssize_t n;
   PyObject *transforms = nullptr, *n_atoms = nullptr, *type_gradients = nullptr;
   bool want_tg = true;
+  bool gradient_words = false;  // keywords of the backward pass alone
   PyObject* workspaces;
   int device = -1;
 };
@@ -87,9 +88,19 @@ bool open(PyObject* const* a, Py_ssize_t nargs, Call& c) {
     while (PyDict_Next(a[2], &at, &k, &v)) {
       if (PyUnicode_CompareWithASCIIString(k, "transforms") == 0) c.transforms = v == Py_None ? nullptr : v;
       else if (PyUnicode_CompareWithASCIIString(k, "n_atoms") == 0) c.n_atoms = v == Py_None ? nullptr : v;
-      else if (PyUnicode_CompareWithASCIIString(k, "type_gradients") == 0) c.type_gradients = v == Py_None ? nullptr : v;
-      else if (PyUnicode_CompareWithASCIIString(k, "want_type_gradients") == 0) c.want_tg = v == Py_True;
-      else return false;
+      else if (PyUnicode_CompareWithASCIIString(k, "type_gradients") == 0) {
+        if (c.n > 6) return false;  // given twice
+        c.type_gradients = v == Py_None ? nullptr : v;
+        c.gradient_words = true;
+      } else if (PyUnicode_CompareWithASCIIString(k, "want_type_gradients") == 0) {
+        const int yes = PyObject_IsTrue(v);
+        if (yes < 0) PyErr_Clear();
+        if (yes < 0) return false;
+        c.want_tg = yes != 0;
+        c.gradient_words = true;
+      } else {
+        return false;
+      }
     }
   }
   return cudaGetDevice(&c.device) == cudaSuccess;
@@ -209,7 +220,7 @@ PyObject* fast_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   void* ws;
   cudaStream_t st;
   PyObject* ret;
-  if (!open(a, nargs, c) || c.n != 5 || c.type_gradients || !atoms(c, A, vec, nr)) Py_RETURN_NONE;
+  if (!open(a, nargs, c) || c.n != 5 || c.gradient_words || !atoms(c, A, vec, nr)) Py_RETURN_NONE;
   const bool batched = THPVariable_Unpack(c.item[1]).dim() == 3;
   if (!grid(c, c.item[4], A, batched, out, T) || (vec && (size_t)A.ntypes != T)) Py_RETURN_NONE;
   A.ntypes = (int)T;
@@ -258,7 +269,7 @@ PyObject* fast_relevance(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   void* ws;
   cudaStream_t st;
   PyObject* ret;
-  if (!open(a, nargs, c) || c.n != 7 || c.type_gradients || !atoms(c, A, vec, nr) || vec || c.g->radii_type_indexed) Py_RETURN_NONE;
+  if (!open(a, nargs, c) || c.n != 7 || c.gradient_words || !atoms(c, A, vec, nr) || vec || c.g->radii_type_indexed) Py_RETURN_NONE;
   const bool batched = THPVariable_Unpack(c.item[1]).dim() == 3;
   if (!grid(c, c.item[4], A, batched, de, T) || !grid(c, c.item[5], A, batched, diff, T2) || T != T2) Py_RETURN_NONE;
   A.ntypes = (int)T;
@@ -279,7 +290,7 @@ PyObject* fast_gradients(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   void* ws;
   cudaStream_t st;
   PyObject* ret;
-  if (!open(a, nargs, c) || c.n != 10 || c.type_gradients || !atoms(c, A, vec, nr) || !vec) Py_RETURN_NONE;
+  if (!open(a, nargs, c) || c.n != 10 || c.gradient_words || !atoms(c, A, vec, nr) || !vec) Py_RETURN_NONE;
   const bool batched = THPVariable_Unpack(c.item[1]).dim() == 3;
   if (batched && c.workspaces == Py_None) Py_RETURN_NONE;
   if (!grid(c, c.item[4], A, batched, diff, T) || !grid(c, c.item[7], A, batched, dd, T2) || T != T2 || (size_t)A.ntypes != T)
