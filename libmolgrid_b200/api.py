@@ -180,8 +180,11 @@ def _fast():
         if os.environ.get("LMG_B200_LIB"):   # another build of the library than the one the module links
             _native = False
         else:
-            from . import molgrid_native
-            _native = molgrid_native
+            try:
+                from . import molgrid_native
+                _native = molgrid_native
+            except ImportError:              # the library alone was built: its calls need no more
+                _native = False
     return _native
 
 
