@@ -113,6 +113,7 @@ class CoordCache(object):
         self.data_root = data_root
         self.cache = None
         self._raw = {}
+        self._loads = 0      # how often structures in memory may have been replaced
         if molcache:
             if not os.path.exists(molcache):
                 molcache = os.path.join(data_root, molcache)
@@ -156,6 +157,7 @@ class CoordCache(object):
             out.write(np.ascontiguousarray(rec).tobytes())
 
     def load_mem_cache(self, inp):
+        self._loads += 1
         (n,) = np.frombuffer(inp.read(8), np.uint64)
         for _ in range(int(n)):
             (ln,) = np.frombuffer(inp.read(4), np.uint32)

@@ -170,15 +170,23 @@ _TABLE_TYPERS = (_py.GninaIndexTyper, _py.FileMappedGninaTyper, _py.NullIndexTyp
 class ExampleProvider(_py.ExampleProvider):
     """The example provider handing out the compiled Example / ExampleVec types."""
 
-    def _native_line(self, i):
+    def _current_lines(self):
+        """The lines made so far, none of them if the settings or the caches have changed since."""
+        made_from = [self.settings.make_vector_types, self.settings.duplicate_first] + \
+            [x for c in self.caches for x in (c, c.typer, c._loads)]
+        if self.__dict__.get("_made_from") != made_from:
+            self._made_from, self._lines = made_from, {}
+        return self._lines
+
+    def _native_line(self, i, lines=None):
         """Line i as the compiled module turns it into Examples (its records, the tables of its
         typers, its labels), made at the line's first use; None where the Python layer has to type
-        the atoms."""
-        lines = self.__dict__.setdefault("_lines", {})
-        if i in lines:
-            return lines[i]
-        ref, line = self.refs[i], None
-        files = self._files(ref)
+        the atoms.  A line that has changed since is made anew."""
+        lines = self._current_lines() if lines is None else lines
+        ref, was = self.refs[i], lines.get(i)
+        if was is not None and was[1:] == (ref.labels, ref.files, ref.group):
+            return was[0]
+        line, files = None, self._files(ref)
         if not self.settings.make_vector_types and all(type(self.caches[c].typer) in _TABLE_TYPERS for _, c in files):
             recs = [self.caches[c].records(f) for f, c in files]
             if all(len(r) == 0 or int(r["type"].min()) >= 0 for r in recs):
@@ -187,7 +195,7 @@ class ExampleProvider(_py.ExampleProvider):
                                              [self.caches[c].num_types() for _, c in files],
                                              [float(v) for v in ref.labels],
                                              int(ref.group) if ref.group is not None else -1)
-        lines[i] = line
+        lines[i] = (line, list(ref.labels), list(ref.files), ref.group)
         return line
 
     def _make(self, ref):
@@ -203,11 +211,13 @@ class ExampleProvider(_py.ExampleProvider):
         B = int(batch_size) or int(self.settings.default_batch_size)
         if hasattr(self._order, "check_batch_size"):
             self._order.check_batch_size(B)
-        if not self._grouped and self.refs:
-            take = self._order.nextref
-            idx = [take() for _ in range(B)]
-            known = self.__dict__.setdefault("_lines", {})
-            lines = [known.get(i) or self._native_line(i) for i in idx]
+        # a class derived from this one may hand out examples of its own
+        own = type(self).next is not ExampleProvider.next or type(self)._make is not ExampleProvider._make
+        if not self._grouped and self.refs and not own:
+            idx, lines, made = [], [], self._current_lines()
+            for _ in range(B):
+                idx.append(self._order.nextref())
+                lines.append(self._native_line(idx[-1], made))
             if None not in lines:
                 return native._make_examples(lines)
             return native.ExampleVec([self._make(self.refs[i]) for i in idx])

@@ -71,3 +71,78 @@ def test_example_batches_on_a_stream(tmp_path, stream):
             # reductions of the same terms in another order: a few roundings of the largest value
             assert torch.allclose(out[i], one, rtol=1e-5, atol=1e-6)
             assert lab[i].tolist() == list(ex.labels)
+
+
+def _provider(tmp_path):
+    import molgrid
+    p = molgrid.ExampleProvider(data_root=str(tmp_path))
+    p.populate(str(tmp_path / "s.types"))
+    return p
+
+
+def test_batches_follow_settings_typers_and_caches(tmp_path):
+    """What a provider's settings, typers, lines and loaded structures are when a batch is asked for, not when its lines were
+    first seen."""
+    import libmolgrid_b200 as lmg
+    import molgrid
+    _lists(tmp_path, 40, 3)
+    p = _provider(tmp_path)
+    before = p.next_batch(3)
+    # structures loaded after the first use take the place of those read before
+    (tmp_path / "other").mkdir()
+    _lists(tmp_path / "other", 16, 3)
+    q = molgrid.ExampleProvider(data_root=str(tmp_path / "other"))
+    q.populate(str(tmp_path / "other" / "s.types"))
+    theirs = q.next_batch(3)
+    q.save_mem_caches(str(tmp_path / "mem"))
+    p.load_mem_caches(str(tmp_path / "mem"))
+    now = p.next_batch(3)
+    for a, b, c in zip(now, theirs, before):
+        assert a.num_coordinates() == b.num_coordinates() != c.num_coordinates()
+    # labels of a line
+    p.refs[0].labels = [5.0, 6.0]
+    p.reset()
+    assert list(p.next_batch(3)[0].labels) == [5.0, 6.0]
+    # another typer
+    p.caches[0].typer = lmg.GninaIndexTyper()
+    p.reset()
+    assert p.next_batch(3)[0].coord_sets[0].max_type == 28
+    # type vectors from now on
+    p.settings.make_vector_types = True
+    p.reset()
+    batch = p.next_batch(3)
+    assert batch[0].coord_sets[0].type_vector.size() > 0 and batch[0].coord_sets[0].type_index.size() == 0
+
+
+def test_a_provider_of_ones_own(tmp_path):
+    """Examples that a derived class makes are in its batches too."""
+    import molgrid
+
+    class Relabelled(molgrid.ExampleProvider):
+        def _make(self, ref):
+            ex = molgrid.ExampleProvider._make(self, ref)
+            ex.labels = [42.0]
+            return ex
+
+    class Every(molgrid.ExampleProvider):
+        def next(self):
+            ex = molgrid.ExampleProvider.next(self)
+            ex.group = 9
+            return ex
+
+    _lists(tmp_path, 10, 3)
+    for cls in (Relabelled, Every):
+        p = cls(data_root=str(tmp_path))
+        p.populate(str(tmp_path / "s.types"))
+        for ex in p.next_batch(3):
+            assert list(ex.labels) == [42.0] if cls is Relabelled else ex.group == 9
+
+
+def test_a_line_that_cannot_be_read_is_not_skipped_with_others(tmp_path):
+    """The example after a missing file is the next one."""
+    _lists(tmp_path, 10, 4)
+    (tmp_path / "r1.gninatypes").unlink()
+    p = _provider(tmp_path)
+    with pytest.raises(ValueError):
+        p.next_batch(3)
+    assert list(p.next_batch(1)[0].labels) == [0.0, 1.0]     # line 2
