@@ -184,7 +184,7 @@ class ExampleProvider(_py.ExampleProvider):
         the atoms.  A line that has changed since is made anew."""
         lines = self._current_lines() if lines is None else lines
         ref, was = self.refs[i], lines.get(i)
-        if was is not None and was[1:] == (ref.labels, ref.files, ref.group):
+        if was is not None and was[1] == ref.__dict__:
             return was[0]
         line, files = None, self._files(ref)
         if not self.settings.make_vector_types and all(type(self.caches[c].typer) in _TABLE_TYPERS for _, c in files):
@@ -195,7 +195,7 @@ class ExampleProvider(_py.ExampleProvider):
                                              [self.caches[c].num_types() for _, c in files],
                                              [float(v) for v in ref.labels],
                                              int(ref.group) if ref.group is not None else -1)
-        lines[i] = (line, list(ref.labels), list(ref.files), ref.group)
+        lines[i] = (line, {k: list(v) if type(v) is list else v for k, v in ref.__dict__.items()})
         return line
 
     def _make(self, ref):
@@ -214,10 +214,12 @@ class ExampleProvider(_py.ExampleProvider):
         # a class derived from this one may hand out examples of its own
         own = type(self).next is not ExampleProvider.next or type(self)._make is not ExampleProvider._make
         if not self._grouped and self.refs and not own:
-            idx, lines, made = [], [], self._current_lines()
+            idx, lines, made, refs, take = [], [], self._current_lines(), self.refs, self._order.nextref
             for _ in range(B):
-                idx.append(self._order.nextref())
-                lines.append(self._native_line(idx[-1], made))
+                i = take()
+                idx.append(i)
+                was = made.get(i)
+                lines.append(was[0] if was is not None and was[1] == refs[i].__dict__ else self._native_line(i, made))
             if None not in lines:
                 return native._make_examples(lines)
             return native.ExampleVec([self._make(self.refs[i]) for i in idx])
