@@ -53,9 +53,21 @@ struct WorkspaceSlot {
   int device = -1;
   cudaStream_t stream = nullptr;
 };
+struct Workspaces {
+  std::vector<WorkspaceSlot> slots;  // the one used last in front
+  // A thread that ends gives its buffers back, also while another one captures a graph, which forbids such calls
+  // unless they are declared to have nothing to do with it.
+  ~Workspaces() {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (slots.empty() || cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return;
+    for (WorkspaceSlot& s : slots)
+      if (s.p) cudaFree(s.p);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+};
 inline std::vector<WorkspaceSlot>& workspaces() {
-  thread_local std::vector<WorkspaceSlot> w;  // the one used last in front
-  return w;
+  thread_local Workspaces w;
+  return w.slots;
 }
 inline const WorkspaceSlot* last_workspace() { return workspaces().empty() ? nullptr : &workspaces().front(); }
 

@@ -777,8 +777,8 @@ int lmg_interpolate(const lmg_interpolater* gi, int batch, int nchannels, const 
   if (out == nullptr) return fail(LMG_ERR_INVALID_ARGUMENT, "Output grid not allocated");
   lmg::InterpArgs I = interp_args(gi, nchannels, in, out);
   // The tiled kernel stages boxes of the input through tensor copies: rows of the input must start
-  // on 16-byte boundaries, and an 8^3 output tile must map into a 16x16x20 box of input voxels under
-  // any rotation (8*sqrt(3)*out_res/in_res + 2 <= 16).
+  // on 16-byte boundaries, and a 12^3 output tile must map into the largest box, 24x24x28 input voxels,
+  // under any rotation (11*sqrt(3)*out_res/in_res + 3 <= 24; a tile that does not is read directly).
   lmg::InterpMaps maps;
   bool tiled = g_interp_tiled && batch > 0 && nchannels > 0 && gi->in_dim > 0 &&
                (uintptr_t)in % 16 == 0 && (gi->in_dim * sizeof(float)) % 16 == 0 &&

@@ -208,19 +208,7 @@ __device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
 
 constexpr float NEG2_LOG2E = -2.8853900817779268f;  // -2*log2(e)
 
-// calc_point<false> (src/grid_maker.cu:95-118) on a precomputed squared distance.
-// Fast form: one ex2, one sqrt, fused arithmetic; within ~1e-6 relative of the reference.
-__device__ __forceinline__ float density_fast(float rsq, float inv_ar2, float Tg, float Tcut,
-                                              float A, float B, float C) {
-  float u = rsq * inv_ar2;
-  float g = ex2_approx(u * NEG2_LOG2E);
-  float s = sqrt_approx(u);
-  float q = fmaxf(fmaf(fmaf(A, s, B), s, C), 0.f);
-  float v = rsq <= Tg ? g : q;
-  return rsq <= Tcut ? v : 0.f;
-}
-
-// Same function with the reference's own operation order and double intermediate.
+// calc_point<false> (src/grid_maker.cu:95-118) on a precomputed squared distance, in the reference's own operation order and double intermediate.
 __device__ __forceinline__ float density_precise(float rsq, float ar, float Tg, float Tcut,
                                                  float A, float B, float C) {
   if (!(rsq <= Tcut)) return 0.f;

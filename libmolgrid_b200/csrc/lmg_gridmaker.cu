@@ -1,7 +1,8 @@
 // sm_100a kernels for GridMaker forward / backward / backward_gradients / backward_relevance.
 //
-// Every pass starts with emit: one thread per atom - fused Transform, exact footprint bounds and
-// distance thresholds -> 64-byte atom record.
+// An atom is prepared once - fused Transform, exact footprint bounds and distance thresholds -> 64-byte atom record -
+// by a thread of k_emit in front of the pass, or, in small passes of index types, by the warps that sweep it
+// (k_forward_self, k_backward_quads_self); binary grids of index types have kernels of their own (lmg_occupancy.cu).
 //
 // Default forward: the output is zero-filled, then one warp per atom (per (atom, channel) with vector
 // types) compacts the columns of the atom's footprint that lie inside the cut-off circle and adds
@@ -125,38 +126,20 @@ __device__ __forceinline__ float gauss_factor(float d2, const ItemParams& P, flo
 // is evaluated as exp(-2 dxy2/ar^2) * exp(-2 dz2/ar^2): one ex2 per column instead of one per voxel.
 // One warp per block in the backward kernels: the kernel waits on its loads of the grid gradient,
 // and a block of several warps keeps its registers until its slowest atom is done.
-#ifndef LMG_BWD_WARPS
-#define LMG_BWD_WARPS 1
-#endif
-#ifndef LMG_SCAT_WARPS
-#define LMG_SCAT_WARPS 4
-#endif
-constexpr int BWD2_WARPS = LMG_BWD_WARPS;    // warps (work items) per block, backward kernels
-constexpr int SCAT_WARPS = LMG_SCAT_WARPS;   // the same for the scatter kernels
+constexpr int BWD2_WARPS = 1;    // warps (work items) per block, backward kernels
+constexpr int SCAT_WARPS = 4;   // the same for the scatter kernels
 // One warp per block for the quad forward kernels whose work items differ a lot in size (an atom's
 // footprint grows with the cube of its radius): a block of several warps keeps its registers and
 // its slot until its slowest item is done.  Measured per batch of 50: index-typed forward 0.266 ->
 // 0.258 ms, one-hot vector forward 0.322 -> 0.286 ms; the binary and the weighted-channel kernels
 // are faster with four and keep SCAT_WARPS.
-#ifndef LMG_QS_WARPS
-#define LMG_QS_WARPS 1
-#endif
-constexpr int QS_WARPS = LMG_QS_WARPS;
-#ifndef LMG_SELF_ATOMS
-#define LMG_SELF_ATOMS 8192
-#endif
-#ifndef LMG_SELF_SPLIT
-#define LMG_SELF_SPLIT 1200
-#endif
-constexpr int SELF_SPLIT = LMG_SELF_SPLIT;   // most of them that four warps each take
-constexpr int SELF_ATOMS = LMG_SELF_ATOMS;   // most atom slots of a backward pass without k_emit
+constexpr int QS_WARPS = 1;
+constexpr int SELF_SPLIT = 1200;   // most of them that four warps each take
+constexpr int SELF_ATOMS = 8192;   // most atom slots of a backward pass without k_emit
 // Gradients on loose rows, whose quads take longer than single voxels do: 2380 slots 12.2 -> 10.3 us, 4760 slots
 // 15.0 and 15.1, 7650 slots 20.0 and 21.5.
 constexpr int LOOSE_SELF_ATOMS = 4096;
-#ifndef LMG_FWD_SELF_ATOMS
-#define LMG_FWD_SELF_ATOMS 32768
-#endif
-constexpr int FWD_SELF_ATOMS = LMG_FWD_SELF_ATOMS;  // the same for the forward pass (densities)
+constexpr int FWD_SELF_ATOMS = 32768;  // the same for the forward pass (densities)
 constexpr int REL_SELF_ATOMS = 2560;                // ... and for relevance, whose kernel is the heaviest
 constexpr int BWD2_COLS = 256;  // compacted columns held per warp at a time
 constexpr int ZSTEPS = 4;       // z positions per lane and chunk; a chunk covers 4*ZSTEPS voxels
@@ -525,11 +508,8 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_gradgrad_scatter(BwdArgs G)
   int bl = blockIdx.y;
   int b = G.b0 + bl;
   if (item >= G.N * G.T) return;
-  if (true) {
-    // an (atom, channel) pair without weight contributes nothing: leave before any other load
-    int ea = item / G.T;
-    if (G.type_vector[((size_t)b * G.N + ea) * G.T + (item - ea * G.T)] == 0.f) return;
-  }
+  // an (atom, channel) pair without weight contributes nothing: leave before any other load
+  if (G.type_vector[((size_t)b * G.N + item / G.T) * G.T + item % G.T] == 0.f) return;
   ColBufD& buf = bufs[wid];
 
   float cx, cy, cz;
@@ -945,10 +925,7 @@ __device__ __forceinline__ void forward_binary_core(const BwdArgs& G, ItemParams
   }
 }
 
-#ifndef LMG_BIN_WARPS
-#define LMG_BIN_WARPS 4
-#endif
-constexpr int BIN_WARPS = LMG_BIN_WARPS;
+constexpr int BIN_WARPS = 4;
 __global__ void __launch_bounds__(BIN_WARPS * 32) k_forward_binary(BwdArgs G) {
   wait_for_stream();
   __shared__ ColBuf bufs[BIN_WARPS];
@@ -1396,7 +1373,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_nz(BwdArgs G
 // the grid receives  density * type_gradient + w * s * (delta . atom_gradient)  (src/grid_maker.cpp:618-634),
 // the atom needs, per column, the sums of diff * alpha * {1, dz, dz^2} and of diff * s (:636-662).
 // Bound by instruction issue: 28x96^3 at 0.25 A, 4 x 3000 atoms of 28 weighted channels each: 6.70 ms as
-// two sweeps with scalar arithmetic, 4.17 ms now (issue 68 %, L1 75 %).
+// two sweeps with scalar arithmetic, 4.17 ms as one (issue 68 %, L1 75 %), 4.25 with values outside the cut-off left out.
 // ---------------------------------------------------------------------------------------------
 constexpr int SO_WARPS = 1;
 // Two lanes share a column, each taking every other quad: a load or reduction of a warp touches 16 lines
@@ -1738,24 +1715,12 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
 // rounds of 16 with 4 loads together 2.79 ms, 8 / 8 2.08 ms, 14 / 7 1.82 ms, 14 / 14 1.70 ms,
 // 16 / 16 2.17 ms, 28 / 14 2.05 ms; capping the registers below what the compiler picks, blocks of
 // several warps, or atoms sorted by cell (for L1 reuse between neighbours) change nothing or lose.
-#ifndef LMG_VA_BCH
-#define LMG_VA_BCH 14
-#endif
-constexpr int VA_BCH = LMG_VA_BCH;
-#ifndef LMG_VA_LD
-#define LMG_VA_LD 14
-#endif
-constexpr int VA_LD = LMG_VA_LD;  // channels whose quads are requested together
+constexpr int VA_BCH = 14;
+constexpr int VA_LD = 14;  // channels whose quads are requested together
 static_assert(VA_BCH % VA_LD == 0, "a round is a whole number of load batches");
 static_assert(VA_BCH <= 32, "a lane per channel of a round reads the weights");
-#ifndef LMG_VA_WARPS
-#define LMG_VA_WARPS BWD2_WARPS
-#endif
-constexpr int VA_WARPS = LMG_VA_WARPS;
-#ifndef LMG_VA_REREAD
-#define LMG_VA_REREAD 2
-#endif
-constexpr int VA_REREAD = LMG_VA_REREAD;  // weighted channels of a round up to which they are re-read from a list
+constexpr int VA_WARPS = BWD2_WARPS;
+constexpr int VA_REREAD = 2;  // weighted channels of a round up to which they are re-read from a list
 
 // per-warp shared state of the kernel below
 struct VaShared {

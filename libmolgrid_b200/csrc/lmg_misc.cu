@@ -241,32 +241,11 @@ __device__ __forceinline__ void tma_load_box(float* dst, const CUtensorMap* map,
       : "memory");
 }
 
-#ifndef LMG_IT_BLOCKS
-#define LMG_IT_BLOCKS 592
-#endif
-#ifndef LMG_IG_BLOCKS
-#define LMG_IG_BLOCKS 592
-#endif
-#ifndef LMG_ID_BLOCKS
-#define LMG_ID_BLOCKS 1184
-#endif
-#ifndef LMG_INTERP_THREADS
-#define LMG_INTERP_THREADS 288
-#endif
-#ifndef LMG_INTERP_MINBLOCKS
-#define LMG_INTERP_MINBLOCKS 2
-#endif
-#ifndef LMG_INTERP_MAXSTAGES
-#define LMG_INTERP_MAXSTAGES 4
-#endif
-constexpr int INT = LMG_INTERP_THREADS;                 // threads that blend; one more warp stages the boxes
+constexpr int INT = 288;                 // threads that blend; one more warp stages the boxes
 constexpr int IVPT = ITILE * ITILE * ITILE / INT;       // voxels per thread
 static_assert(IVPT * INT == ITILE * ITILE * ITILE, "the threads of a block share the tile evenly");
-constexpr int IMAXST = LMG_INTERP_MAXSTAGES;            // most boxes in flight or in use per block
-#ifndef LMG_INTERP_RING
-#define LMG_INTERP_RING 28160  // 110 KB: two blocks per SM
-#endif
-constexpr int IRING = LMG_INTERP_RING;                  // floats of staging per block
+constexpr int IMAXST = 4;            // most boxes in flight or in use per block
+constexpr int IRING = 28160;  // floats of staging per block (110 KB: two blocks per SM)
 static_assert(IMAXST >= 1 && IRING >= ITILE_BOX && IRING % 32 == 0, "the staging area holds at least one box");
 static_assert(ITILE_BX < 1024 && ITILE_BY < 1024 && ITILE_BZ < 1024, "a position in the box is packed into one word");
 
@@ -278,7 +257,7 @@ struct InterpVoxel {
   float xd, yd, zd;
 };
 
-__global__ void __launch_bounds__(INT + 32, LMG_INTERP_MINBLOCKS) k_interpolate_tiled(const __grid_constant__ InterpMaps maps, InterpArgs I) {
+__global__ void __launch_bounds__(INT + 32, 2) k_interpolate_tiled(const __grid_constant__ InterpMaps maps, InterpArgs I) {
   // the staging area is cut into as many slots as boxes of this block's extents fit
   extern __shared__ __align__(128) float ring[];
   __shared__ __align__(8) uint64_t full[IMAXST], empty[IMAXST];
@@ -507,7 +486,7 @@ unsigned interp_tile_count(unsigned out_dim) {
 cudaError_t launch_interpolate_tiled(const InterpMaps& maps, const InterpArgs& I, int nb, cudaStream_t st) {
   unsigned ntiles = interp_tile_count(I.out_dim);
   if (ntiles == 0 || nb == 0 || I.K == 0) return cudaSuccess;
-  dim3 grid(ntiles, nb, channel_shares((unsigned long)ntiles * nb, I.K, LMG_IT_BLOCKS));
+  dim3 grid(ntiles, nb, channel_shares((unsigned long)ntiles * nb, I.K, 592));
   constexpr size_t smem = (size_t)IRING * sizeof(float);
   if (smem > 48 * 1024) {
     // more than the default dynamic shared memory: opted into once per device
@@ -546,10 +525,7 @@ cudaError_t read_tma_timeouts(unsigned* count) {
 constexpr int IG_X = 4, IG_Y = 8, IG_Z = 8;  // input voxels of a block; a warp is a brick of 2 x 2 x 8
 constexpr int IG_THREADS = IG_X * IG_Y * IG_Z;
 constexpr int IG_CAP = 16;                   // entries per list; a list that fills up is worked off in between
-#ifndef LMG_IG_MINB
-#define LMG_IG_MINB 3
-#endif
-constexpr int IG_MINB = LMG_IG_MINB;
+constexpr int IG_MINB = 3;
 
 template <int CH>
 __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(InterpArgs I, GatherFrames G) {
@@ -667,7 +643,7 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
   const unsigned id = I.in_dim, tiles = ((id + IG_X - 1) / IG_X) * ((id + IG_Y - 1) / IG_Y) * ((id + IG_Z - 1) / IG_Z);
   if (tiles == 0 || nb == 0 || I.K == 0) return cudaSuccess;
   // More channels per block mean fewer searches for the same voxel, fewer channels more blocks.
-  const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, LMG_IG_BLOCKS);
+  const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, 592);
   const int per = (I.K + (int)shares - 1) / (int)shares;
   const int ch = per > 16 ? 32 : per > 8 ? 16 : 8;
   InterpArgs J = I;
@@ -687,7 +663,7 @@ cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st) {
   unsigned nv = I.out_dim * I.out_dim * I.out_dim;
   if (nv == 0 || nb == 0 || I.K == 0) return cudaSuccess;
   const unsigned od = I.out_dim, nblk = ((od + 3) / 4) * ((od + 7) / 8) * ((od + 7) / 8);
-  dim3 grid(nblk, nb, channel_shares((unsigned long)nblk * nb, I.K, LMG_ID_BLOCKS));
+  dim3 grid(nblk, nb, channel_shares((unsigned long)nblk * nb, I.K, 1184));
   return launch_early(k_interpolate, grid, 256, 0, st, I);
 }
 

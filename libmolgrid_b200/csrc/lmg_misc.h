@@ -56,14 +56,8 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
 // average, sqrt(3) ITILE at worst.  Each axis of the box takes the smallest of a few fixed extents
 // that hold the tile, one tensor map per combination.  Tiles of 12^3 stage 5.8 input voxels per
 // output voxel on average (8^3: 6.2 after the rounding of the extents, 16^3: 4.6 but one block per SM).
-#ifndef LMG_ITILE
-#define LMG_ITILE 12
-#endif
-#ifndef LMG_ITILE_XYSTEP
-#define LMG_ITILE_XYSTEP 2
-#endif
-constexpr int ITILE = LMG_ITILE;
-constexpr int ITILE_XYSTEP = LMG_ITILE_XYSTEP;
+constexpr int ITILE = 12;
+constexpr int ITILE_XYSTEP = 2;
 constexpr int ITILE_NEED = (int)((ITILE - 1) * 1.7321f + 3.02f);  // largest extent a tile can ask for
 constexpr int ITILE_XY0 = ITILE + 2;                              // smallest x / y extent on offer
 constexpr int ITILE_NXY = (ITILE_NEED + 1 - ITILE_XY0 + ITILE_XYSTEP - 1) / ITILE_XYSTEP + 1;

@@ -134,7 +134,9 @@ int lmg_backward_static(const lmg_gridmaker* g, const lmg_atoms* a, const float*
 
 // The data-dependent check of lmg_backward (a type index >= ntypes) for the static entry point:
 // reads the status word that the last lmg_backward_static call on this device and stream left in
-// the fixed array.  A 4-byte device-to-host copy and a stream synchronisation; allocates nothing.
+// the fixed array.  Two copies to the host, the 24 bytes of the header and then the flags (one byte per 256 atoms, or
+// one per atom: up to 16384, in host memory taken for the purpose), each with a stream synchronisation; no device
+// memory is allocated.
 int lmg_static_check_status(void* stream) {
   char* ws = nullptr;
   int rc = scratch_for_current_device(&ws);

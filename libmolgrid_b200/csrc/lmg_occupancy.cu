@@ -15,7 +15,7 @@ namespace lmg {
 //
 // Bound by the output once enough blocks are at work: 28 x 48^3 is 12.4 MB an example, its mask 387 kB.  Clearing
 // the output and then storing ones into it (a warp per atom) took 207 us for 50 examples of 2000 to 4000
-// atoms, of which 90 were the clearing; this takes 126 us (floor 95).  What counted on the way: the ends of a
+// atoms, of which 90 were the clearing; this takes 126 us (floor 95), and 6 more for k_occupancy_full.  What counted on the way: the ends of a
 // run from its root, with the exact test only near a voxel (170 -> 141 us), and candidates cut to the
 // sphere's own box (141 -> 126 us).
 // ---------------------------------------------------------------------------------------------
