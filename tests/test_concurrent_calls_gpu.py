@@ -116,3 +116,26 @@ def test_captured_calls_have_their_own():
     torch.cuda.synchronize()
     w.check(out)
     x.check(later)
+
+
+def test_threads_that_end_give_their_scratch_memory_back():
+    """Calls of the compiled module on the default stream, from threads that come and go."""
+    gm = molgrid.GridMaker(0.5, 11.5)
+    N, B = 40000, 8
+    c, t, r = torch.zeros(B, N, 3, device="cuda"), torch.zeros(B, N, device="cuda"), torch.ones(B, N, device="cuda")
+    out, cen = torch.empty((B,) + tuple(gm.grid_dimensions(2)), device="cuda"), torch.zeros(B, 3, device="cuda")
+
+    def call():
+        gm.forward(cen, c, t, r, out)
+        torch.cuda.synchronize()
+
+    def once():
+        w = threading.Thread(target=call)
+        w.start()
+        w.join()
+
+    once()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(20):
+        once()
+    assert free - torch.cuda.mem_get_info()[0] < 3 * B * N * 64    # each call takes 64 bytes an atom
