@@ -218,6 +218,55 @@ def test_interpolate_backward_is_the_adjoint(gi):
         g.backward(y, tr, torch.empty_like(y) if din != dout else y)
 
 
+def _adjoint64(y, din, res_in, res_out, q, c, t):
+    """The adjoint of the trilinear resample in 64 bits, by scattering."""
+    dout = y.shape[-1]
+    w, v = q[0], np.asarray(q[1:], float)
+    n = w * w + v @ v
+    S = np.array([[0, -v[2], v[1]], [v[2], 0, -v[0]], [-v[1], v[0], 0]])
+    R = ((w * w - v @ v) * np.eye(3) + 2 * np.outer(v, v) - 2 * w * S) / n     # the inverse rotation
+    ax = (np.arange(dout) - (dout - 1) / 2) * res_out
+    p = np.stack(np.meshgrid(ax, ax, ax, indexing="ij"), -1).reshape(-1, 3)
+    g = ((p - t - c) @ R.T + c) / res_in + (din - 1) / 2
+    lo = np.floor(g).astype(int)
+    fr = g - lo
+    out = np.zeros((y.shape[0], din, din, din))
+    for k in range(8):
+        up = np.array([k >> 2, k >> 1 & 1, k & 1])
+        wt = np.where(up, fr, 1 - fr).prod(1)
+        idx = lo + up
+        ok = ((idx >= 0) & (idx < din)).all(1)
+        i, j, l = idx[ok].T
+        for ch in range(y.shape[0]):
+            np.add.at(out[ch], (i, j, l), wt[ok] * y[ch].reshape(-1)[ok])
+    return out
+
+
+@pytest.mark.parametrize("din,dout,rin,rout", [(16, 16, 0.5, 0.5), (17, 23, 0.5, 0.5), (9, 4, 0.5, 0.5), (3, 30, 0.5, 0.5),
+                                               (25, 13, 0.5, 1.0), (33, 31, 0.375, 0.375), (20, 18, 0.5, 0.45), (1, 1, 0.5, 0.5)])
+@pytest.mark.parametrize("K", [1, 8, 9])
+def test_interpolate_backward_against_64_bits(din, dout, rin, rout, K):
+    """Tiles with and without remainders, output grids as fine, coarser and finer, shares of eight channels with and
+    without a rest, positions on the planes of the input grid (no rotation, and a quarter turn).  A position is off by a
+    few roundings of some ten Angstrom, 1e-6 cells or so, and a weight by as much: 2e-5 of the sum's own norm."""
+    import libmolgrid_b200 as lmg
+    rng = np.random.default_rng(din * 100 + dout)
+    g = lmg.GridInterpolater(rin, (din - 1) * rin, rout, (dout - 1) * rout)
+    turns = [(cases.random_quaternion(rng, 1)[0], (0.25, -0.5, 1.0), (0.75, -0.3, 0.2)), ((1, 0, 0, 0), (0, 0, 0), (0, 0, 0)),
+             ((0.5 ** 0.5, 0, 0, 0.5 ** 0.5), (0, 0, 0), (rin, 0, -rin))]
+    y = rng.normal(size=(len(turns), K, dout, dout, dout)).astype(np.float32)
+    cen = np.zeros((len(turns), 3), np.float32)
+    out = torch.full((len(turns), K, din, din, din), 7.0, device="cuda")
+    trs = [make_transform(*t) for t in turns]
+    g.backward(cen, dev(y), trs, cen, out)
+    for b, (q, c, t) in enumerate(turns):
+        want = _adjoint64(y[b].astype(float), din, rin, rout, np.asarray(q, float), np.asarray(c, float), np.asarray(t, float))
+        assert np.linalg.norm(out[b].cpu().numpy() - want) <= 2e-5 * np.linalg.norm(want) + 1e-6
+    again = torch.full_like(out, 3.0)
+    g.backward(cen, dev(y), trs, cen, again)
+    assert torch.equal(out, again)
+
+
 @pytest.mark.parametrize("layer", ["python", "compiled"])
 def test_transform_known_answers_on_host_arrays_and_in_place(layer):
     """The reference's worked example (test/test_transform.py:65-140): a quarter turn about z through
