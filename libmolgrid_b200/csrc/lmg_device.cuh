@@ -59,19 +59,14 @@ struct __align__(16) ChanParam {
 __device__ __forceinline__ float next_up(float x) { return __int_as_float(__float_as_int(x) + 1); }
 __device__ __forceinline__ float next_down(float x) { return __int_as_float(__float_as_int(x) - 1); }
 
-// Largest t >= 0 with sqrtf(t) <= cut (IEEE round-to-nearest sqrt); -1 if cut is negative or NaN.
+// Largest t >= 0 with sqrtf(t) <= cut (IEEE round-to-nearest sqrt); -1 if cut is negative or NaN.  A root is rounded to
+// `cut` or less where it lies below the middle between `cut` and its successor; that middle has 25 bits, its square is
+// exact in double, and no float is exactly that square.
 __device__ __forceinline__ float sqrt_threshold(float cut) {
   if (!(cut >= 0.f)) return -1.f;
   if (isinf(cut)) return cut;
-  float t = __fmul_rn(cut, cut);
-  if (isinf(t)) t = 3.402823466e38f;
-  for (int i = 0; i < 8 && t > 0.f && __fsqrt_rn(t) > cut; i++) t = next_down(t);
-  for (int i = 0; i < 8; i++) {
-    float n = next_up(t);
-    if (isinf(n) || __fsqrt_rn(n) > cut) break;
-    t = n;
-  }
-  return t;
+  const double middle = 0.5 * ((double)cut + (double)next_up(cut));
+  return fminf(__double2float_rd(middle * middle), 3.402823466e38f);
 }
 
 // Quaternion product with libmolgrid's term order (include/libmolgrid/quaternion.h:82-91).
@@ -174,6 +169,13 @@ __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// a * b + c cut to [0, 1] by the multiply-add itself (comparisons and selections run at half its rate); zero for a NaN
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 // Two floats in a register pair: additions, products and fused multiply-adds of both in one issue slot
