@@ -782,7 +782,7 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
     }
   };
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
-  const float ta = gm.ta, ntb = -gm.tb;
+  const float ta = gm.ta, tb = gm.tb, ntb = -tb;
 
   for (Columns cols(P, part, parts); cols.more();) {
     const unsigned nkept = cols.compact<false>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
@@ -798,17 +798,17 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
       auto quad = [&](unsigned, float dxy2, float exy, const float (&d2v)[4], const float (&ev)[4],
                       const float (&)[4], auto off) {
         float v[4];
-        const Pair xy = pair(dxy2), e2 = pair(exy), ta2 = pair(ta), ntb2 = pair(ntb);
+        const Pair xy = pair(dxy2);
 #pragma unroll
         for (int j = 0; j < 4; j += 2) {
-          float s0, s1, g0, g1, t0, t1;
+          float s0, s1;
           split(add2(xy, pair(d2v[j], d2v[j + 1])), s0, s1);
-          split(mul2(e2, pair(ev[j], ev[j + 1])), g0, g1);
-          split(fma2(ta2, pair(sqrt_approx(s0), sqrt_approx(s1)), ntb2), t0, t1);
-          const Pair tq = pair(fminf(t0, 0.f), fminf(t1, 0.f));  // a NaN gives zero too
-          split(mul2(tq, tq), t0, t1);
-          v[j] = s0 <= sg ? g0 : t0;
-          v[j + 1] = s1 <= sg ? g1 : t1;
+          // the tail's root, tb - ta * distance: at most one where the tail is taken, zero beyond the cut-off and for a
+          // NaN.  Clamps and packed products instead: soft types at 28x96^3 1735 us, like this 1650; 50 x 3000 atoms
+          // on 28x48^3 168 and 164.
+          const float t0 = fma_sat(-ta, sqrt_approx(s0), tb), t1 = fma_sat(-ta, sqrt_approx(s1), tb);
+          v[j] = s0 <= sg ? exy * ev[j] : t0 * t0;
+          v[j + 1] = s1 <= sg ? exy * ev[j + 1] : t1 * t1;
           if (VEC) {
             v[j] *= P.w;
             v[j + 1] *= P.w;
