@@ -136,9 +136,9 @@ constexpr int SCAT_WARPS = 4;   // the same for the scatter kernels
 constexpr int QS_WARPS = 1;
 constexpr int SELF_SPLIT = 1200;   // most of them that four warps each take
 constexpr int SELF_ATOMS = 8192;   // most atom slots of a backward pass without k_emit
-// Gradients on loose rows, whose quads take longer than single voxels do: 2380 slots 12.2 -> 10.3 us, 4760 slots
-// 15.0 and 15.1, 7650 slots 20.0 and 21.5.
-constexpr int LOOSE_SELF_ATOMS = 4096;
+// Gradients on loose rows, whose quads take longer than single voxels do (22x41^3, by quads / by records and single
+// voxels): 1800 slots 9.6 and 9.9 us, 2400 slots 10.4 and 10.4, 3600 slots 13.3 and 12.4.
+constexpr int LOOSE_SELF_ATOMS = 2560;
 constexpr int FWD_SELF_ATOMS = 32768;  // the same for the forward pass (densities)
 constexpr int REL_SELF_ATOMS = 2560;                // ... and for relevance, whose kernel is the heaviest
 constexpr int BWD2_COLS = 256;  // compacted columns held per warp at a time
@@ -283,6 +283,8 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
   }
   const float kexp = P.inv_ar2 * NEG2_LOG2E;
   const float k4 = 4.f * P.inv_ar2, kD = -gm.D * P.inv_ar2, kE = -gm.E * P.inv_ar;  // sign of -(s*dv) folded in
+  const bool has_tail = gm.ta != 0.f || gm.tb != 0.f;
+  const float kDn = has_tail ? -0.25f * gm.D : 0.f, kEn = has_tail ? -0.25f * gm.E * P.ar : 0.f;  // in units of k4
 
   if (P.valid) {
     int grp = lane >> 2, sub = lane & 3;
@@ -319,8 +321,21 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
             dvv[k] = okv[k] ? __ldg(row + 4 * k) : 0.f;
           }
           float fsum = 0.f;  // sum over the column of -(d density / d dist) / dist * dv
+          if constexpr (MODE == 0) {
+            // Without branches: the tail's factor in units of 4 / ar^2 is at most one where it is taken, zero beyond the
+            // cut-off and for a NaN distance.  Bound by issue: 17 x 700 / 1500 / 4000 slots on 22x41^3 26.0 / 41.0 /
+            // 98.1 us with a branch per voxel, 22.7 / 35.4 / 82.9 like this; against 64 bits 2.3e-7 and 1.7e-7, because
+            // the factor's constant is exact in these units.
 #pragma unroll
-          for (int k = 0; k < ZSTEPS; k++) {
+            for (int k = 0; k < ZSTEPS; k++) {
+              const float t = fma_sat(kEn, rsqrt_approx(rsqv[k]), kDn);
+              const float f = (rsqv[k] <= P.Tg ? exy * ezt[k] : t) * dvv[k];
+              fsum += f;
+              agz = fmaf(f, dzt[k], agz);
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < (MODE == 0 ? 0 : ZSTEPS); k++) {
             if (!okv[k]) continue;
             float dz = dzt[k], rsq = rsqv[k], dv = dvv[k];
             float g = exy * ezt[k];  // exp(-2 rsq / ar^2)
@@ -384,6 +399,11 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
       }
       __syncwarp();
     }
+  }
+  if (MODE == 0) {
+    agx *= k4;
+    agy *= k4;
+    agz *= k4;
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
@@ -2314,7 +2334,7 @@ static cudaError_t backward_items(const BwdArgs& G, bool quads, dim3 grid, cudaS
 }
 
 // Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:
-// 72.5 -> 59.8 us; 50 x 3000 on 28x41^3: 525 -> 501).  Gradients with records do not (26.9 us by single voxels, 30.0
+// 72.5 -> 59.8 us; 50 x 3000 on 28x41^3: 525 -> 501).  Gradients with records do not (22.7 us by single voxels, 28.7
 // by quads), nor do type vectors (4 x 1000 atoms, 28 channels of 41^3: 212 and 251 us).
 cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
   long items = (long)G.N * (mode == 1 ? G.T : 1);

@@ -66,6 +66,22 @@ def test_index_types(port, res, points, N, shift):
         np.testing.assert_allclose(rel[b].cpu().numpy(), wrel, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wrel).max())))
 
 
+# gradients on either side of the line between the two kernels, for tails of other shapes and none (a negative multiple)
+@pytest.mark.parametrize("multiple", [1.0, 0.7, 2.5, -1.5])
+@pytest.mark.parametrize("N", [2560, 2561])
+def test_gradients_of_any_tail(port, multiple, N):
+    T = 3
+    g = lmg.GridMaker(0.5, 6.0, gaussian_radius_multiple=multiple)
+    og = port.gm(0.5, 6.0, gaussian_radius_multiple=multiple)
+    coords, types, radii = cases.index_case(5, N, T, 4.0)
+    diff_np = np.random.default_rng(N).normal(size=g.grid_dimensions(T)).astype(np.float32)
+    _, diff = inside(diff_np.shape, dev(diff_np), 0)
+    ag = torch.full((N, 3), 7.0, device="cuda")
+    g.backward((0, 0, 0), dev(coords), dev(types), dev(radii), diff, ag)
+    want = port.backward_index(og, (0, 0, 0), coords, types, radii, diff_np)
+    np.testing.assert_allclose(ag.cpu().numpy(), want, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(want).max())))
+
+
 @pytest.mark.parametrize("res,points,T", [(0.5, 13, 1), (0.5, 14, 9), (0.1, 45, 2), (1.0, 3, 35)])
 @pytest.mark.parametrize("binary", [False, True])
 @pytest.mark.parametrize("rti", [False, True])
