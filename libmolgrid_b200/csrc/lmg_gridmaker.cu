@@ -783,7 +783,9 @@ __device__ __forceinline__ unsigned quad_span(const ItemParams& P) { return (P.h
 
 // The sweep of one work item of the forward pass on aligned quads, whose constants are in P.  Of
 // `parts` warps that share an item, this one takes the `part`-th share of its columns.
-template <bool VEC, bool LOOSE>
+// LATE: the grid is zero only once wait_for_stream() returns, which is called when the first columns are at hand (zeros
+// and sums of 300 atoms in 28x48^3: 5.8 us waiting before the columns, 5.6 like this).
+template <bool VEC, bool LOOSE, bool LATE = false>
 __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemParams& P, int b, float ox, float oy,
                                                    float oz, ColBuf& buf, LooseForward (&tabs)[4], int lane,
                                                    unsigned part = 0, unsigned parts = 1) {
@@ -806,6 +808,7 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
 
   for (Columns cols(P, part, parts); cols.more();) {
     const unsigned nkept = cols.compact<false>(buf, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
+    if (LATE) wait_for_stream();
     __syncwarp();
     // With a tail the density is continuous in the distance, and the squared distances may be taken
     // in units of ar^2 (s = rsq / ar^2: one multiplication per column and z position instead of one per
@@ -1012,12 +1015,15 @@ __global__ void __launch_bounds__(32 * WARPS) k_forward_self(EmitArgs A, BwdArgs
   Rec r;
   float ox, oy, oz;
   const bool bad = make_rec_warp(A, b, a, lane, r, ox, oy, oz);
-  if (ZEROED_BEFORE) wait_for_stream();  // the output is zero
-  if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
   const ItemParams P = item_of(r);
-  if (!P.valid) return;
-  if (BINARY) forward_binary_core(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
-  else forward_quads_core<false, LOOSE>(G, P, b, ox, oy, oz, bufs[w], tabs[w], lane, w, WARPS);
+  if (BINARY) {
+    if (ZEROED_BEFORE) wait_for_stream();  // the output is zero
+    if (P.valid) forward_binary_core(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
+  } else {
+    if (P.valid) forward_quads_core<false, LOOSE, ZEROED_BEFORE>(G, P, b, ox, oy, oz, bufs[w], tabs[w], lane, w, WARPS);
+    if (ZEROED_BEFORE) wait_for_stream();  // nothing to add: not done before the zeros are, either
+  }
+  if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
 }
 
 // Vector types whose radii differ by channel: one warp takes a group of NZ_GROUP consecutive channels
@@ -1643,10 +1649,9 @@ constexpr int VA_CH = 32;  // channels per round
 constexpr int VA_SPARSE = 2;  // rounds with at most this many weighted channels sweep once per channel
 
 template <bool BINARY, bool PRECISE>
-__global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G) {
+__global__ void __launch_bounds__(QS_WARPS * 32, 32) k_forward_quads_atom(BwdArgs G) {
   wait_for_stream();
   __shared__ ColBuf bufs[QS_WARPS];
-  __shared__ ZTabs ztabs[QS_WARPS];
   __shared__ int nz_t[QS_WARPS][VA_CH];
   __shared__ float nz_w[QS_WARPS][VA_CH];
   const GMParams& gm = G.gm;
@@ -1656,7 +1661,6 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
   int b = G.b0 + bl;
   if (item >= G.N) return;
   ColBuf& buf = bufs[wid];
-  ZTabs& zt = ztabs[wid];
 
   float cx, cy, cz;
   if (G.centers != nullptr) {
@@ -1705,7 +1709,7 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
 #pragma unroll
             for (int j = 0; j < 4; j++) {
               float rsq = __fadd_rn(dxy2, d2v[j]);
-              float tq = fminf(fmaf(ta, sqrt_approx(rsq * P.inv_ar2), ntb), 0.f);
+              float tq = fma_sat(-ta, sqrt_approx(rsq * P.inv_ar2), -ntb);
               v[j] = (rsq <= P.Tg ? exy * ev[j] : tq * tq) * wk;
             }
             red_add_v4(out + off, v[0], v[1], v[2], v[3]);
@@ -1715,45 +1719,34 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
         __syncwarp();
         continue;
       }
-      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
-        __syncwarp();
-        fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
-        __syncwarp();
-        unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
-        for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
-          unsigned i = c0 + lane;
-          bool have = i < nkept;
-          unsigned cell = 0;
-          const float dxy2 = have ? buf.get(i, cell) : CUDART_NAN_F;
-          float* row = outb + (size_t)cell * dim + zc;
-          float exy = ex2_approx(dxy2 * kexp);
-          for (unsigned q = 0; q < nq; q++) {
-            float4 d2 = zt.dz2[q], e = zt.ez[q];
-            float d2v[4] = {d2.x, d2.y, d2.z, d2.w}, ev[4] = {e.x, e.y, e.z, e.w}, v[4];
+      // Many weighted channels: densities once, then a reduction for each.  The reductions bound this, by the lines that
+      // they touch: 50 x 3000 atoms on 28x48^3 with 28 / 10 / 5 / 4 weighted channels 4361 / 1782 / 966 / 818 us with a
+      // lane per column, 2964 / 1167 / 628 / 531 like this.
+      auto quad = [&](unsigned, float dxy2, float exy, const float (&d2v)[4], const float (&ev)[4], const float (&)[4],
+                      size_t off) {
+        float v[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              float rsq = __fadd_rn(dxy2, d2v[j]);
-              if (BINARY) {
-                v[j] = rsq < P.Tbin ? 1.f : 0.f;
-              } else if (PRECISE) {
-                v[j] = density_precise(rsq, P.ar, P.Tg, P.Tcut, gm.A, gm.B, gm.C);
-              } else {
-                float tq = fminf(fmaf(ta, sqrt_approx(rsq * P.inv_ar2), ntb), 0.f);
-                v[j] = rsq <= P.Tg ? exy * ev[j] : tq * tq;
-              }
-            }
-            unsigned any = __float_as_uint(v[0]) | __float_as_uint(v[1]) | __float_as_uint(v[2]) |
-                           __float_as_uint(v[3]);
-            if (any != 0u) {
-              for (int k = 0; k < nnz; k++) {
-                float wk = nz_w[wid][k];
-                red_add_v4(row + (size_t)nz_t[wid][k] * chan_stride + 4 * q, v[0] * wk, v[1] * wk, v[2] * wk,
-                           v[3] * wk);
-              }
-            }
+        for (int j = 0; j < 4; j++) {
+          float rsq = __fadd_rn(dxy2, d2v[j]);
+          if (BINARY) {
+            v[j] = rsq < P.Tbin ? 1.f : 0.f;
+          } else if (PRECISE) {
+            v[j] = density_precise(rsq, P.ar, P.Tg, P.Tcut, gm.A, gm.B, gm.C);
+          } else {
+            float tq = fma_sat(-ta, sqrt_approx(rsq * P.inv_ar2), -ntb);
+            v[j] = rsq <= P.Tg ? exy * ev[j] : tq * tq;
           }
         }
-      }
+        const unsigned any = __float_as_uint(v[0]) | __float_as_uint(v[1]) | __float_as_uint(v[2]) | __float_as_uint(v[3]);
+        if (any == 0u) return;
+        float* to = outb + off;
+        for (int k = 0; k < nnz; k++) {
+          const float wk = nz_w[wid][k];
+          red_add_v4(to + (size_t)nz_t[wid][k] * chan_stride, v[0] * wk, v[1] * wk, v[2] * wk, v[3] * wk);
+        }
+      };
+      __syncwarp();
+      qlane_sweep_span(quad_span(P), P, buf, nkept, dim, oz, gm.res, kexp, Tcull, lane, quad);
       __syncwarp();
     }
   }
@@ -1766,14 +1759,17 @@ __global__ void __launch_bounds__(QS_WARPS * 32) k_forward_quads_atom(BwdArgs G)
 // L2: every channel is read under every footprint), so what counts is how many are in flight per SM:
 // registers per warp against loads per warp.  Measured per batch of 50 (28 channels, one-hot types):
 // rounds of 16 with 4 loads together 2.79 ms, 8 / 8 2.08 ms, 14 / 7 1.82 ms, 14 / 14 1.70 ms,
-// 16 / 16 2.17 ms, 28 / 14 2.05 ms; capping the registers below what the compiler picks, blocks of
+// 16 / 16 2.17 ms, 28 / 14 2.05 ms; blocks of
 // several warps, or atoms sorted by cell (for L1 reuse between neighbours) change nothing or lose.
 constexpr int VA_BCH = 14;
 constexpr int VA_LD = 14;  // channels whose quads are requested together
 static_assert(VA_BCH % VA_LD == 0, "a round is a whole number of load batches");
 static_assert(VA_BCH <= 32, "a lane per channel of a round reads the weights");
 constexpr int VA_WARPS = BWD2_WARPS;
-constexpr int VA_REREAD = 2;  // weighted channels of a round up to which they are re-read from a list
+// Resident blocks: 80 registers instead of 128 keep more loads in flight, which the kernel waits on.  50 x 3000 atoms on
+// 28x48^3, one / 2 / 4 / 5 / 28 weighted channels an atom: 1659 / 1792 / 1849 / 2954 / 2127 us with 128 registers and up to
+// two channels of a round read again, 1584 / 1705 / 1804 / 1804 / 1804 with 80 and one.
+constexpr int VA_MINB = 22;
 
 // per-warp shared state of the kernel below
 struct VaShared {
@@ -1786,8 +1782,8 @@ struct VaShared {
 // One round of k_backward_quads_atom: channels [tb, tb + nch) under the whole footprint of the atom.
 // Lanes as (column, z-quad): the lanes of a column read neighbouring 16-byte pieces of one line in
 // every channel, a quarter of the lines a lane-per-column load touches.  The sum over weighted
-// channels that the atom gradient needs is taken inside the channel loop when many channels of the
-// round carry weight (DENSE), and from a re-read of the few that do otherwise (one-hot types: one
+// channels that the atom gradient needs is taken inside the channel loop when several channels of the
+// round carry weight (DENSE), and from a re-read of the one that does otherwise (one-hot types: one
 // extra load per quad in one round, nothing in the others).
 template <bool BINARY, bool DENSE>
 __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, VaShared& sh, const float* diffb,
@@ -1815,7 +1811,7 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
         if (BINARY) {
           v[j] = rsq < P.Tbin ? 1.f : 0.f;
         } else {
-          float tq = fminf(fmaf(ta, sqrt_approx(rsq * P.inv_ar2), ntb), 0.f);
+          float tq = fma_sat(-ta, sqrt_approx(rsq * P.inv_ar2), -ntb);
           v[j] = rsq <= P.Tg ? exy * ev[j] : tq * tq;  // tq is zero beyond the cut-off and for a NaN rsq
         }
       }
@@ -1874,7 +1870,7 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
 }
 
 template <bool BINARY>
-__global__ void __launch_bounds__(VA_WARPS * 32) k_backward_quads_atom(BwdArgs G) {
+__global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(BwdArgs G) {
   wait_for_stream();
   __shared__ VaShared shs[VA_WARPS];
   const GMParams& gm = G.gm;
@@ -1918,7 +1914,7 @@ __global__ void __launch_bounds__(VA_WARPS * 32) k_backward_quads_atom(BwdArgs G
       }
       __syncwarp();
       int nnz = __popc(m);
-      if (nnz > VA_REREAD) va_round<BINARY, true>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
+      if ((m & (m - 1u)) != 0u) va_round<BINARY, true>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
       else va_round<BINARY, false>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
     }
     // type gradients of this round
