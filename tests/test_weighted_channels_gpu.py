@@ -1,5 +1,5 @@
 """Type vectors with radii by atom and one, two, a few and all channels weighted: which of them the forward pass adds one
-by one or together, and from what the backward pass takes the atom gradient, against the CPU checker."""
+by one or together, and from what the backward pass takes the atom gradient, against the CPU oracle."""
 import numpy as np
 import pytest
 import torch
