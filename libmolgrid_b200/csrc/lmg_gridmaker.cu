@@ -401,9 +401,10 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
     }
   }
   if (MODE == 0) {
-    agx *= k4;
-    agy *= k4;
-    agz *= k4;
+    // k4 is infinite for radii below 1.1e-19, within whose reach there is hardly a voxel: nothing times it is nothing
+    agx = agx != 0.f ? agx * k4 : 0.f;
+    agy = agy != 0.f ? agy * k4 : 0.f;
+    agz = agz != 0.f ? agz * k4 : 0.f;
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {

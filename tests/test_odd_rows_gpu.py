@@ -106,3 +106,23 @@ def test_vector_types(port, res, points, T, binary, rti):
         np.testing.assert_allclose(ag.cpu().numpy(), wag, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wag).max())))
         if with_types:
             np.testing.assert_allclose(tg.cpu().numpy(), wtg, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wtg).max())))
+
+
+# radii so small that 1 / radius^2 or 4 / radius^2 is infinite, and one with finite factors, between the grid's points: the
+# kernel that prepares its own atoms, the one with records, rows of any and of 16-byte alignment
+@pytest.mark.parametrize("radius", [1e-20, 1e-19, 1e-15])
+@pytest.mark.parametrize("points,N,shift", [(13, 9, 0), (13, 2561, 0), (13, 9, 1), (16, 9, 0), (16, 9, 1)])
+def test_gradients_of_vanishing_radii(port, radius, points, N, shift):
+    T, extent = 3, (points - 1) * 0.25
+    g, og = lmg.GridMaker(0.5, 2 * extent), port.gm(0.5, 2 * extent)
+    coords, types, radii = cases.index_case(11, N, T, extent, ties=False)
+    on = np.abs(((coords + extent) * 2) % 1 - 0.5).max(axis=1) < 0.5
+    assert on.all()  # no coordinate on a plane of the grid
+    radii[::2] = radius
+    diff_np = np.random.default_rng(N).normal(size=g.grid_dimensions(T)).astype(np.float32)
+    _, diff = inside(diff_np.shape, dev(diff_np), shift)
+    ag = torch.full((N, 3), 7.0, device="cuda")
+    g.backward((0, 0, 0), dev(coords), dev(types), dev(radii), diff, ag)
+    assert not ag[::2].any()
+    want = port.backward_index(og, (0, 0, 0), coords, types, radii, diff_np)
+    np.testing.assert_allclose(ag.cpu().numpy(), want, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(want).max())))
