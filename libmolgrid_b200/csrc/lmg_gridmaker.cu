@@ -136,9 +136,10 @@ constexpr int SCAT_WARPS = 4;   // the same for the scatter kernels
 constexpr int QS_WARPS = 1;
 constexpr int SELF_SPLIT = 1200;   // most of them that four warps each take
 constexpr int SELF_ATOMS = 8192;   // most atom slots of a backward pass without k_emit
-// Gradients on loose rows, whose quads take longer than single voxels do (22x41^3, by quads / by records and single
-// voxels): 1800 slots 9.6 and 9.9 us, 2400 slots 10.4 and 10.4, 3600 slots 13.3 and 12.4.
-constexpr int LOOSE_SELF_ATOMS = 2560;
+// Gradients on loose rows, by quads / by records and single voxels, whose lines cross at different counts: 2600 and 4000
+// slots on 14x25^3 of 1 A 4.9 and 6.6, 6.1 and 7.7 us; on 8x65^3 of 0.375 A 19.6 and 20.3, 24.5 and 26.6; on 22x41^3 of
+// 0.5 A 10.8 and 10.3, 13.6 and 13.2; 4x97^3 of 0.25 A 47.6 and 41.6, 62.1 and 58.8.
+constexpr int LOOSE_SELF_ATOMS = 4096;
 constexpr int FWD_SELF_ATOMS = 32768;  // the same for the forward pass (densities)
 constexpr int REL_SELF_ATOMS = 2560;                // ... and for relevance, whose kernel is the heaviest
 constexpr int BWD2_COLS = 256;  // compacted columns held per warp at a time

@@ -68,7 +68,7 @@ def test_index_types(port, res, points, N, shift):
 
 # gradients on either side of the line between the two kernels, for tails of other shapes and none (a negative multiple)
 @pytest.mark.parametrize("multiple", [1.0, 0.7, 2.5, -1.5])
-@pytest.mark.parametrize("N", [2560, 2561])
+@pytest.mark.parametrize("N", [4096, 4097])
 def test_gradients_of_any_tail(port, multiple, N):
     T = 3
     g = lmg.GridMaker(0.5, 6.0, gaussian_radius_multiple=multiple)
@@ -111,7 +111,7 @@ def test_vector_types(port, res, points, T, binary, rti):
 # radii so small that 1 / radius^2 or 4 / radius^2 is infinite, and one with finite factors, between the grid's points: the
 # kernel that prepares its own atoms, the one with records, rows of any and of 16-byte alignment
 @pytest.mark.parametrize("radius", [1e-20, 1e-19, 1e-15])
-@pytest.mark.parametrize("points,N,shift", [(13, 9, 0), (13, 2561, 0), (13, 9, 1), (16, 9, 0), (16, 9, 1)])
+@pytest.mark.parametrize("points,N,shift", [(13, 9, 0), (13, 4097, 0), (13, 9, 1), (16, 9, 0), (16, 9, 1)])
 def test_gradients_of_vanishing_radii(port, radius, points, N, shift):
     T, extent = 3, (points - 1) * 0.25
     g, og = lmg.GridMaker(0.5, 2 * extent), port.gm(0.5, 2 * extent)
