@@ -1134,7 +1134,13 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
         }
       }
     }
-    if constexpr (MODE == 2) {
+    if constexpr (MODE == 2 && BINARY) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float t = divide_near(dvv[j], dev[j]);
+        if (__fadd_rn(dxy2, d2v[j]) < P.Tbin && dev[j] > 0.f) tg += t;
+      }
+    } else if constexpr (MODE == 2) {
       // density * dv / total density, two voxels at a time with the roundings of tail_quotient() and divide_near();
       // divisors and quotients that the short division cannot take go through the long one afterwards.  The kernel is
       // bound by issue, and this is most of it: 434 -> 388 us for 50 x 3000 atoms on 28x48^3, the same bits.
@@ -1145,28 +1151,21 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
         const Pair r = add2(pair(dxy2), pair(d2v[j], d2v[j + 1])), minus = pair(-1.f);
         float r0, r1;
         split(r, r0, r1);
-        if (BINARY) {
-          v[j] = r0 < P.Tbin ? 1.f : 0.f;
-          v[j + 1] = r1 < P.Tbin ? 1.f : 0.f;
-          in[j] = r0 < P.Tbin;
-          in[j + 1] = r1 < P.Tbin;
-        } else {
-          const Pair y = pair(rsqrt_approx(r0), rsqrt_approx(r1)), s = mul2(r, y);
-          const Pair dist = fma2(fma2(mul2(s, minus), s, r), mul2(pair(0.5f), y), s);
-          const Pair ir = pair(P.inv_ar), q = mul2(dist, ir), dr = fma2(fma2(q, pair(-P.ar), dist), ir, q);
-          const Pair nz = pair(copysignf(0.f, -gm.res));  // see interp_blend(): keeps the products' own roundings
-          const Pair t = add2(fma2(add2(fma2(pair(gm.A), dr, nz), pair(gm.B)), dr, nz), pair(gm.C));
-          float t0, t1, g0, g1;
-          split(t, t0, t1);
-          split(mul2(pair(exy), pair(ev[j], ev[j + 1])), g0, g1);
-          v[j] = r0 <= P.Tg ? g0 : fmaxf(t0, 0.f);
-          v[j + 1] = r1 <= P.Tg ? g1 : fmaxf(t1, 0.f);
-          in[j] = r0 <= P.Tcut && v[j] > 0.f;  // false for a NaN
-          in[j + 1] = r1 <= P.Tcut && v[j + 1] > 0.f;
-        }
+        const Pair y = pair(rsqrt_approx(r0), rsqrt_approx(r1)), s = mul2(r, y);
+        const Pair dist = fma2(fma2(mul2(s, minus), s, r), mul2(pair(0.5f), y), s);
+        const Pair ir = pair(P.inv_ar), q = mul2(dist, ir), dr = fma2(fma2(q, pair(-P.ar), dist), ir, q);
+        const Pair nz = pair(copysignf(0.f, -gm.res));  // see interp_blend(): keeps the products' own roundings
+        const Pair t = add2(fma2(add2(fma2(pair(gm.A), dr, nz), pair(gm.B)), dr, nz), pair(gm.C));
+        float t0, t1, g0, g1;
+        split(t, t0, t1);
+        split(mul2(pair(exy), pair(ev[j], ev[j + 1])), g0, g1);
+        v[j] = r0 <= P.Tg ? g0 : fmaxf(t0, 0.f);
+        v[j + 1] = r1 <= P.Tg ? g1 : fmaxf(t1, 0.f);
+        in[j] = r0 <= P.Tcut && v[j] > 0.f;  // false for a NaN
+        in[j + 1] = r1 <= P.Tcut && v[j + 1] > 0.f;
         const Pair n = mul2(pair(dvv[j], dvv[j + 1]), pair(v[j], v[j + 1])), d = pair(dev[j], dev[j + 1]);
-        const Pair rd = pair(rcp_approx(dev[j]), rcp_approx(dev[j + 1])), q = mul2(n, rd);
-        split(fma2(fma2(q, mul2(d, minus), n), rd, q), c[j], c[j + 1]);
+        const Pair rd = pair(rcp_approx(dev[j]), rcp_approx(dev[j + 1])), share = mul2(n, rd);
+        split(fma2(fma2(share, mul2(d, minus), n), rd, share), c[j], c[j + 1]);
       }
 #pragma unroll
       for (int j = 0; j < 4; j++) {
@@ -1376,8 +1375,15 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32, 32) k_backward_quads(BwdArgs 
 // columns, because so few atoms leave most of the chip idle and the pass lasts as long as one atom.
 // Larger inputs notice that every warp repeats the preparation (with 200 000 slots 0.230-0.316 ms
 // against 0.225 ms for k_emit and the kernel above).
-template <int MODE, bool BINARY, int WARPS, class TABS>
-__global__ void __launch_bounds__(32 * WARPS) k_backward_quads_self(EmitArgs A, BwdArgs G) {
+//
+// Relevance by four warps an atom takes 80 to 94 registers, five or six blocks an SM; up to 1000 atoms are one wave with
+// seven (`tight`; six with the larger tables of loose rows, which need them).  800 / 1000 atoms on 14x24^3 of 1 A 6.3 / 6.6 us
+// and 4.8 / 5.0, occupancy of 1000 6.5 and 4.7; 600 atoms, one wave either way, 4.1 and 4.3.
+constexpr long SELF_ROOMY = 5 * 148;
+constexpr int self_blocks(bool binary, bool loose, bool tight) { return !tight ? 0 : loose ? (binary ? 7 : 6) : binary ? 8 : 7; }
+template <int MODE, bool BINARY, int WARPS, class TABS, bool TIGHT = false>
+__global__ void __launch_bounds__(32 * WARPS, self_blocks(BINARY, !std::is_same<TABS, ZTabs>::value, TIGHT))
+    k_backward_quads_self(EmitArgs A, BwdArgs G) {
   __shared__ ColBufD bufs[WARPS];
   __shared__ TABS zts[WARPS];
   __shared__ float4 sums[WARPS];
@@ -2309,6 +2315,11 @@ template <int WARPS, class TABS>
 static cudaError_t backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st) {
   const dim3 grid(A.N, A.nb);
   if (mode == 0) return launch_early(k_backward_quads_self<0, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
+  if constexpr (WARPS > 1) {
+    if ((long)A.nb * A.N > SELF_ROOMY)
+      return launch_early(A.gm.binary ? k_backward_quads_self<2, true, WARPS, TABS, true> : k_backward_quads_self<2, false, WARPS, TABS, true>,
+                          grid, 32 * WARPS, 0, st, A, G);
+  }
   if (A.gm.binary) return launch_early(k_backward_quads_self<2, true, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
   return launch_early(k_backward_quads_self<2, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
 }

@@ -127,3 +127,25 @@ def test_roots_and_quotients(sweeps, what):
     out = (ctypes.c_uint * 2)()
     assert sweeps.run(what, out) == 0
     assert (out[0], out[1]) == (0, 0)
+
+
+# four warps an atom, on either side of the line between the kernels with room and the tight ones
+@pytest.mark.parametrize("n", [1, 740, 741, 1000])
+@pytest.mark.parametrize("points", [12, 13])
+@pytest.mark.parametrize("binary", [False, True])
+def test_relevance_of_some_atoms(n, points, binary):
+    from libmolgrid_b200 import synthetic as cases
+    from oracle.oracle import CpuOracle
+    port = CpuOracle("port")
+    gm, og = lmg.GridMaker(0.5, (points - 1) * 0.5, binary), port.gm(0.5, (points - 1) * 0.5, binary)
+    coords, types, radii = cases.index_case(n, n, T, 3.0)
+    c, t, r = (torch.from_numpy(a).cuda() for a in (coords, types, radii))
+    grid, out = torch.empty(gm.grid_dimensions(T), device="cuda"), torch.full((n,), 7.0, device="cuda")
+    gm.forward((0.0, 0.0, 0.0), c, t, r, grid)
+    diff = torch.randn_like(grid)
+    diff[0, 0, 0, 0], grid[0, 1, 1, 1] = float("inf"), 1e-35  # one beyond most cut-offs, one that the short division does not take
+    gm.backward_relevance((0.0, 0.0, 0.0), c, t, r, grid, diff, out)
+    want = port.backward_relevance(og, (0, 0, 0), coords, types, radii, grid.cpu().numpy(), diff.cpu().numpy())
+    fine = np.isfinite(want)
+    assert np.array_equal(fine, np.isfinite(out.cpu().numpy()))
+    np.testing.assert_allclose(out.cpu().numpy()[fine], want[fine], rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(want[fine]).max())))
