@@ -787,7 +787,10 @@ __device__ __forceinline__ unsigned quad_span(const ItemParams& P) { return (P.h
 // `parts` warps that share an item, this one takes the `part`-th share of its columns.
 // LATE: the grid is zero only once wait_for_stream() returns, which is called when the first columns are at hand (zeros
 // and sums of 300 atoms in 28x48^3: 5.8 us waiting before the columns, 5.6 like this).
-template <bool VEC, bool LOOSE, bool LATE = false>
+// PACKED: the tail clamped after packed multiply-adds, which is the faster form on loose rows but where four warps share an
+// atom and registers are short.  14 channels of 41^3, 1300 / 5000 atoms 9.0 / 14.4 us with the clamp in the multiply-add,
+// 8.8 / 13.9 packed, 65^3 17.9 / 27.4 and 17.1 / 26.2; 1000 atoms by four warps 7.0 and 8.4.
+template <bool VEC, bool LOOSE, bool LATE = false, bool PACKED = LOOSE>
 __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemParams& P, int b, float ox, float oy,
                                                    float oz, ColBuf& buf, LooseForward (&tabs)[4], int lane,
                                                    unsigned part = 0, unsigned parts = 1) {
@@ -828,12 +831,22 @@ __device__ __forceinline__ void forward_quads_core(const BwdArgs& G, const ItemP
         for (int j = 0; j < 4; j += 2) {
           float s0, s1;
           split(add2(xy, pair(d2v[j], d2v[j + 1])), s0, s1);
-          // the tail's root, tb - ta * distance: at most one where the tail is taken, zero beyond the cut-off and for a
-          // NaN.  Clamps and packed products instead: soft types at 28x96^3 1735 us, like this 1650; 50 x 3000 atoms
-          // on 28x48^3 168 and 164.
-          const float t0 = fma_sat(-ta, sqrt_approx(s0), tb), t1 = fma_sat(-ta, sqrt_approx(s1), tb);
-          v[j] = s0 <= sg ? exy * ev[j] : t0 * t0;
-          v[j + 1] = s1 <= sg ? exy * ev[j + 1] : t1 * t1;
+          if constexpr (PACKED) {
+            float g0, g1, t0, t1;
+            split(mul2(pair(exy), pair(ev[j], ev[j + 1])), g0, g1);
+            split(fma2(pair(ta), pair(sqrt_approx(s0), sqrt_approx(s1)), pair(ntb)), t0, t1);
+            const Pair tq = pair(fminf(t0, 0.f), fminf(t1, 0.f));  // zero beyond the cut-off and for a NaN
+            split(mul2(tq, tq), t0, t1);
+            v[j] = s0 <= sg ? g0 : t0;
+            v[j + 1] = s1 <= sg ? g1 : t1;
+          } else {
+            // the tail's root, tb - ta * distance: at most one where the tail is taken, zero beyond the cut-off and for a
+            // NaN.  Clamps and packed products instead: soft types at 28x96^3 1735 us, like this 1650; 50 x 3000 atoms
+            // on 28x48^3 168 and 164.
+            const float t0 = fma_sat(-ta, sqrt_approx(s0), tb), t1 = fma_sat(-ta, sqrt_approx(s1), tb);
+            v[j] = s0 <= sg ? exy * ev[j] : t0 * t0;
+            v[j + 1] = s1 <= sg ? exy * ev[j + 1] : t1 * t1;
+          }
           if (VEC) {
             v[j] *= P.w;
             v[j + 1] *= P.w;
@@ -1022,7 +1035,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_forward_self(EmitArgs A, BwdArgs
     if (ZEROED_BEFORE) wait_for_stream();  // the output is zero
     if (P.valid) forward_binary_core(G, P, b, ox, oy, oz, bufs[w], lane, w, WARPS);
   } else {
-    if (P.valid) forward_quads_core<false, LOOSE, ZEROED_BEFORE>(G, P, b, ox, oy, oz, bufs[w], tabs[w], lane, w, WARPS);
+    if (P.valid) forward_quads_core<false, LOOSE, ZEROED_BEFORE, LOOSE && WARPS == 1>(G, P, b, ox, oy, oz, bufs[w], tabs[w], lane, w, WARPS);
     if (ZEROED_BEFORE) wait_for_stream();  // nothing to add: not done before the zeros are, either
   }
   if (threadIdx.x == 0) put_flag(A, bl * A.N + a, A.nb * A.N, bad);
