@@ -780,6 +780,35 @@ __device__ __forceinline__ void qlane_sweep_span(unsigned span, const ItemParams
   qlane_sweep_span_t<false>(span, P, buf, nkept, dim, oz, res, kexp, Tcull, 1.f, lane, quad);
 }
 
+// The same with the lanes along z as a variable: one copy of a large `quad` instead of six.  Atoms of one launch differ in
+// their spans, and several copies of such a loop do not fit the instruction cache (k_backward_quads_atom).
+template <class BUF, class QuadFn>
+__device__ __forceinline__ void qlane_sweep_any(unsigned span, const ItemParams& P, const BUF& buf, unsigned nkept,
+                                                size_t dim, float oz, float res, float kexp, float Tcull, int lane,
+                                                QuadFn quad) {
+  const unsigned nq = span <= 2 ? 2u : span <= 6 ? span : 8u, cpi = 32u / nq, cl = lane / nq, zq = lane - cl * nq;
+  for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * nq) {
+    float d2v[4], ev[4], dzv[4];
+    float lo = CUDART_INF_F;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const unsigned zz = zc + 4 * zq + j;
+      dzv[j] = __fsub_rn(voxel_coord(oz, zz, res), P.z);
+      d2v[j] = zz >= P.loz && zz < P.hiz ? __fmul_rn(dzv[j], dzv[j]) : CUDART_NAN_F;
+      ev[j] = ex2_approx(d2v[j] * kexp);
+      lo = fminf(lo, d2v[j]);  // fminf skips the NaN entries
+    }
+    const size_t zoff = zc + 4 * zq;
+#pragma unroll 1
+    for (unsigned i = cl < cpi ? cl : nkept; i < nkept; i += cpi) {
+      unsigned row;
+      const float dxy2 = buf.get(i, row);
+      if (!(__fadd_rn(dxy2, lo) <= Tcull)) continue;  // also false for NaN: no z in range
+      quad(i, dxy2, ex2_approx(dxy2 * kexp), d2v, ev, dzv, (size_t)row * dim + zoff);
+    }
+  }
+}
+
 // number of aligned quads between the first and the last z of a footprint
 __device__ __forceinline__ unsigned quad_span(const ItemParams& P) { return (P.hiz - (P.loz & ~3u) + 3) >> 2; }
 
@@ -1775,22 +1804,25 @@ __global__ void __launch_bounds__(QS_WARPS * 32, 32) k_forward_quads_atom(BwdArg
 
 // Backward for the same layout: atom gradient = sum over voxels of s * delta * (sum_t w_t diff_t),
 // type gradient of EVERY channel = sum over voxels of density * diff_t (src/grid_maker.cpp:508-517).
-// A lane keeps the type gradients of a round's channels in registers; rounds of VA_BCH channels,
-// the quads of VA_LD channels requested together.  The kernel waits on those loads (they come from
-// L2: every channel is read under every footprint), so what counts is how many are in flight per SM:
-// registers per warp against loads per warp.  Measured per batch of 50 (28 channels, one-hot types):
+// A lane keeps the type gradients of a round's CH channels in registers; their quads are requested together.  The kernel
+// waits on those loads (they come from L2: every channel is read under every footprint), so what counts is how many are in
+// flight per SM: registers per warp against loads per warp.  Measured per batch of 50 (28 channels, one-hot types):
 // rounds of 16 with 4 loads together 2.79 ms, 8 / 8 2.08 ms, 14 / 7 1.82 ms, 14 / 14 1.70 ms,
 // 16 / 16 2.17 ms, 28 / 14 2.05 ms; blocks of
 // several warps, or atoms sorted by cell (for L1 reuse between neighbours) change nothing or lose.
+// Few channels get shorter rounds, without loads and sums for channels that there are not (16 x 1000 atoms on 48^3, one /
+// all weighted): 4 channels 100 / 107 us in rounds of 14, 60 / 56 in rounds of 4; 7 channels 102 / 110 and 73 / 74 in
+// rounds of 7.
 constexpr int VA_BCH = 14;
-constexpr int VA_LD = 14;  // channels whose quads are requested together
-static_assert(VA_BCH % VA_LD == 0, "a round is a whole number of load batches");
 static_assert(VA_BCH <= 32, "a lane per channel of a round reads the weights");
 constexpr int VA_WARPS = BWD2_WARPS;
-// Resident blocks: 80 registers instead of 128 keep more loads in flight, which the kernel waits on.  50 x 3000 atoms on
-// 28x48^3, one / 2 / 4 / 5 / 28 weighted channels an atom: 1659 / 1792 / 1849 / 2954 / 2127 us with 128 registers and up to
-// two channels of a round read again, 1584 / 1705 / 1804 / 1804 / 1804 with 80 and one.
-constexpr int VA_MINB = 22;
+// What else counts is the size of the loop.  A round's loop over quads comes in two forms (DENSE below); with a copy of
+// each for every span of quads, atoms that take different ones turn each other's out of the instruction cache.
+// 50 x 3000 atoms on 28x48^3, one / 2 / 5 / 28 weighted channels an atom: copies, 80 registers and 22 blocks an SM
+// 1667 / 3233 / 3364 / 1898 us (an atom's channels of one round are then DENSE, of the other not), copies and 96
+// registers 1741 / 1778 / 2943 / 2222; one copy of each form and 96 registers 1681 / 1630 / 1656 / 1739, with 80 registers
+// 1684 / 1780 / 1846 / 2054, with 128 2447 / 2521 / 2402 / 2451.
+constexpr int VA_MINB = 20;
 
 // per-warp shared state of the kernel below
 struct VaShared {
@@ -1800,16 +1832,31 @@ struct VaShared {
   float nz_w[VA_BCH];
 };
 
+// A quad of the gradient, zero where there is none.  In order: the loads of a round are issued one after the other before
+// any is used.  Placed by the compiler, some waited for others: 2430 us with one weighted channel instead of 1681.
+__device__ __forceinline__ float4 load_quad(const float4* p, bool there) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.u32 q, %5, 0;\n\t"
+      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
+      "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+      "@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+      : "l"(p), "r"((unsigned)there));
+  return v;
+}
+
 // One round of k_backward_quads_atom: channels [tb, tb + nch) under the whole footprint of the atom.
 // Lanes as (column, z-quad): the lanes of a column read neighbouring 16-byte pieces of one line in
 // every channel, a quarter of the lines a lane-per-column load touches.  The sum over weighted
 // channels that the atom gradient needs is taken inside the channel loop when several channels of the
 // round carry weight (DENSE), and from a re-read of the one that does otherwise (one-hot types: one
 // extra load per quad in one round, nothing in the others).
-template <bool BINARY, bool DENSE>
+template <bool BINARY, bool DENSE, int CH>
 __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, VaShared& sh, const float* diffb,
                                          int tb, int nch, int nnz, float ox, float oy, float oz,
-                                         float (&tgacc)[VA_BCH], float& agx, float& agy, float& agz, int lane) {
+                                         float (&tgacc)[CH], float& agx, float& agy, float& agz, int lane) {
   const GMParams& gm = G.gm;
   const size_t dim = gm.dim;
   const size_t cs4 = dim * dim * dim / 4;  // channel stride in quads
@@ -1837,40 +1884,32 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
         }
       }
       const float4* qp = reinterpret_cast<const float4*>(diffb + off) + (size_t)tb * cs4;
+      // the channels requested together, then used
+      float4 dv[CH];
 #pragma unroll
-      for (int c4 = 0; c4 < VA_BCH; c4 += VA_LD) {
-        if (c4 >= nch) break;
-        // a batch of channels requested together, then used
-        float4 dv[VA_LD];
+      for (int u = 0; u < CH; u++) {
+        dv[u] = load_quad(qp, u < nch);
+        qp += cs4;
+      }
 #pragma unroll
-        for (int u = 0; u < VA_LD; u++) {
-          dv[u] = (c4 + u < nch) ? __ldg(qp) : make_float4(0.f, 0.f, 0.f, 0.f);
-          qp += cs4;
-        }
-#pragma unroll
-        for (int u = 0; u < VA_LD; u++) {
-          tgacc[c4 + u] = fmaf(v[0], dv[u].x, fmaf(v[1], dv[u].y, fmaf(v[2], dv[u].z,
-                               fmaf(v[3], dv[u].w, tgacc[c4 + u]))));
-          if (DENSE) {
-            float wk = sh.w[c4 + u];
-            dsum[0] = fmaf(wk, dv[u].x, dsum[0]);
-            dsum[1] = fmaf(wk, dv[u].y, dsum[1]);
-            dsum[2] = fmaf(wk, dv[u].z, dsum[2]);
-            dsum[3] = fmaf(wk, dv[u].w, dsum[3]);
-          }
+      for (int u = 0; u < CH; u++) {
+        tgacc[u] = fmaf(v[0], dv[u].x, fmaf(v[1], dv[u].y, fmaf(v[2], dv[u].z, fmaf(v[3], dv[u].w, tgacc[u]))));
+        if (DENSE) {
+          const float wk = sh.w[u];
+          dsum[0] = fmaf(wk, dv[u].x, dsum[0]);
+          dsum[1] = fmaf(wk, dv[u].y, dsum[1]);
+          dsum[2] = fmaf(wk, dv[u].z, dsum[2]);
+          dsum[3] = fmaf(wk, dv[u].w, dsum[3]);
         }
       }
       if (!DENSE) {
         if (nnz == 0) return;  // the same for every lane
-        const float4* q0 = reinterpret_cast<const float4*>(diffb + off) + (size_t)tb * cs4;
-        for (int k = 0; k < nnz; k++) {
-          float4 d = __ldg(q0 + (size_t)sh.nz_t[k] * cs4);
-          float wk = sh.nz_w[k];
-          dsum[0] = fmaf(wk, d.x, dsum[0]);
-          dsum[1] = fmaf(wk, d.y, dsum[1]);
-          dsum[2] = fmaf(wk, d.z, dsum[2]);
-          dsum[3] = fmaf(wk, d.w, dsum[3]);
-        }
+        const float4 d = __ldg(reinterpret_cast<const float4*>(diffb + off) + (size_t)(tb + sh.nz_t[0]) * cs4);
+        const float wk = sh.nz_w[0];
+        dsum[0] = wk * d.x;
+        dsum[1] = wk * d.y;
+        dsum[2] = wk * d.z;
+        dsum[3] = wk * d.w;
       }
       float fsum = 0.f;
 #pragma unroll
@@ -1885,12 +1924,12 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
       agx = fmaf(fsum, buf.dx[i], agx);
       agy = fmaf(fsum, buf.dy[i], agy);
     };
-    qlane_sweep_span(span, P, buf, nkept, dim, oz, gm.res, kexp, Tcull, lane, quad);
+    qlane_sweep_any(span, P, buf, nkept, dim, oz, gm.res, kexp, Tcull, lane, quad);
     __syncwarp();
   }
 }
 
-template <bool BINARY>
+template <bool BINARY, int CH>
 __global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(BwdArgs G) {
   wait_for_stream();
   __shared__ VaShared shs[VA_WARPS];
@@ -1917,17 +1956,17 @@ __global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(
   const float* wrow = G.type_vector + ai * G.T;
   float agx = 0.f, agy = 0.f, agz = 0.f;
 
-  for (int tb = 0; tb < G.T; tb += VA_BCH) {
-    const int nch = min(VA_BCH, G.T - tb);
-    float tgacc[VA_BCH];
+  for (int tb = 0; tb < G.T; tb += CH) {
+    const int nch = min(CH, G.T - tb);
+    float tgacc[CH];
 #pragma unroll
-    for (int c = 0; c < VA_BCH; c++) tgacc[c] = 0.f;
+    for (int c = 0; c < CH; c++) tgacc[c] = 0.f;
     if (P.valid) {
       // the round's weights, and the list of the channels that carry one
       __syncwarp();
       float w = lane < nch ? wrow[tb + lane] : 0.f;
       unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
-      if (lane < VA_BCH) sh.w[lane] = w;
+      if (lane < CH) sh.w[lane] = w;
       if (w != 0.f) {
         int k = __popc(m & ((1u << lane) - 1u));
         sh.nz_t[k] = lane;
@@ -1935,12 +1974,12 @@ __global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(
       }
       __syncwarp();
       int nnz = __popc(m);
-      if ((m & (m - 1u)) != 0u) va_round<BINARY, true>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
-      else va_round<BINARY, false>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
+      if ((m & (m - 1u)) != 0u) va_round<BINARY, true, CH>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
+      else va_round<BINARY, false, CH>(G, P, sh, diffb, tb, nch, nnz, ox, oy, oz, tgacc, agx, agy, agz, lane);
     }
     // type gradients of this round
 #pragma unroll
-    for (int c = 0; c < VA_BCH; c++) {
+    for (int c = 0; c < CH; c++) {
       float x = tgacc[c];
 #pragma unroll
       for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -2355,6 +2394,13 @@ static cudaError_t backward_items(const BwdArgs& G, bool quads, dim3 grid, cudaS
   return launch_early(k_backward_quads<MODE, BINARY, ZTabs>, grid, BWD2_WARPS * 32, 0, st, G);
 }
 
+template <bool BINARY>
+static cudaError_t backward_quads_atom(const BwdArgs& G, dim3 grid, cudaStream_t st) {
+  return launch_early(G.T <= 4 ? k_backward_quads_atom<BINARY, 4> : G.T <= 7 ? k_backward_quads_atom<BINARY, 7>
+                                                                             : k_backward_quads_atom<BINARY, VA_BCH>,
+                      grid, VA_WARPS * 32, 0, st, G);
+}
+
 // Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:
 // 72.5 -> 59.8 us; 50 x 3000 on 28x41^3: 525 -> 501).  Gradients with records do not (22.7 us by single voxels, 28.7
 // by quads), nor do type vectors (4 x 1000 atoms, 28 channels of 41^3: 212 and 251 us).
@@ -2376,8 +2422,7 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
     dim3 ga((unsigned)((G.N + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
     dim3 gv((unsigned)((G.N + VA_WARPS - 1) / VA_WARPS), G.nb);
     if (G.type_gradients == nullptr) return launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
-    return bin ? launch_early(k_backward_quads_atom<true>, gv, VA_WARPS * 32, 0, st, G)
-               : launch_early(k_backward_quads_atom<false>, gv, VA_WARPS * 32, 0, st, G);
+    return bin ? backward_quads_atom<true>(G, gv, st) : backward_quads_atom<false>(G, gv, st);
   }
   cudaError_t e;
   if (quads && G.type_gradients == nullptr) {

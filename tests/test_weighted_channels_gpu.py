@@ -10,8 +10,8 @@ from libmolgrid_b200 import synthetic as cases
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T", [3, 14, 15, 33])
-@pytest.mark.parametrize("weighted", [0, 1, 2, 3, 40])
+@pytest.mark.parametrize("T", [3, 4, 5, 7, 8, 14, 15, 33])
+@pytest.mark.parametrize("weighted", [0, 1, 2, 3, 13, 40])
 @pytest.mark.parametrize("binary,multiple", [(False, 1.0), (True, 1.0), (False, 3.0), (False, -1.5)])
 def test_weighted_channels(T, weighted, binary, multiple):
     from oracle.oracle import CpuOracle
@@ -20,8 +20,10 @@ def test_weighted_channels(T, weighted, binary, multiple):
     rng = np.random.default_rng(T * 50 + weighted)
     tv[:] = 0
     for a in range(N):  # neighbouring channels, so that several fall into one round, from any first one
+        first = int(rng.integers(T))
         for k in range(min(weighted, T)):
-            tv[a, (int(rng.integers(T)) if k == 0 else int(np.flatnonzero(tv[a])[0]) + k) % T] = rng.uniform(0.1, 1)
+            tv[a, (first + k) % T] = rng.uniform(0.1, 1)
+    assert ((tv != 0).sum(axis=1) == min(weighted, T)).all()
     g = lmg.GridMaker(0.5, 7.5, binary, gaussian_radius_multiple=multiple)
     og = port.gm(0.5, 7.5, binary, gaussian_radius_multiple=multiple)
     assert g.grid_dimensions(T)[1] % 4 == 0
