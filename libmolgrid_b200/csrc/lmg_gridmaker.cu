@@ -1910,6 +1910,23 @@ __device__ __forceinline__ void va_round(const BwdArgs& G, const ItemParams& P, 
         dsum[1] = wk * d.y;
         dsum[2] = wk * d.z;
         dsum[3] = wk * d.w;
+      } else {
+        // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none
+        // either, and the sum is taken again.
+        const float whole = (dsum[0] + dsum[1]) + (dsum[2] + dsum[3]);
+        if (whole != whole) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) dsum[j] = 0.f;
+#pragma unroll 1
+          for (int k = 0; k < nnz; k++) {
+            const float4 d = __ldg(reinterpret_cast<const float4*>(diffb + off) + (size_t)(tb + sh.nz_t[k]) * cs4);
+            const float wk = sh.nz_w[k];
+            dsum[0] = fmaf(wk, d.x, dsum[0]);
+            dsum[1] = fmaf(wk, d.y, dsum[1]);
+            dsum[2] = fmaf(wk, d.z, dsum[2]);
+            dsum[3] = fmaf(wk, d.w, dsum[3]);
+          }
+        }
       }
       float fsum = 0.f;
 #pragma unroll

@@ -38,3 +38,28 @@ def test_weighted_channels(T, weighted, binary, multiple):
     wag, wtg = port.backward_vector(og, (0, 0, 0), coords, tv, radii, diff)
     np.testing.assert_allclose(ag.cpu().numpy(), wag, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wag).max())))
     np.testing.assert_allclose(tg.cpu().numpy(), wtg, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wtg).max())))
+
+
+@pytest.mark.parametrize("T,weighted", [(14, (3, 4)), (15, (0, 13)), (28, (2, 9, 11)), (16, (5,))])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), -3.4e38])
+@pytest.mark.parametrize("binary", [False, True])
+def test_unweighted_channels_do_not_reach_the_atoms(T, weighted, value, binary):
+    """Gradients of the grid that are no numbers, in the channels without weight beside those with one: the atom gradients and
+    the weighted channels' type gradients are those of a grid with zeros there."""
+    from oracle.oracle import CpuOracle
+    port, N = CpuOracle("port"), 13
+    coords, tv, radii = cases.vector_case(T, N, T, 4.0, rti=False)
+    rng = np.random.default_rng(T)
+    tv[:] = 0
+    tv[:, weighted] = rng.uniform(0.1, 1, (N, len(weighted)))
+    g, og = lmg.GridMaker(0.5, 7.5, binary), port.gm(0.5, 7.5, binary)
+    diff = np.zeros(g.grid_dimensions(T), np.float32)
+    diff[list(weighted)] = rng.normal(size=(len(weighted),) + diff.shape[1:])
+    wag, wtg = port.backward_vector(og, (0, 0, 0), coords, tv, radii, diff)
+    diff[[t for t in range(T) if t not in weighted]] = value
+    dc, dt, dr = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (coords, tv, radii))
+    ag, tg = torch.full((N, 3), 7.0, device="cuda"), torch.full((N, T), 7.0, device="cuda")
+    g.backward((0, 0, 0), dc, dt, dr, torch.from_numpy(diff).cuda(), ag, tg)
+    np.testing.assert_allclose(ag.cpu().numpy(), wag, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wag).max())))
+    tg, wtg = tg.cpu().numpy()[:, weighted], wtg[:, weighted]
+    np.testing.assert_allclose(tg, wtg, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wtg).max())))
