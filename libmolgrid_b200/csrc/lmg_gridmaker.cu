@@ -1696,12 +1696,22 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_MINB) k_second_quads_nz(BwdA
 // one work item per (atom, channel).  Channels are handled in rounds of VA_CH.
 // ---------------------------------------------------------------------------------------------
 constexpr int VA_CH = 32;  // channels per round
-constexpr int VA_SPARSE = 2;  // rounds with at most this many weighted channels sweep once per channel
+// Rounds with at most this many weighted channels sweep once per channel, but for densities in the reference's order of
+// operations.  Three: 50 x 3000 atoms on 28x48^3 511 us together and 482 one by one, 8 x 1000 on 28x24^3 of 1 A 14.1 and 15.8.
+// Occupancy with one / two: 8 x 1000 atoms on 28x48^3 30.0 / 33.2 us together, 26.9 / 31.4 one by one.
+constexpr int VA_SPARSE = 2;
+// Densities in the reference's order of operations cost most of the sweep, and a lane per column branches less among them than
+// lanes along z do.  One / 5 / 8 / 28 weighted channels at `grm` 3: 8 x 1000 atoms on 28x48^3 300 / 421 / 598 / 1835 us like that, 467 /
+// 526 / 540 / 1300 along z; 2 x 300 on 28x96^3 of 0.25 A 1040 / 1190 / 1291 / 2793 and 1594 / 1713 / 1698 / 2199; 40 atoms on 28x48^3
+// 144 / 153 / 149 / 257 and 208 / 206 / 202 / 277.
+constexpr int VA_COLUMNS = 6, VA_COLUMNS_FEW = 12;  // most channels for that, and for passes of few atoms
+constexpr long VA_FEW = 1200;
 
 template <bool BINARY, bool PRECISE>
 __global__ void __launch_bounds__(QS_WARPS * 32, 32) k_forward_quads_atom(BwdArgs G) {
   wait_for_stream();
   __shared__ ColBuf bufs[QS_WARPS];
+  __shared__ ZTabs ztabs[PRECISE ? QS_WARPS : 1];
   __shared__ int nz_t[QS_WARPS][VA_CH];
   __shared__ float nz_w[QS_WARPS][VA_CH];
   const GMParams& gm = G.gm;
@@ -1746,7 +1756,37 @@ __global__ void __launch_bounds__(QS_WARPS * 32, 32) k_forward_quads_atom(BwdArg
     __syncwarp();
     for (Columns cols(P); cols.more();) {
       const unsigned nkept = cols.compact<false>(buf, P, Tcull, ox, oy, gm.res, gm.dim, lane);
-      if (!BINARY && !PRECISE && nnz <= VA_SPARSE) {
+      if (PRECISE && nnz <= ((long)G.N * G.nb <= VA_FEW ? VA_COLUMNS_FEW : VA_COLUMNS)) {
+        ZTabs& zt = ztabs[wid];
+        for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+          __syncwarp();
+          fill_ztabs(zt, zc, P, oz, gm.res, kexp, lane);
+          __syncwarp();
+          const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+          for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
+            const unsigned i = c0 + lane;
+            unsigned cell = 0;
+            const float dxy2 = i < nkept ? buf.get(i, cell) : CUDART_NAN_F;
+            float* row = outb + (size_t)cell * dim + zc;
+            for (unsigned q = 0; q < nq; q++) {
+              const float4 d2 = zt.dz2[q];
+              const float d2v[4] = {d2.x, d2.y, d2.z, d2.w};
+              float v[4];
+#pragma unroll
+              for (int j = 0; j < 4; j++)
+                v[j] = density_precise(__fadd_rn(dxy2, d2v[j]), P.ar, P.Tg, P.Tcut, gm.A, gm.B, gm.C);
+              if ((__float_as_uint(v[0]) | __float_as_uint(v[1]) | __float_as_uint(v[2]) | __float_as_uint(v[3])) == 0u) continue;
+              for (int k = 0; k < nnz; k++) {
+                const float wk = nz_w[wid][k];
+                red_add_v4(row + (size_t)nz_t[wid][k] * chan_stride + 4 * q, v[0] * wk, v[1] * wk, v[2] * wk, v[3] * wk);
+              }
+            }
+          }
+        }
+        __syncwarp();
+        continue;
+      }
+      if (!PRECISE && nnz <= VA_SPARSE) {
         // few weighted channels (one-hot types): one sweep per channel in the lane layout of the
         // index-typed forward, whose reductions touch a quarter of the rows
         __syncwarp();
@@ -1760,7 +1800,7 @@ __global__ void __launch_bounds__(QS_WARPS * 32, 32) k_forward_quads_atom(BwdArg
             for (int j = 0; j < 4; j++) {
               float rsq = __fadd_rn(dxy2, d2v[j]);
               float tq = fma_sat(-ta, sqrt_approx(rsq * P.inv_ar2), -ntb);
-              v[j] = (rsq <= P.Tg ? exy * ev[j] : tq * tq) * wk;
+              v[j] = BINARY ? (rsq < P.Tbin ? wk : 0.f) : (rsq <= P.Tg ? exy * ev[j] : tq * tq) * wk;
             }
             red_add_v4(out + off, v[0], v[1], v[2], v[3]);
           };

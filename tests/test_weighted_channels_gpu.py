@@ -63,3 +63,26 @@ def test_unweighted_channels_do_not_reach_the_atoms(T, weighted, value, binary):
     np.testing.assert_allclose(ag.cpu().numpy(), wag, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wag).max())))
     tg, wtg = tg.cpu().numpy()[:, weighted], wtg[:, weighted]
     np.testing.assert_allclose(tg, wtg, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(wtg).max())))
+
+
+# densities in the reference's order of operations: few and many atoms, with few, more and many weighted channels of a round
+@pytest.mark.parametrize("N,weighted", [(30, 12), (30, 13), (1200, 12), (1201, 6), (1201, 7)])
+@pytest.mark.parametrize("points", [12, 40])
+def test_precise_densities_of_weighted_channels(N, weighted, points):
+    from oracle.oracle import CpuOracle
+    port, T = CpuOracle("port"), 16
+    res = 0.5 if points < 20 else 0.125  # footprints of one and of two passes along z
+    if points > 20 and N > 1000:
+        pytest.skip("one size of grid is enough for many atoms")
+    coords, tv, radii = cases.vector_case(N, N, T, (points - 1) * res / 2, rti=False)
+    rng = np.random.default_rng(N)
+    tv[:] = 0
+    for a in range(N):
+        tv[a, rng.permutation(T)[:weighted]] = rng.uniform(0.1, 1, weighted)
+    g = lmg.GridMaker(res, (points - 1) * res, gaussian_radius_multiple=2.5)
+    og = port.gm(res, (points - 1) * res, gaussian_radius_multiple=2.5)
+    out = torch.full(g.grid_dimensions(T), 7.0, device="cuda")
+    g.forward((0, 0, 0), *(torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (coords, tv, radii)), out)
+    want = port.forward_vector(og, (0, 0, 0), coords, tv, radii)
+    # N terms of at most one a voxel in any order: a rounding of the running sum each
+    np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-5, atol=2e-6 * max(1.0, N / 50))
