@@ -817,33 +817,62 @@ __global__ void __launch_bounds__(256) k_interpolate_scatter(InterpArgs I, unsig
   }
 }
 
-cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames& W, int nb, cudaStream_t st) {
+// The examples of one pass, which all take the same kernel.
+static cudaError_t interpolate_backward_run(const InterpArgs& I, const GatherFrames& W, int nb, bool cells, cudaStream_t st) {
   const unsigned id = I.in_dim, tiles = ((id + IG_X - 1) / IG_X) * ((id + IG_Y - 1) / IG_Y) * ((id + IG_Z - 1) / IG_Z);
-  if (tiles == 0 || nb == 0 || I.K == 0) return cudaSuccess;
-  // Each output voxel has a cube of its own, f cells wide and turned, so that no more of them lie in a box of cells than
-  // volumes of such cubes fit in the box widened by their half diagonal on each side: resolutions that differ by 2 %
-  // at most, or a coarser output.  Finer ones would need more room than five blocks an SM have.
-  float slack = 0.f;
-  for (int i = 0; i < nb; i++) slack = fmaxf(slack, W.ex[i].slack);
-  const double f = (double)I.out_res / I.in_res, more = 2.0 * slack + 1.7321 * f;
-  cudaError_t e = cudaSuccess;
-  if (1.005 * (IC_X + more) * (IC_Y + more) * (IC_Z + more) < IC_CAP * f * f * f) {
+  if (cells) {
     // shares of the channels as long as the blocks fit the chip at a time
     const unsigned long room = 148ul * IC_MINB / ((unsigned long)tiles * nb), groups = ((unsigned long)I.K + IC_CH - 1) / IC_CH;
-    e = launch_early(k_interpolate_cells, dim3(tiles, nb, (unsigned)std::max(1ul, std::min(room, groups))), IG_THREADS, 0, st, I, W);
-  } else {
-    // More channels per block mean fewer searches for the same voxel, fewer channels more blocks.
-    const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, 592);
-    const int per = (I.K + (int)shares - 1) / (int)shares;
-    const int ch = per > 16 ? 32 : per > 8 ? 16 : 8;
-    InterpArgs J = I;
-    for (int left = (I.K + ch - 1) / ch; left > 0 && e == cudaSuccess; left -= 65535, J.c0 += 65535 * ch)
-      e = launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>,
-                       dim3(tiles, nb, left < 65535 ? left : 65535), IG_THREADS, 0, st, J, W);
+    return launch_early(k_interpolate_cells, dim3(tiles, nb, (unsigned)std::max(1ul, std::min(room, groups))), IG_THREADS, 0, st, I, W);
   }
+  // More channels per block mean fewer searches for the same voxel, fewer channels more blocks.
+  const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, 592);
+  const int per = (I.K + (int)shares - 1) / (int)shares;
+  const int ch = per > 16 ? 32 : per > 8 ? 16 : 8;
+  InterpArgs J = I;
+  cudaError_t e = cudaSuccess;
+  for (int left = (I.K + ch - 1) / ch; left > 0 && e == cudaSuccess; left -= 65535, J.c0 += 65535 * ch)
+    e = launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>,
+                     dim3(tiles, nb, left < 65535 ? left : 65535), IG_THREADS, 0, st, J, W);
+  return e;
+}
+
+cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames& W, int nb, cudaStream_t st) {
+  if (I.in_dim == 0 || nb == 0 || I.K == 0) return cudaSuccess;
+  // Each output voxel has a cube of its own, f cells wide and turned, so that no more of them lie in a box of cells than
+  // volumes of such cubes fit in the box widened by their half diagonal on each side: resolutions that are equal, with
+  // centres up to some 2600 cells away, outputs up to 0.28 % finer about the origin, and coarser ones.  Finer ones would
+  // need more room than five blocks an SM have.
+  const double f = (double)I.out_res / I.in_res;
+  auto fits = [&](int i) {
+    const double more = 2.0 * W.ex[i].slack + 1.7321 * f;
+    return 1.005 * (IC_X + more) * (IC_Y + more) * (IC_Z + more) < IC_CAP * f * f * f;
+  };
+  // Every example is judged by itself: the kernels sum in different orders, and its gradient is not to depend on the
+  // others of its call.  Neighbours that agree share a launch (nothing is looked up for maps without use, which agree with
+  // any): one for nearly all calls.
   unsigned long long which = 0;
   static_assert(INTERP_MAX_EX <= 64, "a bit per example");
-  for (int i = 0; i < nb; i++) which |= (unsigned long long)(W.ex[i].sane == 0) << i;
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < nb && e == cudaSuccess;) {
+    const int first = i;
+    int cells = -1;
+    for (; i < nb; i++) {
+      if (W.ex[i].sane == 0) which |= 1ull << i;
+      else if (cells < 0) cells = fits(i);
+      else if (cells != (int)fits(i)) break;
+    }
+    if (first == 0 && i == nb) {
+      e = interpolate_backward_run(I, W, nb, cells != 0, st);
+    } else {
+      InterpArgs J = I;
+      GatherFrames V;
+      J.b0 += first;
+      std::copy(I.ex + first, I.ex + i, J.ex);
+      std::copy(W.ex + first, W.ex + i, V.ex);
+      e = interpolate_backward_run(J, V, i - first, cells != 0, st);
+    }
+  }
   if (which == 0 || e != cudaSuccess || I.out_dim == 0) return e;
   const size_t voxels = (size_t)I.out_dim * I.out_dim * I.out_dim;
   return launch_early(k_interpolate_scatter, dim3((unsigned)((voxels + 255) / 256), nb), 256, 0, st, I, which);

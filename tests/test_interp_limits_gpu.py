@@ -1,6 +1,7 @@
 """GridInterpolater at its limits: more channels than a launch has blocks, maps that have no use."""
 import ctypes
 
+import numpy as np
 import pytest
 import torch
 
@@ -67,3 +68,30 @@ def test_backward_of_maps_without_use(odd):
         assert abs(float(left - right)) <= 16 * 2.0 ** -24 * scale
     if odd == "far":
         assert not out[1].any() and not back[1].any()
+
+
+@pytest.mark.parametrize("odd", ["infinite", "nan", "far", "zero", "distant"])
+@pytest.mark.parametrize("rout,K", [(0.5, 3), (0.5, 40), (1.0, 9), (0.45, 9)])
+def test_gradients_do_not_depend_on_the_other_examples(odd, rout, K):
+    """The same bits alone and beside an example whose map has no use, or whose positions are rounded so far from the origin
+    (a rotation about a point 3000 cells away) that the sums take another order for it."""
+    n, m = 18, 17
+    gi = lmg.GridInterpolater(0.5, (n - 1) * 0.5, rout, (m - 1) * rout)
+    inf, nan = float("inf"), float("nan")
+    one = lmg.Quaternion(1, 0, 0, 0)
+    t = {"infinite": lmg.Transform(one, (0, 0, 0), (inf, 0, 0)), "nan": lmg.Transform(lmg.Quaternion(nan, 0, 0, 0)),
+         "far": lmg.Transform(one, (0, 0, 0), (3e7, 0, 0)), "zero": lmg.Transform(lmg.Quaternion(0, 0, 0, 0)),
+         "distant": lmg.Transform(lmg.Quaternion(0.8, 0.6, 0, 0), (1500.0, 0, 0), (0.25, -0.5, 0))}[odd]
+    trs = [lmg.Transform(lmg.Quaternion(0.6, 0, 0.8, 0), (0, 0, 0), (0.3, -0.2, 0.1)), t,
+           lmg.Transform(lmg.Quaternion(0.5, -0.5, 0.1, 0.7), (0.25, 1, -0.5), (0.7, 0.1, -0.4))]
+    cen = np.zeros((3, 3), np.float32)
+    g = torch.randn((3, K, m, m, m), device="cuda")
+    together = torch.full((3, K, n, n, n), 7.0, device="cuda")
+    gi.backward(cen, g, trs, cen, together)
+    for b in range(3):
+        if b == 1 and odd not in ("far", "distant"):
+            continue  # positions that are no numbers: added up by reductions, in no fixed order
+        alone = torch.full((1, K, n, n, n), 8.0, device="cuda")
+        gi.backward(cen[b:b + 1], g[b:b + 1].clone(), trs[b:b + 1], cen[b:b + 1], alone)
+        assert torch.equal(alone[0], together[b])
+        assert bool(alone.any()) == (b != 1 or odd == "distant")
