@@ -529,7 +529,9 @@ constexpr int IG_THREADS = IG_X * IG_Y * IG_Z;
 constexpr int IG_CAP = 16;                   // entries per list; a list that fills up is worked off in between
 constexpr int IG_MINB = 3;
 
-template <int CH>
+// BIG: an output grid of 2^32 voxels or more; offsets are then counted from the plane of the first candidate of a list, whose
+// entries, neighbours, span few planes.
+template <int CH, bool BIG = false>
 __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(InterpArgs I, GatherFrames G) {
   __shared__ uint2 list[IG_CAP][IG_THREADS];  // first the candidates (i << 16 | j, k), then (weight, offset)
   const int tid = threadIdx.x, bl = blockIdx.y;
@@ -551,6 +553,7 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
   int n = 0;
   auto work_off = [&]() {
     int m = 0;
+    const unsigned plane = BIG && n > 0 ? list[0][tid].x >> 16 : 0u;
     for (int e = 0; e < n; e++) {
       const uint2 cand = list[e][tid];
       const unsigned i = cand.x >> 16, j = cand.x & 0xffffu, k = cand.y;
@@ -560,14 +563,14 @@ __global__ void __launch_bounds__(IG_THREADS, IG_MINB) k_interpolate_gather(Inte
       const float wx = x == C.xl ? C.xm : x == C.xh ? C.xd : 0.f, wy = y == C.yl ? C.ym : y == C.yh ? C.yd : 0.f,
                   wz = z == C.zl ? C.zm : z == C.zh ? C.zd : 0.f;
       const float w = wx * wy * wz;
-      if (w != 0.f) list[m++][tid] = make_uint2(__float_as_uint(w), (i * od + j) * od + k);
+      if (w != 0.f) list[m++][tid] = make_uint2(__float_as_uint(w), ((i - plane) * od + j) * od + k);
     }
     n = 0;
     wait_for_stream();
     for (int e = 0; e < m; e++) {
       const uint2 t = list[e][tid];
       const float w = __uint_as_float(t.x);
-      const float* p = gout + t.y;
+      const float* p = gout + (size_t)plane * od * od + t.y;
 #pragma unroll
       for (int c = 0; c < CH; c++)
         if (c < nch) acc[c] = fmaf(w, __ldg(p + c * ochan), acc[c]);
@@ -628,6 +631,8 @@ constexpr int IC_CELLS = IC_X * IC_Y * IC_Z, IC_SCAN = (IC_CELLS + 1 + 31) / 32;
 constexpr int IC_CAP = 790;  // output voxels of a block: what fits for equal resolutions, and five blocks an SM
 constexpr int IC_CH = 8, IC_MINB = 5;
 
+// BIG: an output grid of 2^32 voxels or more; offsets are then counted from the block's first plane.
+template <bool BIG>
 __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(InterpArgs I, GatherFrames G) {
   // entries as they were found (weights of the upper corners, offset in a channel), then gradients by place
   __shared__ float4 val[2][IC_CAP];
@@ -647,7 +652,7 @@ __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(Inter
   for (int c = tid; c < 32 * IC_SCAN; c += IG_THREADS) start[c] = 0;
   if (tid == 0) count = 0;
   __syncthreads();
-  int found = 0;
+  int found = 0, plane = 0;
   if (W.sane) {
     const float h[3] = {0.5f * IC_X + W.slack, 0.5f * IC_Y + W.slack, 0.5f * IC_Z + W.slack};
     const float d[3] = {(float)x0 - 1.f + 0.5f * IC_X - W.g0[0], (float)y0 - 1.f + 0.5f * IC_Y - W.g0[1],
@@ -661,6 +666,7 @@ __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(Inter
       lo[i] = max(0, (int)ceilf(fmaxf(at[i] - e, -1.f)));  // inside [-1, od] before the conversions
       n[i] = max(0, min(od - 1, (int)floorf(fminf(at[i] + e, (float)od))) - lo[i] + 1);
     }
+    if (BIG) plane = lo[0];
     const int njk = n[1] * n[2], all = n[0] * njk;
     const float inv_njk = __fdividef(1.f, (float)njk), inv_nk = __fdividef(1.f, (float)n[2]);
     for (int c0 = 0; c0 < all; c0 += IG_THREADS) {
@@ -689,7 +695,7 @@ __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(Inter
       if (cx >= 0 && cx < IC_X && cy >= 0 && cy < IC_Y && cz >= 0 && cz < IC_Z) {
         const unsigned cell = (cx * IC_Y + cy) * IC_Z + cz;
         key = cell | atomicAdd(&start[cell], 1u) << 16;
-        entry[e] = make_float4(C.xd, C.yd, C.zd, __uint_as_float((i * od + j) * od + k));
+        entry[e] = make_float4(C.xd, C.yd, C.zd, __uint_as_float(((i - plane) * od + j) * od + k));
       }
       cand[e] = key;
     }
@@ -744,7 +750,7 @@ __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(Inter
   float* gin = I.out + b * I.K * ichan + ((size_t)(x0 + x) * id + y0 + y) * id + z0 + z;
   wait_for_stream();
   for (int c0 = R.c0; c0 < R.c1; c0 += IC_CH) {
-    const float* gout = I.in + (b * I.K + c0) * ochan;
+    const float* gout = I.in + (b * I.K + c0) * ochan + (size_t)plane * od * od;
     const int nch = min(IC_CH, R.c1 - c0);
     for (int e = tid; e < found; e += IG_THREADS) {
       const unsigned p = cand[e];
@@ -820,19 +826,20 @@ __global__ void __launch_bounds__(256) k_interpolate_scatter(InterpArgs I, unsig
 // The examples of one pass, which all take the same kernel.
 static cudaError_t interpolate_backward_run(const InterpArgs& I, const GatherFrames& W, int nb, bool cells, cudaStream_t st) {
   const unsigned id = I.in_dim, tiles = ((id + IG_X - 1) / IG_X) * ((id + IG_Y - 1) / IG_Y) * ((id + IG_Z - 1) / IG_Z);
+  const bool big = (unsigned long long)I.out_dim * I.out_dim * I.out_dim >> 32 != 0;
   if (cells) {
     // shares of the channels as long as the blocks fit the chip at a time
     const unsigned long room = 148ul * IC_MINB / ((unsigned long)tiles * nb), groups = ((unsigned long)I.K + IC_CH - 1) / IC_CH;
-    return launch_early(k_interpolate_cells, dim3(tiles, nb, (unsigned)std::max(1ul, std::min(room, groups))), IG_THREADS, 0, st, I, W);
+    return launch_early(big ? k_interpolate_cells<true> : k_interpolate_cells<false>, dim3(tiles, nb, (unsigned)std::max(1ul, std::min(room, groups))), IG_THREADS, 0, st, I, W);
   }
   // More channels per block mean fewer searches for the same voxel, fewer channels more blocks.
   const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, 592);
   const int per = (I.K + (int)shares - 1) / (int)shares;
-  const int ch = per > 16 ? 32 : per > 8 ? 16 : 8;
+  const int ch = big ? 8 : per > 16 ? 32 : per > 8 ? 16 : 8;
   InterpArgs J = I;
   cudaError_t e = cudaSuccess;
   for (int left = (I.K + ch - 1) / ch; left > 0 && e == cudaSuccess; left -= 65535, J.c0 += 65535 * ch)
-    e = launch_early(ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>,
+    e = launch_early(big ? k_interpolate_gather<8, true> : ch == 32 ? k_interpolate_gather<32> : ch == 16 ? k_interpolate_gather<16> : k_interpolate_gather<8>,
                      dim3(tiles, nb, left < 65535 ? left : 65535), IG_THREADS, 0, st, J, W);
   return e;
 }

@@ -95,3 +95,29 @@ def test_gradients_do_not_depend_on_the_other_examples(odd, rout, K):
         gi.backward(cen[b:b + 1], g[b:b + 1].clone(), trs[b:b + 1], cen[b:b + 1], alone)
         assert torch.equal(alone[0], together[b])
         assert bool(alone.any()) == (b != 1 or odd == "distant")
+
+
+def _adjoint_axis(din, dout, f, shift):
+    """The weights of an axis without rotation: output voxel o at input index f * (o - (dout - 1) / 2) - shift + (din - 1) / 2."""
+    g = f * (np.arange(dout) - (dout - 1) / 2) - shift + (din - 1) / 2
+    return np.maximum(0.0, 1.0 - np.abs(np.arange(din)[:, None] - g[None, :]))
+
+
+@pytest.mark.parametrize("rout", [0.5, 0.25])
+def test_backward_from_a_grid_of_more_voxels_than_32_bits_count(rout):
+    """1626^3 output voxels, of which the last planes lie in the input grid (a translation by whole quarters of a voxel, so
+    that every weight and sum is exact): by cells, and by the search for a finer output."""
+    din, m = 9, 1626
+    gi = lmg.GridInterpolater(0.5, (din - 1) * 0.5, rout, (m - 1) * rout)
+    rng = np.random.default_rng(3)
+    keep = 24
+    corner = rng.integers(-8, 8, (keep,) * 3).astype(np.float32)
+    g = torch.zeros((1, m, m, m), device="cuda")
+    g[0, -keep:, -keep:, -keep:] = torch.from_numpy(corner).cuda()
+    shift = rout / 0.5 * (m - 1) / 2 - (din - 1) / 2  # the last output voxel on the last of the input
+    back = torch.full((1, din, din, din), 7.0, device="cuda")
+    gi.backward(g, lmg.Transform(lmg.Quaternion(1, 0, 0, 0), (0, 0, 0), (shift * 0.5,) * 3), back)
+    w = _adjoint_axis(din, m, rout / 0.5, shift)[:, -keep:]
+    assert w.sum() > din - 1
+    want = np.einsum("ai,bj,ck,ijk->abc", w, w, w, corner.astype(float))
+    assert np.array_equal(back[0].cpu().numpy(), want)
