@@ -632,7 +632,10 @@ constexpr int IC_CAP = 790;  // output voxels of a block: what fits for equal re
 constexpr int IC_CH = 8, IC_MINB = 5;
 
 // BIG: an output grid of 2^32 voxels or more; offsets are then counted from the block's first plane.
-template <bool BIG>
+// OUTSIDE: blocks without output voxels skip the rounds over the channels.  64^3 from 16^3 of the same resolution, 48 x 14
+// channels, 330 -> 254 us, 48^3 from 48^3 616 -> 588; from outputs twice as coarse, which leave few such blocks, 234 -> 242, so
+// these go without.
+template <bool BIG, bool OUTSIDE>
 __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(InterpArgs I, GatherFrames G) {
   // entries as they were found (weights of the upper corners, offset in a channel), then gradients by place
   __shared__ float4 val[2][IC_CAP];
@@ -749,6 +752,11 @@ __global__ void __launch_bounds__(IG_THREADS, IC_MINB) k_interpolate_cells(Inter
   const ChannelRange R(I.K, IC_CH);
   float* gin = I.out + b * I.K * ichan + ((size_t)(x0 + x) * id + y0 + y) * id + z0 + z;
   wait_for_stream();
+  if (OUTSIDE && found == 0) {
+    if (live)
+      for (int c = R.c0; c < R.c1; c++) gin[c * ichan] = 0.f;
+    return;
+  }
   for (int c0 = R.c0; c0 < R.c1; c0 += IC_CH) {
     const float* gout = I.in + (b * I.K + c0) * ochan + (size_t)plane * od * od;
     const int nch = min(IC_CH, R.c1 - c0);
@@ -830,7 +838,7 @@ static cudaError_t interpolate_backward_run(const InterpArgs& I, const GatherFra
   if (cells) {
     // shares of the channels as long as the blocks fit the chip at a time
     const unsigned long room = 148ul * IC_MINB / ((unsigned long)tiles * nb), groups = ((unsigned long)I.K + IC_CH - 1) / IC_CH;
-    return launch_early(big ? k_interpolate_cells<true> : k_interpolate_cells<false>, dim3(tiles, nb, (unsigned)std::max(1ul, std::min(room, groups))), IG_THREADS, 0, st, I, W);
+    return launch_early(big ? k_interpolate_cells<true, true> : I.out_res < 1.5f * I.in_res ? k_interpolate_cells<false, true> : k_interpolate_cells<false, false>, dim3(tiles, nb, (unsigned)std::max(1ul, std::min(room, groups))), IG_THREADS, 0, st, I, W);
   }
   // More channels per block mean fewer searches for the same voxel, fewer channels more blocks.
   const unsigned long shares = channel_shares((unsigned long)tiles * nb, I.K, 592);
@@ -851,7 +859,14 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
   // centres up to some 2600 cells away, outputs up to 0.28 % finer about the origin, and coarser ones.  Finer ones would
   // need more room than five blocks an SM have.
   const double f = (double)I.out_res / I.in_res;
+  // Much coarser outputs leave a block few voxels to look up, in rounds of eight channels, where the search takes up to 32
+  // together.  96^3 of 0.25 A, cells / search: from 0.5 A 4 / 24 / 28 / 40 channels 27 / 59 / 72 / 93 and 35 / 67 / 67 / 117 us, from 0.7 A
+  // 4 / 28 channels 25 / 60 and 22 / 52, from 1 A 22 / 54 and 19 / 42; one wave of blocks, 28 x 48^3 from outputs twice as coarse
+  // 11.7 and 15.0.
+  const unsigned long tiles = (unsigned long)((I.in_dim + IG_X - 1) / IG_X) * ((I.in_dim + IG_Y - 1) / IG_Y) * ((I.in_dim + IG_Z - 1) / IG_Z);
+  const bool few = f >= 2.5 || (f >= 1.75 && (I.K + 7) / 8 % 4 == 0 && tiles > 148 * IC_MINB);
   auto fits = [&](int i) {
+    if (few) return false;
     const double more = 2.0 * W.ex[i].slack + 1.7321 * f;
     return 1.005 * (IC_X + more) * (IC_Y + more) * (IC_Z + more) < IC_CAP * f * f * f;
   };

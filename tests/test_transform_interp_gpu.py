@@ -267,6 +267,30 @@ def test_interpolate_backward_against_64_bits(din, dout, rin, rout, K):
     assert torch.equal(out, again)
 
 
+# either side of every line between the two kernels: outputs a little finer, centres far away (in cells), outputs coarser by
+# more and less than 2.5 and, in grids of many tiles, twice as coarse with channels that make whole groups and others
+@pytest.mark.parametrize("din,dout,rin,rout,far,K,B", [
+    (17, 18, 0.5, 0.499, 0, 1, 24), (17, 18, 0.5, 0.498, 0, 1, 24), (17, 18, 0.5, 0.5, 2580, 1, 24), (17, 18, 0.5, 0.5, 2720, 1, 24),
+    (30, 12, 0.5, 1.24, 0, 2, 24), (30, 12, 0.5, 1.25, 0, 2, 24), (30, 13, 0.5, 0.87, 0, 32, 2), (61, 14, 0.5, 0.875, 0, 32, 2),
+    (61, 14, 0.5, 0.875, 0, 33, 1), (29, 5, 0.5, 0.7, 0, 9, 8), (29, 5, 0.5, 0.8, 0, 9, 8)])
+def test_interpolate_backward_on_either_side_of_the_lines(din, dout, rin, rout, far, K, B):
+    """Random rotations of grids of several tiles.  Positions of `far` cells are off by a few roundings of that size, and
+    the weights by as much."""
+    import libmolgrid_b200 as lmg
+    rng = np.random.default_rng(din + 7 * dout + far)
+    g = lmg.GridInterpolater(rin, (din - 1) * rin, rout, (dout - 1) * rout)
+    center = np.array([far * rin, 0, 0], np.float32)
+    q, t = cases.random_quaternion(rng, B), rng.uniform(-1, 1, (B, 3)).astype(np.float32)
+    y = rng.normal(size=(B, K, dout, dout, dout)).astype(np.float32)
+    out = torch.full((B, K, din, din, din), 7.0, device="cuda")
+    cen = np.tile(center, (B, 1))
+    g.backward(cen, dev(y), [make_transform(q[b], center, t[b]) for b in range(B)], cen, out)
+    # one rounding of a position for each of about sixteen operations, in the worst case along all axes
+    for b in range(B):
+        want = _adjoint64(y[b].astype(float), din, rin, rout, q[b].astype(float), np.zeros(3), t[b].astype(float))
+        assert np.linalg.norm(out[b].cpu().numpy() - want) <= (2e-5 + 16 * 2.0 ** -24 * far) * np.linalg.norm(want) + 1e-6
+
+
 @pytest.mark.parametrize("layer", ["python", "compiled"])
 def test_transform_known_answers_on_host_arrays_and_in_place(layer):
     """The reference's worked example (test/test_transform.py:65-140): a quarter turn about z through
