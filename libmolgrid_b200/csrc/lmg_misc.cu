@@ -901,8 +901,7 @@ cudaError_t launch_interpolate_backward(const InterpArgs& I, const GatherFrames&
 }
 
 cudaError_t launch_interpolate(const InterpArgs& I, int nb, cudaStream_t st) {
-  unsigned nv = I.out_dim * I.out_dim * I.out_dim;
-  if (nv == 0 || nb == 0 || I.K == 0) return cudaSuccess;
+  if (I.out_dim == 0 || nb == 0 || I.K == 0) return cudaSuccess;
   const unsigned od = I.out_dim, nblk = ((od + 3) / 4) * ((od + 7) / 8) * ((od + 7) / 8);
   dim3 grid(nblk, nb, channel_shares((unsigned long)nblk * nb, I.K, 1184));
   return launch_early(k_interpolate, grid, 256, 0, st, I);

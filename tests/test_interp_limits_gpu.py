@@ -121,3 +121,17 @@ def test_backward_from_a_grid_of_more_voxels_than_32_bits_count(rout):
     assert w.sum() > din - 1
     want = np.einsum("ai,bj,ck,ijk->abc", w, w, w, corner.astype(float))
     assert np.array_equal(back[0].cpu().numpy(), want)
+
+
+def test_forward_to_a_grid_of_2048_voxels_a_side():
+    """2^33 output voxels, a count of zero in 32 bits."""
+    din, m = 5, 2048
+    gi = lmg.GridInterpolater(0.5, (din - 1) * 0.5, 0.5, (m - 1) * 0.5)
+    src = torch.rand((1, din, din, din), device="cuda")
+    out = torch.full((1, m, m, m), 7.0, device="cuda")
+    gi.forward(src, lmg.Transform(lmg.Quaternion(1, 0, 0, 0), (0, 0, 0), (0.25, 0.25, 0.25)), out)
+    lo = (m - din) // 2  # an odd difference: half a voxel that the translation makes up for
+    inside = out[0, lo - 1:lo + din + 2, lo - 1:lo + din + 2, lo - 1:lo + din + 2].clone()
+    assert torch.equal(inside[inside != 0].sort().values, src[0].flatten().sort().values)
+    out[0, lo - 1:lo + din + 2, lo - 1:lo + din + 2, lo - 1:lo + din + 2] = 0
+    assert not out.any()
