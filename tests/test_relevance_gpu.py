@@ -129,8 +129,8 @@ def test_roots_and_quotients(sweeps, what):
     assert (out[0], out[1]) == (0, 0)
 
 
-# four warps an atom, on either side of the line between the kernels with room and the tight ones
-@pytest.mark.parametrize("n", [1, 740, 741, 1000])
+# four warps an atom, on either side of the lines between the kernels with room and the tight ones
+@pytest.mark.parametrize("n", [1, 740, 741, 889, 1037, 1185])
 @pytest.mark.parametrize("points", [12, 13])
 @pytest.mark.parametrize("binary", [False, True])
 def test_relevance_of_some_atoms(n, points, binary):
