@@ -57,7 +57,6 @@ struct __align__(16) ChanParam {
 };
 
 __device__ __forceinline__ float next_up(float x) { return __int_as_float(__float_as_int(x) + 1); }
-__device__ __forceinline__ float next_down(float x) { return __int_as_float(__float_as_int(x) - 1); }
 
 // Largest t >= 0 with sqrtf(t) <= cut (IEEE round-to-nearest sqrt); -1 if cut is negative or NaN.  A root is rounded to
 // `cut` or less where it lies below the middle between `cut` and its successor; that middle has 25 bits, its square is

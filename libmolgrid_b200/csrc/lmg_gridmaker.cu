@@ -600,10 +600,11 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_gradgrad_scatter(BwdArgs G)
 // 16-byte load, so a warp has 32 columns x 4 quads in flight per round trip to memory instead of
 // 8 columns x 4 voxels.  What depends on z alone sits in a small shared table per warp (one pass
 // covers 32 z positions from the aligned start of the footprint).  This lane-per-column layout
-// serves the backward passes and the per-atom vector kernels, which spend their time issuing
-// instructions and amortise the per-column terms over the quads of a column; the forward pass of
-// index types and of (atom, channel) items is bound by the lines its reductions touch and uses
-// the (column, z-quad) layout of qlane_sweep instead.
+// serves the backward passes of index types and of (atom, channel) items, the atom gradients alone of
+// type vectors and their densities in the reference's order of operations, which spend their time
+// issuing instructions and amortise the per-column terms over the quads of a column; the other forward
+// passes and the type gradients by atom are bound by the lines that they touch and use the (column,
+// z-quad) layout of qlane_sweep instead.
 // ---------------------------------------------------------------------------------------------
 constexpr int QPASS = 8;  // quads per pass
 
