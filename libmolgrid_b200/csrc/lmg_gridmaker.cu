@@ -1422,7 +1422,8 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32, 32) k_backward_quads(BwdArgs 
 // Relevance by four warps an atom takes 80 to 94 registers, five or six blocks an SM.  The `tight` variant, of which six to
 // eight fit (loose rows need larger tables), is for the counts that are one wave with it and two without: 800 / 1000 atoms on
 // 14x24^3 of 1 A 6.3 / 6.6 us with room and 4.8 / 5.0 tight, occupancy of 1000 6.5 and 4.7; one wave or two either way, 600
-// atoms 4.1 and 4.3, 1200 on 14x41^3 14.9 and 15.2.
+// atoms 4.1 and 4.3, 1200 on 14x41^3 14.9 and 15.2.  Examples with counts of their own: the slots behind them leave at once
+// and are taken for a quarter (16 x 26 to 53 atoms in 848 slots on 31x48^3 8.1 and 8.7).
 constexpr long SELF_ROOMY = 5 * 148;
 constexpr int self_blocks(bool binary, bool loose, bool tight) { return !tight ? 0 : loose ? (binary ? 7 : 6) : binary ? 8 : 7; }
 template <int MODE, bool BINARY, int WARPS, class TABS, bool TIGHT = false>
@@ -2427,7 +2428,7 @@ static cudaError_t backward_self(const EmitArgs& A, const BwdArgs& G, int mode, 
   const dim3 grid(A.N, A.nb);
   if (mode == 0) return launch_early(k_backward_quads_self<0, false, WARPS, TABS>, grid, 32 * WARPS, 0, st, A, G);
   if constexpr (WARPS > 1) {
-    const long atoms = (long)A.nb * A.N;
+    const long slots = (long)A.nb * A.N, atoms = A.n_atoms != nullptr ? slots * 3 / 4 : slots;
     if (atoms > SELF_ROOMY && atoms <= 148 * self_blocks(A.gm.binary != 0, !std::is_same<TABS, ZTabs>::value, true))
       return launch_early(A.gm.binary ? k_backward_quads_self<2, true, WARPS, TABS, true> : k_backward_quads_self<2, false, WARPS, TABS, true>,
                           grid, 32 * WARPS, 0, st, A, G);
