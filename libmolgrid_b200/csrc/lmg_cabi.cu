@@ -266,6 +266,10 @@ lmg::InterpArgs interp_args(const lmg_interpolater* gi, int nchannels, const flo
 struct Layout {
   size_t flags, recs, chanp, partial, total;
   size_t per_example;
+  // type gradients by copies of the grid gradient (instead of the partial sums, in their place): examples copied together,
+  // 0 if that is not the way, the copies and where they end
+  int copies;
+  size_t copy, copy_end;
 };
 
 constexpr size_t STATUS_BYTES = 256;
@@ -284,7 +288,15 @@ Layout layout(const lmg_gridmaker* g, int op, int nb, int N, int T, int vec) {
   L.recs = o; o += recs * nb;
   L.chanp = o; o += chanp * nb;
   L.partial = o; o += partial * nb;
-  L.total = o;
+  const lmg::GMParams gm = lmg::to_params(g);
+  // the rows of an aligned tensor; of another one with such rows it is not known here
+  if (partial != 0 && op == LMG_OP_BACKWARD && lmg::type_copies_serve(gm, nb, N, T, g->dim % 4 == 0)) {
+    const size_t each = lmg::type_copy_bytes(gm, T);
+    L.copies = (int)std::max<size_t>(1, std::min<size_t>(nb, lmg::TYPE_COPIES / each));
+    L.copy = L.partial;
+    L.copy_end = L.copy + L.copies * each;
+  }
+  L.total = std::max(o, L.copy_end);
   return L;
 }
 
@@ -622,13 +634,18 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
     }
     if (e != cudaSuccess) return cuda_fail(e, "emit");
     g_launches += 1 + ((vec && g->radii_type_indexed) ? 1 : 0);
+    // a workspace that is too small for the copies is enough for the kernels that need none
+    const bool copies = type_gradients != nullptr && L.copies > 0 && L.copy_end <= workspace_bytes && g_quads;
     ProfRec* pr = prof_begin(1, st);
     {
       Range r(mode == 2 ? "backward relevance" : "backward");
-      e = lmg::launch_backward(B, mode, st);
+      if (copies)
+        e = lmg::launch_type_gradients(B, reinterpret_cast<float*>(ws + L.copy), L.copies, &g_launches, st);
+      else
+        e = lmg::launch_backward(B, mode, st);
     }
     prof_end(pr, st);
-    g_launches += mode == 1 ? 2 : 1;
+    if (!copies) g_launches += mode == 1 ? 2 : 1;
     if (e != cudaSuccess) return cuda_fail(e, "backward");
   }
   return LMG_OK;

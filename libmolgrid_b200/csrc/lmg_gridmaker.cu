@@ -2059,6 +2059,366 @@ __global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same for many atoms a grid: every channel is read under every footprint, and above the L1 takes a clock for each line
+// that a request touches, 85 columns in each of 28 channels.  A copy of the gradient with the channels of a voxel next to
+// each other makes that one line a voxel, and the sums are bound by the L2 instead (50 x 3000 atoms on 28x48^3: 12.7 GB at 12
+// TB/s, 22 % of the time waiting for issue slots).  Blocks of one warp: several atoms a block, neighbours by Morton's curve,
+// meet too few lines of each other's in the L1 (hits 22 to 35 %, as without order) for what the wait for the slowest costs
+// (1590 us for 1225).  Quads of a column and voxels of a lane requested together, blocks an SM: 4 / 4 / 20 1226 us, 2 / 4 / 20
+// 1301, 4 / 4 / 24 1297 to 1505 (the L1 gets what shared memory leaves), 4 / 6 / 20 1267.
+// ---------------------------------------------------------------------------------------------
+constexpr int CL_VOXELS = 128, CL_PITCH = CL_VOXELS + 1;
+
+// Channels [0, T) of the voxels to rows of TQ quads a voxel, filled up with zeros, and a row of zeros behind the last.  A
+// block of TQ warps turns 128 voxels: a warp reads four channels, a thread writes one quad of channels of every 32nd voxel.
+// Bound by memory: 4 examples of 28x48^3 17 us, 6.2 TB/s.
+template <int TQ>
+__global__ void __launch_bounds__(32 * TQ) k_channel_last(const float* diff, float4* copy, unsigned voxels, int T) {
+  __shared__ float tile[4 * TQ * CL_PITCH];
+  wait_for_stream();
+  let_next_begin();
+  const unsigned v0 = blockIdx.x * CL_VOXELS, lane = threadIdx.x & 31, c0 = threadIdx.x >> 5 << 2, n = min((unsigned)CL_VOXELS, voxels - v0);
+  const float* src = diff + (size_t)blockIdx.y * T * voxels + (size_t)c0 * voxels + v0 + lane;
+  float d[4][4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) d[c][k] = c0 + c < T && lane + 32 * k < n ? __ldcs(src + 32 * k) : 0.f;
+    src += voxels;
+  }
+  float* to = tile + c0 * CL_PITCH + lane;
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) to[c * CL_PITCH + 32 * k] = d[c][k];
+  __syncthreads();
+  const unsigned v = threadIdx.x / TQ, q = threadIdx.x % TQ;
+  const float* p = tile + 4 * q * CL_PITCH + v;
+  float4* dst = copy + ((size_t)blockIdx.y * (voxels + 1) + v0) * TQ + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (v + 32 * k < n) dst[32 * k * TQ] = make_float4(p[32 * k], p[CL_PITCH + 32 * k], p[2 * CL_PITCH + 32 * k], p[3 * CL_PITCH + 32 * k]);
+  if (v0 + n == voxels && threadIdx.x < TQ) copy[((size_t)blockIdx.y * (voxels + 1) + voxels) * TQ + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+constexpr int TG_MINB = 20;       // blocks of one warp an SM
+constexpr int TG_COLS = 128;
+constexpr int TG_Q = 4;           // quads of a column that are requested together
+constexpr int TG_U = 4;           // voxels of a lane that are requested together
+constexpr int TG_DIRECT = 4;      // most weighted channels that the atom gradient reads where they lie
+
+// Eight channels of a voxel in one load.
+struct __align__(32) Eight {
+  Pair p[4];
+};
+__device__ __forceinline__ Eight load_eight(const Eight* p) {
+  Eight v;
+  asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v.p[0].v), "=l"(v.p[1].v), "=l"(v.p[2].v), "=l"(v.p[3].v) : "l"(p) : "memory");
+  return v;
+}
+
+struct TgArgs {
+  BwdArgs G;
+  const Eight* copy;  // [examples of the launch][voxels + 1][TO]
+  int first;          // first example of the launch, counted in the pass
+};
+
+// TO: eights of channels a voxel.  The lanes are (voxel, eight) while voxels are added up, VOXELS at a time.
+template <int TO>
+struct __align__(16) TgShared {
+  static constexpr unsigned VOXELS = 32 / TO, BATCH = TG_U * VOXELS;
+  // voxels within reach, filled up to a whole batch: place in the copy and density; for atoms of many weighted channels
+  // place, density and its gradient by the atom's position, of one step (128 voxels at most)
+  static constexpr unsigned CAP = 128 * TG_Q + BATCH, DENSE_CAP = 128 + BATCH;
+  union {
+    uint2 list[CAP];
+    struct {
+      unsigned place[DENSE_CAP];
+      float v[DENSE_CAP], slope[3][DENSE_CAP];
+    } dense;
+    float sums[32][9];
+  };
+  ColBufT<TG_COLS> cols;
+  ZTabs zt;
+};
+
+// Sums of the n listed voxels; places up to a whole batch are the copy's row of zeros.  `mine` is the lane's eight of voxel 0.
+template <int TO, bool DENSE>
+__device__ __forceinline__ void tg_add(TgShared<TO>& sh, unsigned n, const Eight* mine, unsigned zeros, int lane, Pair (&tg)[4],
+                                       const Pair (&w)[4], float (&ag)[3]) {
+  constexpr unsigned VOXELS = TgShared<TO>::VOXELS, BATCH = TgShared<TO>::BATCH;
+  const unsigned whole = (n + BATCH - 1) / BATCH * BATCH, g = min((unsigned)lane / TO, VOXELS - 1u);
+  for (unsigned i = n + lane; i < whole; i += 32) {
+    if (DENSE) {
+      sh.dense.place[i] = zeros;
+      sh.dense.v[i] = sh.dense.slope[0][i] = sh.dense.slope[1][i] = sh.dense.slope[2][i] = 0.f;
+    } else {
+      sh.list[i] = make_uint2(zeros, 0u);
+    }
+  }
+  __syncwarp();
+  Pair acc[4] = {pair(0.f), pair(0.f), pair(0.f), pair(0.f)};
+  float own[3] = {0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (unsigned i = g; i < whole; i += BATCH) {
+    uint2 e[TG_U];
+    Eight d[TG_U];
+#pragma unroll
+    for (int u = 0; u < TG_U; u++) {
+      const unsigned k = i + u * VOXELS;
+      e[u] = DENSE ? make_uint2(sh.dense.place[k], __float_as_uint(sh.dense.v[k])) : sh.list[k];
+    }
+#pragma unroll
+    for (int u = 0; u < TG_U; u++) d[u] = load_eight(mine + e[u].x);
+    // by batches, then by calls, then for the atom: sums of few terms each
+    Pair sum[4];
+    float a[3];
+#pragma unroll
+    for (int u = 0; u < TG_U; u++) {
+      const Pair v = pair(__uint_as_float(e[u].y));
+#pragma unroll
+      for (int c = 0; c < 4; c++) sum[c] = u == 0 ? mul2(v, d[u].p[c]) : fma2(v, d[u].p[c], sum[c]);
+      if (DENSE) {
+        float x, y;
+        split(fma2(w[0], d[u].p[0], fma2(w[1], d[u].p[1], fma2(w[2], d[u].p[2], mul2(w[3], d[u].p[3])))), x, y);
+        const unsigned k = i + u * VOXELS;
+#pragma unroll
+        for (int j = 0; j < 3; j++) a[j] = u == 0 ? sh.dense.slope[j][k] * (x + y) : fmaf(sh.dense.slope[j][k], x + y, a[j]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[c] = add2(acc[c], sum[c]);
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (DENSE) own[j] += a[j];
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++) tg[c] = add2(tg[c], acc[c]);
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+    if (DENSE) ag[j] += own[j];
+  __syncwarp();
+}
+
+// One atom.  Its weights `w` are those of a lane's channel, `m` tells which there are.  A lane owns a column, as in
+// backward_quads_core(), and lists the voxels of its quads that lie within reach.  The atom gradient takes the weighted
+// channels' values where they lie; of many (DENSE) from the copy, by the gradients of the density that are listed too.
+template <int TO, bool BINARY, bool DENSE>
+__device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, TgShared<TO>& sh, const float* diffb, const Eight* mine,
+                                        float ox, float oy, float oz, float w, unsigned m, Pair (&tg)[4], float (&ag)[3], int lane) {
+  const GMParams& gm = A.G.gm;
+  const unsigned dim = gm.dim, voxels = dim * dim * dim;
+  const bool aligned = dim % 4 == 0 && (uintptr_t)A.G.diff % 16 == 0;
+  const float Tcull = fmaxf(P.Tcut, BINARY ? P.Tbin : -1.f);
+  const float kexp = P.inv_ar2 * NEG2_LOG2E;
+  const bool tail = gm.ta != 0.f || gm.tb != 0.f;
+  const float k4 = 4.f * P.inv_ar2, kD = tail ? -gm.D * P.inv_ar2 : 0.f, kE = tail ? -gm.E * P.inv_ar : 0.f;
+  const float inv_dim = 1.f / small_float(dim);
+  // the first weighted channel
+  const int t1 = m != 0u ? __ffs(m) - 1 : 0;
+  const float w1 = __shfl_sync(0xffffffffu, w, t1);
+  const float* one = diffb + (size_t)t1 * voxels;
+  Pair w8[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    w8[c] = pair(0.f);
+    if (DENSE) w8[c] = pair(__shfl_sync(0xffffffffu, w, lane % TO * 8 + 2 * c), __shfl_sync(0xffffffffu, w, lane % TO * 8 + 2 * c + 1));
+  }
+  Pair az = pair(0.f);
+  unsigned n = 0;
+  for (Columns cols(P); cols.more();) {
+    const unsigned nkept = cols.compact<false>(sh.cols, P, Tcull, ox, oy, gm.res, dim, lane);
+    for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+      __syncwarp();
+      fill_ztabs(sh.zt, zc, P, oz, gm.res, kexp, lane);
+      __syncwarp();
+      const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+#pragma unroll 1
+      for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
+        const unsigned i = c0 + lane;
+        unsigned row = 0;
+        const float dxy2 = i < nkept ? sh.cols.get(i, row) : CUDART_NAN_F;
+        const unsigned voxel = row * dim + zc;
+        float dx = 0.f, dy = 0.f;
+        auto from_atom = [&] {
+          const unsigned x = (unsigned)((small_float(row) + 0.5f) * inv_dim);
+          dx = __fsub_rn(voxel_coord(ox, x, gm.res), P.x);
+          dy = __fsub_rn(voxel_coord(oy, row - x * dim, gm.res), P.y);
+        };
+        if (DENSE) from_atom();
+        const float exy = ex2_approx(dxy2 * kexp);
+        const Pair xy = pair(dxy2);
+        Pair fs = pair(0.f);
+#pragma unroll 1
+        for (unsigned q0 = 0; q0 < nq; q0 += TG_Q) {
+          float4 dv[TG_Q];
+          bool live[TG_Q];
+#pragma unroll
+          for (int u = 0; u < TG_Q; u++) {
+            live[u] = q0 + u < nq && __fadd_rn(dxy2, sh.zt.lo[q0 + u]) <= Tcull;  // false for a NaN
+            if (DENSE) continue;
+            dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* p = one + voxel + 4 * (q0 + u);
+            if (aligned) {
+              if (live[u]) dv[u] = __ldg(reinterpret_cast<const float4*>(p));
+            } else if (live[u]) {
+              const unsigned z = zc + 4 * (q0 + u);
+              if (z >= P.loz && z < P.hiz) dv[u].x = __ldg(p);
+              if (z + 1 >= P.loz && z + 1 < P.hiz) dv[u].y = __ldg(p + 1);
+              if (z + 2 >= P.loz && z + 2 < P.hiz) dv[u].z = __ldg(p + 2);
+              if (z + 3 >= P.loz && z + 3 < P.hiz) dv[u].w = __ldg(p + 3);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < TG_Q; u++) {
+            if (!__any_sync(0xffffffffu, live[u])) continue;
+            const float4 d2 = sh.zt.dz2[q0 + u], e = sh.zt.ez[q0 + u], dz = sh.zt.dz[q0 + u];
+            const Pair d2p[2] = {pair(d2.x, d2.y), pair(d2.z, d2.w)}, ep[2] = {pair(e.x, e.y), pair(e.z, e.w)},
+                       dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)};
+            float v[4], s[4];
+            bool listed[4];
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+              float r0, r1, a0, a1, b0, b1;
+              const Pair r = add2(xy, d2p[j / 2]), gauss = mul2(pair(exy), ep[j / 2]);
+              split(r, r0, r1);
+              const Pair id = pair(rsqrt_approx(r0), rsqrt_approx(r1));
+              split(fma2(pair(kE), id, pair(kD)), a0, a1);  // zero at the cut-off and negative beyond it
+              split(mul2(pair(k4), gauss), b0, b1);
+              const bool g0 = r0 <= P.Tg, g1 = r1 <= P.Tg, in0 = r0 <= Tcull, in1 = r1 <= Tcull;
+              s[j] = g0 ? b0 : fmaxf(a0, 0.f);
+              s[j + 1] = g1 ? b1 : fmaxf(a1, 0.f);
+              listed[j] = BINARY && !DENSE ? r0 < P.Tbin : in0;
+              listed[j + 1] = BINARY && !DENSE ? r1 < P.Tbin : in1;
+              if (BINARY) {
+                v[j] = r0 < P.Tbin ? 1.f : 0.f;
+                v[j + 1] = r1 < P.Tbin ? 1.f : 0.f;
+              } else {
+                // from a root of its own: through the reciprocal one of the gradient it is 5 to 14 % further from 64 bits
+                split(mul2(r, pair(P.inv_ar2)), a0, a1);
+                a0 = fma_sat(-gm.ta, sqrt_approx(a0), gm.tb);
+                a1 = fma_sat(-gm.ta, sqrt_approx(a1), gm.tb);
+                split(gauss, b0, b1);
+                v[j] = g0 ? b0 : a0 * a0;
+                v[j + 1] = g1 ? b1 : a1 * a1;
+              }
+              if (!DENSE) {
+                float x0, x1;
+                split(mul2(pair(w1), j == 0 ? pair(dv[u].x, dv[u].y) : pair(dv[u].z, dv[u].w)), x0, x1);
+                // the other weighted channels, one after the other
+                for (unsigned left = m & (m - 1u); left != 0u; left &= left - 1u) {
+                  const int t = __ffs(left) - 1;
+                  const float wt = __shfl_sync(0xffffffffu, w, t);
+                  const float* p = diffb + (size_t)t * voxels + voxel + 4 * (q0 + u) + j;
+                  if (in0) x0 = fmaf(wt, __ldg(p), x0);
+                  if (in1) x1 = fmaf(wt, __ldg(p + 1), x1);
+                }
+                split(mul2(pair(s[j], s[j + 1]), pair(x0, x1)), x0, x1);
+                const Pair f = pair(in0 ? x0 : 0.f, in1 ? x1 : 0.f);  // a neighbour's value may be anything
+                fs = add2(fs, f);
+                az = fma2(f, dzp[j / 2], az);
+              }
+            }
+            unsigned place = (voxel + 4 * (q0 + u)) * TO;
+            const float dzv[4] = {dz.x, dz.y, dz.z, dz.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const unsigned them = __ballot_sync(0xffffffffu, listed[j]), at = n + __popc(them & ((1u << lane) - 1u));
+              if (DENSE) {
+                if (listed[j]) {
+                  sh.dense.place[at] = place;
+                  sh.dense.v[at] = v[j];
+                  sh.dense.slope[0][at] = s[j] * dx;
+                  sh.dense.slope[1][at] = s[j] * dy;
+                  sh.dense.slope[2][at] = s[j] * dzv[j];
+                }
+              } else if (listed[j]) {
+                sh.list[at] = make_uint2(place, __float_as_uint(v[j]));
+              }
+              n += __popc(them);
+              place += TO;
+            }
+            if (DENSE) {
+              tg_add<TO, DENSE>(sh, n, mine, voxels * TO, lane, tg, w8, ag);
+              n = 0;
+            }
+          }
+          if (!DENSE && n != 0) {
+            tg_add<TO, DENSE>(sh, n, mine, voxels * TO, lane, tg, w8, ag);
+            n = 0;
+          }
+        }
+        if (!DENSE) {
+          float f0, f1;
+          split(fs, f0, f1);
+          from_atom();
+          ag[0] = fmaf(f0 + f1, dx, ag[0]);
+          ag[1] = fmaf(f0 + f1, dy, ag[1]);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (!DENSE) {
+    float z0, z1;
+    split(az, z0, z1);
+    ag[2] += z0 + z1;
+  } else if (lane / TO >= (int)TgShared<TO>::VOXELS) {
+    ag[0] = ag[1] = ag[2] = 0.f;  // a lane too many for whole voxels
+  }
+}
+
+template <int TO, bool BINARY>
+__global__ void __launch_bounds__(32, TG_MINB) k_type_gradients(TgArgs A) {
+  wait_for_stream();
+  __shared__ TgShared<TO> sh;
+  const BwdArgs& G = A.G;
+  const GMParams& gm = G.gm;
+  const int lane = threadIdx.x, item = blockIdx.x, bl = A.first + blockIdx.y, b = G.b0 + bl;
+  float cx, cy, cz;
+  if (G.centers != nullptr) {
+    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
+  } else {
+    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
+  }
+  const float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
+  const ItemParams P = load_item<false>(G, bl, b, item, ox, oy, oz);
+  const size_t voxels = (size_t)gm.dim * gm.dim * gm.dim, ai = (size_t)b * G.N + item;
+  const float* diffb = G.diff + (size_t)b * G.T * voxels;
+  const Eight* mine = A.copy + blockIdx.y * (voxels + 1) * TO + lane % TO;
+  const float w = lane < G.T ? G.type_vector[ai * G.T + lane] : 0.f;
+  const unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
+  Pair tg[4];
+  float ag[3];
+  for (bool dense = __popc(m) > TG_DIRECT;; dense = false) {
+    tg[0] = tg[1] = tg[2] = tg[3] = pair(0.f);
+    ag[0] = ag[1] = ag[2] = 0.f;
+    if (!P.valid) break;
+    if (dense) tg_atom<TO, BINARY, true>(A, P, sh, diffb, mine, ox, oy, oz, w, m, tg, ag, lane);
+    else tg_atom<TO, BINARY, false>(A, P, sh, diffb, mine, ox, oy, oz, w, m, tg, ag, lane);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) ag[c] += __shfl_xor_sync(0xffffffffu, ag[c], o);
+    }
+    // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either,
+    // and the sums are taken again from the others alone.
+    const float whole = (ag[0] + ag[1]) + ag[2];
+    if (!dense || whole == whole) break;
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++) split(tg[c], sh.sums[lane][2 * c], sh.sums[lane][2 * c + 1]);
+  __syncwarp();
+  if (lane < G.T) {
+    float sum = 0.f;
+#pragma unroll
+    for (unsigned g = 0; g < TgShared<TO>::VOXELS; g++) sum += sh.sums[g * TO + (lane >> 3)][lane & 7];
+    G.type_gradients[ai * G.T + lane] = sum;
+  }
+  if (lane < 3) G.atom_gradients[ai * 3 + lane] = lane == 0 ? ag[0] : lane == 1 ? ag[1] : ag[2];
+}
+
 // The same without type gradients (the caller passed none: types that are inputs, not parameters):
 // only the channels that carry weight are read.
 __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_quads_atom_ag(BwdArgs G) {
@@ -2460,6 +2820,47 @@ static cudaError_t backward_quads_atom(const BwdArgs& G, dim3 grid, cudaStream_t
   return launch_early(G.T <= 4 ? k_backward_quads_atom<BINARY, 4> : G.T <= 7 ? k_backward_quads_atom<BINARY, 7>
                                                                              : k_backward_quads_atom<BINARY, VA_BCH>,
                       grid, VA_WARPS * 32, 0, st, G);
+}
+
+// Enough atoms a grid pay for the copy, which costs the same for any of them, and enough (atom, channel) pairs in all fill the
+// chip.  50 x 3000 atoms of one channel on 28x48^3, in order 1705 us by single atoms from the gradient as it lies, 1276 like
+// this; with 28 weighted channels 1747 and 1537.
+// Loose rows have their pairs one by one otherwise: 14 channels of 41^3 of 0.5 A, 40 x 1500 / 8 x 400 / 1 x 1500 atoms 1483 /
+// 96 / 51 and 388 / 48 / 29 us, 28 channels of 65^3, 8 x 400 atoms 199 and 171, but 8 x 50 48 and 163, and 8 channels of 25^3
+// of 1 A, 1 x 1500 atoms 22 and 23.
+// Aligned rows have rounds of 14 channels, and up to 16 are as fast without the copy (40 x 1500 atoms on 14x48^3 of 0.5 A,
+// 0.11 atoms per cubic A: 389 and 464 us).  More channels, one / all weighted: 20 there 615 / 673 and 608 / 735, 28 698 / 712
+// and 657 / 743, 32 897 / 1008 and 669 / 753; 8 x 400 atoms (0.03) 28 85 and 91, 32 111 and 92; 28 channels of 24^3 of 1 A,
+// 8 x 2000 / 8 x 400 atoms 56 / 21 and 37 / 23.
+bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned) {
+  if (gm.rti || T > 32 || type_copy_bytes(gm, T) > TYPE_COPY_MOST) return false;
+  const double side = (double)gm.dim * gm.res, dense = N / (side * side * side), pairs = (double)nb * N * T;
+  if (!aligned) return T >= 8 && dense >= 0.011 && pairs >= 16000;
+  return T > 16 && dense >= (T > 28 ? 0.025 : T > 24 ? 0.12 : 0.2) && pairs >= 300e3 * gm.res * gm.res * gm.res;
+}
+
+template <int TO>
+static cudaError_t type_gradients(const TgArgs& A, unsigned voxels, float* copy, int n, cudaStream_t st) {
+  const BwdArgs& G = A.G;
+  const cudaError_t e = launch_early(k_channel_last<2 * TO>, dim3((voxels + CL_VOXELS - 1) / CL_VOXELS, n), 64 * TO, 0, st,
+                                     G.diff + (size_t)(G.b0 + A.first) * G.T * voxels, reinterpret_cast<float4*>(copy), voxels, G.T);
+  if (e != cudaSuccess) return e;
+  return launch_early(G.gm.binary ? k_type_gradients<TO, true> : k_type_gradients<TO, false>, dim3(G.N, n), 32, 0, st, A);
+}
+
+cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, long* launches, cudaStream_t st) {
+  if (G.N == 0 || G.nb == 0) return cudaSuccess;
+  TgArgs A;
+  A.G = G;
+  A.copy = reinterpret_cast<const Eight*>(copy);
+  const unsigned voxels = G.gm.dim * G.gm.dim * G.gm.dim;
+  cudaError_t e = cudaSuccess;
+  for (A.first = 0; e == cudaSuccess && A.first < G.nb; A.first += per_copy, *launches += 2) {
+    const int n = std::min(per_copy, G.nb - A.first);
+    e = G.T <= 8 ? type_gradients<1>(A, voxels, copy, n, st) : G.T <= 16 ? type_gradients<2>(A, voxels, copy, n, st)
+        : G.T <= 24 ? type_gradients<3>(A, voxels, copy, n, st) : type_gradients<4>(A, voxels, copy, n, st);
+  }
+  return e;
 }
 
 // Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:

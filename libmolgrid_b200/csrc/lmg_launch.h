@@ -116,6 +116,15 @@ cudaError_t launch_forward_self(const EmitArgs& A, const BwdArgs& G, bool early,
 // the same for the backward passes (modes 0 and 2, aligned tensors)
 bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode);
 cudaError_t launch_backward_self(const EmitArgs& A, const BwdArgs& G, int mode, cudaStream_t st);
+// type and atom gradients of type vectors from copies of the grid gradient with the channels of a voxel next to each
+// other: `per_copy` examples at a time into `copy`
+constexpr size_t TYPE_COPY_MOST = (size_t)256 << 20;   // largest copy of one example
+// of the examples that are copied together, if more than one: 50 x 3000 atoms on 28x48^3 in copies of 64 / 128 / 256 MB 1478 /
+// 1354 / 1276 us (each launch ends with its slowest atoms; two copies that take turns do not help)
+constexpr size_t TYPE_COPIES = (size_t)256 << 20;
+inline size_t type_copy_bytes(const GMParams& gm, int T) { return ((size_t)gm.dim * gm.dim * gm.dim + 1) * ((T + 7) / 8) * 32; }
+bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned);
+cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, long* launches, cudaStream_t st);
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st);
 // both terms of backward_gradients: out_grid (zero-filled before) and atom_gradients
 cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st);

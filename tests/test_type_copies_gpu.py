@@ -1,0 +1,111 @@
+"""Gradients of type vectors with radii by atom where the grid gradient is copied with the channels of a voxel next to each
+other (many atoms a grid): against the CPU oracle and against the kernels that read it where it lies, at the edges of the
+copy's channels and voxels, for atoms with none to many weighted channels."""
+import numpy as np
+import pytest
+import torch
+
+import libmolgrid_b200 as lmg
+from libmolgrid_b200 import api
+from libmolgrid_b200 import synthetic as cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(seed, B, N, T, side):
+    rng = np.random.default_rng(seed)
+    coords = rng.uniform(-side / 2 - 1, side / 2 + 1, (B, N, 3)).astype(np.float32)
+    radii = rng.uniform(1.0, 2.2, (B, N)).astype(np.float32)
+    types = np.zeros((B, N, T), np.float32)
+    for b in range(B):
+        for a in range(N):
+            k = (0, 1, 2, 4, 5, T)[a % 6]
+            types[b, a, rng.permutation(T)[:k]] = rng.uniform(0.1, 1, k)
+    return coords, types, radii
+
+
+def _close(got, want):
+    # sums of up to some hundred terms in another order, as for the other gradients
+    np.testing.assert_allclose(got, want, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(want).max())))
+
+
+def _gradients(g, data, diff, quads=1, **more):
+    lib = api._cabi.lib()
+    ag = torch.full(data[0].shape, 7.0, device="cuda")
+    tg = torch.full(data[1].shape, 7.0, device="cuda")
+    lib.lmg_set_quads(quads)
+    try:
+        g.backward(torch.zeros(len(ag), 3, device="cuda"), *data, diff, ag, tg, **more)
+    finally:
+        lib.lmg_set_quads(1)
+    return ag.cpu().numpy(), tg.cpu().numpy()
+
+
+@pytest.mark.parametrize("points,T,B,N", [(25, 8, 10, 200), (25, 9, 9, 200), (25, 16, 7, 200), (25, 17, 5, 200), (25, 24, 4, 200),
+                                          (25, 25, 4, 200), (25, 32, 3, 200), (24, 29, 27, 400), (24, 25, 8, 1700), (24, 17, 7, 2800),
+                                          (13, 31, 3, 200)])
+@pytest.mark.parametrize("binary,multiple", [(False, 1.0), (True, 1.0), (False, -1.5)])
+def test_copies(port, points, T, B, N, binary, multiple):
+    coords, types, radii = _batch(points * T, B, N, T, points - 1.0)
+    g = lmg.GridMaker(1.0, points - 1.0, binary, gaussian_radius_multiple=multiple)
+    og = port.gm(1.0, points - 1.0, binary, gaussian_radius_multiple=multiple)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    shape = (B,) + tuple(g.grid_dimensions(T))
+    diff = torch.randn(shape, device="cuda")
+    n = torch.tensor([N - 3 * b for b in range(B)], dtype=torch.int32, device="cuda")
+    ag, tg = _gradients(g, data, diff, n_atoms=n)
+    for a, b in zip((ag, tg), _gradients(g, data, diff, quads=0, n_atoms=n)):
+        _close(a, b)
+    for b in (0, B - 1):
+        m = N - 3 * b
+        wag, wtg = port.backward_vector(og, (0, 0, 0), coords[b, :m], types[b, :m], radii[b, :m], diff[b].cpu().numpy())
+        _close(ag[b, :m], wag)
+        _close(tg[b, :m], wtg)
+        assert not ag[b, m:].any() and not tg[b, m:].any()
+    again = _gradients(g, data, diff, n_atoms=n)
+    assert np.array_equal(ag, again[0]) and np.array_equal(tg, again[1])
+    # the same floats off a 16-byte boundary, and a workspace that has no room for copies
+    loose = torch.empty(diff.numel() + 1, device="cuda")[1:].view(shape).copy_(diff)
+    old = api.MAX_WORKSPACE_BYTES
+    try:
+        for d, room in ((loose, old), (diff, 2 * (N * (64 + 12 * T) + 4096))):
+            api.MAX_WORKSPACE_BYTES = room
+            api._workspaces.clear()
+            for a, b in zip(_gradients(g, data, d, n_atoms=n), (ag, tg)):
+                _close(a, b)
+    finally:
+        api.MAX_WORKSPACE_BYTES = old
+        api._workspaces.clear()
+
+
+def test_several_copies_and_one_example_more():
+    """More examples than are copied at a time, the last copy of a single one."""
+    points, T, N = 65, 32, 400
+    each = (points ** 3 + 1) * 128
+    B = (256 << 20) // each + 1
+    coords, types, radii = _batch(3, B, N, T, 32.0)
+    g = lmg.GridMaker(0.5, 32.0)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
+    for a, b in zip(_gradients(g, data, diff), _gradients(g, data, diff, quads=0)):
+        _close(a, b)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_values_beyond_reach_and_without_weight(value):
+    """Values that are no numbers, in voxels that no atom reaches and in channels without weight."""
+    points, T, B, N = 25, 14, 6, 200
+    coords, types, radii = _batch(5, B, N, T, 8.0)
+    types[:, :, 3] = 0
+    g = lmg.GridMaker(1.0, points - 1.0)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
+    ag, tg = _gradients(g, data, diff)
+    diff[:, :, :2], diff[:, :, :, :2], diff[..., :2], diff[..., -2:] = value, value, value, value
+    diff[:, 3] = value
+    ag2, tg2 = _gradients(g, data, diff)
+    assert np.isfinite(ag2).all()
+    _close(ag2, ag)
+    keep = [t for t in range(T) if t != 3]
+    _close(tg2[..., keep], tg[..., keep])
+    assert not np.isfinite(tg2[..., 3]).any()
