@@ -14,7 +14,8 @@ void lmg_set_precise(int mode);
  * red.global.add.v4.f32) where dim % 4 == 0 and the grid is 16-byte aligned; 0: never. */
 void lmg_set_quads(int on);
 /* 1 (default): GridInterpolater stages input boxes through tensor copies where rows of the input
- * are 16-byte aligned and out_resolution <= in_resolution; 0: always the direct-read kernel. */
+ * are 16-byte aligned, out_resolution <= in_resolution and the call is large enough for it to pay;
+ * 2: of any size; 0: always the direct-read kernel. */
 void lmg_set_interp_tiled(int on);
 /* Blocks of the tiled interpolation kernel that ever gave up a bounded wait for a staged box (they
  * finish through direct reads, so results stay correct); 0xffffffff if the counter cannot be read. */

@@ -18,7 +18,7 @@ namespace {
 thread_local std::string g_err;
 std::default_random_engine g_engine;  // same engine type as libmolgrid::random_engine
 int g_precise = -1;                   // -1 auto, 0 fast density, 1 reference-order density
-int g_interp_tiled = 1;               // tensor-copy staged interpolation where the input allows it
+int g_interp_tiled = 1;               // tensor-copy staged interpolation where the input allows it and it pays
 int g_quads = 1;                      // aligned-quad kernels where the grid allows them
 
 // ---- optional per-kernel timing (bench support; off by default) --------------------------------
@@ -801,6 +801,7 @@ int lmg_interpolate(const lmg_interpolater* gi, int batch, int nchannels, const 
                (uintptr_t)in % 16 == 0 && (gi->in_dim * sizeof(float)) % 16 == 0 &&
                gi->out_resolution <= 1.008f * gi->in_resolution &&
                (size_t)batch * nchannels < (size_t)1 << 31 &&
+               (g_interp_tiled > 1 || lmg::interp_tiles_pay(gi->in_dim, gi->out_dim, std::min(batch, lmg::INTERP_MAX_EX), nchannels)) &&
                make_input_maps(&maps, in, gi->in_dim, (size_t)batch * nchannels);
   for (int b0 = 0; b0 < batch; b0 += lmg::INTERP_MAX_EX) {
     int nb = std::min(lmg::INTERP_MAX_EX, batch - b0);

@@ -72,6 +72,8 @@ struct alignas(64) InterpMaps {
   CUtensorMap m[ITILE_NXY * ITILE_NXY * ITILE_NZ];
 };
 // the maps describe the input as a 4-d tensor {z, y, x, example*channels}
+// whether they are worth it: enough of them in a launch of nb examples
+bool interp_tiles_pay(unsigned in_dim, unsigned out_dim, int nb, int K);
 cudaError_t launch_interpolate_tiled(const InterpMaps& maps, const InterpArgs& I, int nb, cudaStream_t st);
 // how many blocks ever gave up waiting for a staged box (they finish through direct reads)
 cudaError_t read_tma_timeouts(unsigned* count);
