@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(SCAT_WARPS * 32) k_gradgrad_scatter(BwdArgs G)
 constexpr int QPASS = 8;  // quads per pass
 
 struct __align__(16) ZTabs {
-  float4 dz2[QPASS];  // (gz-az)^2, NaN outside [loz, hiz)
+  float4 dz2[QPASS];  // (gz-az)^2 (relevance: negated), NaN outside [loz, hiz)
   float4 ez[QPASS];   // exp(-2 dz2 / ar^2)
   float4 dz[QPASS];   // gz-az
   float lo[QPASS];    // smallest dz2 of the quad (NaN when no z of it lies in the footprint)
@@ -622,7 +622,7 @@ __device__ __forceinline__ void fill_ztabs(ZTabs& zt, unsigned zc, const ItemPar
   float dz = __fsub_rn(voxel_coord(oz, zz, res), P.z);
   bool in = zz >= P.loz && zz < P.hiz;
   float d2 = in ? __fmul_rn(dz, dz) : CUDART_NAN_F;
-  reinterpret_cast<float*>(zt.dz2)[lane] = d2;
+  reinterpret_cast<float*>(zt.dz2)[lane] = MODE == 2 ? -d2 : d2;  // relevance wants it negated
   reinterpret_cast<float*>(zt.ez)[lane] = gauss_factor<MODE>(d2, P, kexp);
   reinterpret_cast<float*>(zt.dz)[lane] = dz;
   float lo = fminf(d2, __shfl_xor_sync(0xffffffffu, d2, 1));  // fminf skips the NaN entries
@@ -660,7 +660,7 @@ __device__ __forceinline__ void fill_loose(TAB (&f)[4], unsigned zc, const ItemP
     const float dz = in ? __fsub_rn(voxel_coord(oz, zz, res), P.z) : 0.f;
     float d2 = in ? __fmul_rn(dz, dz) : CUDART_NAN_F;
     if (SCALED) d2 *= scale;
-    reinterpret_cast<float*>(f[t].dz2)[lane] = d2;
+    reinterpret_cast<float*>(f[t].dz2)[lane] = MODE == 2 ? -d2 : d2;
     reinterpret_cast<float*>(f[t].ez)[lane] = gauss_factor<MODE>(d2, P, kexp);
     if constexpr (std::is_same<TAB, LooseBackward>::value) reinterpret_cast<float*>(f[t].dz)[lane] = dz;
     float lo = fminf(d2, __shfl_xor_sync(0xffffffffu, d2, 1));
@@ -1181,47 +1181,50 @@ __device__ __forceinline__ BwdSums backward_quads_core(const BwdArgs& G, const I
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const float t = divide_near(dvv[j], dev[j]);
-        if (__fadd_rn(dxy2, d2v[j]) < P.Tbin && dev[j] > 0.f) tg += t;
+        if (__fsub_rn(dxy2, d2v[j]) < P.Tbin && dev[j] > 0.f) tg += t;
       }
     } else if constexpr (MODE == 2) {
-      // density * dv / total density, two voxels at a time with the roundings of tail_quotient() and divide_near();
-      // divisors and quotients that the short division cannot take go through the long one afterwards.  The kernel is
-      // bound by issue, and this is most of it: 434 -> 388 us for 50 x 3000 atoms on 28x48^3, the same bits.
+      // density * dv / total density, two voxels at a time with the roundings of tail_quotient() and divide_near(): the
+      // negated numbers of these where that saves a negation.  Divisors and quotients that the short division cannot take go
+      // through the long one afterwards; such a quotient is no number, and neither is the sum then.  The kernel is bound by
+      // issue, and this is most of it: 434 -> 388 us for 50 x 3000 atoms on 28x48^3, the same bits.
       float v[4], c[4];
       bool in[4], odd = false;
 #pragma unroll
       for (int j = 0; j < 4; j += 2) {
-        const Pair r = add2(pair(dxy2), pair(d2v[j], d2v[j + 1])), minus = pair(-1.f);
-        float r0, r1;
+        // the squared distance, its root and the root over the radius, all three negated
+        const Pair r = add2(pair(-dxy2), pair(d2v[j], d2v[j + 1]));
+        float r0, r1, t0, t1, g0, g1;
         split(r, r0, r1);
+        r0 = -r0;
+        r1 = -r1;
         const Pair y = pair(rsqrt_approx(r0), rsqrt_approx(r1)), s = mul2(r, y);
-        const Pair dist = fma2(fma2(mul2(s, minus), s, r), mul2(pair(0.5f), y), s);
+        const Pair dist = fma2(fma2(s, s, r), mul2(pair(0.5f), y), s);
         const Pair ir = pair(P.inv_ar), q = mul2(dist, ir), dr = fma2(fma2(q, pair(-P.ar), dist), ir, q);
         const Pair nz = pair(copysignf(0.f, -gm.res));  // see interp_blend(): keeps the products' own roundings
-        const Pair t = add2(fma2(add2(fma2(pair(gm.A), dr, nz), pair(gm.B)), dr, nz), pair(gm.C));
-        float t0, t1, g0, g1;
+        const Pair t = add2(fma2(add2(fma2(pair(gm.A), dr, nz), pair(-gm.B)), dr, nz), pair(gm.C));
         split(t, t0, t1);
         split(mul2(pair(exy), pair(ev[j], ev[j + 1])), g0, g1);
         v[j] = r0 <= P.Tg ? g0 : fmaxf(t0, 0.f);
         v[j + 1] = r1 <= P.Tg ? g1 : fmaxf(t1, 0.f);
-        in[j] = r0 <= P.Tcut && v[j] > 0.f;  // false for a NaN
-        in[j + 1] = r1 <= P.Tcut && v[j + 1] > 0.f;
+        in[j] = r0 <= P.Tcut && v[j] > 0.f && dev[j] > 0.f;  // false for a NaN
+        in[j + 1] = r1 <= P.Tcut && v[j + 1] > 0.f && dev[j + 1] > 0.f;
         const Pair n = mul2(pair(dvv[j], dvv[j + 1]), pair(v[j], v[j + 1])), d = pair(dev[j], dev[j + 1]);
-        const Pair rd = pair(rcp_approx(dev[j]), rcp_approx(dev[j + 1])), share = mul2(n, rd);
-        split(fma2(fma2(share, mul2(d, minus), n), rd, share), c[j], c[j + 1]);
+        const Pair rd = pair(rcp_approx(-dev[j]), rcp_approx(-dev[j + 1])), share = mul2(n, rd);  // and the quotient
+        split(fma2(fma2(share, d, n), rd, share), c[j], c[j + 1]);
+        odd = odd || (in[j] && dev[j] < 1e-30f) || (in[j + 1] && dev[j + 1] < 1e-30f);
       }
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        in[j] = in[j] && dev[j] > 0.f;
-        odd = odd || (in[j] && (dev[j] < 1e-30f || c[j] != c[j]));
-      }
-      if (odd) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) c[j] = divide_near(__fmul_rn(dvv[j], v[j]), dev[j]);
-      }
+      float sum = tg;
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (in[j]) tg += c[j];
+        if (in[j]) sum -= c[j];
+      if (odd || sum != sum) {
+        sum = tg;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (in[j]) sum += divide_near(__fmul_rn(dvv[j], v[j]), dev[j]);
+      }
+      tg = sum;
     }
   };
 
