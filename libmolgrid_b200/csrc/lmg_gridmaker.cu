@@ -2729,9 +2729,19 @@ bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode) {
          quads_of(G, G.diff, mode == 2 ? G.density : nullptr);
 }
 
+// Densities of many atoms a grid, whose sums outlast the zeros, have records of k_emit earlier: us with and without, all slots
+// atoms, 8 x 1500 / 8 x 3000 atoms on 22x41^3 30.4 / 44.3 and 31.9 / 49.7, on 14x33^3 17.6 / 26.4 and 18.7 / 31.2, 16 x 1900 on
+// 14x24^3 of 1 A 23.1 and 27.0, 8 x 3000 on 28x48^3 46.1 and 49.0; but 4 x 2000 on 14x24^3 10.6 and 9.4, 16 x 1900 on 28x48^3
+// 80.3 and 76.6.  With half of the slots empty, which leave at once, 16 x 1900 on 22x41^3 43.7 and 45.9, on 14x24^3 22.4 and 20.6:
+// only on loose rows, whose tables make a warp's own preparation the longer one.
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G) {
-  if (A.vec || (long)A.nb * A.N > FWD_SELF_ATOMS) return false;
-  return A.gm.binary || (!G.precise && quads_of(G, G.out_grid));
+  const long slots = (long)A.nb * A.N;
+  if (A.vec || slots > FWD_SELF_ATOMS) return false;
+  if (A.gm.binary) return true;
+  const bool loose = loose_rows(G);
+  const double voxels = (double)A.T * A.gm.dim * A.gm.dim * A.gm.dim;
+  if (voxels <= 1500.0 * A.N && (A.n_atoms == nullptr ? slots >= (loose ? 12000 : 14000) : loose && slots >= 20000)) return false;
+  return !G.precise && quads_of(G, G.out_grid);
 }
 
 template <bool BINARY, int WARPS, bool LOOSE>
