@@ -2677,6 +2677,219 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
   if (lane < 3) G.atom_gradients[ai * 3 + lane] = lane == 0 ? agx : lane == 1 ? agy : agz;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Type vectors whose radii differ by channel, all channels wanted: the footprints of an atom's channels lie in each other, so
+// a warp takes up to RT_CH channels of an ATOM, and what depends on the place alone - column, squared distance, its roots,
+// the address - is computed once for all of them.  A warp lists the quads that the largest sphere reaches and takes 32 at a
+// time, whose lines are mostly neighbours; a channel whose sphere reaches none of these is skipped.
+// Bound by issue.  Item by item the L1 bounded it (95 %: a lane per column touches 32 lines a load): soft types, 28 channels,
+// 4 x 3000 atoms on 96^3 of 0.25 A 2473 us, 4 x 1500 on 48^3 of 0.5 A 284, 8 x 1000 with 20 channels on 40^3 of 0.75 A 176; like this
+// 2014, 184 and 84.  On the way: lanes as (column, z-quad) of the whole footprint 3338 / 255 / 109, the list 2271 / 196 / 88; quads
+// in three shells by distance 2202 / 195 / 95; the tails of all channels apart 2514 / 221 / 105; channels by radius, blocks of an
+// atom's warps 2870 / 250 / 110, of one warp 2267 / 209 / 94; blocks of one warp, channels as they come 2185 / 194 / 86, then no test of
+// a weight for each.
+// ---------------------------------------------------------------------------------------------
+constexpr int RT_CH = 16, RT_WARPS = 4;  // channels a warp, most warps an atom
+constexpr int RT_MINB = 20;              // blocks of one warp an SM: 96 registers (16 / 24: 2395 / 2313 us instead of 2267)
+constexpr int RT_COLS = 128;
+constexpr int RT_LOADS = 4;              // channels that are requested together
+
+struct __align__(16) RtChannel {
+  float kexp, Tg, Tcut, inv_ar;
+  float k4, kE, kD, w;
+};
+struct __align__(16) RtShared {
+  RtChannel ch[RT_CH];
+  union {
+    ColBufDT<RT_COLS> cols;
+    float sums[RT_CH][33];
+  };
+  ZTabs zt;
+  float4 ez[RT_CH][QPASS];                // exp(-2 dz2 / ar^2) for each channel
+  unsigned short list[RT_COLS * QPASS];   // quads within reach: column | quad << 8
+};
+
+__global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, int per, int warps) {
+  wait_for_stream();
+  __shared__ RtShared sh;
+  const GMParams& gm = G.gm;
+  const int lane = threadIdx.x, item = blockIdx.x / warps, wid = blockIdx.x - item * warps, bl = blockIdx.y, b = G.b0 + bl;
+  float cx, cy, cz;
+  if (G.centers != nullptr) {
+    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
+  } else {
+    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
+  }
+  const float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
+  const ItemParams P = item_of(G.recs[(size_t)bl * G.N + item]);  // of the largest radius
+  const size_t dim = gm.dim, cs4 = dim * dim * dim / 4, ai = (size_t)b * G.N + item;
+  const int t0 = wid * per, nch = min(per, G.T - t0);
+  const ChanParam* params = G.chanp + (size_t)bl * G.T;
+  if (lane < RT_CH) {
+    RtChannel c = {0.f, -1.f, -1.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (lane < nch) {
+      const float4 p = params[t0 + lane].p;
+      c.kexp = p.x * NEG2_LOG2E; c.Tg = p.y; c.Tcut = p.w; c.inv_ar = p.z;
+      c.k4 = 4.f * p.x; c.kE = -gm.E * p.z; c.kD = -gm.D * p.x;
+      c.w = G.type_vector[ai * G.T + t0 + lane];
+    }
+    sh.ch[lane] = c;
+  }
+  __syncwarp();
+  const float4* diff = reinterpret_cast<const float4*>(G.diff) + ((size_t)b * G.T + t0) * cs4;
+  float tg[RT_CH], agx, agy, agz;
+  // SKIP: channels without weight stay out of the atom gradient
+  auto sweep = [&](auto skip) {
+    constexpr bool SKIP = decltype(skip)::value;
+#pragma unroll
+    for (int c = 0; c < RT_CH; c++) tg[c] = 0.f;
+    agx = agy = 0.f;
+    Pair az = pair(0.f);
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(sh.cols, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
+      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+        __syncwarp();
+        fill_ztabs(sh.zt, zc, P, oz, gm.res, 0.f, lane);
+        __syncwarp();
+        for (int c = 0; c < nch; c++) reinterpret_cast<float*>(sh.ez[c])[lane] = ex2_approx(reinterpret_cast<const float*>(sh.zt.dz2)[lane] * sh.ch[c].kexp);
+        const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
+        unsigned n = 0;
+        for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
+          const unsigned i = c0 + lane;
+          const float dxy2 = i < nkept ? sh.cols.dxy2[i] : CUDART_NAN_F;
+          unsigned mask = 0;
+#pragma unroll
+          for (unsigned q = 0; q < QPASS; q++)
+            if (q < nq && __fadd_rn(dxy2, sh.zt.lo[q]) <= P.Tcut) mask |= 1u << q;  // false for a NaN
+          unsigned upto = __popc(mask);
+          const unsigned own = upto;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const unsigned x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+          }
+          for (unsigned at = n + upto - own; mask != 0u; mask &= mask - 1u) sh.list[at++] = (unsigned short)(i | (__ffs(mask) - 1) << 8);
+          n += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (unsigned e0 = 0; e0 < n; e0 += 32) {
+          const unsigned e = sh.list[min(e0 + lane, n - 1u)], i = e & 255u, zq = e >> 8;
+          const float dxy2 = sh.cols.dxy2[i], near = e0 + lane < n ? __fadd_rn(dxy2, sh.zt.lo[zq]) : CUDART_NAN_F;
+          const float4* from = diff + (((size_t)sh.cols.row[i] * dim + zc) / 4 + zq);
+          const float4 d2 = sh.zt.dz2[zq];
+          const float d2v[4] = {d2.x, d2.y, d2.z, d2.w};
+          float r[4], root[4], id[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            r[j] = __fadd_rn(dxy2, d2v[j]);
+            // the root to the last place (root(), from the reciprocal root at hand): shared by the channels it costs little, and
+            // the type gradients are 3 to 17 % nearer to 64 bits than with the approximate one
+            id[j] = rsqrt_approx(r[j]);
+            const float x = __fmul_rn(r[j], id[j]);
+            root[j] = fmaf(fmaf(-x, x, r[j]), 0.5f * id[j], x);
+          }
+          Pair f[2] = {pair(0.f), pair(0.f)};
+#pragma unroll
+          for (int q = 0; q < RT_CH; q += RT_LOADS) {
+            if (q >= nch) break;
+            float4 dv[RT_LOADS];
+            bool live[RT_LOADS];
+#pragma unroll
+            for (int u = 0; u < RT_LOADS; u++) {
+              live[u] = near <= sh.ch[q + u].Tcut;  // false for a NaN, and for a channel that there is not
+              dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (live[u]) dv[u] = __ldg(from);
+              from += cs4;
+            }
+#pragma unroll
+            for (int u = 0; u < RT_LOADS; u++) {
+              if (!__any_sync(0xffffffffu, live[u])) continue;
+              const RtChannel& C = sh.ch[q + u];
+              const Pair dvp[2] = {pair(dv[u].x, dv[u].y), pair(dv[u].z, dv[u].w)};
+              const float4 e = sh.ez[q + u][zq];
+              const Pair exy = pair(ex2_approx(dxy2 * C.kexp)), ep[2] = {pair(e.x, e.y), pair(e.z, e.w)};
+              Pair sum = pair(0.f);
+#pragma unroll
+              for (int j = 0; j < 2; j++) {
+                float e0, e1, x0, x1, a0, a1, b0, b1;
+                split(mul2(exy, ep[j]), e0, e1);
+                const bool g0 = r[2 * j] <= C.Tg, g1 = r[2 * j + 1] <= C.Tg;
+                split(mul2(pair(root[2 * j], root[2 * j + 1]), pair(C.inv_ar)), x0, x1);
+                x0 = fma_sat(-gm.ta, x0, gm.tb);
+                x1 = fma_sat(-gm.ta, x1, gm.tb);
+                const Pair v = pair(g0 ? e0 : x0 * x0, g1 ? e1 : x1 * x1);
+                sum = j == 0 ? mul2(v, dvp[0]) : fma2(v, dvp[1], sum);
+                split(fma2(pair(C.kE), pair(id[2 * j], id[2 * j + 1]), pair(C.kD)), a0, a1);  // negative beyond the cut-off
+                split(mul2(pair(C.k4), pair(e0, e1)), b0, b1);
+                if (!SKIP || C.w != 0.f)  // the same for every lane
+                  f[j] = fma2(mul2(pair(g0 ? b0 : fmaxf(a0, 0.f), g1 ? b1 : fmaxf(a1, 0.f)), pair(C.w)), dvp[j], f[j]);
+              }
+              float sum0, sum1;
+              split(sum, sum0, sum1);
+              tg[q + u] += sum0 + sum1;
+            }
+          }
+          float f0, f1;
+          split(add2(f[0], f[1]), f0, f1);
+          agx = fmaf(f0 + f1, sh.cols.dx[i], agx);
+          agy = fmaf(f0 + f1, sh.cols.dy[i], agy);
+          const float4 dz = sh.zt.dz[zq];
+          az = fma2(f[0], pair(dz.x, dz.y), fma2(f[1], pair(dz.z, dz.w), az));
+        }
+      }
+      __syncwarp();
+    }
+    float z1;
+    split(az, agz, z1);
+    agz += z1;
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      agx += __shfl_xor_sync(0xffffffffu, agx, o);
+      agy += __shfl_xor_sync(0xffffffffu, agy, o);
+      agz += __shfl_xor_sync(0xffffffffu, agz, o);
+    }
+  };
+  agx = agy = agz = 0.f;
+#pragma unroll
+  for (int c = 0; c < RT_CH; c++) tg[c] = 0.f;
+  if (P.valid) {
+    // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either, and
+    // the sums are taken again.  Most without weight: left out at once.  28 channels of 96^3, 4 x 3000 atoms, all / one
+    // weighted: a test in any case 2185 / 1904 us, none 2075 / 2063.
+    const int weighted = __popc(__ballot_sync(0xffffffffu, lane < nch && sh.ch[lane & (RT_CH - 1)].w != 0.f));
+    bool again = 2 * weighted < nch;
+    if (!again) {
+      sweep(std::false_type());
+      const float whole = (agx + agy) + agz;
+      again = weighted < nch && whole != whole;
+    }
+    if (again) sweep(std::true_type());
+  }
+  // of several warps an atom, k_sum_parts adds up the parts
+  float* to = warps == 1 ? G.atom_gradients + ai * 3 : G.partial + (((size_t)bl * G.N + item) * warps + wid) * 3;
+  if (lane < 3) to[lane] = lane == 0 ? agx : lane == 1 ? agy : agz;
+#pragma unroll
+  for (int c = 0; c < RT_CH; c++) sh.sums[c][lane] = tg[c];
+  __syncwarp();
+  static_assert(RT_CH == 16, "two lanes a channel");
+  float sum = 0.f;
+#pragma unroll
+  for (int k = 0; k < 16; k++) sum += sh.sums[lane & 15][(lane & 16) + k];
+  sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+  if (lane < nch) G.type_gradients[ai * G.T + t0 + lane] = sum;
+}
+
+__global__ void __launch_bounds__(256) k_sum_parts(BwdArgs G, int warps) {
+  wait_for_stream();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= G.nb * G.N * 3) return;
+  const int a = i / 3, axis = i - a * 3;
+  float sum = 0.f;
+  for (int w = 0; w < warps; w++) sum += G.partial[((size_t)a * warps + w) * 3 + axis];
+  G.atom_gradients[(size_t)G.b0 * G.N * 3 + i] = sum;
+}
+
 // atom_gradients[a] = sum over channels in ascending order of partial[a][t] * w[a][t] for w != 0
 // (src/grid_maker.cpp:508-515)
 __global__ void __launch_bounds__(256) k_reduce_types(BwdArgs G) {
@@ -2876,6 +3089,18 @@ cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, l
   return e;
 }
 
+// Warps that share an atom's places among its channels serve coarse grids at any count, finer ones where there is work enough
+// for warps that last 4 to 16 times as long: us item by item / together, soft types, 28 channels, 8 x 1500 / 1 x 200 / 1 x 16 atoms on
+// 24^3 of 1 A 279 / 17.8 / 11.9 and 88 / 10.5 / 9.5, on 40^3 of 0.75 A 352 / 19.7 / 12.5 and 157 / 13.7 / 12.3, on 48^3 of 0.5 A 551 /
+// 24.7 / 14.6 and 360 / 23.6 / 21.1, 4 channels there 86 / 11.5 / 10.4 and 73 / 14.4 / 13.9; on 96^3 of 0.25 A 4 x 3000 / 8 x 400 / 1 x 1500
+// 2473 / 691 / 328 and 2075 / 855 / 446, which have most of their spheres' quads in the tail and in full columns.
+static bool channels_together(const BwdArgs& G) {
+  if (G.type_gradients == nullptr || G.T < 4 || G.T > RT_CH * RT_WARPS || G.gm.binary) return false;
+  if (G.gm.ta == 0.f && G.gm.tb == 0.f) return false;  // a Gaussian without a tail is cut by each channel's own footprint too
+  const double pairs = (double)G.N * G.nb * G.T;
+  return G.gm.res >= 0.7f ? pairs >= 600 : G.gm.res >= 0.4f ? pairs >= 12000 : G.gm.res >= 0.2f && G.T > 8 && pairs >= 300e3;
+}
+
 // Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:
 // 72.5 -> 59.8 us; 50 x 3000 on 28x41^3: 525 -> 501).  Gradients with records do not (22.7 us by single voxels, 28.7
 // by quads), nor do type vectors (4 x 1000 atoms, 28 channels of 41^3: 212 and 251 us).
@@ -2898,6 +3123,15 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
     dim3 gv((unsigned)((G.N + VA_WARPS - 1) / VA_WARPS), G.nb);
     if (G.type_gradients == nullptr) return launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
     return bin ? backward_quads_atom<true>(G, gv, st) : backward_quads_atom<false>(G, gv, st);
+  }
+  if (quads && channels_together(G)) {
+    // as few warps an atom as its channels need, more while the atoms alone leave the chip idle
+    const long atoms = (long)G.N * G.nb;
+    const int most = std::min(RT_WARPS, (G.T + 3) / 4), warps = std::max((G.T + RT_CH - 1) / RT_CH, (int)std::min((long)most, 8000 / atoms));
+    const int per = (G.T + warps - 1) / warps;
+    const cudaError_t e = launch_early(k_backward_channels, dim3(G.N * warps, G.nb), 32, 0, st, G, per, warps);
+    if (e != cudaSuccess || warps == 1) return e;
+    return launch_early(k_sum_parts, dim3((G.nb * G.N * 3 + 255) / 256), 256, 0, st, G, warps);
   }
   cudaError_t e;
   if (quads && G.type_gradients == nullptr) {

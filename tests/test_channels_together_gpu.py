@@ -1,0 +1,67 @@
+"""Gradients of type vectors with radii by channel where a warp takes several channels of an atom: against the CPU oracle, at the
+edges of the channels a warp takes, for atoms with no, one and all channels weighted."""
+import numpy as np
+import pytest
+import torch
+
+import libmolgrid_b200 as lmg
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(seed, N, T, side):
+    rng = np.random.default_rng(seed)
+    coords = rng.uniform(-side / 2 - 2, side / 2 + 2, (N, 3)).astype(np.float32)
+    radii = rng.uniform(0.6, 2.6, T).astype(np.float32)
+    radii[T // 2] = 0.0  # a channel that reaches nothing
+    types = np.zeros((N, T), np.float32)
+    for a in range(N):
+        k = (0, 1, T // 2 + 1, T)[a % 4]
+        types[a, rng.permutation(T)[:k]] = rng.uniform(0.1, 1, k)
+    return coords, types, radii
+
+
+def _close(got, want):
+    np.testing.assert_allclose(got, want, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(want).max())))
+
+
+# channels, atoms, points, resolution: one warp an atom to four, footprints of more columns than are held at a time
+@pytest.mark.parametrize("T,N,points,res", [(4, 160, 24, 1.0), (5, 2000, 16, 1.0), (16, 700, 24, 1.0), (16, 9000, 12, 1.0), (17, 100, 24, 1.0),
+                                            (17, 9000, 12, 1.0), (33, 60, 24, 1.0), (64, 20, 24, 1.0), (64, 3000, 8, 1.0), (28, 440, 32, 0.5),
+                                            (9, 40000, 16, 0.25), (14, 50, 36, 0.75)])
+@pytest.mark.parametrize("multiple", [1.0, 0.4, 2.5])
+def test_gradients(port, T, N, points, res, multiple):
+    side = (points - 1) * res
+    coords, types, radii = _case(T * points, N, T, side)
+    g, og = lmg.GridMaker(res, side, False, True, 1.0, multiple), port.gm(res, side, False, True, 1.0, multiple)
+    diff = torch.randn(g.grid_dimensions(T), device="cuda")
+    dc, dt, dr = (torch.from_numpy(x).cuda() for x in (coords, types, radii))
+    out = []
+    for _ in range(2):
+        ag, tg = torch.full((N, 3), 7.0, device="cuda"), torch.full((N, T), 7.0, device="cuda")
+        g.backward((0, 0, 0), dc, dt, dr, diff, ag, tg)
+        out.append((ag, tg))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    m = min(N, 40)
+    wag, wtg = port.backward_vector(og, (0, 0, 0), coords[:m], types[:m], radii, diff.cpu().numpy())
+    _close(out[0][0][:m].cpu().numpy(), wag)
+    _close(out[0][1][:m].cpu().numpy(), wtg)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("weighted", [(3,), (0, 1, 2, 4, 5, 6, 7, 8, 9, 10)])
+def test_channels_without_weight_do_not_reach_the_atoms(value, weighted):
+    T, N = 11, 200
+    coords, types, radii = _case(7, N, T, 20.0)
+    types[:] = 0
+    types[:, weighted] = np.random.default_rng(1).uniform(0.1, 1, (N, len(weighted)))
+    g = lmg.GridMaker(1.0, 23.0, False, True)
+    diff = torch.randn(g.grid_dimensions(T), device="cuda")
+    data = [torch.from_numpy(x.astype(np.float32)).cuda() for x in (coords, types, radii)]
+    grads = []
+    for v in (0.0, value):
+        diff[[t for t in range(T) if t not in weighted]] = v
+        grads.append((torch.empty(N, 3, device="cuda"), torch.empty(N, T, device="cuda")))
+        g.backward((0, 0, 0), *data, diff, *grads[-1])
+    _close(grads[1][0].cpu().numpy(), grads[0][0].cpu().numpy())
+    assert torch.equal(grads[0][1][:, list(weighted)], grads[1][1][:, list(weighted)])
