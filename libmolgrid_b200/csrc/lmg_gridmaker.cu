@@ -2709,6 +2709,30 @@ struct __align__(16) RtShared {
   unsigned short list[RT_COLS * QPASS];   // quads within reach: column | quad << 8
 };
 
+// Lists the quads of the nkept columns whose nearest voxel lies within Tcut; returns how many.
+__device__ __forceinline__ unsigned list_quads(unsigned short* list, const ColBufDT<RT_COLS>& cols, const ZTabs& zt, unsigned nkept,
+                                               unsigned nq, float Tcut, int lane) {
+  unsigned n = 0;
+  for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
+    const unsigned i = c0 + lane;
+    const float dxy2 = i < nkept ? cols.dxy2[i] : CUDART_NAN_F;
+    unsigned mask = 0;
+#pragma unroll
+    for (unsigned q = 0; q < QPASS; q++)
+      if (q < nq && __fadd_rn(dxy2, zt.lo[q]) <= Tcut) mask |= 1u << q;  // false for a NaN
+    unsigned upto = __popc(mask);
+    const unsigned own = upto;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
+    }
+    for (unsigned at = n + upto - own; mask != 0u; mask &= mask - 1u) list[at++] = (unsigned short)(i | (__ffs(mask) - 1) << 8);
+    n += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return n;
+}
+
 __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, int per, int warps) {
   wait_for_stream();
   __shared__ RtShared sh;
@@ -2752,25 +2776,7 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
         fill_ztabs(sh.zt, zc, P, oz, gm.res, 0.f, lane);
         __syncwarp();
         for (int c = 0; c < nch; c++) reinterpret_cast<float*>(sh.ez[c])[lane] = ex2_approx(reinterpret_cast<const float*>(sh.zt.dz2)[lane] * sh.ch[c].kexp);
-        const unsigned nq = min((unsigned)QPASS, (P.hiz - zc + 3) >> 2);
-        unsigned n = 0;
-        for (unsigned c0 = 0; c0 < nkept; c0 += 32) {
-          const unsigned i = c0 + lane;
-          const float dxy2 = i < nkept ? sh.cols.dxy2[i] : CUDART_NAN_F;
-          unsigned mask = 0;
-#pragma unroll
-          for (unsigned q = 0; q < QPASS; q++)
-            if (q < nq && __fadd_rn(dxy2, sh.zt.lo[q]) <= P.Tcut) mask |= 1u << q;  // false for a NaN
-          unsigned upto = __popc(mask);
-          const unsigned own = upto;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const unsigned x = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += x;
-          }
-          for (unsigned at = n + upto - own; mask != 0u; mask &= mask - 1u) sh.list[at++] = (unsigned short)(i | (__ffs(mask) - 1) << 8);
-          n += __shfl_sync(0xffffffffu, upto, 31);
-        }
+        const unsigned n = list_quads(sh.list, sh.cols, sh.zt, nkept, min((unsigned)QPASS, (P.hiz - zc + 3) >> 2), P.Tcut, lane);
         __syncwarp();
 #pragma unroll 1
         for (unsigned e0 = 0; e0 < n; e0 += 32) {
@@ -2878,6 +2884,190 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
   for (int k = 0; k < 16; k++) sum += sh.sums[lane & 15][(lane & 16) + k];
   sum += __shfl_xor_sync(0xffffffffu, sum, 16);
   if (lane < nch) G.type_gradients[ai * G.T + t0 + lane] = sum;
+}
+
+// backward_gradients for the same layout (see k_second_quads_nz for the terms): the sums over an atom's channels that its
+// term needs, with the weights w and the incoming type gradients t, are taken voxel by voxel - of w alpha diff and t alpha diff for
+// the products of distances, of w s diff and t s diff for the rest.  Only channels that carry weight take part.
+// Bound by issue at few warps: 20 blocks an SM spill and gain nothing (soft types, 4 x 1500 atoms on 28x48^3 of 0.5 A: item by item
+// 543 us, like this 350, with 20 360).
+constexpr int RS_MINB = 16;
+constexpr int RS_LOADS = 2;
+__global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int per, int warps) {
+  wait_for_stream();
+  __shared__ RtShared sh;
+  __shared__ float tgrad[RT_CH];
+  __shared__ size_t offset[RT_CH];  // of the weighted channels, from the first of the warp's
+  const GMParams& gm = G.gm;
+  const int lane = threadIdx.x, item = blockIdx.x / warps, wid = blockIdx.x - item * warps, bl = blockIdx.y, b = G.b0 + bl;
+  float cx, cy, cz;
+  if (G.centers != nullptr) {
+    cx = G.centers[b * 3]; cy = G.centers[b * 3 + 1]; cz = G.centers[b * 3 + 2];
+  } else {
+    cx = G.center_host[0]; cy = G.center_host[1]; cz = G.center_host[2];
+  }
+  const float ox = __fsub_rn(cx, gm.half), oy = __fsub_rn(cy, gm.half), oz = __fsub_rn(cz, gm.half);
+  ItemParams P = item_of(G.recs[(size_t)bl * G.N + item]);
+  const size_t dim = gm.dim, cs = dim * dim * dim, ai = (size_t)b * G.N + item;
+  const int t0 = wid * per, nch = min(per, G.T - t0);
+  const float inx = G.ag_in[ai * 3], iny = G.ag_in[ai * 3 + 1], inz = G.ag_in[ai * 3 + 2];
+  bool strange = false;
+  float cut = -1.f;
+  const float weight = lane < nch ? G.type_vector[ai * G.T + t0 + lane] : 0.f;
+  const unsigned weighted = __ballot_sync(0xffffffffu, weight != 0.f);
+  const int count = __popc(weighted);
+  if (lane < RT_CH) {
+    sh.ch[lane].Tcut = -1.f;
+    offset[lane] = 0;
+  }
+  __syncwarp();
+  if (weight != 0.f) {
+    const float4 p = G.chanp[(size_t)bl * G.T + t0 + lane].p;
+    RtChannel c;
+    c.kexp = p.x * NEG2_LOG2E; c.Tg = p.y; c.Tcut = cut = p.w; c.inv_ar = p.z;
+    c.k4 = 4.f * p.x; c.kE = -gm.E * p.z; c.kD = -gm.D * p.x;
+    c.w = weight;
+    const float t = G.tg_in[ai * G.T + t0 + lane];
+    strange = !finite3(weight * inx, weight * iny, weight * inz) || !finite3(t, 0.f, 0.f);
+    const int slot = __popc(weighted & ((1u << lane) - 1u));
+    sh.ch[slot] = c;
+    tgrad[slot] = t;
+    offset[slot] = lane * cs;
+  }
+  const bool odd = __any_sync(0xffffffffu, strange);
+  // the footprint of the largest of the weighted channels, which the others lie in
+  float most = cut;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+  P.valid = P.valid && most >= 0.f;
+  if (P.valid) {
+    const ChanParam big = G.chanp[(size_t)bl * G.T + t0 + __ffs(__ballot_sync(0xffffffffu, cut == most)) - 1];
+    P.Tcut = big.p.w;
+    bounds_1d(ox, P.x, big.q.z, gm.res, gm.dim, P.lox, P.hix);
+    bounds_1d(oy, P.y, big.q.z, gm.res, gm.dim, P.loy, P.hiy);
+    bounds_1d(oz, P.z, big.q.z, gm.res, gm.dim, P.loz, P.hiz);
+    P.valid = P.hix > P.lox && P.hiy > P.loy && P.hiz > P.loz;
+  }
+  __syncwarp();
+  float agx = 0.f, agy = 0.f, agz = 0.f;
+  Pair sb1 = pair(0.f), sb2 = pair(0.f);  // sums of w s diff and t s diff
+  const size_t first = ((size_t)b * G.T + t0) * cs;
+  auto sweep = [&](auto odd) {
+    for (Columns cols(P); cols.more();) {
+      const unsigned nkept = cols.compact<true>(sh.cols, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
+      for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
+        __syncwarp();
+        fill_ztabs(sh.zt, zc, P, oz, gm.res, 0.f, lane);
+        __syncwarp();
+        for (int c = 0; c < count; c++) reinterpret_cast<float*>(sh.ez[c])[lane] = ex2_approx(reinterpret_cast<const float*>(sh.zt.dz2)[lane] * sh.ch[c].kexp);
+        const unsigned n = list_quads(sh.list, sh.cols, sh.zt, nkept, min((unsigned)QPASS, (P.hiz - zc + 3) >> 2), P.Tcut, lane);
+        __syncwarp();
+#pragma unroll 1
+        for (unsigned e0 = 0; e0 < n; e0 += 32) {
+          const unsigned e = sh.list[min(e0 + lane, n - 1u)], i = e & 255u, zq = e >> 8;
+          const float dxy2 = sh.cols.dxy2[i], dx = sh.cols.dx[i], dy = sh.cols.dy[i];
+          const float near = e0 + lane < n ? __fadd_rn(dxy2, sh.zt.lo[zq]) : CUDART_NAN_F;
+          const size_t off = first + (size_t)sh.cols.row[i] * dim + zc + 4 * zq;
+          const float* from = G.diff + off;
+          float* to = G.out_grid + off;
+          const float4 d2 = sh.zt.dz2[zq], dz = sh.zt.dz[zq];
+          const Pair r[2] = {add2(pair(dxy2), pair(d2.x, d2.y)), add2(pair(dxy2), pair(d2.z, d2.w))}, dzp[2] = {pair(dz.x, dz.y), pair(dz.z, dz.w)};
+          const float dotxy = fmaf(dx, inx, dy * iny);
+          float rv[4];
+          Pair id[2], id2[2], dist[2], dot[2], a1[2], a2[2], b1 = pair(0.f), b2 = pair(0.f);
+#pragma unroll
+          for (int j = 0; j < 2; j++) {
+            split(r[j], rv[2 * j], rv[2 * j + 1]);
+            id[j] = pair(rsqrt_approx(rv[2 * j]), rsqrt_approx(rv[2 * j + 1]));
+            id2[j] = mul2(id[j], id[j]);
+            dist[j] = mul2(r[j], id[j]);
+            dot[j] = fma2(dzp[j], pair(inz), pair(dotxy));
+            a1[j] = a2[j] = pair(0.f);
+          }
+#pragma unroll 1
+          for (int q = 0; q < count; q += RS_LOADS) {
+            float4 dv[RS_LOADS];
+            bool live[RS_LOADS];
+#pragma unroll
+            for (int u = 0; u < RS_LOADS; u++) {
+              live[u] = near <= sh.ch[q + u].Tcut;  // false for a NaN, and for a channel that there is not
+              dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (live[u]) dv[u] = __ldg(reinterpret_cast<const float4*>(from + offset[q + u]));
+            }
+#pragma unroll
+            for (int u = 0; u < RS_LOADS; u++) {
+              if (!__any_sync(0xffffffffu, live[u])) continue;
+              const RtChannel& C = sh.ch[q + u];
+              const float4 e = sh.ez[q + u][zq];
+              const Pair exy = pair(ex2_approx(dxy2 * C.kexp)), ep[2] = {pair(e.x, e.y), pair(e.z, e.w)}, w = pair(C.w), t = pair(tgrad[q + u]);
+              float v[4];
+#pragma unroll
+              for (int j = 0; j < 2; j++) {
+                float g0, g1, x0, x1, y0, y1;
+                const bool gauss0 = rv[2 * j] <= C.Tg, gauss1 = rv[2 * j + 1] <= C.Tg, in0 = rv[2 * j] <= C.Tcut, in1 = rv[2 * j + 1] <= C.Tcut;
+                const Pair g = mul2(exy, ep[j]), kid = mul2(pair(C.kE), id[j]), sg = mul2(pair(C.k4), g);
+                split(mul2(dist[j], pair(C.inv_ar)), x0, x1);
+                x0 = fma_sat(-gm.ta, x0, gm.tb);
+                x1 = fma_sat(-gm.ta, x1, gm.tb);
+                split(g, g0, g1);
+                const Pair val = pair(gauss0 ? g0 : x0 * x0, gauss1 ? g1 : x1 * x1);
+                split(sg, g0, g1);
+                split(add2(kid, pair(C.kD)), x0, x1);
+                const Pair sl = pair(gauss0 ? g0 : fmaxf(x0, 0.f), gauss1 ? g1 : fmaxf(x1, 0.f));
+                split(mul2(pair(C.k4), sg), g0, g1);
+                split(mul2(kid, id2[j]), y0, y1);
+                const Pair alpha = pair(gauss0 ? g0 : in0 ? y0 : 0.f, gauss1 ? g1 : in1 ? y1 : 0.f);
+                Pair sd = mul2(sl, mul2(dot[j], w));
+                if constexpr (odd.value) sd = only_off_atom(sd, r[j], in0, in1);
+                Pair out2 = fma2(val, t, sd);
+                if constexpr (odd.value) out2 = only(out2, in0, in1);
+                split(out2, v[2 * j], v[2 * j + 1]);
+                // a neighbour's value may be anything
+                const Pair d = only(j == 0 ? pair(dv[u].x, dv[u].y) : pair(dv[u].z, dv[u].w), in0, in1);
+                const Pair da = mul2(d, alpha), ds = mul2(d, sl);
+                a1[j] = fma2(w, da, a1[j]);
+                a2[j] = fma2(t, da, a2[j]);
+                b1 = fma2(w, ds, b1);
+                b2 = fma2(t, ds, b2);
+              }
+              if (live[u]) red_add_v4(to + offset[q + u], v[0], v[1], v[2], v[3]);
+            }
+          }
+          sb1 = add2(sb1, b1);
+          sb2 = add2(sb2, b2);
+          float x0, x1, y0, y1, z0, z1;
+          const Pair p[2] = {mul2(a1[0], dot[0]), mul2(a1[1], dot[1])};
+          split(add2(p[0], p[1]), x0, x1);
+          split(add2(a2[0], a2[1]), y0, y1);
+          split(fma2(dzp[0], fma2(a2[0], dzp[0], p[0]), mul2(dzp[1], fma2(a2[1], dzp[1], p[1]))), z0, z1);
+          agx = fmaf(dx, fmaf(y0 + y1, dx, x0 + x1), agx);
+          agy = fmaf(dy, fmaf(y0 + y1, dy, x0 + x1), agy);
+          agz += z0 + z1;
+        }
+      }
+      __syncwarp();
+    }
+  };
+  if (P.valid) {
+    if (odd) sweep(std::true_type());
+    else sweep(std::false_type());
+    float x0, x1, y0, y1;
+    split(sb1, x0, x1);
+    split(sb2, y0, y1);
+    x0 += x1;
+    y0 += y1;
+    agx -= fmaf(x0, inx, y0);
+    agy -= fmaf(x0, iny, y0);
+    agz -= fmaf(x0, inz, y0);
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    agx += __shfl_xor_sync(0xffffffffu, agx, o);
+    agy += __shfl_xor_sync(0xffffffffu, agy, o);
+    agz += __shfl_xor_sync(0xffffffffu, agz, o);
+  }
+  float* parts = warps == 1 ? G.atom_gradients + ai * 3 : G.partial + (((size_t)bl * G.N + item) * warps + wid) * 3;
+  if (lane < 3) parts[lane] = lane == 0 ? agx : lane == 1 ? agy : agz;
 }
 
 __global__ void __launch_bounds__(256) k_sum_parts(BwdArgs G, int warps) {
@@ -3095,10 +3285,19 @@ cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, l
 // 24.7 / 14.6 and 360 / 23.6 / 21.1, 4 channels there 86 / 11.5 / 10.4 and 73 / 14.4 / 13.9; on 96^3 of 0.25 A 4 x 3000 / 8 x 400 / 1 x 1500
 // 2473 / 691 / 328 and 2075 / 855 / 446, which have most of their spheres' quads in the tail and in full columns.
 static bool channels_together(const BwdArgs& G) {
-  if (G.type_gradients == nullptr || G.T < 4 || G.T > RT_CH * RT_WARPS || G.gm.binary) return false;
+  if (G.T < 4 || G.T > RT_CH * RT_WARPS || G.gm.binary) return false;
   if (G.gm.ta == 0.f && G.gm.tb == 0.f) return false;  // a Gaussian without a tail is cut by each channel's own footprint too
   const double pairs = (double)G.N * G.nb * G.T;
   return G.gm.res >= 0.7f ? pairs >= 600 : G.gm.res >= 0.4f ? pairs >= 12000 : G.gm.res >= 0.2f && G.T > 8 && pairs >= 300e3;
+}
+
+static cudaError_t channels_together_launch(void (*kernel)(BwdArgs, int, int), const BwdArgs& G, long enough, cudaStream_t st) {
+  // as few warps an atom as its channels need, more while the atoms alone leave the chip idle
+  const long atoms = (long)G.N * G.nb;
+  const int most = std::min(RT_WARPS, (G.T + 3) / 4), warps = std::max((G.T + RT_CH - 1) / RT_CH, (int)std::min((long)most, enough / atoms));
+  const cudaError_t e = launch_early(kernel, dim3(G.N * warps, G.nb), 32, 0, st, G, (G.T + warps - 1) / warps, warps);
+  if (e != cudaSuccess || warps == 1) return e;
+  return launch_early(k_sum_parts, dim3((G.nb * G.N * 3 + 255) / 256), 256, 0, st, G, warps);
 }
 
 // Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:
@@ -3124,14 +3323,8 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
     if (G.type_gradients == nullptr) return launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
     return bin ? backward_quads_atom<true>(G, gv, st) : backward_quads_atom<false>(G, gv, st);
   }
-  if (quads && channels_together(G)) {
-    // as few warps an atom as its channels need, more while the atoms alone leave the chip idle
-    const long atoms = (long)G.N * G.nb;
-    const int most = std::min(RT_WARPS, (G.T + 3) / 4), warps = std::max((G.T + RT_CH - 1) / RT_CH, (int)std::min((long)most, 8000 / atoms));
-    const int per = (G.T + warps - 1) / warps;
-    const cudaError_t e = launch_early(k_backward_channels, dim3(G.N * warps, G.nb), 32, 0, st, G, per, warps);
-    if (e != cudaSuccess || warps == 1) return e;
-    return launch_early(k_sum_parts, dim3((G.nb * G.N * 3 + 255) / 256), 256, 0, st, G, warps);
+  if (quads && G.type_gradients != nullptr && channels_together(G)) {
+    return channels_together_launch(k_backward_channels, G, 8000, st);
   }
   cudaError_t e;
   if (quads && G.type_gradients == nullptr) {
@@ -3154,6 +3347,11 @@ cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
   if (quads && !G.gm.rti) {
     return launch_early(k_second_quads_atom, dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st, G);
   }
+  // Item by item only the weighted channels have warps, so one of many (as one-hot types have) gains less: us item by item /
+  // together, 28 channels, soft / one-hot types, 8 x 1500 atoms on 24^3 of 1 A 446 / 62 and 161 / 49, 4 x 1500 on 48^3 of 0.5 A 543 / 74 and
+  // 350 / 71, but 8 channels there, 8 x 1500 atoms one-hot 69 and 80, and 28 of 96^3 of 0.25 A, 4 x 3000 atoms 4241 / 356 and 4177 / 456.
+  if (quads && (G.gm.res >= 0.7f || (G.gm.res >= 0.4f && G.T >= 24)) && channels_together(G))
+    return channels_together_launch(k_second_channels, G, 3000, st);
   cudaError_t e;
   if (quads) {
     const long units = (long)G.N * nz_groups(G.T);

@@ -65,3 +65,30 @@ def test_channels_without_weight_do_not_reach_the_atoms(value, weighted):
         g.backward((0, 0, 0), *data, diff, *grads[-1])
     _close(grads[1][0].cpu().numpy(), grads[0][0].cpu().numpy())
     assert torch.equal(grads[0][1][:, list(weighted)], grads[1][1][:, list(weighted)])
+
+
+@pytest.mark.parametrize("T,N,points,res", [(4, 160, 24, 1.0), (16, 60, 24, 1.0), (17, 60, 24, 1.0), (33, 60, 24, 1.0), (64, 20, 24, 1.0),
+                                            (28, 440, 32, 0.5), (14, 50, 36, 0.75)])
+@pytest.mark.parametrize("multiple", [1.0, 2.0])
+@pytest.mark.parametrize("infinite", [False, True])
+def test_second_derivatives(port, T, N, points, res, multiple, infinite):
+    side = (points - 1) * res
+    coords, types, radii = _case(T + points, N, T, side)
+    rng = np.random.default_rng(T)
+    ca, ct = rng.normal(size=(N, 3)).astype(np.float32), rng.normal(size=(N, T)).astype(np.float32)
+    diff = rng.normal(size=(T, points, points, points)).astype(np.float32)
+    if infinite:  # an incoming gradient that is no number stays within its atom's reach
+        coords[5] = 0.0
+        ca[5, 1] = np.inf
+    g, og = lmg.GridMaker(res, side, False, True, 1.0, multiple), port.gm(res, side, False, True, 1.0, multiple)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii, diff, ca, ct)]
+    dd, da, dt = torch.full(diff.shape, 7.0, device="cuda"), torch.full((N, 3), 7.0, device="cuda"), torch.full((N, T), 7.0, device="cuda")
+    g.backward_gradients((0, 0, 0), *data, dd, da, dt)
+    wd, wa, wt = port.backward_gradients(og, (0, 0, 0), coords, types, radii, diff, ca, ct)
+    got, keep = dd.cpu().numpy(), np.isfinite(wd)
+    if infinite:
+        assert keep.mean() > 0.5 and np.isfinite(got[keep]).all()
+    _close(got[keep], wd[keep])
+    rows = [a for a in range(N) if not (infinite and a == 5)]
+    _close(da.cpu().numpy()[rows], wa[rows])
+    assert not dt.any()
