@@ -2065,11 +2065,11 @@ __global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(
 // ---------------------------------------------------------------------------------------------
 // The same for many atoms a grid: every channel is read under every footprint, and above the L1 takes a clock for each line
 // that a request touches, 85 columns in each of 28 channels.  A copy of the gradient with the channels of a voxel next to
-// each other makes that one line a voxel, and the sums are bound by the L2 instead (50 x 3000 atoms on 28x48^3: 12.7 GB at 12
-// TB/s, 22 % of the time waiting for issue slots).  Blocks of one warp: several atoms a block, neighbours by Morton's curve,
-// meet too few lines of each other's in the L1 (hits 22 to 35 %, as without order) for what the wait for the slowest costs
-// (1590 us for 1225).  Quads of a column and voxels of a lane requested together, blocks an SM: 4 / 4 / 20 1226 us, 2 / 4 / 20
-// 1301, 4 / 4 / 24 1297 to 1505 (the L1 gets what shared memory leaves), 4 / 6 / 20 1267.
+// each other makes that one line a voxel, and what bounds the sums are the loads from the L2 (83 kB an atom, 11 TB/s; L1 62 %,
+// issue 48 %).  Blocks of one warp: several atoms a block, neighbours by Morton's curve, meet too few lines of each other's
+// in the L1 (hits 22 to 35 %, as without order) for what the wait for the slowest costs (50 x 3000 atoms on 28x48^3: 1590 us for
+// 1225).  Quads of a column and voxels of a lane requested together, blocks an SM: 4 / 4 / 20 1226 us, 2 / 4 / 20 1301, 4 / 4 / 24
+// 1297 to 1505 (the L1 gets what shared memory leaves), 4 / 6 / 20 1267; with the atoms of many weighted channels beside, 1271.
 // ---------------------------------------------------------------------------------------------
 constexpr int CL_VOXELS = 128, CL_PITCH = CL_VOXELS + 1;
 
