@@ -288,13 +288,15 @@ Layout layout(const lmg_gridmaker* g, int op, int nb, int N, int T, int vec) {
   L.recs = o; o += recs * nb;
   L.chanp = o; o += chanp * nb;
   L.partial = o; o += partial * nb;
-  const lmg::GMParams gm = lmg::to_params(g);
-  // the rows of an aligned tensor; of another one with such rows it is not known here
-  if (partial != 0 && op == LMG_OP_BACKWARD && lmg::type_copies_serve(gm, nb, N, T, g->dim % 4 == 0)) {
-    const size_t each = lmg::type_copy_bytes(gm, T);
-    L.copies = (int)std::max<size_t>(1, std::min<size_t>(nb, lmg::TYPE_COPIES / each));
-    L.copy = L.partial;
-    L.copy_end = L.copy + L.copies * each;
+  if (partial != 0 && op == LMG_OP_BACKWARD) {
+    const lmg::GMParams gm = lmg::to_params(g);
+    // the rows of an aligned tensor; of another one with such rows it is not known here
+    if (lmg::type_copies_serve(gm, nb, N, T, g->dim % 4 == 0)) {
+      const size_t each = lmg::type_copy_bytes(gm, T);
+      L.copies = (int)std::max<size_t>(1, std::min<size_t>(nb, lmg::TYPE_COPIES / each));
+      L.copy = L.partial;
+      L.copy_end = L.copy + L.copies * each;
+    }
   }
   L.total = std::max(o, L.copy_end);
   return L;
@@ -634,8 +636,10 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
     }
     if (e != cudaSuccess) return cuda_fail(e, "emit");
     g_launches += 1 + ((vec && g->radii_type_indexed) ? 1 : 0);
-    // a workspace that is too small for the copies is enough for the kernels that need none
-    const bool copies = type_gradients != nullptr && L.copies > 0 && L.copy_end <= workspace_bytes && g_quads;
+    // a workspace that is too small for the copies, or off the boundary that their 32-byte loads want, is enough for the
+    // kernels that need none
+    const bool copies = type_gradients != nullptr && L.copies > 0 && L.copy_end <= workspace_bytes && g_quads &&
+                        ((uintptr_t)ws + L.copy) % 32 == 0;
     ProfRec* pr = prof_begin(1, st);
     {
       Range r(mode == 2 ? "backward relevance" : "backward");

@@ -109,3 +109,27 @@ def test_values_beyond_reach_and_without_weight(value):
     keep = [t for t in range(T) if t != 3]
     _close(tg2[..., keep], tg[..., keep])
     assert not np.isfinite(tg2[..., 3]).any()
+
+
+def test_workspace_off_the_boundary_of_the_copies():
+    """A workspace 16 bytes off a 32-byte boundary takes the kernels that need no copies."""
+    import ctypes
+    from libmolgrid_b200 import _cabi
+    lib, points, T, B, N = _cabi.lib(), 25, 16, 7, 200
+    coords, types, radii = _batch(11, B, N, T, points - 1.0)
+    g = lmg.GridMaker(1.0, points - 1.0)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
+    want = _gradients(g, data, diff)
+    a = _cabi.AtomsStruct()
+    a.batch, a.max_atoms, a.ntypes = B, N, T
+    a.coords, a.type_vector, a.radii = (t.data_ptr() for t in data)
+    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD, B, N, T, 1)
+    room = torch.empty(need + 64, dtype=torch.uint8, device="cuda")
+    for off in (0, 16):
+        ag, tg = torch.full((B, N, 3), 7.0, device="cuda"), torch.full((B, N, T), 7.0, device="cuda")
+        rc = lib.lmg_backward(ctypes.byref(g.s), ctypes.byref(a), diff.data_ptr(), ag.data_ptr(), tg.data_ptr(),
+                              room.data_ptr() + off, need, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, lib.lmg_last_error()
+        _close(ag.cpu().numpy(), want[0])
+        _close(tg.cpu().numpy(), want[1])
