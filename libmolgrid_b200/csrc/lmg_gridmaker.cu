@@ -2410,6 +2410,7 @@ __global__ void __launch_bounds__(32, TG_MINB) k_type_gradients(TgArgs A) {
     const float whole = (ag[0] + ag[1]) + ag[2];
     if (!dense || whole == whole) break;
   }
+  if (m == 0u) ag[0] = ag[1] = ag[2] = 0.f;  // no channel is the atom's, and the first was read all the same
 #pragma unroll
   for (int c = 0; c < 4; c++) split(tg[c], sh.sums[lane][2 * c], sh.sums[lane][2 * c + 1]);
   __syncwarp();

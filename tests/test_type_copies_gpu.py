@@ -111,6 +111,23 @@ def test_values_beyond_reach_and_without_weight(value):
     assert not np.isfinite(tg2[..., 3]).any()
 
 
+@pytest.mark.parametrize("points,T,B,N", [(25, 8, 10, 200), (25, 14, 6, 200), (24, 29, 27, 400)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_atoms_without_weight_take_no_channel(points, T, B, N, value):
+    """The first channel is no number anywhere and carries no weight: atoms without any weight have exactly no gradient."""
+    coords, types, radii = _batch(points + T, B, N, T, points - 1.0)
+    types[:, :, 0] = 0
+    g = lmg.GridMaker(1.0, points - 1.0)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
+    ag, tg = _gradients(g, data, diff)
+    diff[:, 0] = value
+    ag2, tg2 = _gradients(g, data, diff)
+    assert not ag2[~types.any(-1)].any()
+    _close(ag2, ag)
+    _close(tg2[..., 1:], tg[..., 1:])
+
+
 def test_workspace_off_the_boundary_of_the_copies():
     """A workspace 16 bytes off a 32-byte boundary takes the kernels that need no copies."""
     import ctypes
