@@ -2734,6 +2734,20 @@ __device__ __forceinline__ unsigned list_quads(unsigned short* list, const ColBu
   return n;
 }
 
+// A channel whose sphere is smaller than a voxel reaches the voxel nearest to the atom at most, and not even that where its
+// own footprint leaves it out: beside a coordinate a radius of 1e-7 times it is nothing, and the footprint is empty.
+// The footprint that it shares with larger channels does not tell.
+__device__ __forceinline__ bool reaches_nothing(const GMParams& gm, float densityrad, const ItemParams& P, float ox, float oy, float oz) {
+  if (!(densityrad < 0.5f * gm.res)) return false;
+  auto along = [&](float origin, float at) {
+    unsigned lo, hi;
+    bounds_1d(origin, at, densityrad, gm.res, gm.dim, lo, hi);
+    const float nearest = rintf(__fdiv_rn(__fsub_rn(at, origin), gm.res));
+    return nearest >= (float)lo && nearest < (float)hi;
+  };
+  return !(along(ox, P.x) && along(oy, P.y) && along(oz, P.z));
+}
+
 __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, int per, int warps) {
   wait_for_stream();
   __shared__ RtShared sh;
@@ -2753,8 +2767,10 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
   if (lane < RT_CH) {
     RtChannel c = {0.f, -1.f, -1.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (lane < nch) {
-      const float4 p = params[t0 + lane].p;
-      c.kexp = p.x * NEG2_LOG2E; c.Tg = p.y; c.Tcut = p.w; c.inv_ar = p.z;
+      const ChanParam cp = params[t0 + lane];
+      const float4 p = cp.p;
+      c.kexp = p.x * NEG2_LOG2E; c.Tg = p.y; c.inv_ar = p.z;
+      c.Tcut = reaches_nothing(gm, cp.q.z, P, ox, oy, oz) ? -1.f : p.w;
       c.k4 = 4.f * p.x; c.kE = -gm.E * p.z; c.kD = -gm.D * p.x;
       c.w = G.type_vector[ai * G.T + t0 + lane];
     }
@@ -2923,9 +2939,11 @@ __global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int 
   }
   __syncwarp();
   if (weight != 0.f) {
-    const float4 p = G.chanp[(size_t)bl * G.T + t0 + lane].p;
+    const ChanParam cp = G.chanp[(size_t)bl * G.T + t0 + lane];
+    const float4 p = cp.p;
     RtChannel c;
-    c.kexp = p.x * NEG2_LOG2E; c.Tg = p.y; c.Tcut = cut = p.w; c.inv_ar = p.z;
+    c.kexp = p.x * NEG2_LOG2E; c.Tg = p.y; c.inv_ar = p.z;
+    c.Tcut = cut = reaches_nothing(gm, cp.q.z, P, ox, oy, oz) ? -1.f : p.w;
     c.k4 = 4.f * p.x; c.kE = -gm.E * p.z; c.kD = -gm.D * p.x;
     c.w = weight;
     const float t = G.tg_in[ai * G.T + t0 + lane];

@@ -92,3 +92,32 @@ def test_second_derivatives(port, T, N, points, res, multiple, infinite):
     rows = [a for a in range(N) if not (infinite and a == 5)]
     _close(da.cpu().numpy()[rows], wa[rows])
     assert not dt.any()
+
+
+# Radii so small that an atom's own footprint is empty beside its coordinates, and others that reach one voxel at most, for
+# atoms on grid points and off them.
+@pytest.mark.parametrize("T,N,points,res", [(4, 160, 24, 1.0), (16, 60, 24, 1.0), (33, 60, 24, 1.0), (28, 440, 32, 0.5)])
+@pytest.mark.parametrize("multiple", [1.0, 2.5])
+@pytest.mark.parametrize("on_points", [False, True])
+def test_radii_below_a_voxel(port, T, N, points, res, multiple, on_points):
+    side = (points - 1) * res
+    coords, types, radii = _case(T * points + 1, N, T, side)
+    if on_points:
+        coords = (np.round((coords + side / 2) / res) * res - side / 2).astype(np.float32)
+    rng = np.random.default_rng(T)
+    small = rng.choice([1e-38, 1e-20, 1e-12, 1e-7, 4e-7, 1e-6, 2e-6, 1e-4, 0.03, 0.15], T).astype(np.float32)
+    radii = np.where(np.arange(T) % 3 == 1, radii, small).astype(np.float32)
+    ca, ct = rng.normal(size=(N, 3)).astype(np.float32), rng.normal(size=(N, T)).astype(np.float32)
+    diff = rng.normal(size=(T, points, points, points)).astype(np.float32)
+    g, og = lmg.GridMaker(res, side, False, True, 1.0, multiple), port.gm(res, side, False, True, 1.0, multiple)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii, diff)]
+    ag, tg = torch.full((N, 3), 7.0, device="cuda"), torch.full((N, T), 7.0, device="cuda")
+    g.backward((0, 0, 0), *data, ag, tg)
+    wag, wtg = port.backward_vector(og, (0, 0, 0), coords, types, radii, diff)
+    _close(ag.cpu().numpy(), wag)
+    _close(tg.cpu().numpy(), wtg)
+    dd, da, dt = torch.empty_like(data[3]), torch.empty_like(ag), torch.empty_like(tg)
+    g.backward_gradients((0, 0, 0), *data, torch.from_numpy(ca).cuda(), torch.from_numpy(ct).cuda(), dd, da, dt)
+    wd, wa, _ = port.backward_gradients(og, (0, 0, 0), coords, types, radii, diff, ca, ct)
+    _close(dd.cpu().numpy(), wd)
+    _close(da.cpu().numpy(), wa)
