@@ -2372,6 +2372,12 @@ __device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, Tg
   }
 }
 
+// Whether a sum over voxels of weight * slope * value has to be taken of slope * value alone and weighted afterwards: an
+// infinite weight is no number where slope or value is zero, and a huge one makes the products overflow before the sum does.
+__device__ __forceinline__ bool weigh_afterwards(float w, float inv_ar2) {
+  return w != 0.f && !(fabsf(w) * fmaxf(1.f, 4.f * inv_ar2) < 1e30f);
+}
+
 template <int TO, bool BINARY>
 __global__ void __launch_bounds__(32, TG_MINB) k_type_gradients(TgArgs A) {
   wait_for_stream();
@@ -2393,17 +2399,28 @@ __global__ void __launch_bounds__(32, TG_MINB) k_type_gradients(TgArgs A) {
   const float w = lane < G.T ? G.type_vector[ai * G.T + lane] : 0.f;
   const unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
   Pair tg[4];
-  float ag[3];
-  for (bool dense = __popc(m) > TG_DIRECT;; dense = false) {
+  float ag[3], sum = 0.f;
+  // channel by channel, a lane per axis adding up, or all weighted channels in one sweep
+  const bool apart = __any_sync(0xffffffffu, weigh_afterwards(w, P.inv_ar2));
+  unsigned left = m;
+  for (bool dense = !apart && __popc(m) > TG_DIRECT;; dense = false) {
     tg[0] = tg[1] = tg[2] = tg[3] = pair(0.f);
     ag[0] = ag[1] = ag[2] = 0.f;
     if (!P.valid) break;
     if (dense) tg_atom<TO, BINARY, true>(A, P, sh, diffb, mine, ox, oy, oz, w, m, tg, ag, lane);
-    else tg_atom<TO, BINARY, false>(A, P, sh, diffb, mine, ox, oy, oz, w, m, tg, ag, lane);
+    else tg_atom<TO, BINARY, false>(A, P, sh, diffb, mine, ox, oy, oz, apart ? 1.f : w, apart ? left & (0u - left) : m, tg, ag, lane);
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
 #pragma unroll
       for (int c = 0; c < 3; c++) ag[c] += __shfl_xor_sync(0xffffffffu, ag[c], o);
+    }
+    if (apart) {
+      sum = fmaf(lane == 0 ? ag[0] : lane == 1 ? ag[1] : ag[2], __shfl_sync(0xffffffffu, w, __ffs(left) - 1), sum);
+      left &= left - 1u;
+      if (left != 0u) continue;
+#pragma unroll
+      for (int c = 0; c < 3; c++) ag[c] = __shfl_sync(0xffffffffu, sum, c);
+      break;
     }
     // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either,
     // and the sums are taken again from the others alone.
@@ -2880,14 +2897,33 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
     // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either, and
     // the sums are taken again.  Most without weight: left out at once.  28 channels of 96^3, 4 x 3000 atoms, all / one
     // weighted: a test in any case 2185 / 1904 us, none 2075 / 2063.
-    const int weighted = __popc(__ballot_sync(0xffffffffu, lane < nch && sh.ch[lane & (RT_CH - 1)].w != 0.f));
-    bool again = 2 * weighted < nch;
+    const RtChannel& own = sh.ch[lane & (RT_CH - 1)];
+    const float w = lane < nch ? own.w : 0.f;
+    const unsigned weighted = __ballot_sync(0xffffffffu, w != 0.f);
+    const bool apart = __any_sync(0xffffffffu, weigh_afterwards(w, 0.25f * own.k4));
+    bool again = apart || 2 * __popc(weighted) < nch;
     if (!again) {
       sweep(std::false_type());
       const float whole = (agx + agy) + agz;
-      again = weighted < nch && whole != whole;
+      again = __popc(weighted) < nch && whole != whole;
     }
-    if (again) sweep(std::true_type());
+    if (again) {
+      float sum = 0.f;  // of an axis a lane, channel by channel
+      unsigned left = apart ? weighted : 1u;
+      do {
+        __syncwarp();
+        if (apart && lane < nch) sh.ch[lane].w = lane == __ffs(left) - 1 ? 1.f : 0.f;
+        __syncwarp();
+        sweep(std::true_type());
+        if (apart) sum = fmaf(lane == 0 ? agx : lane == 1 ? agy : agz, __shfl_sync(0xffffffffu, w, __ffs(left) - 1), sum);
+        left &= left - 1u;
+      } while (left != 0u);
+      if (apart) {
+        agx = __shfl_sync(0xffffffffu, sum, 0);
+        agy = __shfl_sync(0xffffffffu, sum, 1);
+        agz = __shfl_sync(0xffffffffu, sum, 2);
+      }
+    }
   }
   // of several warps an atom, k_sum_parts adds up the parts
   float* to = warps == 1 ? G.atom_gradients + ai * 3 : G.partial + (((size_t)bl * G.N + item) * warps + wid) * 3;

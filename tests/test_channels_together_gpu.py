@@ -121,3 +121,29 @@ def test_radii_below_a_voxel(port, T, N, points, res, multiple, on_points):
     wd, wa, _ = port.backward_gradients(og, (0, 0, 0), coords, types, radii, diff, ca, ct)
     _close(dd.cpu().numpy(), wd)
     _close(da.cpu().numpy(), wa)
+
+
+@pytest.mark.parametrize("weight", [float("inf"), -3.4e38, 1e37])
+@pytest.mark.parametrize("by_channel,T,N,points", [(True, 16, 60, 24), (True, 17, 60, 24), (True, 28, 60, 24), (False, 14, 1200, 25)])
+def test_infinite_and_huge_weights(port, weight, by_channel, T, N, points):
+    """An atom's gradient is the weighted sum of its channels' own: infinite, not undefined, where a weight is."""
+    side = points - 1.0
+    coords, types, radii = _case(T + 3 * points, N, T, side)
+    # huge ones in a single channel: sums of several may overflow on the way or not, as they are added up
+    rows = types[::2] if np.isinf(weight) else types[1::4]
+    rows[rows != 0] = weight
+    if not by_channel:
+        radii = np.random.default_rng(1).uniform(0.8, 2.2, N).astype(np.float32)
+    g, og = lmg.GridMaker(1.0, side, False, by_channel), port.gm(1.0, side, False, by_channel)
+    diff = np.random.default_rng(T).normal(size=(T, points, points, points)).astype(np.float32)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii, diff)]
+    ag, tg = torch.full((N, 3), 7.0, device="cuda"), torch.full((N, T), 7.0, device="cuda")
+    g.backward((0, 0, 0), *data, ag, tg)
+    m = min(N, 200)
+    wag, wtg = port.backward_vector(og, (0, 0, 0), coords[:m], types[:m], radii if by_channel else radii[:m], diff)
+    ag, keep = ag[:m].cpu().numpy(), np.isfinite(wag)
+    assert np.array_equal(np.isnan(ag), np.isnan(wag)) and np.array_equal(ag[~keep & ~np.isnan(wag)], wag[~keep & ~np.isnan(wag)])
+    # gradients of weights that differ by up to 1e38: each against its own atom's
+    scale = np.maximum(np.nanmax(np.where(keep, np.abs(wag), 0), axis=1, keepdims=True), 1.0) + np.zeros((1, 3))
+    np.testing.assert_array_less(np.abs(ag[keep] / scale[keep] - wag[keep] / scale[keep]), 2e-4)
+    _close(tg[:m].cpu().numpy(), wtg)
