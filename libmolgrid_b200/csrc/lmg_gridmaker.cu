@@ -3304,7 +3304,7 @@ static cudaError_t backward_quads_atom(const BwdArgs& G, dim3 grid, cudaStream_t
 // and 657 / 743, 32 897 / 1008 and 669 / 753; 8 x 400 atoms (0.03) 28 85 and 91, 32 111 and 92; 28 channels of 24^3 of 1 A,
 // 8 x 2000 / 8 x 400 atoms 56 / 21 and 37 / 23.
 bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned) {
-  if (gm.rti || T > 32 || type_copy_bytes(gm, T) > TYPE_COPY_MOST) return false;
+  if (gm.rti || T > 32 || gm.dim == 0 || type_copy_bytes(gm, T) > TYPE_COPY_MOST) return false;
   const double side = (double)gm.dim * gm.res, dense = N / (side * side * side), pairs = (double)nb * N * T;
   if (!aligned) return T >= 8 && dense >= 0.011 && pairs >= 16000;
   return T > 16 && dense >= (T > 28 ? 0.025 : T > 24 ? 0.12 : 0.2) && pairs >= 300e3 * gm.res * gm.res * gm.res;

@@ -150,3 +150,23 @@ def test_workspace_off_the_boundary_of_the_copies():
         assert rc == 0, lib.lmg_last_error()
         _close(ag.cpu().numpy(), want[0])
         _close(tg.cpu().numpy(), want[1])
+
+
+@pytest.mark.parametrize("T", [17, 32])
+def test_a_grid_without_points(T):
+    """No voxel: every gradient is zero, whatever the number of atoms."""
+    import ctypes
+    from libmolgrid_b200 import _cabi
+    lib, N = _cabi.lib(), 20000
+    g = lmg.GridMaker(1.0, -1.0)
+    assert g.s.dim == 0
+    data = [torch.randn(1, N, 3, device="cuda"), torch.rand(1, N, T, device="cuda"), torch.rand(1, N, device="cuda") + 1]
+    a = _cabi.AtomsStruct()
+    a.batch, a.max_atoms, a.ntypes = 1, N, T
+    a.coords, a.type_vector, a.radii = (t.data_ptr() for t in data)
+    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD, 1, N, T, 1)
+    room, ag, tg = torch.empty(need, dtype=torch.uint8, device="cuda"), torch.full_like(data[0], 7.0), torch.full_like(data[1], 7.0)
+    rc = lib.lmg_backward(ctypes.byref(g.s), ctypes.byref(a), room.data_ptr(), ag.data_ptr(), tg.data_ptr(), room.data_ptr(), need,
+                          torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, lib.lmg_last_error()
+    assert not ag.any() and not tg.any()
