@@ -2372,6 +2372,16 @@ __device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, Tg
   }
 }
 
+// Sum by pairs, then pairs of pairs: as near to 64 bits as lanes that add up by shuffles.
+template <int N>
+__device__ __forceinline__ float tree_sum(float (&v)[N]) {
+#pragma unroll
+  for (int step = 1; step < N; step *= 2)
+#pragma unroll
+    for (int k = 0; k + step < N; k += 2 * step) v[k] += v[k + step];
+  return v[0];
+}
+
 // Whether a sum over voxels of weight * slope * value has to be taken of slope * value alone and weighted afterwards: an
 // infinite weight is no number where slope or value is zero, and a huge one makes the products overflow before the sum does.
 __device__ __forceinline__ bool weigh_afterwards(float w, float inv_ar2) {
@@ -2432,10 +2442,10 @@ __global__ void __launch_bounds__(32, TG_MINB) k_type_gradients(TgArgs A) {
   for (int c = 0; c < 4; c++) split(tg[c], sh.sums[lane][2 * c], sh.sums[lane][2 * c + 1]);
   __syncwarp();
   if (lane < G.T) {
-    float sum = 0.f;
+    float part[TgShared<TO>::VOXELS];
 #pragma unroll
-    for (unsigned g = 0; g < TgShared<TO>::VOXELS; g++) sum += sh.sums[g * TO + (lane >> 3)][lane & 7];
-    G.type_gradients[ai * G.T + lane] = sum;
+    for (unsigned g = 0; g < TgShared<TO>::VOXELS; g++) part[g] = sh.sums[g * TO + (lane >> 3)][lane & 7];
+    G.type_gradients[ai * G.T + lane] = tree_sum(part);
   }
   if (lane < 3) G.atom_gradients[ai * 3 + lane] = lane == 0 ? ag[0] : lane == 1 ? ag[1] : ag[2];
 }
@@ -2932,9 +2942,10 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
   for (int c = 0; c < RT_CH; c++) sh.sums[c][lane] = tg[c];
   __syncwarp();
   static_assert(RT_CH == 16, "two lanes a channel");
-  float sum = 0.f;
+  float part[16];
 #pragma unroll
-  for (int k = 0; k < 16; k++) sum += sh.sums[lane & 15][(lane & 16) + k];
+  for (int k = 0; k < 16; k++) part[k] = sh.sums[lane & 15][(lane & 16) + k];
+  float sum = tree_sum(part);
   sum += __shfl_xor_sync(0xffffffffu, sum, 16);
   if (lane < nch) G.type_gradients[ai * G.T + t0 + lane] = sum;
 }
