@@ -147,3 +147,35 @@ def test_infinite_and_huge_weights(port, weight, by_channel, T, N, points):
     scale = np.maximum(np.nanmax(np.where(keep, np.abs(wag), 0), axis=1, keepdims=True), 1.0) + np.zeros((1, 3))
     np.testing.assert_array_less(np.abs(ag[keep] / scale[keep] - wag[keep] / scale[keep]), 2e-4)
     _close(tg[:m].cpu().numpy(), wtg)
+
+
+@pytest.mark.parametrize("soft", [False, True])
+def test_large_spheres_against_64_bits(soft):
+    """Some thousand voxels an atom and channel, 28 distinct atoms of many: a lane's sums are as near to 64 bits as those of a warp
+    for each channel, whose relative error (2-norm) here is 2.2e-7 with one weighted channel and 2.4e-7 with all."""
+    points, res, T, grm, N, k = 96, 0.25, 14, 2.0, 28, 800
+    torch.manual_seed(1)
+    coords = (torch.rand(N, 3, device="cuda") - 0.5) * 16
+    types = torch.rand(N, T, device="cuda") ** 4 if soft else torch.nn.functional.one_hot(torch.arange(N, device="cuda") % T, T).float()
+    radii = 1.2 + torch.rand(T, device="cuda")
+    g = lmg.GridMaker(res, (points - 1) * res, False, True, 1.0, grm)
+    diff = torch.randn(g.grid_dimensions(T), device="cuda")
+    ag, tg = torch.empty(N * k, 3, device="cuda"), torch.empty(N * k, T, device="cuda")
+    g.backward((0, 0, 0), coords.repeat(k, 1), types.repeat(k, 1), radii, diff, ag, tg)
+    assert torch.equal(ag[:N], ag[-N:]) and torch.equal(tg[:N], tg[-N:])
+    e = np.exp(-2 * grm * grm)
+    A, B, C = 4 * grm ** 2 * e, -e * (4 * grm + 8 * grm ** 3), e * (4 * grm ** 4 + 4 * grm ** 2 + 1)
+    axis = torch.arange(points, device="cuda", dtype=torch.float64) * res - (points - 1) * res / 2
+    wag, wtg = torch.zeros(N, 3, dtype=torch.float64, device="cuda"), torch.zeros(N, T, dtype=torch.float64, device="cuda")
+    for a in range(N):
+        d = [(axis - coords[a, c].double()).reshape([-1 if i == c else 1 for i in range(3)]) for c in range(3)]
+        r = (d[0] ** 2 + d[1] ** 2 + d[2] ** 2).sqrt()
+        for t in range(T):
+            ar = radii[t].double()
+            q = r / ar
+            gauss, inside = torch.exp(-2 * q * q), q <= (1 + 2 * grm * grm) / (2 * grm)
+            wtg[a, t] = (torch.where(q <= grm, gauss, (A * q + B) * q + C) * inside * diff[t].double()).sum()
+            f = torch.where(q <= grm, 4 * gauss / ar ** 2, -(2 * A * q + B) / ar / r) * inside * diff[t].double() * types[a, t].double()
+            wag[a] += torch.stack([(f * x).sum() for x in d])
+    assert ((ag[:N].double() - wag).norm() / wag.norm()).item() < 2.4e-7
+    assert ((tg[:N].double() - wtg).norm() / wtg.norm()).item() < 3.1e-7  # 2.6e-7 measured, 3.0e-7 a warp for each channel
