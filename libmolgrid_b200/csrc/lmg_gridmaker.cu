@@ -2721,7 +2721,7 @@ constexpr int RT_CH = 16, RT_WARPS = 4;  // channels a warp, most warps an atom
 constexpr int RT_MINB = 20;              // blocks of one warp an SM: 96 registers (16 / 24: 2395 / 2313 us instead of 2267)
 constexpr int RT_COLS = 128;
 constexpr int RT_LOADS = 4;              // channels that are requested together
-constexpr int RT_STEPS = 8;              // groups of 32 quads whose atom gradients are summed by themselves
+constexpr unsigned RT_STEPS = 8;         // groups of 32 quads whose atom gradients are summed by themselves
 
 struct __align__(16) RtChannel {
   float kexp, Tg, Tcut, inv_ar;
@@ -2735,7 +2735,7 @@ struct __align__(16) RtShared {
   };
   ZTabs zt;
   float4 ez[RT_CH][QPASS];                // exp(-2 dz2 / ar^2) for each channel
-  float atom[4][32];                      // a lane's sums for the atom gradient: x, y, z of even and odd voxels
+  float atom[5][32];                      // a lane's sums for the atom gradient: x, y, z of even and odd voxels; or as k_second_channels has them
   unsigned short list[RT_COLS * QPASS];   // quads within reach: column | quad << 8
 };
 
@@ -2767,7 +2767,7 @@ __device__ __forceinline__ unsigned list_quads(unsigned short* list, const ColBu
 // own footprint leaves it out: beside a coordinate a radius of 1e-7 times it is nothing, and the footprint is empty.
 // The footprint that it shares with larger channels does not tell.
 __device__ __forceinline__ bool reaches_nothing(const GMParams& gm, float densityrad, const ItemParams& P, float ox, float oy, float oz) {
-  if (!(densityrad < 0.5f * gm.res)) return false;
+  if (!(densityrad < 0.5f * gm.res && densityrad > 0.f)) return false;
   auto along = [&](float origin, float at) {
     unsigned lo, hi;
     bounds_1d(origin, at, densityrad, gm.res, gm.dim, lo, hi);
@@ -2815,6 +2815,18 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
     for (int c = 0; c < RT_CH; c++) tg[c] = 0.f;
 #pragma unroll
     for (int c = 0; c < 4; c++) sh.atom[c][lane] = 0.f;
+    agx = agy = 0.f;
+    Pair az = pair(0.f);
+    auto put_by = [&] {
+      float z0, z1;
+      split(az, z0, z1);
+      sh.atom[0][lane] += agx;
+      sh.atom[1][lane] += agy;
+      sh.atom[2][lane] += z0;
+      sh.atom[3][lane] += z1;
+      agx = agy = 0.f;
+      az = pair(0.f);
+    };
     for (Columns cols(P); cols.more();) {
       const unsigned nkept = cols.compact<true>(sh.cols, P, P.Tcut, ox, oy, gm.res, gm.dim, lane);
       for (unsigned zc = P.loz & ~3u; zc < P.hiz; zc += 4 * QPASS) {
@@ -2825,86 +2837,75 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
         const unsigned n = list_quads(sh.list, sh.cols, sh.zt, nkept, min((unsigned)QPASS, (P.hiz - zc + 3) >> 2), P.Tcut, lane);
         __syncwarp();
 #pragma unroll 1
-        for (unsigned e0 = 0; e0 < n;) {
-          // by RT_STEPS at a time, then for the atom: sums of few terms each
-          const unsigned stop = min(n, e0 + 32 * RT_STEPS);
-          float bx = 0.f, by = 0.f;
-          Pair bz = pair(0.f);
-#pragma unroll 1
-          for (; e0 < stop; e0 += 32) {
-            const unsigned e = sh.list[min(e0 + lane, n - 1u)], i = e & 255u, zq = e >> 8;
-            const float dxy2 = sh.cols.dxy2[i], near = e0 + lane < n ? __fadd_rn(dxy2, sh.zt.lo[zq]) : CUDART_NAN_F;
-            const float4* from = diff + (((size_t)sh.cols.row[i] * dim + zc) / 4 + zq);
-            const float4 d2 = sh.zt.dz2[zq];
-            const float d2v[4] = {d2.x, d2.y, d2.z, d2.w};
-            float r[4], root[4], id[4];
+        for (unsigned e0 = 0; e0 < n; e0 += 32) {
+          const unsigned e = sh.list[min(e0 + lane, n - 1u)], i = e & 255u, zq = e >> 8;
+          const float dxy2 = sh.cols.dxy2[i], near = e0 + lane < n ? __fadd_rn(dxy2, sh.zt.lo[zq]) : CUDART_NAN_F;
+          const float4* from = diff + (((size_t)sh.cols.row[i] * dim + zc) / 4 + zq);
+          const float4 d2 = sh.zt.dz2[zq];
+          const float d2v[4] = {d2.x, d2.y, d2.z, d2.w};
+          float r[4], root[4], id[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              r[j] = __fadd_rn(dxy2, d2v[j]);
-              // the root to the last place (root(), from the reciprocal root at hand): shared by the channels it costs little, and
-              // the type gradients are 3 to 17 % nearer to 64 bits than with the approximate one
-              id[j] = rsqrt_approx(r[j]);
-              const float x = __fmul_rn(r[j], id[j]);
-              root[j] = fmaf(fmaf(-x, x, r[j]), 0.5f * id[j], x);
-            }
-            Pair f[2] = {pair(0.f), pair(0.f)};
-#pragma unroll
-            for (int q = 0; q < RT_CH; q += RT_LOADS) {
-              if (q >= nch) break;
-              float4 dv[RT_LOADS];
-              bool live[RT_LOADS];
-#pragma unroll
-              for (int u = 0; u < RT_LOADS; u++) {
-                live[u] = near <= sh.ch[q + u].Tcut;  // false for a NaN, and for a channel that there is not
-                dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (live[u]) dv[u] = __ldg(from);
-                from += cs4;
-              }
-#pragma unroll
-              for (int u = 0; u < RT_LOADS; u++) {
-                if (!__any_sync(0xffffffffu, live[u])) continue;
-                const RtChannel& C = sh.ch[q + u];
-                const Pair dvp[2] = {pair(dv[u].x, dv[u].y), pair(dv[u].z, dv[u].w)};
-                const float4 e = sh.ez[q + u][zq];
-                const Pair exy = pair(ex2_approx(dxy2 * C.kexp)), ep[2] = {pair(e.x, e.y), pair(e.z, e.w)};
-                Pair sum = pair(0.f);
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                  float e0, e1, x0, x1, a0, a1, b0, b1;
-                  split(mul2(exy, ep[j]), e0, e1);
-                  const bool g0 = r[2 * j] <= C.Tg, g1 = r[2 * j + 1] <= C.Tg;
-                  split(mul2(pair(root[2 * j], root[2 * j + 1]), pair(C.inv_ar)), x0, x1);
-                  x0 = fma_sat(-gm.ta, x0, gm.tb);
-                  x1 = fma_sat(-gm.ta, x1, gm.tb);
-                  const Pair v = pair(g0 ? e0 : x0 * x0, g1 ? e1 : x1 * x1);
-                  sum = j == 0 ? mul2(v, dvp[0]) : fma2(v, dvp[1], sum);
-                  split(fma2(pair(C.kE), pair(id[2 * j], id[2 * j + 1]), pair(C.kD)), a0, a1);  // negative beyond the cut-off
-                  split(mul2(pair(C.k4), pair(e0, e1)), b0, b1);
-                  if (!SKIP || C.w != 0.f)  // the same for every lane
-                    f[j] = fma2(mul2(pair(g0 ? b0 : fmaxf(a0, 0.f), g1 ? b1 : fmaxf(a1, 0.f)), pair(C.w)), dvp[j], f[j]);
-                }
-                float sum0, sum1;
-                split(sum, sum0, sum1);
-                tg[q + u] += sum0 + sum1;
-              }
-            }
-            float f0, f1;
-            split(add2(f[0], f[1]), f0, f1);
-            bx = fmaf(f0 + f1, sh.cols.dx[i], bx);
-            by = fmaf(f0 + f1, sh.cols.dy[i], by);
-            const float4 dz = sh.zt.dz[zq];
-            bz = fma2(f[0], pair(dz.x, dz.y), fma2(f[1], pair(dz.z, dz.w), bz));
+          for (int j = 0; j < 4; j++) {
+            r[j] = __fadd_rn(dxy2, d2v[j]);
+            // the root to the last place (root(), from the reciprocal root at hand): shared by the channels it costs little, and
+            // the type gradients are 3 to 17 % nearer to 64 bits than with the approximate one
+            id[j] = rsqrt_approx(r[j]);
+            const float x = __fmul_rn(r[j], id[j]);
+            root[j] = fmaf(fmaf(-x, x, r[j]), 0.5f * id[j], x);
           }
-          float z0, z1;
-          split(bz, z0, z1);
-          sh.atom[0][lane] += bx;
-          sh.atom[1][lane] += by;
-          sh.atom[2][lane] += z0;
-          sh.atom[3][lane] += z1;
+          Pair f[2] = {pair(0.f), pair(0.f)};
+#pragma unroll
+          for (int q = 0; q < RT_CH; q += RT_LOADS) {
+            if (q >= nch) break;
+            float4 dv[RT_LOADS];
+            bool live[RT_LOADS];
+#pragma unroll
+            for (int u = 0; u < RT_LOADS; u++) {
+              live[u] = near <= sh.ch[q + u].Tcut;  // false for a NaN, and for a channel that there is not
+              dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (live[u]) dv[u] = __ldg(from);
+              from += cs4;
+            }
+#pragma unroll
+            for (int u = 0; u < RT_LOADS; u++) {
+              if (!__any_sync(0xffffffffu, live[u])) continue;
+              const RtChannel& C = sh.ch[q + u];
+              const Pair dvp[2] = {pair(dv[u].x, dv[u].y), pair(dv[u].z, dv[u].w)};
+              const float4 e = sh.ez[q + u][zq];
+              const Pair exy = pair(ex2_approx(dxy2 * C.kexp)), ep[2] = {pair(e.x, e.y), pair(e.z, e.w)};
+              Pair sum = pair(0.f);
+#pragma unroll
+              for (int j = 0; j < 2; j++) {
+                float e0, e1, x0, x1, a0, a1, b0, b1;
+                split(mul2(exy, ep[j]), e0, e1);
+                const bool g0 = r[2 * j] <= C.Tg, g1 = r[2 * j + 1] <= C.Tg;
+                split(mul2(pair(root[2 * j], root[2 * j + 1]), pair(C.inv_ar)), x0, x1);
+                x0 = fma_sat(-gm.ta, x0, gm.tb);
+                x1 = fma_sat(-gm.ta, x1, gm.tb);
+                const Pair v = pair(g0 ? e0 : x0 * x0, g1 ? e1 : x1 * x1);
+                sum = j == 0 ? mul2(v, dvp[0]) : fma2(v, dvp[1], sum);
+                split(fma2(pair(C.kE), pair(id[2 * j], id[2 * j + 1]), pair(C.kD)), a0, a1);  // negative beyond the cut-off
+                split(mul2(pair(C.k4), pair(e0, e1)), b0, b1);
+                if (!SKIP || C.w != 0.f)  // the same for every lane
+                  f[j] = fma2(mul2(pair(g0 ? b0 : fmaxf(a0, 0.f), g1 ? b1 : fmaxf(a1, 0.f)), pair(C.w)), dvp[j], f[j]);
+              }
+              float sum0, sum1;
+              split(sum, sum0, sum1);
+              tg[q + u] += sum0 + sum1;
+            }
+          }
+          float f0, f1;
+          split(add2(f[0], f[1]), f0, f1);
+          agx = fmaf(f0 + f1, sh.cols.dx[i], agx);
+          agy = fmaf(f0 + f1, sh.cols.dy[i], agy);
+          const float4 dz = sh.zt.dz[zq];
+          az = fma2(f[0], pair(dz.x, dz.y), fma2(f[1], pair(dz.z, dz.w), az));
+          if ((e0 & 32 * (RT_STEPS - 1)) == 32 * (RT_STEPS - 1)) put_by();  // sums of few terms each
         }
       }
       __syncwarp();
     }
+    put_by();
     agx = sh.atom[0][lane];
     agy = sh.atom[1][lane];
     agz = sh.atom[2][lane] + sh.atom[3][lane];
@@ -2922,9 +2923,9 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
     // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either, and
     // the sums are taken again.  Most without weight: left out at once.  28 channels of 96^3, 4 x 3000 atoms, all / one
     // weighted: a test in any case 2185 / 1904 us, none 2075 / 2063.
-    auto weight = [&] { return lane < nch ? G.type_vector[ai * G.T + t0 + lane] : 0.f; };
-    const unsigned weighted = __ballot_sync(0xffffffffu, weight() != 0.f);
-    const bool apart = __any_sync(0xffffffffu, weigh_afterwards(weight(), 0.25f * sh.ch[lane & (RT_CH - 1)].k4));
+    const RtChannel& own = sh.ch[lane & (RT_CH - 1)];
+    const unsigned weighted = __ballot_sync(0xffffffffu, lane < nch && own.w != 0.f);
+    const bool apart = __any_sync(0xffffffffu, weigh_afterwards(own.w, 0.25f * own.k4));
     bool again = apart || 2 * __popc(weighted) < nch;
     if (!again) {
       sweep(std::false_type());
@@ -2939,7 +2940,7 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
         if (apart && lane < nch) sh.ch[lane].w = lane == __ffs(left) - 1 ? 1.f : 0.f;
         __syncwarp();
         sweep(std::true_type());
-        if (apart) sum = fmaf(lane == 0 ? agx : lane == 1 ? agy : agz, __shfl_sync(0xffffffffu, weight(), __ffs(left) - 1), sum);
+        if (apart) sum = fmaf(lane == 0 ? agx : lane == 1 ? agy : agz, G.type_vector[ai * G.T + t0 + __ffs(left) - 1], sum);
         left &= left - 1u;
       } while (left != 0u);
       if (apart) {
@@ -3030,7 +3031,22 @@ __global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int 
   }
   __syncwarp();
   float agx = 0.f, agy = 0.f, agz = 0.f;
-  Pair sb1 = pair(0.f), sb2 = pair(0.f);  // sums of w s diff and t s diff
+  // a lane's sums: of the products of distances by axis, of w s diff and t s diff
+  Pair sb1 = pair(0.f), sb2 = pair(0.f);
+#pragma unroll
+  for (int c = 0; c < 5; c++) sh.atom[c][lane] = 0.f;
+  auto put_by = [&] {
+    sh.atom[0][lane] += agx;
+    sh.atom[1][lane] += agy;
+    sh.atom[2][lane] += agz;
+    float x0, x1, y0, y1;
+    split(sb1, x0, x1);
+    split(sb2, y0, y1);
+    sh.atom[3][lane] += x0 + x1;
+    sh.atom[4][lane] += y0 + y1;
+    agx = agy = agz = 0.f;
+    sb1 = sb2 = pair(0.f);
+  };
   const size_t first = ((size_t)b * G.T + t0) * cs;
   auto sweep = [&](auto odd) {
     for (Columns cols(P); cols.more();) {
@@ -3113,9 +3129,9 @@ __global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int 
               if (live[u]) red_add_v4(to + offset[q + u], v[0], v[1], v[2], v[3]);
             }
           }
+          float x0, x1, y0, y1, z0, z1;
           sb1 = add2(sb1, b1);
           sb2 = add2(sb2, b2);
-          float x0, x1, y0, y1, z0, z1;
           const Pair p[2] = {mul2(a1[0], dot[0]), mul2(a1[1], dot[1])};
           split(add2(p[0], p[1]), x0, x1);
           split(add2(a2[0], a2[1]), y0, y1);
@@ -3123,6 +3139,7 @@ __global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int 
           agx = fmaf(dx, fmaf(y0 + y1, dx, x0 + x1), agx);
           agy = fmaf(dy, fmaf(y0 + y1, dy, x0 + x1), agy);
           agz += z0 + z1;
+          if ((e0 & 32 * (RT_STEPS - 1)) == 32 * (RT_STEPS - 1)) put_by();  // sums of few terms each
         }
       }
       __syncwarp();
@@ -3131,14 +3148,11 @@ __global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int 
   if (P.valid) {
     if (odd) sweep(std::true_type());
     else sweep(std::false_type());
-    float x0, x1, y0, y1;
-    split(sb1, x0, x1);
-    split(sb2, y0, y1);
-    x0 += x1;
-    y0 += y1;
-    agx -= fmaf(x0, inx, y0);
-    agy -= fmaf(x0, iny, y0);
-    agz -= fmaf(x0, inz, y0);
+    put_by();
+    const float s1 = sh.atom[3][lane], s2 = sh.atom[4][lane];
+    agx = sh.atom[0][lane] - fmaf(s1, inx, s2);
+    agy = sh.atom[1][lane] - fmaf(s1, iny, s2);
+    agz = sh.atom[2][lane] - fmaf(s1, inz, s2);
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
