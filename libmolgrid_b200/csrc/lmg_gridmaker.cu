@@ -2919,7 +2919,7 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
   agx = agy = agz = 0.f;
 #pragma unroll
   for (int c = 0; c < RT_CH; c++) tg[c] = 0.f;
-  if (P.valid) {
+  if (P.valid && __any_sync(0xffffffffu, sh.ch[lane & (RT_CH - 1)].Tcut >= 0.f)) {
     // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either, and
     // the sums are taken again.  Most without weight: left out at once.  28 channels of 96^3, 4 x 3000 atoms, all / one
     // weighted: a test in any case 2185 / 1904 us, none 2075 / 2063.
