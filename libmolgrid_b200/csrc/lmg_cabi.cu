@@ -613,6 +613,7 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
     lmg::BwdArgs B;
     std::memset(&B, 0, sizeof B);
     B.gm = E.gm; B.b0 = b0; B.nb = nb; B.N = E.N; B.T = E.T;
+    B.first_nb = std::min(per_pass, a->batch);
     B.type_vector = a->type_vector;
     B.centers = a->centers;
     for (int i = 0; i < 3; i++) B.center_host[i] = a->center_host[i];
@@ -736,6 +737,7 @@ int lmg_backward_gradients(const lmg_gridmaker* g, const lmg_atoms* a, const flo
     lmg::BwdArgs B;
     std::memset(&B, 0, sizeof B);
     B.gm = E.gm; B.b0 = b0; B.nb = nb; B.N = E.N; B.T = E.T;
+    B.first_nb = std::min(per_pass, a->batch);
     B.type_vector = a->type_vector;
     B.centers = a->centers;
     for (int i = 0; i < 3; i++) B.center_host[i] = a->center_host[i];

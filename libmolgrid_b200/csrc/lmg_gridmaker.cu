@@ -3381,13 +3381,13 @@ cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, l
 static bool channels_together(const BwdArgs& G) {
   if (G.T < 4 || G.T > RT_CH * RT_WARPS || G.gm.binary) return false;
   if (G.gm.ta == 0.f && G.gm.tb == 0.f) return false;  // a Gaussian without a tail is cut by each channel's own footprint too
-  const double pairs = (double)G.N * G.nb * G.T;
+  const double pairs = (double)G.N * G.first_nb * G.T;
   return G.gm.res >= 0.7f ? pairs >= 600 : G.gm.res >= 0.4f ? pairs >= 12000 : G.gm.res >= 0.2f && G.T > 8 && pairs >= 300e3;
 }
 
 static cudaError_t channels_together_launch(void (*kernel)(BwdArgs, int, int), const BwdArgs& G, long enough, cudaStream_t st) {
   // as few warps an atom as its channels need, more while the atoms alone leave the chip idle
-  const long atoms = (long)G.N * G.nb;
+  const long atoms = (long)G.N * G.first_nb;
   const int most = std::min(RT_WARPS, (G.T + 3) / 4), warps = std::max((G.T + RT_CH - 1) / RT_CH, (int)std::min((long)most, enough / atoms));
   const cudaError_t e = launch_early(kernel, dim3(G.N * warps, G.nb), 32, 0, st, G, (G.T + warps - 1) / warps, warps);
   if (e != cudaSuccess || warps == 1) return e;

@@ -73,6 +73,7 @@ struct EmitArgs {
 struct BwdArgs {
   GMParams gm;
   int b0, nb, N, T;
+  int first_nb;  // examples of the call's first and largest pass, by which the kernels of all its passes are chosen
   const float* type_vector;
   const float* centers;
   float center_host[3];

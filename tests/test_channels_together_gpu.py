@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import libmolgrid_b200 as lmg
+from libmolgrid_b200 import _cabi, api
 
 pytestmark = pytest.mark.gpu
 
@@ -179,3 +180,51 @@ def test_large_spheres_against_64_bits(soft):
             wag[a] += torch.stack([(f * x).sum() for x in d])
     assert ((ag[:N].double() - wag).norm() / wag.norm()).item() < 2.4e-7
     assert ((tg[:N].double() - wtg).norm() / wtg.norm()).item() < 3.1e-7  # 2.6e-7 measured, 3.0e-7 a warp for each channel
+
+
+def _batch(seed, B, N, T, side):
+    """Examples of their own, with a centre, a rotation and a translation each."""
+    from libmolgrid_b200 import synthetic
+    rng = np.random.default_rng(seed)
+    coords, types, radii = (np.stack(x) for x in zip(*(_case(seed + b, N, T, side) for b in range(B))))
+    q = synthetic.random_quaternion(rng, B)
+    rows = np.concatenate([q, rng.uniform(-1, 1, (B, 6)).astype(np.float32)], 1).astype(np.float32)
+    return coords, types, radii, rng.uniform(-1, 1, (B, 3)).astype(np.float32), rows
+
+
+class _Room:
+    """Workspaces of at most this many bytes."""
+    def __init__(self, nbytes):
+        self.nbytes = nbytes
+
+    def __enter__(self):
+        self.old, api.MAX_WORKSPACE_BYTES = api.MAX_WORKSPACE_BYTES, self.nbytes
+        api._workspaces.clear()
+
+    def __exit__(self, *a):
+        api.MAX_WORKSPACE_BYTES = self.old
+        api._workspaces.clear()
+
+
+def _bytes(g, op, B, N, T):
+    import ctypes
+    return _cabi.lib().lmg_workspace_bytes(ctypes.byref(g.s), op, B, N, T, 1)
+
+
+@pytest.mark.parametrize("T,N,points,res", [(8, 50, 24, 1.0), (16, 130, 24, 1.0), (28, 160, 32, 0.5)])
+def test_passes_of_a_call_take_the_same_kernel(T, N, points, res):
+    """Five times the same example, two a pass: the last one alone has the bits of the others."""
+    side = (points - 1) * res
+    coords, types, radii = (torch.from_numpy(x).cuda()[None].repeat(5, *[1] * x.ndim) for x in _case(T, N, T, side))
+    g = lmg.GridMaker(res, side, False, True)
+    diff = torch.randn(g.grid_dimensions(T), device="cuda")[None].repeat(5, 1, 1, 1, 1)
+    ca, ct = torch.randn(N, 3, device="cuda")[None].repeat(5, 1, 1), torch.randn(N, T, device="cuda")[None].repeat(5, 1, 1)
+    centers = torch.zeros(5, 3, device="cuda")
+    ag, tg = torch.empty_like(coords), torch.empty_like(types)
+    with _Room(_bytes(g, _cabi.OP_BACKWARD, 2, N, T)):
+        g.backward(centers, coords, types, radii, diff, ag, tg)
+    dd, da, dt = torch.empty_like(diff), torch.empty_like(coords), torch.empty_like(types)
+    with _Room(_bytes(g, _cabi.OP_BACKWARD_GRADIENTS, 2, N, T)):
+        g.backward_gradients(centers, coords, types, radii, diff, ca, ct, dd, da, dt)
+    for x in (ag, tg, da):
+        assert all(torch.equal(x[0], x[b]) for b in range(1, 5))
