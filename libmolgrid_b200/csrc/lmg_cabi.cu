@@ -647,10 +647,9 @@ static int backward_common(const lmg_gridmaker* g, const lmg_atoms* a, int op, i
       if (copies)
         e = lmg::launch_type_gradients(B, reinterpret_cast<float*>(ws + L.copy), L.copies, &g_launches, st);
       else
-        e = lmg::launch_backward(B, mode, st);
+        e = lmg::launch_backward(B, mode, &g_launches, st);
     }
     prof_end(pr, st);
-    if (!copies) g_launches += mode == 1 ? 2 : 1;
     if (e != cudaSuccess) return cuda_fail(e, "backward");
   }
   return LMG_OK;
@@ -751,9 +750,9 @@ int lmg_backward_gradients(const lmg_gridmaker* g, const lmg_atoms* a, const flo
     B.quads = g_quads;
     e = lmg::launch_emit(E, st);
     if (e != cudaSuccess) return cuda_fail(e, "emit");
-    e = lmg::launch_second_order(B, st);
+    e = lmg::launch_second_order(B, &g_launches, st);
     if (e != cudaSuccess) return cuda_fail(e, "backward_gradients");
-    g_launches += 2 + (g->radii_type_indexed ? 2 : 0);
+    g_launches += 1 + (g->radii_type_indexed ? 1 : 0);
   }
   return LMG_OK;
 }

@@ -3385,24 +3385,29 @@ static bool channels_together(const BwdArgs& G) {
   return G.gm.res >= 0.7f ? pairs >= 600 : G.gm.res >= 0.4f ? pairs >= 12000 : G.gm.res >= 0.2f && G.T > 8 && pairs >= 300e3;
 }
 
-static cudaError_t channels_together_launch(void (*kernel)(BwdArgs, int, int), const BwdArgs& G, long enough, cudaStream_t st) {
+static cudaError_t channels_together_launch(void (*kernel)(BwdArgs, int, int), const BwdArgs& G, long enough, long* launches, cudaStream_t st) {
   // as few warps an atom as its channels need, more while the atoms alone leave the chip idle
   const long atoms = (long)G.N * G.first_nb;
   const int most = std::min(RT_WARPS, (G.T + 3) / 4), warps = std::max((G.T + RT_CH - 1) / RT_CH, (int)std::min((long)most, enough / atoms));
   const cudaError_t e = launch_early(kernel, dim3(G.N * warps, G.nb), 32, 0, st, G, (G.T + warps - 1) / warps, warps);
+  ++*launches;
   if (e != cudaSuccess || warps == 1) return e;
+  ++*launches;
   return launch_early(k_sum_parts, dim3((G.nb * G.N * 3 + 255) / 256), 256, 0, st, G, warps);
 }
 
 // Loose rows: relevance, which reads two tensors and divides, gains at every size (17 x 700 atoms on 22x41^3:
 // 72.5 -> 59.8 us; 50 x 3000 on 28x41^3: 525 -> 501).  Gradients with records do not (22.7 us by single voxels, 28.7
 // by quads), nor do type vectors (4 x 1000 atoms, 28 channels of 41^3: 212 and 251 us).
-cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
+cudaError_t launch_backward(const BwdArgs& G, int mode, long* launches, cudaStream_t st) {
   long items = (long)G.N * (mode == 1 ? G.T : 1);
   if (items == 0 || G.nb == 0) return cudaSuccess;
   dim3 grid((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb);
   const bool bin = G.gm.binary != 0, any = quads_of(G, G.diff, mode == 2 ? G.density : nullptr), loose = any && loose_rows(G);
   const bool quads = any && !loose;
+  if (quads && mode == 1 && G.gm.rti && G.type_gradients != nullptr && channels_together(G))
+    return channels_together_launch(k_backward_channels, G, 8000, launches, st);
+  ++*launches;
   if (mode == 0) return backward_items<0, false>(G, quads, grid, st);
   if (mode == 2) {
     if (loose)
@@ -3417,9 +3422,6 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
     if (G.type_gradients == nullptr) return launch_early(k_backward_quads_atom_ag, ga, BWD2_WARPS * 32, 0, st, G);
     return bin ? backward_quads_atom<true>(G, gv, st) : backward_quads_atom<false>(G, gv, st);
   }
-  if (quads && G.type_gradients != nullptr && channels_together(G)) {
-    return channels_together_launch(k_backward_channels, G, 8000, st);
-  }
   cudaError_t e;
   if (quads && G.type_gradients == nullptr) {
     // radii by channel, no type gradients wanted: only the weighted channels of each atom
@@ -3430,22 +3432,25 @@ cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st) {
     e = bin ? backward_items<1, true>(G, quads, grid, st) : backward_items<1, false>(G, quads, grid, st);
   }
   if (e != cudaSuccess) return e;
+  ++*launches;
   const int n = G.nb * G.N;
   return launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
 }
 
-cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
+cudaError_t launch_second_order(const BwdArgs& G, long* launches, cudaStream_t st) {
   const long items = (long)G.N * G.T;
   if (items == 0 || G.nb == 0) return cudaSuccess;
   const bool quads = G.quads && G.gm.dim % 4 == 0 && (uintptr_t)G.out_grid % 16 == 0 && (uintptr_t)G.diff % 16 == 0;
   if (quads && !G.gm.rti) {
+    ++*launches;
     return launch_early(k_second_quads_atom, dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st, G);
   }
   // Item by item only the weighted channels have warps, so one of many (as one-hot types have) gains less: us item by item /
   // together, 28 channels, soft / one-hot types, 8 x 1500 atoms on 24^3 of 1 A 446 / 62 and 161 / 49, 4 x 1500 on 48^3 of 0.5 A 543 / 74 and
   // 350 / 71, but 8 channels there, 8 x 1500 atoms one-hot 69 and 80, and 28 of 96^3 of 0.25 A, 4 x 3000 atoms 4241 / 356 and 4177 / 456.
   if (quads && (G.gm.res >= 0.7f || (G.gm.res >= 0.4f && G.T >= 24)) && channels_together(G))
-    return channels_together_launch(k_second_channels, G, 3000, st);
+    return channels_together_launch(k_second_channels, G, 3000, launches, st);
+  *launches += quads ? 1 : 2;
   cudaError_t e;
   if (quads) {
     const long units = (long)G.N * nz_groups(G.T);
@@ -3456,6 +3461,7 @@ cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st) {
       e = launch_early(k_backward_warp<3, false>, dim3((unsigned)((items + BWD2_WARPS - 1) / BWD2_WARPS), G.nb), BWD2_WARPS * 32, 0, st, G);
   }
   if (e != cudaSuccess) return e;
+  ++*launches;
   const int n = G.nb * G.N;
   return launch_early(k_reduce_types, dim3((n + 255) / 256), 256, 0, st, G);
 }

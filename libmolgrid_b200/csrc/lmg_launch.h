@@ -98,7 +98,10 @@ struct BwdArgs {
 // kernel before it, whose results the zeros do not touch, is still at work
 cudaError_t launch_zero(float* p, size_t n, bool beside, cudaStream_t st);
 cudaError_t launch_emit(const EmitArgs& A, cudaStream_t st);
-cudaError_t launch_backward(const BwdArgs& G, int mode, cudaStream_t st);
+// counts its launches, as does the next
+cudaError_t launch_backward(const BwdArgs& G, int mode, long* launches, cudaStream_t st);
+// both terms of backward_gradients: out_grid (zero-filled before) and atom_gradients
+cudaError_t launch_second_order(const BwdArgs& G, long* launches, cudaStream_t st);
 // occupancy of index types that writes every voxel once, but for channels that hold many atoms (lmg_occupancy.cu);
 // counts its launches
 bool occupancy_serves(const EmitArgs& A);
@@ -127,8 +130,6 @@ inline size_t type_copy_bytes(const GMParams& gm, int T) { return ((size_t)gm.di
 bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned);
 cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, long* launches, cudaStream_t st);
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st);
-// both terms of backward_gradients: out_grid (zero-filled before) and atom_gradients
-cudaError_t launch_second_order(const BwdArgs& G, cudaStream_t st);
 
 }  // namespace lmg
 

@@ -126,7 +126,8 @@ int lmg_backward_static(const lmg_gridmaker* g, const lmg_atoms* a, const float*
   } else {
     e = lmg::launch_emit(E, st);
     if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: emit: ") + cudaGetErrorString(e));
-    e = lmg::launch_backward(B, 0, st);
+    long launches = 0;
+    e = lmg::launch_backward(B, 0, &launches, st);
   }
   if (e != cudaSuccess) return fail(LMG_ERR_CUDA, std::string("CUDA Error: backward: ") + cudaGetErrorString(e));
   return LMG_OK;

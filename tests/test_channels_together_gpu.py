@@ -228,3 +228,27 @@ def test_passes_of_a_call_take_the_same_kernel(T, N, points, res):
         g.backward_gradients(centers, coords, types, radii, diff, ca, ct, dd, da, dt)
     for x in (ag, tg, da):
         assert all(torch.equal(x[0], x[b]) for b in range(1, 5))
+
+
+# by (atom, channel) or by atom: records (and the channels' constants), sums, their reduction if there is one
+@pytest.mark.parametrize("by_channel,quads,T,N,first,second", [(True, 1, 16, 9000, 3, 3), (True, 1, 17, 100, 4, 4), (True, 0, 17, 100, 4, 5),
+                                                               (True, 1, 3, 100, 4, 4), (False, 1, 5, 100, 2, 2), (False, 0, 5, 100, 3, 4)])
+def test_launches_are_counted(by_channel, quads, T, N, first, second):
+    lib, side = _cabi.lib(), 23.0
+    coords, types, radii = _case(3, N, T, side)
+    if not by_channel:
+        radii = np.ones(N, np.float32)
+    g = lmg.GridMaker(1.0, side, False, by_channel)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff, ag, tg = torch.randn(g.grid_dimensions(T), device="cuda"), torch.empty_like(data[0]), torch.empty_like(data[1])
+    outs = torch.empty_like(diff), torch.empty_like(ag), torch.empty_like(tg)
+    lib.lmg_set_quads(quads)
+    try:
+        n = [lib.lmg_launch_count()]
+        g.backward((0, 0, 0), *data, diff, ag, tg)
+        n.append(lib.lmg_launch_count())
+        g.backward_gradients((0, 0, 0), *data, diff, ag, tg, *outs)
+        n.append(lib.lmg_launch_count())
+    finally:
+        lib.lmg_set_quads(1)
+    assert (n[1] - n[0], n[2] - n[1]) == (first, second)
