@@ -486,7 +486,7 @@ class GridMaker(object):
 
     def _ws(self, dev, op, B, N, T, vec):
         # the size depends on the shapes and the settings: asked once per combination
-        key = (op, B, N, T, vec, self.s.radii_type_indexed, self.s.binary, self.s.dim)
+        key = (op, B, N, T, vec, self.s.radii_type_indexed, self.s.binary, self.s.dim, self.s.resolution)
         sizes = self.__dict__.setdefault("_ws_sizes", {})
         need = sizes.get(key)
         if need is None:

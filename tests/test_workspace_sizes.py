@@ -1,0 +1,20 @@
+"""Scratch sizes that the Python layer asks for: those of the settings at the time of the call."""
+import ctypes
+
+import libmolgrid_b200 as lmg
+from libmolgrid_b200 import _cabi, api
+
+
+def test_sizes_follow_the_resolution(monkeypatch):
+    """Type gradients by copies go by the resolution too: two resolutions of the same points do not share a size."""
+    monkeypatch.setattr(api, "_workspace", lambda device, nbytes, *more: nbytes)
+    g, B, N, T = lmg.GridMaker(1.0, 23.0), 8, 2000, 28
+    ops = range(4)
+    sizes = []
+    for res in (1.0, 2.0, 1.0):
+        g.set_resolution(res)
+        g.set_dimension(23.0 * res)
+        assert g.s.dim == 24
+        sizes.append([g._ws("cuda:0", op, B, N, T, True) for op in ops])
+        assert sizes[-1] == [_cabi.lib().lmg_workspace_bytes(ctypes.byref(g.s), op, B, N, T, 1) for op in ops]
+    assert sizes[0] == sizes[2] != sizes[1]
