@@ -100,12 +100,22 @@ enum {
   LMG_OP_FORWARD = 0,
   LMG_OP_BACKWARD = 1,
   LMG_OP_BACKWARD_GRADIENTS = 2,
-  LMG_OP_BACKWARD_RELEVANCE = 3
+  LMG_OP_BACKWARD_RELEVANCE = 3,
+  LMG_OP_BACKWARD_TYPES = 4 /* lmg_backward with type gradients, at its fastest: see below */
 };
 
 /* Scratch bytes that let the given op process the whole batch in one pass.  A smaller
  * workspace makes the op run the batch in several passes; it fails with LMG_ERR_WORKSPACE
- * only if not even one example fits.  `vector_types` != 0 for type_vector input. */
+ * only if not even one example fits.  `vector_types` != 0 for type_vector input.
+ *
+ * LMG_OP_BACKWARD is enough for any lmg_backward.  Type gradients of many atoms with radii by atom are
+ * faster from a copy of the grid gradient, up to 256 MB of it: LMG_OP_BACKWARD_TYPES has room for it.  Where
+ * the workspace does not, or does not start on a 32-byte boundary, lmg_backward takes the kernels that
+ * need no copy, whose sums have other last bits.
+ *
+ * Which kernels a call takes, and with them the last bits of its floating-point sums, goes by its settings,
+ * its sizes (the batch among them), the alignment of its grids and its workspace.  The same call has the same bits
+ * again, and all passes of a call take the same kernels. */
 size_t lmg_workspace_bytes(const lmg_gridmaker* g, int op, int batch, int max_atoms, int ntypes,
                            int vector_types);
 

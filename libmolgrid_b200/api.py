@@ -216,18 +216,26 @@ _workspaces = _Workspaces()
 _transform_ring = {}   # (device, batch) -> pinned staging buffers of GridMaker.batch_transforms
 
 
-def _workspace(device, nbytes):
+def _workspace(device, nbytes, least=None):
     """Scratch buffer of the current stream, reused across calls (grown on demand).  Given up, it goes back to
     torch's allocator for that stream, whose order keeps it from calls still under way.  A call that is being captured has
-    one of its own, in the memory of its graph."""
+    one of its own, in the memory of its graph.  Where there is no room for ``nbytes``, one of ``least``."""
+    def room():
+        try:
+            return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            if least is None or least >= nbytes:
+                raise
+        return torch.empty(int(least), dtype=torch.uint8, device=device)
+
     if torch.cuda.is_current_stream_capturing():
-        return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        return room()
     by, key = _workspaces.by, torch._C._cuda_getCurrentRawStream(device.index) << 6 | device.index
     ws = by.pop(key, None)
     if ws is None or ws.numel() < nbytes:
         if len(by) >= _Workspaces.KEPT:
             del by[next(iter(by))]
-        ws = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        ws = room()
     by[key] = ws
     return ws
 
@@ -484,14 +492,18 @@ class GridMaker(object):
         self._last_ws = ws
         return True
 
-    def _ws(self, dev, op, B, N, T, vec):
+    def _bytes(self, op, B, N, T, vec):
         # the size depends on the shapes and the settings: asked once per combination
         key = (op, B, N, T, vec, self.s.radii_type_indexed, self.s.binary, self.s.dim, self.s.resolution)
         sizes = self.__dict__.setdefault("_ws_sizes", {})
         need = sizes.get(key)
         if need is None:
             need = sizes[key] = _cabi.lib().lmg_workspace_bytes(ctypes.byref(self.s), op, B, N, T, int(vec))
-        return _workspace(dev, min(need, MAX_WORKSPACE_BYTES))
+        return min(need, MAX_WORKSPACE_BYTES)
+
+    def _ws(self, dev, op, B, N, T, vec):
+        least = self._bytes(_cabi.OP_BACKWARD, B, N, T, vec) if op == _cabi.OP_BACKWARD_TYPES else None
+        return _workspace(dev, self._bytes(op, B, N, T, vec), least)
 
     # --- forward -----------------------------------------------------------------------------
     def forward(self, *args, **kw):
@@ -731,7 +743,7 @@ class GridMaker(object):
             raise TypeError("type_gradients given with index types")
         A.ntypes = T
         self._check_radii(vec, N, T, nr, ValueError)
-        ws = self._ws(dev, _cabi.OP_BACKWARD, B, N, T, vec)
+        ws = self._ws(dev, _cabi.OP_BACKWARD if tg is None else _cabi.OP_BACKWARD_TYPES, B, N, T, vec)
         check(_cabi.lib().lmg_backward(ctypes.byref(self.s), ctypes.byref(A), df.ptr, ag.ptr,
                                        tg.ptr if tg is not None else None,
                                        ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(dev)))

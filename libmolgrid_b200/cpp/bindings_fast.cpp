@@ -169,11 +169,11 @@ bool per_atom(const Call& c, PyObject* o, const lmg_atoms& A, bool batched, size
 }
 
 // where the call runs, `ret` a new reference; false leaves it to the general route (no workspace of that size yet, or
-// a call that is being captured)
-bool place(const Call& c, size_t bytes, void** ws, size_t* ws_bytes, cudaStream_t* st, PyObject** ret) {
+// a call that is being captured).  The compiled module's own buffers may hold no more than `least`.
+bool place(const Call& c, size_t bytes, size_t least, void** ws, size_t* ws_bytes, cudaStream_t* st, PyObject** ret) {
   if (c.workspaces == Py_None) {
     try {
-      *ws = libmolgrid::detail::workspace(bytes);
+      *ws = libmolgrid::detail::workspace_or_less(bytes, least);
     } catch (std::exception&) {
       return false;
     }
@@ -225,7 +225,8 @@ PyObject* fast_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!grid(c, c.item[4], A, batched, out, T) || (vec && (size_t)A.ntypes != T)) Py_RETURN_NONE;
   A.ntypes = (int)T;
   if (!radii_fit(c, vec, nr, A.max_atoms, T)) Py_RETURN_NONE;
-  if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_FORWARD, A.batch, A.max_atoms, A.ntypes, vec), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
+  const size_t bytes = lmg_workspace_bytes(c.g, LMG_OP_FORWARD, A.batch, A.max_atoms, A.ntypes, vec);
+  if (!place(c, bytes, bytes, &ws, &wb, &st, &ret)) Py_RETURN_NONE;
   return finish([&] {
     Released r;
     return lmg_forward(c.g, &A, out.f(), ws, wb, st);
@@ -253,7 +254,9 @@ PyObject* fast_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   } else if (!vec && (tgo != nullptr || c.g->radii_type_indexed)) {
     Py_RETURN_NONE;
   }
-  if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_BACKWARD, A.batch, A.max_atoms, A.ntypes, vec), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
+  const size_t least = lmg_workspace_bytes(c.g, LMG_OP_BACKWARD, A.batch, A.max_atoms, A.ntypes, vec);
+  const size_t bytes = tg.ptr != nullptr ? lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_TYPES, A.batch, A.max_atoms, A.ntypes, vec) : least;
+  if (!place(c, bytes, least, &ws, &wb, &st, &ret)) Py_RETURN_NONE;
   return finish([&] {
     Released r;
     return lmg_backward(c.g, &A, diff.f(), ag.f(), tg.f(), ws, wb, st);
@@ -274,7 +277,8 @@ PyObject* fast_relevance(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!grid(c, c.item[4], A, batched, de, T) || !grid(c, c.item[5], A, batched, diff, T2) || T != T2) Py_RETURN_NONE;
   A.ntypes = (int)T;
   if (!per_atom(c, c.item[6], A, batched, 0, rel) || nr != (size_t)A.max_atoms) Py_RETURN_NONE;
-  if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_RELEVANCE, A.batch, A.max_atoms, A.ntypes, 0), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
+  const size_t bytes = lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_RELEVANCE, A.batch, A.max_atoms, A.ntypes, 0);
+  if (!place(c, bytes, bytes, &ws, &wb, &st, &ret)) Py_RETURN_NONE;
   return finish([&] {
     Released r;
     return lmg_backward_relevance(c.g, &A, de.f(), diff.f(), rel.f(), ws, wb, st);
@@ -299,7 +303,8 @@ PyObject* fast_gradients(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       !per_atom(c, c.item[8], A, batched, 3, add) || !per_atom(c, c.item[9], A, batched, T, tdd) ||
       !radii_fit(c, vec, nr, A.max_atoms, T))
     Py_RETURN_NONE;
-  if (!place(c, lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_GRADIENTS, A.batch, A.max_atoms, A.ntypes, 1), &ws, &wb, &st, &ret)) Py_RETURN_NONE;
+  const size_t bytes = lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_GRADIENTS, A.batch, A.max_atoms, A.ntypes, 1);
+  if (!place(c, bytes, bytes, &ws, &wb, &st, &ret)) Py_RETURN_NONE;
   return finish([&] {
     Released r;
     return lmg_backward_gradients(c.g, &A, diff.f(), ag.f(), tg.f(), dd.f(), add.f(), tdd.f(), ws, wb, st);

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <condition_variable>
 #include <cstddef>
 #include <mutex>
@@ -71,7 +72,8 @@ inline std::vector<WorkspaceSlot>& workspaces() {
 }
 inline const WorkspaceSlot* last_workspace() { return workspaces().empty() ? nullptr : &workspaces().front(); }
 
-inline void* workspace(size_t bytes, cudaStream_t stream = nullptr) {
+// The buffer of the calling thread, its device and the stream, as large as it is.
+inline WorkspaceSlot& workspace_slot(cudaStream_t stream) {
   std::vector<WorkspaceSlot>& w = workspaces();
   int dev = 0;
   LMG_CUDA_CHECK(cudaGetDevice(&dev));
@@ -89,7 +91,11 @@ inline void* workspace(size_t bytes, cudaStream_t stream = nullptr) {
     w.push_back(n);
   }
   if (i != 0) std::swap(w[0], w[i]);
-  WorkspaceSlot& s = w[0];
+  return w[0];
+}
+
+inline void* workspace(size_t bytes, cudaStream_t stream = nullptr) {
+  WorkspaceSlot& s = workspace_slot(stream);
   if (bytes > s.cap) {
     if (s.p) cudaFree(s.p);
     s.p = nullptr;
@@ -98,6 +104,22 @@ inline void* workspace(size_t bytes, cudaStream_t stream = nullptr) {
     s.cap = bytes;
   }
   return s.p;
+}
+
+// The same with `least` bytes at least where there is no room for `bytes`, which is then set to what there is.
+inline void* workspace_or_less(size_t& bytes, size_t least, cudaStream_t stream = nullptr) {
+  WorkspaceSlot& s = workspace_slot(stream);
+  if (bytes <= s.cap || least >= bytes) return workspace(bytes, stream);
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) {
+    if (s.p) cudaFree(s.p);  // waits for the work that uses it
+    s.p = p;
+    s.cap = bytes;
+  } else {
+    cudaGetLastError();  // not to be found by a later check
+    bytes = std::max(least, s.cap);
+  }
+  return workspace(bytes, stream);
 }
 
 // Device copy of a host array for the duration of one call (host-grid overloads compute on the

@@ -146,8 +146,7 @@ class GridMaker {
     a.coords = coords.data(); a.radii = radii.data(); a.centers = centers.data();
     a.transforms = transforms; a.n_atoms = n_atoms;
     if (N == 2) a.type_index = types.data(); else a.type_vector = types.data();
-    size_t bytes = lmg_workspace_bytes(&s_, LMG_OP_BACKWARD, (int)B, (int)n, (int)T, N == 3);
-    detail::check(lmg_backward(&s_, &a, diff.data(), atom_gradients.data(), type_gradients, detail::workspace(bytes), bytes, nullptr));
+    backward_call(a, diff.data(), atom_gradients.data(), type_gradients);
   }
 
   void forward(float3 grid_center, const CoordinateSet& in, Grid<float, 4, true>& out, const Transform* transform = nullptr) const {
@@ -284,8 +283,7 @@ class GridMaker {
     check_diff(diff);
     lmg_atoms a = single(grid_center, n, diff.dimension(0), coords.data(), radii.data(), transform);
     a.type_index = type_index.data();
-    size_t bytes = lmg_workspace_bytes(&s_, LMG_OP_BACKWARD, 1, (int)n, a.ntypes, 0);
-    detail::check(lmg_backward(&s_, &a, diff.data(), atom_gradients.data(), nullptr, detail::workspace(bytes), bytes, nullptr));
+    backward_call(a, diff.data(), atom_gradients.data(), nullptr);
   }
 
   void backward(float3 grid_center, const Grid<float, 2, true>& coords, const Grid<float, 2, true>& type_vector,
@@ -302,8 +300,7 @@ class GridMaker {
     check_diff(diff);
     lmg_atoms a = single(grid_center, n, T, coords.data(), radii.data(), transform);
     a.type_vector = type_vector.data();
-    size_t bytes = lmg_workspace_bytes(&s_, LMG_OP_BACKWARD, 1, (int)n, (int)T, 1);
-    detail::check(lmg_backward(&s_, &a, diff.data(), atom_gradients.data(), type_gradients.data(), detail::workspace(bytes), bytes, nullptr));
+    backward_call(a, diff.data(), atom_gradients.data(), type_gradients.data());
   }
 
   void backward(float3 grid_center, const CoordinateSet& in, const Grid<float, 4, true>& diff, Grid<float, 2, true>& atomic_gradients) const {
@@ -500,6 +497,13 @@ class GridMaker {
     a.center_host[0] = center.x; a.center_host[1] = center.y; a.center_host[2] = center.z;
     if (tr) { tr_ = tr->c_struct(); a.transform_host = &tr_; }
     return a;
+  }
+  void backward_call(const lmg_atoms& a, const float* diff, float* atom_gradients, float* type_gradients) const {
+    const int vec = a.type_vector != nullptr;
+    const size_t least = lmg_workspace_bytes(&s_, LMG_OP_BACKWARD, a.batch, a.max_atoms, a.ntypes, vec);
+    size_t bytes = type_gradients == nullptr ? least : lmg_workspace_bytes(&s_, LMG_OP_BACKWARD_TYPES, a.batch, a.max_atoms, a.ntypes, vec);
+    void* w = detail::workspace_or_less(bytes, least);
+    detail::check(lmg_backward(&s_, &a, diff, atom_gradients, type_gradients, w, bytes, nullptr));
   }
   void run_forward(const lmg_atoms& a, float* out, int vec, cudaStream_t stream = nullptr) const {
     size_t bytes = lmg_workspace_bytes(&s_, LMG_OP_FORWARD, a.batch, a.max_atoms, a.ntypes, vec);

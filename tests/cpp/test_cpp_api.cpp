@@ -417,6 +417,17 @@ int main(int argc, char** argv) {
     EXPECT_THROW(mixed.merge_coordinates(), std::invalid_argument);
   }
 
+  // scratch that cannot be had: the least that will do, and no error left behind for a later check
+  {
+    const size_t none = (size_t)1 << 50;
+    size_t bytes = none;
+    EXPECT(detail::workspace_or_less(bytes, 4096) != nullptr && bytes >= 4096 && bytes < none);
+    EXPECT(cudaGetLastError() == cudaSuccess);
+    const size_t more = 2 * detail::last_workspace()->cap;
+    bytes = more;
+    EXPECT(detail::workspace_or_less(bytes, 4096) != nullptr && bytes == more && detail::last_workspace()->cap == more);
+  }
+
   std::fclose(out);
   std::fclose(in);
   std::printf(failures ? "%d checks FAILED\n" : "all checks passed\n", failures);

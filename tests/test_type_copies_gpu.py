@@ -141,7 +141,7 @@ def test_workspace_off_the_boundary_of_the_copies():
     a = _cabi.AtomsStruct()
     a.batch, a.max_atoms, a.ntypes = B, N, T
     a.coords, a.type_vector, a.radii = (t.data_ptr() for t in data)
-    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD, B, N, T, 1)
+    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD_TYPES, B, N, T, 1)
     room = torch.empty(need + 64, dtype=torch.uint8, device="cuda")
     for off in (0, 16):
         ag, tg = torch.full((B, N, 3), 7.0, device="cuda"), torch.full((B, N, T), 7.0, device="cuda")
@@ -164,9 +164,64 @@ def test_a_grid_without_points(T):
     a = _cabi.AtomsStruct()
     a.batch, a.max_atoms, a.ntypes = 1, N, T
     a.coords, a.type_vector, a.radii = (t.data_ptr() for t in data)
-    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD, 1, N, T, 1)
+    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD_TYPES, 1, N, T, 1)
     room, ag, tg = torch.empty(need, dtype=torch.uint8, device="cuda"), torch.full_like(data[0], 7.0), torch.full_like(data[1], 7.0)
     rc = lib.lmg_backward(ctypes.byref(g.s), ctypes.byref(a), room.data_ptr(), ag.data_ptr(), tg.data_ptr(), room.data_ptr(), need,
                           torch.cuda.current_stream().cuda_stream)
     assert rc == 0, lib.lmg_last_error()
     assert not ag.any() and not tg.any()
+
+
+def test_room_for_copies_short_by_a_byte():
+    """Copies are made where they fit and nowhere else: nothing is written behind the workspace, and one byte less takes the
+    kernels that need none (records and two launches more by copies, records, sums and their reduction without)."""
+    import ctypes
+    from libmolgrid_b200 import _cabi
+    lib, points, T, B, N = _cabi.lib(), 25, 16, 7, 200
+    coords, types, radii = _batch(12, B, N, T, points - 1.0)
+    g = lmg.GridMaker(1.0, points - 1.0)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
+    a = _cabi.AtomsStruct()
+    a.batch, a.max_atoms, a.ntypes = B, N, T
+    a.coords, a.type_vector, a.radii = (t.data_ptr() for t in data)
+    need = lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD_TYPES, B, N, T, 1)
+    assert need > lib.lmg_workspace_bytes(ctypes.byref(g.s), _cabi.OP_BACKWARD, B, N, T, 1)
+    out = []
+    for size in (need, need - 1):
+        room = torch.full((need + 4096,), 0xAB, dtype=torch.uint8, device="cuda")
+        ag, tg = torch.full((B, N, 3), 7.0, device="cuda"), torch.full((B, N, T), 7.0, device="cuda")
+        rc = lib.lmg_backward(ctypes.byref(g.s), ctypes.byref(a), diff.data_ptr(), ag.data_ptr(), tg.data_ptr(), room.data_ptr(), size,
+                              torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, lib.lmg_last_error()
+        assert bool((room[size:] == 0xAB).all())
+        out.append((ag.cpu().numpy(), tg.cpu().numpy()))
+    _close(out[0][0], out[1][0])
+    _close(out[0][1], out[1][1])
+    assert not np.array_equal(out[0][1], out[1][1])  # other kernels, other last bits
+
+
+def test_no_memory_for_copies(monkeypatch):
+    """Where the scratch of the copies cannot be had, that of the kernels that need none is enough."""
+    points, T, B, N = 25, 16, 7, 200
+    coords, types, radii = _batch(13, B, N, T, points - 1.0)
+    g = lmg.GridMaker(1.0, points - 1.0)
+    data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
+    diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
+    want = _gradients(g, data, diff)
+    from libmolgrid_b200 import _cabi
+    least, real = g._bytes(_cabi.OP_BACKWARD, B, N, T, True), torch.empty
+
+    def empty(*a, **k):
+        if k.get("dtype") is torch.uint8 and a[0] > least:
+            raise torch.OutOfMemoryError("no room")
+        return real(*a, **k)
+    api._workspaces.clear()
+    monkeypatch.setattr(torch, "empty", empty)
+    try:
+        for _ in range(2):
+            got = _gradients(g, data, diff)
+            _close(got[0], want[0])
+            _close(got[1], want[1])
+    finally:
+        api._workspaces.clear()
