@@ -2109,7 +2109,6 @@ constexpr int TG_MINB = 20;       // blocks of one warp an SM
 constexpr int TG_COLS = 128;
 constexpr int TG_Q = 4;           // quads of a column that are requested together
 constexpr int TG_U = 4;           // voxels of a lane that are requested together
-constexpr int TG_DIRECT = 4;      // most weighted channels that the atom gradient reads where they lie
 
 // Eight channels of a voxel in one load.
 struct __align__(32) Eight {
@@ -2204,12 +2203,12 @@ __device__ __forceinline__ void tg_add(TgShared<TO>& sh, unsigned n, const Eight
   __syncwarp();
 }
 
-// One atom.  Its weights `w` are those of a lane's channel, `m` tells which there are.  A lane owns a column, as in
-// backward_quads_core(), and lists the voxels of its quads that lie within reach.  The atom gradient takes the weighted
-// channels' values where they lie; of many (DENSE) from the copy, by the gradients of the density that are listed too.
+// One atom, whose weights `w` are those of a lane's channel.  A lane owns a column, as in backward_quads_core(), and lists the
+// voxels of its quads that lie within reach.  The atom gradient takes the values of channel `one`, not weighted, where they lie, or
+// of all channels (DENSE) from the copy, by the gradients of the density that are listed too.
 template <int TO, bool BINARY, bool DENSE>
 __device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, TgShared<TO>& sh, const float* diffb, const Eight* mine,
-                                        float ox, float oy, float oz, float w, unsigned m, Pair (&tg)[4], float (&ag)[3], int lane) {
+                                        float ox, float oy, float oz, float w, int channel, Pair (&tg)[4], float (&ag)[3], int lane) {
   const GMParams& gm = A.G.gm;
   const unsigned dim = gm.dim, voxels = dim * dim * dim;
   const bool aligned = dim % 4 == 0 && (uintptr_t)A.G.diff % 16 == 0;
@@ -2218,10 +2217,7 @@ __device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, Tg
   const bool tail = gm.ta != 0.f || gm.tb != 0.f;
   const float k4 = 4.f * P.inv_ar2, kD = tail ? -gm.D * P.inv_ar2 : 0.f, kE = tail ? -gm.E * P.inv_ar : 0.f;
   const float inv_dim = 1.f / small_float(dim);
-  // the first weighted channel
-  const int t1 = m != 0u ? __ffs(m) - 1 : 0;
-  const float w1 = __shfl_sync(0xffffffffu, w, t1);
-  const float* one = diffb + (size_t)t1 * voxels;
+  const float* one = diffb + (size_t)channel * voxels;
   Pair w8[4];
 #pragma unroll
   for (int c = 0; c < 4; c++) {
@@ -2308,16 +2304,7 @@ __device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, Tg
               }
               if (!DENSE) {
                 float x0, x1;
-                split(mul2(pair(w1), j == 0 ? pair(dv[u].x, dv[u].y) : pair(dv[u].z, dv[u].w)), x0, x1);
-                // the other weighted channels, one after the other
-                for (unsigned left = m & (m - 1u); left != 0u; left &= left - 1u) {
-                  const int t = __ffs(left) - 1;
-                  const float wt = __shfl_sync(0xffffffffu, w, t);
-                  const float* p = diffb + (size_t)t * voxels + voxel + 4 * (q0 + u) + j;
-                  if (in0) x0 = fmaf(wt, __ldg(p), x0);
-                  if (in1) x1 = fmaf(wt, __ldg(p + 1), x1);
-                }
-                split(mul2(pair(s[j], s[j + 1]), pair(x0, x1)), x0, x1);
+                split(mul2(pair(s[j], s[j + 1]), j == 0 ? pair(dv[u].x, dv[u].y) : pair(dv[u].z, dv[u].w)), x0, x1);
                 const Pair f = pair(in0 ? x0 : 0.f, in1 ? x1 : 0.f);  // a neighbour's value may be anything
                 fs = add2(fs, f);
                 az = fma2(f, dzp[j / 2], az);
@@ -2409,35 +2396,35 @@ __global__ void __launch_bounds__(32, TG_MINB) k_type_gradients(TgArgs A) {
   const float w = lane < G.T ? G.type_vector[ai * G.T + lane] : 0.f;
   const unsigned m = __ballot_sync(0xffffffffu, w != 0.f);
   Pair tg[4];
-  float ag[3], sum = 0.f;
-  // channel by channel, a lane per axis adding up, or all weighted channels in one sweep
-  const bool apart = __any_sync(0xffffffffu, weigh_afterwards(w, P.inv_ar2));
+  float ag[3] = {0.f, 0.f, 0.f}, sum = 0.f;
   unsigned left = m;
-  for (bool dense = !apart && __popc(m) > TG_DIRECT;; dense = false) {
+  tg[0] = tg[1] = tg[2] = tg[3] = pair(0.f);
+  for (bool dense = (m & (m - 1u)) != 0u; P.valid; dense = false) {
     tg[0] = tg[1] = tg[2] = tg[3] = pair(0.f);
     ag[0] = ag[1] = ag[2] = 0.f;
-    if (!P.valid) break;
-    if (dense) tg_atom<TO, BINARY, true>(A, P, sh, diffb, mine, ox, oy, oz, w, m, tg, ag, lane);
-    else tg_atom<TO, BINARY, false>(A, P, sh, diffb, mine, ox, oy, oz, apart ? 1.f : w, apart ? left & (0u - left) : m, tg, ag, lane);
+    if (dense) tg_atom<TO, BINARY, true>(A, P, sh, diffb, mine, ox, oy, oz, w, 0, tg, ag, lane);
+    else tg_atom<TO, BINARY, false>(A, P, sh, diffb, mine, ox, oy, oz, 0.f, left != 0u ? __ffs(left) - 1 : 0, tg, ag, lane);
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
 #pragma unroll
       for (int c = 0; c < 3; c++) ag[c] += __shfl_xor_sync(0xffffffffu, ag[c], o);
     }
-    if (apart) {
+    if (dense) {
+      // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either.  An
+      // infinite weight is none where slope or value is zero, and a huge one overflows before the sum does.  Then the weighted
+      // channels are summed one by one and weighted afterwards, as a single one is.
+      if (fabsf((ag[0] + ag[1]) + ag[2]) < CUDART_INF_F && !__any_sync(0xffffffffu, fabsf(w) == CUDART_INF_F)) break;
+      continue;
+    }
+    if (left != 0u) {
       sum = fmaf(lane == 0 ? ag[0] : lane == 1 ? ag[1] : ag[2], __shfl_sync(0xffffffffu, w, __ffs(left) - 1), sum);
       left &= left - 1u;
       if (left != 0u) continue;
-#pragma unroll
-      for (int c = 0; c < 3; c++) ag[c] = __shfl_sync(0xffffffffu, sum, c);
-      break;
     }
-    // What stands in a channel without weight is not the atom's: where it was no number, zero times it is none either,
-    // and the sums are taken again from the others alone.
-    const float whole = (ag[0] + ag[1]) + ag[2];
-    if (!dense || whole == whole) break;
+#pragma unroll
+    for (int c = 0; c < 3; c++) ag[c] = __shfl_sync(0xffffffffu, sum, c);
+    break;
   }
-  if (m == 0u) ag[0] = ag[1] = ag[2] = 0.f;  // no channel is the atom's, and the first was read all the same
 #pragma unroll
   for (int c = 0; c < 4; c++) split(tg[c], sh.sums[lane][2 * c], sh.sums[lane][2 * c + 1]);
   __syncwarp();
