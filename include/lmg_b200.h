@@ -101,7 +101,8 @@ enum {
   LMG_OP_BACKWARD = 1,
   LMG_OP_BACKWARD_GRADIENTS = 2,
   LMG_OP_BACKWARD_RELEVANCE = 3,
-  LMG_OP_BACKWARD_TYPES = 4 /* lmg_backward with type gradients, at its fastest: see below */
+  LMG_OP_BACKWARD_TYPES = 4,        /* lmg_backward with type gradients, at its fastest: see below */
+  LMG_OP_BACKWARD_TYPES_COUNTED = 5 /* the same with n_atoms given */
 };
 
 /* Scratch bytes that let the given op process the whole batch in one pass.  A smaller
@@ -109,8 +110,9 @@ enum {
  * only if not even one example fits.  `vector_types` != 0 for type_vector input.
  *
  * LMG_OP_BACKWARD is enough for any lmg_backward.  Type gradients of many atoms with radii by atom are
- * faster from a copy of the grid gradient, up to 256 MB of it: LMG_OP_BACKWARD_TYPES has room for it.  Where
- * the workspace does not, or does not start on a 32-byte boundary, lmg_backward takes the kernels that
+ * faster from a copy of the grid gradient, up to 256 MB of it: LMG_OP_BACKWARD_TYPES has room for it.  A copy
+ * costs the same however many of the slots are atoms, so calls with n_atoms go by a rule of their own.  Where
+ * the workspace has no room, or does not start on a 32-byte boundary, lmg_backward takes the kernels that
  * need no copy, whose sums have other last bits.
  *
  * Which kernels a call takes, and with them the last bits of its floating-point sums, goes by its settings,

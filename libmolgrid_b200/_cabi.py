@@ -10,7 +10,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("LMG_B200_LIB") or os.path.join(HERE, "liblmg_b200.so")
 
 LMG_OK, LMG_ERR_OUT_OF_RANGE, LMG_ERR_INVALID_ARGUMENT, LMG_ERR_CUDA, LMG_ERR_WORKSPACE = range(5)
-OP_FORWARD, OP_BACKWARD, OP_BACKWARD_GRADIENTS, OP_BACKWARD_RELEVANCE, OP_BACKWARD_TYPES = range(5)
+OP_FORWARD, OP_BACKWARD, OP_BACKWARD_GRADIENTS, OP_BACKWARD_RELEVANCE, OP_BACKWARD_TYPES, OP_BACKWARD_TYPES_COUNTED = range(6)
 
 c_float_p = ctypes.POINTER(ctypes.c_float)
 c_int_p = ctypes.POINTER(ctypes.c_int)

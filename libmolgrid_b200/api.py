@@ -502,7 +502,7 @@ class GridMaker(object):
         return min(need, MAX_WORKSPACE_BYTES)
 
     def _ws(self, dev, op, B, N, T, vec):
-        least = self._bytes(_cabi.OP_BACKWARD, B, N, T, vec) if op == _cabi.OP_BACKWARD_TYPES else None
+        least = self._bytes(_cabi.OP_BACKWARD, B, N, T, vec) if op >= _cabi.OP_BACKWARD_TYPES else None
         return _workspace(dev, self._bytes(op, B, N, T, vec), least)
 
     # --- forward -----------------------------------------------------------------------------
@@ -743,7 +743,8 @@ class GridMaker(object):
             raise TypeError("type_gradients given with index types")
         A.ntypes = T
         self._check_radii(vec, N, T, nr, ValueError)
-        ws = self._ws(dev, _cabi.OP_BACKWARD if tg is None else _cabi.OP_BACKWARD_TYPES, B, N, T, vec)
+        ws = self._ws(dev, _cabi.OP_BACKWARD if tg is None else _cabi.OP_BACKWARD_TYPES_COUNTED if A.n_atoms else _cabi.OP_BACKWARD_TYPES,
+                      B, N, T, vec)
         check(_cabi.lib().lmg_backward(ctypes.byref(self.s), ctypes.byref(A), df.ptr, ag.ptr,
                                        tg.ptr if tg is not None else None,
                                        ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(dev)))

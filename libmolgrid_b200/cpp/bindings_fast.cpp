@@ -255,7 +255,8 @@ PyObject* fast_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   }
   const size_t least = lmg_workspace_bytes(c.g, LMG_OP_BACKWARD, A.batch, A.max_atoms, A.ntypes, vec);
-  const size_t bytes = tg.ptr != nullptr ? lmg_workspace_bytes(c.g, LMG_OP_BACKWARD_TYPES, A.batch, A.max_atoms, A.ntypes, vec) : least;
+  const int op = A.n_atoms != nullptr ? LMG_OP_BACKWARD_TYPES_COUNTED : LMG_OP_BACKWARD_TYPES;
+  const size_t bytes = tg.ptr != nullptr ? lmg_workspace_bytes(c.g, op, A.batch, A.max_atoms, A.ntypes, vec) : least;
   if (!place(c, bytes, least, &ws, &wb, &st, &ret)) Py_RETURN_NONE;
   return finish([&] {
     Released r;

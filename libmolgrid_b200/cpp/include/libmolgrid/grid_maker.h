@@ -501,7 +501,8 @@ class GridMaker {
   void backward_call(const lmg_atoms& a, const float* diff, float* atom_gradients, float* type_gradients) const {
     const int vec = a.type_vector != nullptr;
     const size_t least = lmg_workspace_bytes(&s_, LMG_OP_BACKWARD, a.batch, a.max_atoms, a.ntypes, vec);
-    size_t bytes = type_gradients == nullptr ? least : lmg_workspace_bytes(&s_, LMG_OP_BACKWARD_TYPES, a.batch, a.max_atoms, a.ntypes, vec);
+    const int op = a.n_atoms != nullptr ? LMG_OP_BACKWARD_TYPES_COUNTED : LMG_OP_BACKWARD_TYPES;
+    size_t bytes = type_gradients == nullptr ? least : lmg_workspace_bytes(&s_, op, a.batch, a.max_atoms, a.ntypes, vec);
     void* w = detail::workspace_or_less(bytes, least);
     detail::check(lmg_backward(&s_, &a, diff, atom_gradients, type_gradients, w, bytes, nullptr));
   }

@@ -279,7 +279,7 @@ Layout layout(const lmg_gridmaker* g, int op, int nb, int N, int T, int vec) {
   std::memset(&L, 0, sizeof L);
   size_t recs = align_up((size_t)N * sizeof(lmg::Rec));
   size_t chanp = (vec && g->radii_type_indexed) ? align_up((size_t)T * sizeof(lmg::ChanParam)) : 0;
-  size_t partial = (vec && (op == LMG_OP_BACKWARD || op == LMG_OP_BACKWARD_TYPES || op == LMG_OP_BACKWARD_GRADIENTS))
+  size_t partial = (vec && (op != LMG_OP_FORWARD && op != LMG_OP_BACKWARD_RELEVANCE))
                        ? align_up((size_t)N * T * 3 * 4) : 0;
   size_t flags = align_up((size_t)N / 256 + 1);  // one byte per block of k_emit
   L.per_example = flags + recs + chanp + partial;
@@ -288,10 +288,10 @@ Layout layout(const lmg_gridmaker* g, int op, int nb, int N, int T, int vec) {
   L.recs = o; o += recs * nb;
   L.chanp = o; o += chanp * nb;
   L.partial = o; o += partial * nb;
-  if (partial != 0 && op == LMG_OP_BACKWARD_TYPES) {
+  if (partial != 0 && (op == LMG_OP_BACKWARD_TYPES || op == LMG_OP_BACKWARD_TYPES_COUNTED)) {
     const lmg::GMParams gm = lmg::to_params(g);
     // the rows of an aligned tensor; of another one with such rows it is not known here
-    if (lmg::type_copies_serve(gm, nb, N, T, g->dim % 4 == 0)) {
+    if (lmg::type_copies_serve(gm, nb, N, T, g->dim % 4 == 0, op == LMG_OP_BACKWARD_TYPES_COUNTED)) {
       const size_t each = lmg::type_copy_bytes(gm, T);
       L.copies = (int)std::max<size_t>(1, std::min<size_t>(nb, lmg::TYPE_COPIES / each));
       L.copy = L.partial;
@@ -665,7 +665,8 @@ int lmg_backward(const lmg_gridmaker* g, const lmg_atoms* a, const float* diff, 
     return fail(LMG_ERR_INVALID_ARGUMENT, "diff/atom_gradients missing memory");
   if (!vec && type_gradients != nullptr)
     return fail(LMG_ERR_INVALID_ARGUMENT, "type_gradients given with index types");
-  return backward_common(g, a, type_gradients != nullptr ? LMG_OP_BACKWARD_TYPES : LMG_OP_BACKWARD, vec ? 1 : 0, diff, nullptr, atom_gradients,
+  const int op = type_gradients == nullptr ? LMG_OP_BACKWARD : a->n_atoms == nullptr ? LMG_OP_BACKWARD_TYPES : LMG_OP_BACKWARD_TYPES_COUNTED;
+  return backward_common(g, a, op, vec ? 1 : 0, diff, nullptr, atom_gradients,
                          type_gradients, nullptr, workspace, workspace_bytes, stream);
 }
 

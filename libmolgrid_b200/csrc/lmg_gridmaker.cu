@@ -3320,20 +3320,30 @@ static cudaError_t backward_quads_atom(const BwdArgs& G, dim3 grid, cudaStream_t
 }
 
 // Enough atoms a grid pay for the copy, which costs the same for any of them, and enough (atom, channel) pairs in all fill the
-// chip.  50 x 3000 atoms of one channel on 28x48^3, in order 1705 us by single atoms from the gradient as it lies, 1276 like
-// this; with 28 weighted channels 1747 and 1537.
-// Loose rows have their pairs one by one otherwise: 14 channels of 41^3 of 0.5 A, 40 x 1500 / 8 x 400 / 1 x 1500 atoms 1483 /
-// 96 / 51 and 388 / 48 / 29 us, 28 channels of 65^3, 8 x 400 atoms 199 and 171, but 8 x 50 48 and 163, and 8 channels of 25^3
-// of 1 A, 1 x 1500 atoms 22 and 23.
-// Aligned rows have rounds of 14 channels, and up to 16 are as fast without the copy (40 x 1500 atoms on 14x48^3 of 0.5 A,
-// 0.11 atoms per cubic A: 389 and 464 us).  More channels, one / all weighted: 20 there 615 / 673 and 608 / 735, 28 698 / 712
-// and 657 / 743, 32 897 / 1008 and 669 / 753; 8 x 400 atoms (0.03) 28 85 and 91, 32 111 and 92; 28 channels of 24^3 of 1 A,
-// 8 x 2000 / 8 x 400 atoms 56 / 21 and 37 / 23.
-bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned) {
+// chip.  What counts is atoms that reach the grid; known here are slots: those of a call without counts may lie beside the grid,
+// of one with counts be empty, and the kernels without a copy are quick with both.
+// Loose rows have their pairs one by one otherwise, an empty slot's too: us without / with a copy, one weighted channel, all slots
+// atoms: 14 channels of 41^3 of 0.5 A, 40 x 1500 / 8 x 400 / 1 x 1500 atoms 1483 / 96 / 51 and 388 / 48 / 29.  With a copy over
+// without, for all slots atoms / 7 of 8 atoms beside the grid / 1 slot of 10 an atom, 14 channels of 41^3 by slots a voxel: 0.003,
+// 8 x 207 0.73 / 1.26 / 1.61, 40 x 207 0.58 / 0.85 / 1.20; 0.005, 8 x 345 0.51 / 0.95 / 1.29; 0.008, 8 x 551 0.45 / 0.70 / 0.98; of one
+// example on 57^3 0.008 (21e3 pairs) 0.63 / 1.15 / 1.97, 0.012 (31e3) 0.47 / 0.91 / 1.43, 0.02 (52e3) 0.39 / 0.67 / 0.91.
+// Aligned rows have rounds of 14 channels, and up to 24 are about as fast without the copy (40 x 3000 atoms, 20 channels of 48^3 of 0.5
+// A, one / 3 / all weighted 1086 / 1151 / 1197 and 950 / 1183 / 1183 us, a fifth of the slots atoms 336 and 407).  More channels, one / 3 /
+// all weighted: 28, 50 x 3000 atoms 1540 / 1583 / 1571 and 1197 / 1525 / 1525, half / a fifth of the slots atoms 865 / 454 and 825 / 604
+// with one, 885 / 463 and 1000 / 705 with all; of 24^3 of 1 A, 8 x 2000 atoms 56 / 24 and 37 / 21 with all slots / a twentieth atoms; 32,
+// 8 x 400 on 48^3 103 / 105 / 105 and 95 / 111 / 111.  Still the slower way: 28 channels, 50 x 3000 atoms 7 of 8 beside the grid 465 and 617,
+// all of 0.5 to 0.9 A 442 and 478.
+bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned, bool counted) {
   if (gm.rti || T > 32 || gm.dim == 0 || type_copy_bytes(gm, T) > TYPE_COPY_MOST) return false;
   const double side = (double)gm.dim * gm.res, dense = N / (side * side * side), pairs = (double)nb * N * T;
-  if (!aligned) return T >= 8 && dense >= 0.011 && pairs >= 16000;
-  return T > 16 && dense >= (T > 28 ? 0.025 : T > 24 ? 0.12 : 0.2) && pairs >= 300e3 * gm.res * gm.res * gm.res;
+  const double slots = N / ((double)gm.dim * gm.dim * gm.dim);  // a voxel
+  if (!aligned) {
+    if (T < 8 || dense < 0.011 || pairs < 16000) return false;
+    if (counted) return nb >= 4 ? slots >= 0.005 : slots >= 0.012 && pairs >= 30000;
+    return slots >= 0.003 && (nb >= 4 || slots >= 0.02 || pairs >= 30000);
+  }
+  if (counted && T <= 28 && slots < 0.1) return false;
+  return T > 24 && dense >= (T > 28 ? 0.05 : 0.12) && pairs >= 300e3 * gm.res * gm.res * gm.res;
 }
 
 template <int TO>

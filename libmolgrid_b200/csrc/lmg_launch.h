@@ -127,7 +127,8 @@ constexpr size_t TYPE_COPY_MOST = (size_t)256 << 20;   // largest copy of one ex
 // 1354 / 1276 us (each launch ends with its slowest atoms; two copies that take turns do not help)
 constexpr size_t TYPE_COPIES = (size_t)256 << 20;
 inline size_t type_copy_bytes(const GMParams& gm, int T) { return ((size_t)gm.dim * gm.dim * gm.dim + 1) * ((T + 7) / 8) * 32; }
-bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned);
+// `counted`: not all slots are atoms
+bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned, bool counted);
 cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, long* launches, cudaStream_t st);
 cudaError_t launch_forward_scatter(const BwdArgs& G, bool vec, cudaStream_t st);
 

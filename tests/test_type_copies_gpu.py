@@ -41,9 +41,15 @@ def _gradients(g, data, diff, quads=1, **more):
     return ag.cpu().numpy(), tg.cpu().numpy()
 
 
+def _copied(g, B, N, T, counted):
+    """Whether the call is one that goes by copies: then its scratch has room for them."""
+    from libmolgrid_b200 import _cabi
+    return g._bytes(_cabi.OP_BACKWARD_TYPES_COUNTED if counted else _cabi.OP_BACKWARD_TYPES, B, N, T, True) > g._bytes(_cabi.OP_BACKWARD, B, N, T, True)
+
+
 @pytest.mark.parametrize("points,T,B,N", [(25, 8, 10, 200), (25, 9, 9, 200), (25, 16, 7, 200), (25, 17, 5, 200), (25, 24, 4, 200),
-                                          (25, 25, 4, 200), (25, 32, 3, 200), (24, 29, 27, 400), (24, 25, 8, 1700), (24, 17, 7, 2800),
-                                          (13, 31, 3, 200)])
+                                          (25, 25, 4, 200), (25, 32, 4, 200), (24, 29, 15, 700), (24, 25, 8, 1700), (24, 28, 7, 1700),
+                                          (13, 31, 9, 200), (25, 32, 3, 200), (24, 17, 7, 2800), (13, 31, 3, 200)])
 @pytest.mark.parametrize("binary,multiple", [(False, 1.0), (True, 1.0), (False, -1.5)])
 def test_copies(port, points, T, B, N, binary, multiple):
     coords, types, radii = _batch(points * T, B, N, T, points - 1.0)
@@ -52,6 +58,7 @@ def test_copies(port, points, T, B, N, binary, multiple):
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     shape = (B,) + tuple(g.grid_dimensions(T))
     diff = torch.randn(shape, device="cuda")
+    assert _copied(g, B, N, T, True) == ((points, T, B) not in ((25, 32, 3), (24, 17, 7), (13, 31, 3)))
     n = torch.tensor([N - 3 * b for b in range(B)], dtype=torch.int32, device="cuda")
     ag, tg = _gradients(g, data, diff, n_atoms=n)
     for a, b in zip((ag, tg), _gradients(g, data, diff, quads=0, n_atoms=n)):
@@ -80,11 +87,12 @@ def test_copies(port, points, T, B, N, binary, multiple):
 
 def test_several_copies_and_one_example_more():
     """More examples than are copied at a time, the last copy of a single one."""
-    points, T, N = 65, 32, 400
+    points, T, N = 65, 32, 1400
     each = (points ** 3 + 1) * 128
     B = (256 << 20) // each + 1
     coords, types, radii = _batch(3, B, N, T, 32.0)
     g = lmg.GridMaker(0.5, 32.0)
+    assert _copied(g, B, N, T, False)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
     for a, b in zip(_gradients(g, data, diff), _gradients(g, data, diff, quads=0)):
@@ -98,6 +106,7 @@ def test_values_beyond_reach_and_without_weight(value):
     coords, types, radii = _batch(5, B, N, T, 8.0)
     types[:, :, 3] = 0
     g = lmg.GridMaker(1.0, points - 1.0)
+    assert _copied(g, B, N, T, False)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
     ag, tg = _gradients(g, data, diff)
@@ -111,13 +120,14 @@ def test_values_beyond_reach_and_without_weight(value):
     assert not np.isfinite(tg2[..., 3]).any()
 
 
-@pytest.mark.parametrize("points,T,B,N", [(25, 8, 10, 200), (25, 14, 6, 200), (24, 29, 27, 400)])
+@pytest.mark.parametrize("points,T,B,N", [(25, 8, 10, 200), (25, 14, 6, 200), (24, 29, 15, 700)])
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_atoms_without_weight_take_no_channel(points, T, B, N, value):
     """The first channel is no number anywhere and carries no weight: atoms without any weight have exactly no gradient."""
     coords, types, radii = _batch(points + T, B, N, T, points - 1.0)
     types[:, :, 0] = 0
     g = lmg.GridMaker(1.0, points - 1.0)
+    assert _copied(g, B, N, T, False)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
     ag, tg = _gradients(g, data, diff)
@@ -135,6 +145,7 @@ def test_workspace_off_the_boundary_of_the_copies():
     lib, points, T, B, N = _cabi.lib(), 25, 16, 7, 200
     coords, types, radii = _batch(11, B, N, T, points - 1.0)
     g = lmg.GridMaker(1.0, points - 1.0)
+    assert _copied(g, B, N, T, False)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
     want = _gradients(g, data, diff)
@@ -180,6 +191,7 @@ def test_room_for_copies_short_by_a_byte():
     lib, points, T, B, N = _cabi.lib(), 25, 16, 7, 200
     coords, types, radii = _batch(12, B, N, T, points - 1.0)
     g = lmg.GridMaker(1.0, points - 1.0)
+    assert _copied(g, B, N, T, False)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
     a = _cabi.AtomsStruct()
@@ -206,6 +218,7 @@ def test_no_memory_for_copies(monkeypatch):
     points, T, B, N = 25, 16, 7, 200
     coords, types, radii = _batch(13, B, N, T, points - 1.0)
     g = lmg.GridMaker(1.0, points - 1.0)
+    assert _copied(g, B, N, T, False)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     diff = torch.randn((B,) + tuple(g.grid_dimensions(T)), device="cuda")
     want = _gradients(g, data, diff)
