@@ -3213,18 +3213,18 @@ bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode) {
          quads_of(G, G.diff, mode == 2 ? G.density : nullptr);
 }
 
-// Densities of many atoms a grid, whose sums outlast the zeros, have records of k_emit earlier: us with and without, all slots
-// atoms, 8 x 1500 / 8 x 3000 atoms on 22x41^3 30.4 / 44.3 and 31.9 / 49.7, on 14x33^3 17.6 / 26.4 and 18.7 / 31.2, 16 x 1900 on
-// 14x24^3 of 1 A 23.1 and 27.0, 8 x 3000 on 28x48^3 46.1 and 49.0; but 4 x 2000 on 14x24^3 10.6 and 9.4, 16 x 1900 on 28x48^3
-// 80.3 and 76.6.  With half of the slots empty, which leave at once, 16 x 1900 on 22x41^3 43.7 and 45.9, on 14x24^3 22.4 and 20.6:
-// only on loose rows, whose tables make a warp's own preparation the longer one.
+// Densities of many atoms a grid, whose sums outlast the zeros, have records of k_emit earlier on loose rows, whose tables make a
+// warp's own preparation the longer one: us without and with, all slots atoms, 8 x 2500 / 8 x 4000 atoms on 14x33^3 36.0 / 52.5 and
+// 34.8 / 48.8, on 22x41^3 41.6 / 58.5 and 39.7 / 54.0, on 14x25^3 of 1 A 19.2 / 28.2 and 18.0 / 24.5; 4 x 4000 15.9 and 15.5, 3 x 4000
+// 12.8 and 13.2.  An atom beside the grid leaves at once without (8 x 2500 atoms, 7 of 8 of them there: 20.5 / 25.9 / 14.1 and 21.0 / 25.5 /
+// 16.2), as an empty slot does, so calls with counts stay there (a tenth atoms: 17.9 / 22.9 / 13.2 and 19.9 / 24.4 / 15.7), and aligned
+// rows gain nothing (8 x 2500 / 8 x 4000 atoms on 28x48^3 43.0 / 54.5 and 44.8 / 53.1, on 14x24^3 of 1 A 16.0 / 23.5 and 16.6 / 22.8).
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G) {
   const long slots = (long)A.nb * A.N;
   if (A.vec || slots > FWD_SELF_ATOMS) return false;
   if (A.gm.binary) return true;
-  const bool loose = loose_rows(G);
   const double voxels = (double)A.T * A.gm.dim * A.gm.dim * A.gm.dim;
-  if (voxels <= 1500.0 * A.N && (A.n_atoms == nullptr ? slots >= (loose ? 12000 : 14000) : loose && slots >= 20000)) return false;
+  if (loose_rows(G) && A.n_atoms == nullptr && slots >= 20000 && voxels <= 1500.0 * A.N) return false;
   return !G.precise && quads_of(G, G.out_grid);
 }
 

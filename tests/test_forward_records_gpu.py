@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("points,B,N,ragged", [(13, 6, 1999, False), (13, 6, 2000, False), (13, 4, 5000, True), (13, 4, 4999, True),
-                                               (12, 7, 2000, False), (12, 7, 1999, False), (17, 4, 3000, False), (18, 12, 1000, False)])
+                                               (12, 7, 2000, False), (12, 7, 1999, False), (17, 4, 3000, False), (18, 12, 1000, False),
+                                               (13, 10, 1999, False), (13, 10, 2000, False), (14, 5, 4000, False)])
 def test_densities_at_the_lines(port, points, B, N, ragged):
     T, side = 5, points - 1.0
     rng = np.random.default_rng(points * N)
