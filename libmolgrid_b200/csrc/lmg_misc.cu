@@ -486,15 +486,18 @@ unsigned interp_tile_count(unsigned out_dim) {
 }
 
 // Tiles cost a block's start (positions, choice of a box) before the first channel, and the voxels that the last of a row has
-// too many.  Tiles / direct, us: 48^3 from 48^3, 1 x 4 / 3 x 4 / 2 x 14 channels 7.8 / 18.8 / 22.0 and 6.3 / 12.3 / 23.5; 41^3 from 48^3,
-// 1 x 4 / 1 x 14 / 4 x 14 7.6 / 15.2 / 31.8 and 5.3 / 12.0 / 35.6; 57^3 from 64^3, 1 x 4 / 2 x 4 15.5 / 18.1 and 13.2 / 19.0; 17^3 from
-// 40^3, 8 x 28 22.9 and 14.4.  Input channels that fit the L1 are read there: 24^3 from 24^3, 1 x 14 / 8 x 28 / 16 x 28 5.7 / 21.4 /
-// 36.4 and 4.2 / 18.7 / 38.0.
+// too many.  Of 1064 calls (1 to 40 examples, 1 to 28 channels, 20^3 to 96^3) direct reads are taken where they are no slower but for
+// one, by 1.08.  Tiles / direct, us: 48^3 from 48^3, 1 x 4 / 2 x 4 channels 7.8 / 12.3 and 6.3 / 8.5; 41^3 from 48^3, 1 x 4 / 1 x 14 7.6 / 15.2
+// and 5.3 / 12.0; 57^3 from 64^3, 1 x 4 15.5 and 13.2; 17^3 from 40^3, 8 x 28 22.9 and 14.4.  Input channels that fit the L1 are read there:
+// 24^3 from 24^3, 1 x 14 / 8 x 28 / 16 x 28 5.7 / 21.4 / 36.4 and 4.2 / 18.7 / 38.0.  A single channel is the slower directly, because a
+// thread's position serves it alone: 33^3 from 64^3, 40 examples 25.5 and 29.3, 47^3 from 24^3 50.1 and 59.4.  What the line leaves to the
+// tiles because calls beside it lose: 3 x 4 channels of 48^3 18.8 and 12.3, 8 x 8 of 40^3 36.1 and 27.1.
 bool interp_tiles_pay(unsigned in_dim, unsigned out_dim, int nb, int K) {
   const double tiles = (double)interp_tile_count(out_dim) * nb * K * (ITILE * ITILE * ITILE);
-  if (in_dim <= 25) return tiles > 5e6;
   const double waste = tiles / ((double)out_dim * out_dim * out_dim * nb * K);
-  return tiles > 1.2e6 * waste * waste;
+  if (K == 1 && waste < 1.35) return tiles > 0.4e6;
+  if (in_dim <= 25) return tiles > (K > 2 ? 5e6 : 2.5e6);
+  return tiles > (waste < 1.35 ? 1.0e6 * waste : 1.2e6 * waste * waste);
 }
 
 cudaError_t launch_interpolate_tiled(const InterpMaps& maps, const InterpArgs& I, int nb, cudaStream_t st) {

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 # batch, channels, input and output points: tiny, ragged tiles, and just below and above the lines of the choice
 @pytest.mark.parametrize("shape", [(1, 1, 8, 4), (1, 7, 24, 24), (3, 8, 12, 25), (2, 33, 16, 13), (49, 2, 8, 8), (2, 12, 28, 36),
-                                   (2, 13, 28, 36), (13, 27, 24, 24), (13, 28, 24, 24)])
+                                   (2, 13, 28, 36), (13, 27, 24, 24), (13, 28, 24, 24), (2, 10, 28, 36), (2, 11, 28, 36),
+                                   (8, 1, 28, 36), (9, 1, 28, 36), (26, 2, 24, 36), (27, 2, 24, 36)])
 @pytest.mark.parametrize("identity", [False, True])
 def test_tiles_and_direct_reads_agree(shape, identity):
     B, K, n, m = shape
