@@ -40,3 +40,12 @@ def lib():
     build.build_library()
     from libmolgrid_b200 import _cabi
     return _cabi.lib()
+
+
+@pytest.fixture(params=[1, 2], ids=["by size", "staged"])
+def interpolation(request):
+    """GridInterpolater as calls of that size take it, then staged by tensor copies wherever the input allows it."""
+    from libmolgrid_b200 import _cabi
+    _cabi.lib().lmg_set_interp_tiled(request.param)
+    yield
+    _cabi.lib().lmg_set_interp_tiled(1)

@@ -117,6 +117,7 @@ def test_interpolate_28x48_rotated_against_oracle(port):
     assert _cabi.lib().lmg_tma_timeouts() == 0
 
 
+@pytest.mark.usefixtures("interpolation")
 @pytest.mark.parametrize("axis_angle", [((1.0, 0.0, 0.0), 0.0), ((0.0, 0.0, 1.0), 90.0), ((0.0, 0.0, 1.0), 45.0),
                                         ((1.0, -1.0, 0.0), 54.735610317245346), ((1.0, 1.0, 1.0), 60.0)])
 def test_interpolate_48_cubed_special_rotations(port, axis_angle):
@@ -235,6 +236,7 @@ def test_guard_words_vector_passes(port, rti, shift):
     assert not tdd.check("type_diffdiff").any()
 
 
+@pytest.mark.usefixtures("interpolation")
 def test_guard_words_transform_and_interpolation(port):
     import libmolgrid_b200 as lmg
     rng = np.random.default_rng(9)

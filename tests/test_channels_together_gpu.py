@@ -211,6 +211,49 @@ def _bytes(g, op, B, N, T):
     return _cabi.lib().lmg_workspace_bytes(ctypes.byref(g.s), op, B, N, T, 1)
 
 
+# one warp an atom and several; in one pass and in passes of two and one
+@pytest.mark.parametrize("T,N,points,res", [(5, 160, 16, 1.0), (14, 3000, 12, 1.0), (17, 60, 24, 1.0), (28, 160, 32, 0.5)])
+@pytest.mark.parametrize("passes", [False, True])
+def test_batches(port, T, N, points, res, passes):
+    """Examples with a centre, a transform and a count each: every one against the oracle, with nothing behind the counts."""
+    B, side = 5, (points - 1) * res
+    coords, types, radii, centers, rows = _batch(T * N, B, N, T, side)
+    n = np.array([N, N - 7, N // 2, 1, 0], np.int32)
+    rng = np.random.default_rng(N)
+    diff = rng.normal(size=(B, T, points, points, points)).astype(np.float32)
+    ca, ct = rng.normal(size=(B, N, 3)).astype(np.float32), rng.normal(size=(B, N, T)).astype(np.float32)
+    g, og = lmg.GridMaker(res, side, False, True), port.gm(res, side, False, True)
+    d = [torch.from_numpy(x).cuda() for x in (centers, coords, types, radii, diff, ca, ct)]
+    more = dict(transforms=torch.from_numpy(rows).cuda(), n_atoms=torch.from_numpy(n).cuda())
+    shapes = (B, N, 3), (B, N, T), diff.shape, (B, N, 3), (B, N, T)
+    rooms = [torch.full((int(np.prod(x)) + 64,), 7.0, device="cuda") for x in shapes]
+    ag, tg, dd, da, dt = (r[32:-32].view(x) for r, x in zip(rooms, shapes))
+    launches = [_cabi.lib().lmg_launch_count()]
+    with _Room(_bytes(g, _cabi.OP_BACKWARD, 2, N, T) if passes else api.MAX_WORKSPACE_BYTES):
+        g.backward(*d[:5], ag, tg, **more)
+    launches.append(_cabi.lib().lmg_launch_count())
+    with _Room(_bytes(g, _cabi.OP_BACKWARD_GRADIENTS, 2, N, T) if passes else api.MAX_WORKSPACE_BYTES):
+        g.backward_gradients(*d[:5], d[5], d[6], dd, da, dt, **more)
+    launches.append(_cabi.lib().lmg_launch_count())
+    # constants, records and sums, and the parts of atoms that several warps share
+    assert all((b - a) in ((9, 12) if passes else (3, 4)) for a, b in zip(launches, launches[1:]))
+    assert all(bool((r[:32] == 7.0).all() and (r[-32:] == 7.0).all()) for r in rooms)  # nothing beside the outputs
+    for b in range(B):
+        m = int(n[b])
+        assert not ag[b, m:].any() and not tg[b, m:].any() and not da[b, m:].any()
+        if m == 0:
+            assert not dd[b].any()
+            continue
+        k = min(m, 60)
+        moved = port.transform_forward(port.tr(rows[b, :4], rows[b, 4:7], rows[b, 7:]), coords[b, :m])
+        wag, wtg = port.backward_vector(og, centers[b], moved[:k], types[b, :k], radii[b], diff[b])
+        _close(ag[b, :k].cpu().numpy(), wag)
+        _close(tg[b, :k].cpu().numpy(), wtg)
+        wd, wa, _ = port.backward_gradients(og, centers[b], moved, types[b, :m], radii[b], diff[b], ca[b, :m], ct[b, :m])
+        _close(dd[b].cpu().numpy(), wd)
+        _close(da[b, :m].cpu().numpy(), wa)
+
+
 @pytest.mark.parametrize("T,N,points,res", [(8, 50, 24, 1.0), (16, 130, 24, 1.0), (28, 160, 32, 0.5)])
 def test_passes_of_a_call_take_the_same_kernel(T, N, points, res):
     """Five times the same example, two a pass: the last one alone has the bits of the others."""

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 # batch, channels, input and output points, resolutions
 SHAPES = [(1, 1, 5, 4, 0.5, 0.5), (1, 7, 24, 24, 0.5, 0.5), (3, 8, 12, 25, 0.5, 0.5), (1, 9, 13, 12, 0.375, 0.375),
-          (2, 33, 16, 13, 1.0, 1.0), (1, 17, 20, 9, 0.375, 1.0), (1, 3, 8, 40, 1.0, 0.125), (49, 2, 8, 8, 0.5, 0.5)]
+          (2, 33, 16, 13, 1.0, 1.0), (1, 17, 20, 9, 0.375, 1.0), (1, 3, 8, 40, 1.0, 0.125), (49, 2, 8, 8, 0.5, 0.5),
+          (1, 5, 20, 39, 0.5, 0.25), (2, 3, 28, 28, 0.75, 0.75)]
 
 
 def transforms(rng, B, kind):
@@ -36,12 +37,13 @@ def test_forward_both_ways_and_backward_is_its_adjoint(shape, kind):
     out = torch.full((B, K, m, m, m), 7.0, device="cuda")
     gi.forward(src, trs, out)
     try:
-        _cabi.lib().lmg_set_interp_tiled(0)
-        direct = torch.full_like(out, 8.0)
-        gi.forward(src, trs, direct)
+        for mode in (0, 2):                  # read directly, staged wherever the input allows it
+            _cabi.lib().lmg_set_interp_tiled(mode)
+            other = torch.full_like(out, 8.0)
+            gi.forward(src, trs, other)
+            assert torch.equal(out, other)   # the same roundings
     finally:
         _cabi.lib().lmg_set_interp_tiled(1)
-    assert torch.equal(out, direct)          # the same roundings
     gout = torch.randn_like(out)
     gin, again = torch.full_like(src, 7.0), torch.full_like(src, 8.0)
     gi.backward(gout, trs, gin)

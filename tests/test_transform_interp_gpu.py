@@ -75,6 +75,7 @@ def test_transform_roundtrip_large():
     assert torch.allclose(b, pts, atol=1e-4)
 
 
+@pytest.mark.usefixtures("interpolation")
 @pytest.mark.parametrize("gi", [(0.5, 11.5, 0.5, 11.5), (0.5, 11.5, 0.25, 8.0), (0.25, 6.0, 0.5, 9.5)])
 def test_interpolate(port, gi):
     import libmolgrid_b200 as lmg
@@ -96,6 +97,7 @@ def test_interpolate(port, gi):
         assert np.array_equal(got, want)
 
 
+@pytest.mark.usefixtures("interpolation")
 def test_interpolate_batched_and_identity(port):
     import libmolgrid_b200 as lmg
     rng = np.random.default_rng(9)
@@ -155,6 +157,7 @@ def test_interpolate_tiled_equals_direct_at_benchmark_shape():
     assert torch.equal(one, tiled[3])
 
 
+@pytest.mark.usefixtures("interpolation")
 @pytest.mark.parametrize("gi", [(0.5, 23.5, 0.6, 21.0), (0.5, 23.5, 0.41, 15.17), (0.5, 15.5, 1.5, 30.0)])
 def test_interpolate_staged_resampling(port, gi):
     """Coarser and finer output grids than the input (input rows 16-byte aligned: the finer one

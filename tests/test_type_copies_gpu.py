@@ -7,7 +7,6 @@ import torch
 
 import libmolgrid_b200 as lmg
 from libmolgrid_b200 import api
-from libmolgrid_b200 import synthetic as cases
 
 pytestmark = pytest.mark.gpu
 
@@ -29,15 +28,23 @@ def _close(got, want):
     np.testing.assert_allclose(got, want, rtol=1e-4, atol=1e-5 * max(1.0, float(np.abs(want).max())))
 
 
+def _between_guards(shape):
+    """A tensor of sevens and the floats around it, which no call writes."""
+    n = int(np.prod(shape))
+    room = torch.full((n + 64,), 7.0, device="cuda")
+    return room[32:32 + n].view(shape), (room[:32], room[32 + n:])
+
+
 def _gradients(g, data, diff, quads=1, **more):
     lib = api._cabi.lib()
-    ag = torch.full(data[0].shape, 7.0, device="cuda")
-    tg = torch.full(data[1].shape, 7.0, device="cuda")
+    ag, around_ag = _between_guards(data[0].shape)
+    tg, around_tg = _between_guards(data[1].shape)
     lib.lmg_set_quads(quads)
     try:
         g.backward(torch.zeros(len(ag), 3, device="cuda"), *data, diff, ag, tg, **more)
     finally:
         lib.lmg_set_quads(1)
+    assert all(bool((x == 7.0).all()) for x in around_ag + around_tg)
     return ag.cpu().numpy(), tg.cpu().numpy()
 
 
