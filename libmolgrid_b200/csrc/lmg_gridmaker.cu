@@ -3217,14 +3217,16 @@ bool backward_self_serves(const EmitArgs& A, const BwdArgs& G, int mode) {
 // warp's own preparation the longer one: us without and with, all slots atoms, 8 x 2500 / 8 x 4000 atoms on 14x33^3 36.0 / 52.5 and
 // 34.8 / 48.8, on 22x41^3 41.6 / 58.5 and 39.7 / 54.0, on 14x25^3 of 1 A 19.2 / 28.2 and 18.0 / 24.5; 4 x 4000 15.9 and 15.5, 3 x 4000
 // 12.8 and 13.2.  An atom beside the grid leaves at once without (8 x 2500 atoms, 7 of 8 of them there: 20.5 / 25.9 / 14.1 and 21.0 / 25.5 /
-// 16.2), as an empty slot does, so calls with counts stay there (a tenth atoms: 17.9 / 22.9 / 13.2 and 19.9 / 24.4 / 15.7), and aligned
-// rows gain nothing (8 x 2500 / 8 x 4000 atoms on 28x48^3 43.0 / 54.5 and 44.8 / 53.1, on 14x24^3 of 1 A 16.0 / 23.5 and 16.6 / 22.8).
+// 16.2), as an empty slot does: calls with counts have them on fine grids, where half of 8 x 3000 slots pay (27.1 / 32.7 / 16.1 and 26.8 /
+// 31.4 / 18.0 with half of them atoms, 34.4 / 40.0 / 18.6 and 33.1 / 38.0 / 18.9 with three quarters).  Aligned rows gain nothing
+// (8 x 2500 / 8 x 4000 atoms on 28x48^3 43.0 / 54.5 and 44.8 / 53.1, on 14x24^3 of 1 A 16.0 / 23.5 and 16.6 / 22.8).
 bool forward_self_serves(const EmitArgs& A, const BwdArgs& G) {
   const long slots = (long)A.nb * A.N;
   if (A.vec || slots > FWD_SELF_ATOMS) return false;
   if (A.gm.binary) return true;
   const double voxels = (double)A.T * A.gm.dim * A.gm.dim * A.gm.dim;
-  if (loose_rows(G) && A.n_atoms == nullptr && slots >= 20000 && voxels <= 1500.0 * A.N) return false;
+  if (loose_rows(G) && slots >= (A.n_atoms == nullptr ? 20000 : 24000) && (A.n_atoms == nullptr || A.gm.res <= 0.6f) && voxels <= 1500.0 * A.N)
+    return false;
   return !G.precise && quads_of(G, G.out_grid);
 }
 

@@ -12,16 +12,18 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("points,B,N,ragged", [(13, 6, 1999, False), (13, 6, 2000, False), (13, 4, 5000, True), (13, 4, 4999, True),
                                                (12, 7, 2000, False), (12, 7, 1999, False), (17, 4, 3000, False), (18, 12, 1000, False),
-                                               (13, 10, 1999, False), (13, 10, 2000, False), (14, 5, 4000, False)])
+                                               (13, 10, 1999, False), (13, 10, 2000, False), (14, 5, 4000, False),
+                                               (13, 6, 4000, True), (13, 6, 3999, True)])
 def test_densities_at_the_lines(port, points, B, N, ragged):
-    T, side = 5, points - 1.0
+    T, res = 5, 0.5 if ragged and N in (3999, 4000) else 1.0
+    side = (points - 1) * res
     rng = np.random.default_rng(points * N)
     coords = rng.uniform(-side / 2 - 1, side / 2 + 1, (B, N, 3)).astype(np.float32)
     types = rng.integers(-1, T, (B, N)).astype(np.float32)
     radii = rng.uniform(1.0, 2.0, (B, N)).astype(np.float32)
     n = [N - 1700 * b if ragged else N for b in range(B)]
     more = dict(n_atoms=torch.tensor(n, dtype=torch.int32, device="cuda").clamp_min(0)) if ragged else {}
-    g, og = lmg.GridMaker(1.0, side), port.gm(1.0, side)
+    g, og = lmg.GridMaker(res, side), port.gm(res, side)
     data = [torch.from_numpy(x).cuda() for x in (coords, types, radii)]
     out = []
     for quads in (1, 0):
