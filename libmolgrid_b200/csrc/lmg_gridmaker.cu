@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(BWD2_WARPS * 32) k_backward_warp(BwdArgs G) {
           float fsum = 0.f;  // sum over the column of -(d density / d dist) / dist * dv
           if constexpr (MODE == 0) {
             // Without branches: the tail's factor in units of 4 / ar^2 is at most one where it is taken, zero beyond the
-            // cut-off and for a NaN distance.  Bound by issue: 17 x 700 / 1500 / 4000 slots on 22x41^3 26.0 / 41.0 /
+            // cut-off and for a NaN distance.  Waits on its loads at half of the issue rate: 17 x 700 / 1500 / 4000 slots on 22x41^3 26.0 / 41.0 /
             // 98.1 us with a branch per voxel, 22.7 / 35.4 / 82.9 like this; against 64 bits 2.3e-7 and 1.7e-7, because
             // the factor's constant is exact in these units.
 #pragma unroll
@@ -2065,11 +2065,13 @@ __global__ void __launch_bounds__(VA_WARPS * 32, VA_MINB) k_backward_quads_atom(
 // ---------------------------------------------------------------------------------------------
 // The same for many atoms a grid: every channel is read under every footprint, and above the L1 takes a clock for each line
 // that a request touches, 85 columns in each of 28 channels.  A copy of the gradient with the channels of a voxel next to
-// each other makes that one line a voxel, and what bounds the sums are the loads from the L2 (83 kB an atom, 11 TB/s; L1 62 %,
-// issue 48 %).  Blocks of one warp: several atoms a block, neighbours by Morton's curve, meet too few lines of each other's
-// in the L1 (hits 22 to 35 %, as without order) for what the wait for the slowest costs (50 x 3000 atoms on 28x48^3: 1590 us for
-// 1225).  Quads of a column and voxels of a lane requested together, blocks an SM: 4 / 4 / 20 1226 us, 2 / 4 / 20 1301, 4 / 4 / 24
-// 1297 to 1505 (the L1 gets what shared memory leaves), 4 / 6 / 20 1267; with the atoms of many weighted channels beside, 1271.
+// each other makes that one line a voxel, and what bounds the sums are the loads from the L2 (83 kB an atom, 11.8 TB/s; L1 69 %
+// with 8 % hits, issue 47 %).  50 x 3000 atoms on 28x48^3, one / all weighted, 1690 / 1730 us without a copy and 1171 / 1661 like this.
+// Blocks of one warp: eight atoms a block, neighbours by Morton's curve, meet too few lines of each other's in the L1 (hits 22 to
+// 35 %, with the order and without) for what the wait for the slowest costs: 1590 us where blocks of one warp had 1225.  In the build
+// of that time, quads of a column and voxels of a lane requested together, blocks an SM: 4 / 4 / 20 1226 us, 2 / 4 / 20 1301, 4 / 4 / 24
+// 1297 to 1505 (the L1 gets what shared memory leaves), 4 / 6 / 20 1267; with the atoms of many weighted channels beside, 1271; with a
+// single channel's values weighted afterwards 1171.
 // ---------------------------------------------------------------------------------------------
 constexpr int CL_VOXELS = 128, CL_PITCH = CL_VOXELS + 1;
 
@@ -2698,11 +2700,13 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
 // the address - is computed once for all of them.  A warp lists the quads that the largest sphere reaches and takes 32 at a
 // time, whose lines are mostly neighbours; a channel whose sphere reaches none of these is skipped.
 // Bound by issue.  Item by item the L1 bounded it (95 %: a lane per column touches 32 lines a load): soft types, 28 channels,
-// 4 x 3000 atoms on 96^3 of 0.25 A 2473 us, 4 x 1500 on 48^3 of 0.5 A 284, 8 x 1000 with 20 channels on 40^3 of 0.75 A 176; like this
-// 2014, 184 and 84.  On the way: lanes as (column, z-quad) of the whole footprint 3338 / 255 / 109, the list 2271 / 196 / 88; quads
+// 4 x 3000 atoms on 96^3 of 0.25 A 2469 us, 4 x 1500 on 48^3 of 0.5 A 283, 8 x 1000 with 20 channels on 40^3 of 0.75 A 173; like this
+// 2045, 188 and 85, of which sums of few terms (RT_STEPS) take 1 to 2 %.  On the way: lanes as (column, z-quad) of the whole footprint 3338 / 255 / 109, the list 2271 / 196 / 88; quads
 // in three shells by distance 2202 / 195 / 95; the tails of all channels apart 2514 / 221 / 105; channels by radius, blocks of an
 // atom's warps 2870 / 250 / 110, of one warp 2267 / 209 / 94; blocks of one warp, channels as they come 2185 / 194 / 86, then no test of
-// a weight for each.
+// a weight for each.  A channel much smaller than the largest is listed with it all the same: see channels_together() for what that
+// costs.  Tried against it: a vote for four channels together before their loads 10 % slower with all channels weighted; sweeps of
+// their own for channels of half the radius and less 3 (0.25 A) to 20 % (24^3 of 1 A) slower where there are none.
 // ---------------------------------------------------------------------------------------------
 constexpr int RT_CH = 16, RT_WARPS = 4;  // channels a warp, most warps an atom
 constexpr int RT_MINB = 20;              // blocks of one warp an SM: 96 registers (16 / 24: 2395 / 2313 us instead of 2267)
@@ -2956,7 +2960,7 @@ __global__ void __launch_bounds__(32, RT_MINB) k_backward_channels(BwdArgs G, in
 // term needs, with the weights w and the incoming type gradients t, are taken voxel by voxel - of w alpha diff and t alpha diff for
 // the products of distances, of w s diff and t s diff for the rest.  Only channels that carry weight take part.
 // Bound by issue at few warps: 20 blocks an SM spill and gain nothing (soft types, 4 x 1500 atoms on 28x48^3 of 0.5 A: item by item
-// 543 us, like this 350, with 20 360).
+// 542 us, like this 353, with 20 some 10 more).
 constexpr int RS_MINB = 16;
 constexpr int RS_LOADS = 2;
 __global__ void __launch_bounds__(32, RS_MINB) k_second_channels(BwdArgs G, int per, int warps) {
@@ -3325,16 +3329,16 @@ static cudaError_t backward_quads_atom(const BwdArgs& G, dim3 grid, cudaStream_t
 // chip.  What counts is atoms that reach the grid; known here are slots: those of a call without counts may lie beside the grid,
 // of one with counts be empty, and the kernels without a copy are quick with both.
 // Loose rows have their pairs one by one otherwise, an empty slot's too: us without / with a copy, one weighted channel, all slots
-// atoms: 14 channels of 41^3 of 0.5 A, 40 x 1500 / 8 x 400 / 1 x 1500 atoms 1483 / 96 / 51 and 388 / 48 / 29.  With a copy over
+// atoms: 14 channels of 41^3 of 0.5 A, 40 x 1500 / 8 x 400 / 1 x 1500 atoms 1530 / 99 / 52 and 366 / 44 / 26.  With a copy over
 // without, for all slots atoms / 7 of 8 atoms beside the grid / 1 slot of 10 an atom, 14 channels of 41^3 by slots a voxel: 0.003,
-// 8 x 207 0.73 / 1.26 / 1.61, 40 x 207 0.58 / 0.85 / 1.20; 0.005, 8 x 345 0.51 / 0.95 / 1.29; 0.008, 8 x 551 0.45 / 0.70 / 0.98; of one
+// 8 x 207 0.67 / 1.15 / 1.61, 40 x 207 0.56 / 0.82 / 1.20; 0.005, 8 x 345 0.48 / 0.86 / 1.29; 0.008, 8 x 551 0.42 / 0.63 / 0.98; of one
 // example on 57^3 0.008 (21e3 pairs) 0.63 / 1.15 / 1.97, 0.012 (31e3) 0.47 / 0.91 / 1.43, 0.02 (52e3) 0.39 / 0.67 / 0.91.
 // Aligned rows have rounds of 14 channels, and up to 24 are about as fast without the copy (40 x 3000 atoms, 20 channels of 48^3 of 0.5
 // A, one / 3 / all weighted 1086 / 1151 / 1197 and 950 / 1183 / 1183 us, a fifth of the slots atoms 336 and 407).  More channels, one / 3 /
-// all weighted: 28, 50 x 3000 atoms 1540 / 1583 / 1571 and 1197 / 1525 / 1525, half / a fifth of the slots atoms 865 / 454 and 825 / 604
+// all weighted: 28, 50 x 3000 atoms 1541 / 1585 / 1573 and 1120 / 1541 / 1541, half / a fifth of the slots atoms 865 / 454 and 825 / 604
 // with one, 885 / 463 and 1000 / 705 with all; of 24^3 of 1 A, 8 x 2000 atoms 56 / 24 and 37 / 21 with all slots / a twentieth atoms; 32,
-// 8 x 400 on 48^3 103 / 105 / 105 and 95 / 111 / 111.  Still the slower way: 28 channels, 50 x 3000 atoms 7 of 8 beside the grid 465 and 617,
-// all of 0.5 to 0.9 A 442 and 478.
+// 8 x 400 on 48^3 103 / 105 / 105 and 95 / 111 / 111.  Still the slower way: 28 channels, 50 x 3000 atoms 7 of 8 beside the grid 466 and 591,
+// all of 0.5 to 0.9 A 442 and 467.  (Which examples are copied, decided on the GPU by their atoms' footprints, cost 5 % of full calls.)
 bool type_copies_serve(const GMParams& gm, int nb, int N, int T, bool aligned, bool counted) {
   if (gm.rti || T > 32 || gm.dim == 0 || type_copy_bytes(gm, T) > TYPE_COPY_MOST) return false;
   const double side = (double)gm.dim * gm.res, dense = N / (side * side * side), pairs = (double)nb * N * T;
@@ -3376,7 +3380,11 @@ cudaError_t launch_type_gradients(const BwdArgs& G, float* copy, int per_copy, l
 // for warps that last 4 to 16 times as long: us item by item / together, soft types, 28 channels, 8 x 1500 / 1 x 200 / 1 x 16 atoms on
 // 24^3 of 1 A 279 / 17.8 / 11.9 and 88 / 10.5 / 9.5, on 40^3 of 0.75 A 352 / 19.7 / 12.5 and 157 / 13.7 / 12.3, on 48^3 of 0.5 A 551 /
 // 24.7 / 14.6 and 360 / 23.6 / 21.1, 4 channels there 86 / 11.5 / 10.4 and 73 / 14.4 / 13.9; on 96^3 of 0.25 A 4 x 3000 / 8 x 400 / 1 x 1500
-// 2473 / 691 / 328 and 2075 / 855 / 446, which have most of their spheres' quads in the tail and in full columns.
+// 2473 / 691 / 328 and 2075 / 855 / 446, which have most of their spheres' quads in the tail and in full columns.  (By the rule, with
+// sums of few terms: 279 / 17.7 and 86 / 11.6, 351 / 19.6 and 146 / 14.5, 552 and 345, 85 and 70, 2469 and 2045.)
+// Radii are not known here.  Still slower together: one radius of 4 A among channels of 0.8 to 1.2 (28 channels, 4 x 3000 atoms on
+// 96^3 1660 and 5500, 4 x 1500 on 48^3 246 and 454, 4 channels there 177 and 249, but 8 x 1500 on 24^3 279 and 181); three quarters
+// of the radii zero on 96^3 783 and 930; 7 of 8 atoms beside that grid 568 and 702.
 static bool channels_together(const BwdArgs& G) {
   if (G.T < 4 || G.T > RT_CH * RT_WARPS || G.gm.binary) return false;
   if (G.gm.ta == 0.f && G.gm.tb == 0.f) return false;  // a Gaussian without a tail is cut by each channel's own footprint too
@@ -3445,8 +3453,8 @@ cudaError_t launch_second_order(const BwdArgs& G, long* launches, cudaStream_t s
     return launch_early(k_second_quads_atom, dim3((G.N + SO_WARPS - 1) / SO_WARPS, G.nb), SO_WARPS * 32, 0, st, G);
   }
   // Item by item only the weighted channels have warps, so one of many (as one-hot types have) gains less: us item by item /
-  // together, 28 channels, soft / one-hot types, 8 x 1500 atoms on 24^3 of 1 A 446 / 62 and 161 / 49, 4 x 1500 on 48^3 of 0.5 A 543 / 74 and
-  // 350 / 71, but 8 channels there, 8 x 1500 atoms one-hot 69 and 80, and 28 of 96^3 of 0.25 A, 4 x 3000 atoms 4241 / 356 and 4177 / 456.
+  // together, 28 channels, soft / one-hot types, 8 x 1500 atoms on 24^3 of 1 A 447 / 61 and 163 / 50, 4 x 1500 on 48^3 of 0.5 A 542 / 73 and
+  // 353 / 71, but 8 channels there, 8 x 1500 atoms one-hot 69 and 80, and 28 of 96^3 of 0.25 A, 4 x 3000 atoms 4241 / 356 and 4177 / 456.
   if (quads && (G.gm.res >= 0.7f || (G.gm.res >= 0.4f && G.T >= 24)) && channels_together(G))
     return channels_together_launch(k_second_channels, G, 3000, launches, st);
   *launches += quads ? 1 : 2;
