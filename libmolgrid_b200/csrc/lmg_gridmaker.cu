@@ -2206,7 +2206,7 @@ __device__ __forceinline__ void tg_add(TgShared<TO>& sh, unsigned n, const Eight
 }
 
 // One atom, whose weights `w` are those of a lane's channel.  A lane owns a column, as in backward_quads_core(), and lists the
-// voxels of its quads that lie within reach.  The atom gradient takes the values of channel `one`, not weighted, where they lie, or
+// voxels of its quads that lie within reach.  The atom gradient takes the values of `channel`, not weighted, where they lie, or
 // of all channels (DENSE) from the copy, by the gradients of the density that are listed too.
 template <int TO, bool BINARY, bool DENSE>
 __device__ __forceinline__ void tg_atom(const TgArgs& A, const ItemParams& P, TgShared<TO>& sh, const float* diffb, const Eight* mine,
@@ -2699,14 +2699,15 @@ __global__ void __launch_bounds__(SO_WARPS * 32, SO_ATOM_MINB) k_second_quads_at
 // a warp takes up to RT_CH channels of an ATOM, and what depends on the place alone - column, squared distance, its roots,
 // the address - is computed once for all of them.  A warp lists the quads that the largest sphere reaches and takes 32 at a
 // time, whose lines are mostly neighbours; a channel whose sphere reaches none of these is skipped.
-// Bound by issue.  Item by item the L1 bounded it (95 %: a lane per column touches 32 lines a load): soft types, 28 channels,
-// 4 x 3000 atoms on 96^3 of 0.25 A 2469 us, 4 x 1500 on 48^3 of 0.5 A 283, 8 x 1000 with 20 channels on 40^3 of 0.75 A 173; like this
-// 2045, 188 and 85, of which sums of few terms (RT_STEPS) take 1 to 2 %.  On the way: lanes as (column, z-quad) of the whole footprint 3338 / 255 / 109, the list 2271 / 196 / 88; quads
-// in three shells by distance 2202 / 195 / 95; the tails of all channels apart 2514 / 221 / 105; channels by radius, blocks of an
-// atom's warps 2870 / 250 / 110, of one warp 2267 / 209 / 94; blocks of one warp, channels as they come 2185 / 194 / 86, then no test of
-// a weight for each.  A channel much smaller than the largest is listed with it all the same: see channels_together() for what that
-// costs.  Tried against it: a vote for four channels together before their loads 10 % slower with all channels weighted; sweeps of
-// their own for channels of half the radius and less 3 (0.25 A) to 20 % (24^3 of 1 A) slower where there are none.
+// Bound by issue.  Item by item the L1 bounded it (95 %: a lane per column touches 32 lines a load): soft types, 28 channels, 4 x
+// 3000 atoms on 96^3 of 0.25 A 2469 us, 4 x 1500 on 48^3 of 0.5 A 283, 8 x 1000 with 20 channels on 40^3 of 0.75 A 173; like this
+// 2045, 188 and 85, of which sums of few terms (RT_STEPS) take 1 to 2 %.  On the way: lanes as (column, z-quad) of the whole
+// footprint 3338 / 255 / 109, the list 2271 / 196 / 88; quads in three shells by distance 2202 / 195 / 95; the tails of all
+// channels apart 2514 / 221 / 105; channels by radius, blocks of an atom's warps 2870 / 250 / 110, of one warp 2267 / 209 / 94;
+// blocks of one warp, channels as they come 2185 / 194 / 86, then no test of a weight for each.  A channel much smaller than the
+// largest is listed with it all the same: see channels_together() for what that costs.  Tried against it: a vote for four channels
+// together before their loads 10 % slower with all channels weighted; sweeps of their own for channels of half the radius and less
+// 3 (0.25 A) to 20 % (24^3 of 1 A) slower where there are none.
 // ---------------------------------------------------------------------------------------------
 constexpr int RT_CH = 16, RT_WARPS = 4;  // channels a warp, most warps an atom
 constexpr int RT_MINB = 20;              // blocks of one warp an SM: 96 registers (16 / 24: 2395 / 2313 us instead of 2267)
